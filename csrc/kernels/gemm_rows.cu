@@ -1,0 +1,243 @@
+// Matrix products with few rows: D[M, N] = epilogue(alpha * X[M, K] W[N, K]^T) for M <= 96, bf16 operands, fp32 accumulation.
+//
+// With few rows the product is bound by reading W once, so the kernel is built to have as much of W in flight as the memory wants.
+// W takes the 128-row side of tcgen05.mma and the rows of X its N side (rounded up to 16), so nothing is multiplied for padding beyond
+// that; 128 rows of W form a tile, and a cluster of up to 8 CTAs shares a tile: each CTA contracts over its part of K with its own ring
+// of TMA stages, leaves its partial sums in shared memory, and takes its share of the tile's results, adding the partial sums of all
+// CTAs in rank order through distributed shared memory (bit-reproducible, no workspace, no second kernel).  Measured on one B200, one
+// row, in a captured chain: 28672 x 4096 41 us = 5.7 TB/s (the tile kernel: 54), 65536 x 4096 6.5 TB/s, 2048 x 2048 5.4 us (12.0), of which
+// launch, first load, exchange and last store are about 4.
+//
+// Roles: warp 0 TMA, warp 1 MMA issue and TMEM, warps 2 to 5 accumulator -> shared memory; then all warps the epilogue.
+#include "gemm_rows.h"
+
+#include "pdl.cuh"
+#include "rb_common.cuh"
+
+namespace rb {
+
+constexpr int kRowsThreads = 192;
+constexpr int kRowsTile = 128;                         // rows of W of a tile
+constexpr int kRowsWBytes = kRowsTile * 128;           // one stage of W: 64 columns
+
+struct RowsEpi {
+  void* d;
+  long long ldd;
+  const __nv_bfloat16* bias;
+  const __nv_bfloat16* residual;
+  long long ldr;
+  int act, out_f32;
+  float alpha;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ float rows_act(int act, float v) {
+  if (act == RB_ACT_GELU) return gelu_tanh_fast(v);
+  if (act == RB_ACT_SILU) return silu(v);
+  if (act == RB_ACT_RELU || act == RB_ACT_RELU2) {
+    v = fmaxf(v, 0.f);
+    return act == RB_ACT_RELU ? v : v * v;
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kRowsThreads)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, int M, int N, int K, int mpad,
+                 int parts, int stages, const RowsEpi ep, unsigned int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t base = smem_u32(smem);
+  const uint32_t stage_bytes = kRowsWBytes + mpad * 128;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + stages * stage_bytes);
+  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * stages, bar_acc = bar_empty + 8 * stages;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * stages + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / parts, part = blockIdx.x - tile * parts;
+  const uint32_t tmem_cols = mpad <= 32 ? 32 : mpad <= 64 ? 64 : 128;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2 * stages + 1; ++s) mbar_init(bar_full + 8 * s, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_ptr), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
+  const int num_kb = (K + 63) / 64;
+  const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * part / parts);
+  const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (part + 1) / parts);
+
+  if (warp == 0) {
+    if (elect_one()) {
+      pdl_wait();
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int it = kb - kb0, s = it % stages;
+        if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag, status, 81)) break;
+        mbar_arrive_expect_tx(bar_full + 8 * s, stage_bytes);
+        tma_load_2d(base + s * stage_bytes, &tmW, kb * 64, tile * kRowsTile, bar_full + 8 * s);
+        tma_load_2d(base + s * stage_bytes + kRowsWBytes, &tmX, kb * 64, 0, bar_full + 8 * s);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc_bf16(kRowsTile, mpad, 0, 0);
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int it = kb - kb0, s = it % stages;
+        if (!mbar_wait(bar_full + 8 * s, (it / stages) & 1, abort_flag, status, 82)) { ok = false; break; }
+        tc_fence_after();
+        uint64_t dw = umma_smem_desc_sw128(base + s * stage_bytes, 16, 1024);
+        uint64_t dx = umma_smem_desc_sw128(base + s * stage_bytes + kRowsWBytes, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_bf16_ss(tmem, dw + 2 * k, dx + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+        umma_commit(bar_empty + 8 * s);
+      }
+      if (ok) umma_commit(bar_acc);
+    }
+  } else {
+    pdl_wait();
+    pdl_launch();
+    // Every load of the ring has been consumed when the accumulator is complete: its memory takes the partial sums [M][128].
+    if (mbar_wait(bar_acc, 0, abort_flag, status, 83)) {
+      tc_fence_after();
+      const int q = warp & 3;                            // the quarter of the TMEM lanes that this warp may read
+      float* dst = reinterpret_cast<float*>(smem) + q * 32 + lane;
+      for (int c = 0; c < mpad; c += 16) {
+        uint32_t r[16];
+        tmem_ld_32x16(tmem + (static_cast<uint32_t>(q * 32) << 16) + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c + j < M) dst[(c + j) * kRowsTile] = __uint_as_float(r[j]);
+      }
+      tc_fence_before();
+    }
+  }
+  __syncwarp();
+  if (warp < 2) pdl_wait();
+  if (parts > 1) cluster_sync_all();
+  else __syncthreads();
+
+  // ---- results: four neighbouring columns per item, items dealt to the CTAs of the cluster
+  if (!*abort_flag) {
+    for (int i = part * kRowsThreads + threadIdx.x; i < M * (kRowsTile / 4); i += parts * kRowsThreads) {
+      const int m = i >> 5, n = (i & 31) * 4, col = tile * kRowsTile + n;
+      if (col >= N) continue;
+      const uint32_t off = base + (m * kRowsTile + n) * 4;
+      float4 a;
+      if (parts > 1) {
+        a = ld_cluster_f4(mapa_shared(off, 0));
+        for (int s = 1; s < parts; ++s) {
+          const float4 b = ld_cluster_f4(mapa_shared(off, s));
+          a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+      } else {
+        a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem) + m * kRowsTile + n);
+      }
+      float v[4] = {a.x * ep.alpha, a.y * ep.alpha, a.z * ep.alpha, a.w * ep.alpha};
+      const bool full = col + 4 <= N;
+      if (ep.bias) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (full || col + j < N) v[j] += __bfloat162float(__ldg(ep.bias + col + j));
+      }
+      if (ep.act != RB_ACT_NONE) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = rows_act(ep.act, v[j]);
+      }
+      if (ep.residual) {
+        const __nv_bfloat16* r = ep.residual + m * ep.ldr + col;
+        if (full) {
+          const uint2 u = *reinterpret_cast<const uint2*>(r);
+          const float2 r0 = unpack_bf16x2(u.x), r1 = unpack_bf16x2(u.y);
+          v[0] += r0.x; v[1] += r0.y; v[2] += r1.x; v[3] += r1.y;
+        } else {
+          for (int j = 0; col + j < N; ++j) v[j] += __bfloat162float(r[j]);
+        }
+      }
+      if (ep.out_f32) {
+        float* d = reinterpret_cast<float*>(ep.d) + m * ep.ldd + col;
+        if (full) *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+        else for (int j = 0; col + j < N; ++j) d[j] = v[j];
+      } else {
+        __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(ep.d) + m * ep.ldd + col;
+        if (full) *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+        else for (int j = 0; col + j < N; ++j) d[j] = __float2bfloat16(v[j]);
+      }
+    }
+  }
+  if (parts > 1) cluster_sync_all();                     // nobody leaves while another CTA still reads its partial sums
+  else __syncthreads();
+  if (warp == 1) {
+    if (*abort_flag) {
+      // give copies and MMAs that are still in flight time to land before TMEM is released
+      const unsigned long long t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+    tc_fence_after();
+    tmem_dealloc(tmem, tmem_cols);
+  }
+}
+
+}  // namespace rb
+
+namespace rbhost {
+
+// Up to 96 rows this kernel is the faster one (us per product in a captured chain, tile kernel / this one; 1 row: 768 x 768 8.1 / 3.7,
+// 2048 x 2048 12.0 / 5.4, 28672 x 4096 54.0 / 41.3; 96 rows: 8.7 / 6.3, 12.2 / 9.4, 48.1 / 48.9, 65536 x 4096 126 / 100).  With 128 rows the two
+// cross (2048 x 8192 16.3 / 17.1).  From 49 rows on a short contraction under many tiles is all results and little reading: 50304 x 768
+// with 64 rows 20.8 / 24.8, with 24 rows 21.5 / 20.0.
+bool gemm_rows_takes(const RbGemmArgs& g) {
+  if (g.M > 96 || (g.M > 48 && g.K < 1024 && g.N > 148 * rb::kRowsTile)) return false;
+  return !g.a_mn_major && !g.b_mn_major && !g.accumulate && !g.aux_out && !g.aux_in && g.group_mode == 0 && g.peer_mode == 0 && !g.ab_fp8 &&
+         !g.a_scale && !g.b_scale && g.block_n == 0 && g.group_m == 0 && g.max_ctas == 0 && g.splits <= 1;
+}
+
+int gemm_rows(const RbGemmArgs& g, cudaStream_t stream) {
+  const int mpad = (g.M + 15) / 16 * 16;
+  const int tiles = (g.N + rb::kRowsTile - 1) / rb::kRowsTile, num_kb = (g.K + 63) / 64;
+  // About 100 CTAs or more read at the memory's rate; each further part of K costs another CTA's partial sums.  One row, us per product
+  // in a captured chain with 1 / 2 / 4 / 8 parts: 768 x 768 5.7 / 4.6 / 4.0 / 3.9, 2048 x 8192 36.9 / 20.6 / 12.5 / 9.6, 16384 x 2048
+  // 14.1 / 14.2 / 17.9 / 25.0.
+  int parts = 1;
+  while (parts < 8 && tiles * parts < 100 && num_kb / (parts + 1) >= 2) ++parts;
+  // The ring is kept below half of an SM's shared memory: with one CTA per SM, clusters of 8 no longer all fit side by side (2048 x 2048,
+  // 64 rows, 8 parts: 8.1 us with 4 stages, 13.7 with 6).
+  const int stage_bytes = rb::kRowsWBytes + mpad * 128;
+  const int stages = (111 * 1024) / stage_bytes < 6 ? (111 * 1024) / stage_bytes : 6;
+  int err = 0;
+  const CUtensorMap* tw = get_tmap_2d(g.b, 2, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb, 64, rb::kRowsTile, 1, &err);
+  if (!tw) return err ? err : -5;
+  const CUtensorMap* tx = get_tmap_2d(g.a, 2, (uint64_t)g.K, (uint64_t)g.M, (uint64_t)g.lda, 64, (uint32_t)mpad, 1, &err);
+  if (!tx) return err ? err : -5;
+  const int smem = stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024;
+  static bool configured_dev[64] = {false};
+  bool& configured = configured_dev[device_slot()];
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(rb::gemm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 114 * 1024);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  rb::RowsEpi ep;
+  ep.d = g.d; ep.ldd = g.ldd;
+  ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
+  ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual); ep.ldr = g.ldr;
+  ep.act = g.act; ep.out_f32 = g.out_f32; ep.alpha = g.alpha;
+  return static_cast<int>(launch_pdl(rb::gemm_rows_kernel, dim3(tiles * parts), dim3(rb::kRowsThreads), smem, stream, parts, *tw, *tx,
+                                     g.M, g.N, g.K, mpad, parts, stages, ep, status_ptr()));
+}
+
+}  // namespace rbhost

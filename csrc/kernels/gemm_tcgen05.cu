@@ -18,6 +18,8 @@
 // op sequences (crates/candle-backend/src/lib.rs:220-312).
 #include "gemm_tcgen05.h"
 
+#include "gemm_rows.h"
+
 #include <stdlib.h>
 #include <string.h>
 
@@ -1536,6 +1538,7 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
   }
   const int sms = rbhost::device_sm_count();
   if (g.block_n != 0 && g.block_n != 64 && g.block_n != 128 && g.block_n != 192 && g.block_n != 256) return -6;
+  if (rbhost::gemm_rows_takes(g)) return rbhost::gemm_rows(g, stream);
   int bn = 128, splits = 1;
   pick_plan(g, sms, bn, splits);
   if (g.splits > 1 && splits != g.splits) return -7;   // a forced split count that cannot be honoured

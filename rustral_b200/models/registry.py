@@ -52,11 +52,11 @@ def _layered_weights(cfg, device, dtype, tensors, seed):
     return InferenceWeights.layered(cfg, device, dtype, tensors, seed)
 
 
-_GPT_KERNELS = ("gemm_tcgen05", "embedding", "elementwise", "norm", "rope", "attention", "attention_tc", "attention_fwd2",
+_GPT_KERNELS = ("gemm_tcgen05", "gemm_rows", "embedding", "elementwise", "norm", "rope", "attention", "attention_tc", "attention_fwd2",
                 "paged_attention", "optim")
-_LAYERED_KERNELS = ("gemm_tcgen05", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe",
+_LAYERED_KERNELS = ("gemm_tcgen05", "gemm_rows", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe",
                     "attention_fwd2", "paged_attention")
-_HYBRID_KERNELS = ("gemm_tcgen05", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe", "attention_fwd2",
+_HYBRID_KERNELS = ("gemm_tcgen05", "gemm_rows", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe", "attention_fwd2",
                    "paged_attention", "short_conv", "state_space", "state_space_chunk", "delta_rule",
                    "delta_rule_chunk", "gated_norm")
 

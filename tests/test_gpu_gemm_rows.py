@@ -1,0 +1,60 @@
+"""The product kernel for few rows (gemm_rows.cu) at the edges of its tiles, parts and rule, against 64-bit arithmetic and the tile kernel."""
+import pytest
+import torch
+
+from rustral_b200.ops.matmul import gemm
+
+pytestmark = pytest.mark.gpu
+
+# (N, K): one tile and less, ragged columns, a last K block of 8, one block only, parts of unequal length, more tiles than SMs
+SIZES = [(8, 64), (128, 8), (130, 72), (520, 200), (768, 768), (1000, 1016), (2048, 8192), (19200, 136)]
+
+
+def _operands(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    ld = (K + 15) // 8 * 8                                             # rows that do not follow each other
+    return rnd(M, ld)[:, :K], rnd(N, ld)[:, :K], rnd(N), rnd(M, (N + 15) // 8 * 8)[:, :N]
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 48, 49, 96, 97])
+@pytest.mark.parametrize("N,K", SIZES)
+def test_matches_64_bit_and_the_tile_kernel(M, N, K, cuda_status):
+    x, w, bias, res = _operands(M, N, K)
+    ref = x.double() @ w.double().T
+    # fp32 sums of K products in any order: K * 2^-24 of the sum of magnitudes
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-6
+    y = torch.empty(M, (N + 7) // 4 * 4, device="cuda")[:, :N]
+    gemm(x, w, out=y)
+    assert ((y.double() - ref).abs() <= bound).all()
+    assert ((gemm(x, w, out=torch.empty_like(y, memory_format=torch.preserve_format), group_m=8).double() - ref).abs() <= bound).all()
+    if N % 8 == 0:
+        for act, f in (("none", lambda t: t), ("relu2", lambda t: torch.relu(t) ** 2), ("silu", torch.nn.functional.silu),
+                       ("gelu", lambda t: torch.nn.functional.gelu(t, approximate="tanh"))):
+            got = gemm(x, w, bias=bias, act=act, residual=res, alpha=0.5)
+            want = f(0.5 * ref + bias.double()) + res.double()
+            # bf16 result (2^-8), fp32 sums, tanh.approx of gelu (5e-4 relative)
+            assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * (want - res.double()).abs() + 1e-2 * bound + 1e-3).all(), act
+            assert torch.equal(got, gemm(x, w, bias=bias, act=act, residual=res, alpha=0.5))
+
+
+def test_residual_in_place_and_graph_replay(cuda_status):
+    """The result may replace the residual; a captured chain of dependent products gives what the eager one gives."""
+    x, w, _, _ = _operands(5, 256, 256)
+    w = (w.float() * 0.05).bfloat16()
+
+    def chain(t, r):
+        for _ in range(6):
+            gemm(t, w, residual=r, out=r)
+            t = gemm(r, w, act="relu")
+        return t
+
+    r0 = x.flip(0).contiguous()
+    want = chain(x, r0.clone())
+    r = r0.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(x, r)
+    r.copy_(r0)
+    graph.replay()
+    assert torch.equal(got, want)
