@@ -26,6 +26,7 @@
 // reference's dense attention gradient (crates/autodiff/src/lib.rs:645-806 applied to crates/nn/src/attention.rs:640-836).
 #include "attention.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -85,6 +86,8 @@ __global__ void __launch_bounds__(kB2Threads, 1)
 attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, B2Params p,
                  unsigned int* status) {
+  pdl_wait();
+  pdl_launch();
   using L = B2Smem<D, MODE>;
   constexpr int ST = L::kStages, RS = L::kResStages, SB = L::kSBufs, DB = L::kDpBufs;
   extern __shared__ uint8_t smem_raw[];
@@ -545,7 +548,7 @@ int b2_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* t
     if (e != cudaSuccess) return static_cast<int>(e);
     cfg = true;
   }
-  kern<<<grid, rb::kB2Threads, smem, stream>>>(*tq, *tk, *tv, *tdo, p, rbhost::status_ptr());
+  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kB2Threads), smem, stream, 1, *tq, *tk, *tv, *tdo, p, rbhost::status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 }  // namespace

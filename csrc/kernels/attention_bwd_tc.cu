@@ -20,6 +20,7 @@
 // Same semantics as the mma.sync backward in attention.cu (causal alignment to the end of the keys, GQA).
 #include "attention.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -71,6 +72,8 @@ template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_tc_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
                      long long bs, long long rs, long long hs, int heads, int seq_q) {
+  pdl_wait();
+  pdl_launch();
   // delta[b, h, r] = sum_d dO * O.  D / 8 adjacent lanes share a row (one 16-byte load of each tensor per lane).
   constexpr int TPR = D / 8;                       // threads per row: 8 or 16
   constexpr int RPB = 256 / TPR;                   // rows per block
@@ -534,10 +537,10 @@ RB_API int rb_attention_delta_tc(const RbAttnArgs* a, void* stream_v) {
   const __nv_bfloat16* o = reinterpret_cast<const __nv_bfloat16*>(a->o);
   const __nv_bfloat16* d_o = reinterpret_cast<const __nv_bfloat16*>(a->d_o);
   if (D == 64)
-    rb::attn_delta_tc_kernel<64><<<dgrid, 256, 0, stream>>>(o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
+    rbhost::launch_pdl(rb::attn_delta_tc_kernel<64>, dim3(dgrid), dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
                                                              a->o_strides[2], a->heads, a->seq_q);
   else
-    rb::attn_delta_tc_kernel<128><<<dgrid, 256, 0, stream>>>(o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
+    rbhost::launch_pdl(rb::attn_delta_tc_kernel<128>, dim3(dgrid), dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
                                                               a->o_strides[2], a->heads, a->seq_q);
   return static_cast<int>(cudaGetLastError());
 }

@@ -24,6 +24,7 @@
 // Replaces the reference's materialised-score attention (crates/nn/src/attention.rs:640-836).
 #include "attention.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -242,6 +243,8 @@ __global__ void __launch_bounds__(kF2Threads, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQr,
                  const __grid_constant__ CUtensorMap tmKr, F2Params p, unsigned int* status) {
+  pdl_wait();
+  pdl_launch();
   using L = F2Smem<D + DR, DV>;
   constexpr int kStages = L::kStages, kVStages = L::kVStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -670,7 +673,7 @@ int f2_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* t
     if (e != cudaSuccess) return static_cast<int>(e);
     cfg = true;
   }
-  kern<<<grid, rb::kF2Threads, smem, stream>>>(*tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk, p, rbhost::status_ptr());
+  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kF2Threads), smem, stream, 1, *tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk, p, rbhost::status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 }  // namespace

@@ -6,6 +6,7 @@
 // One templated grid-stride kernel per family; 128-bit accesses when the pointers allow it.
 #include "elementwise.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -66,6 +67,8 @@ __device__ __forceinline__ float scalar_apply(int op, float a, float s) {
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
 pointwise_kernel(int op, const T* __restrict__ a, const T* __restrict__ b, float s, T* __restrict__ out, long long n) {
+  pdl_wait();
+  pdl_launch();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const float x = (MODE == 2 && op == RB_FILL) ? 0.f : Cvt<T>::ld(a + i);
@@ -83,6 +86,8 @@ pointwise_kernel(int op, const T* __restrict__ a, const T* __restrict__ b, float
 template <int MODE>
 __global__ void __launch_bounds__(256)
 pointwise_bf16x8_kernel(int op, const uint4* __restrict__ a, const uint4* __restrict__ b, float s, uint4* __restrict__ out, long long n8) {
+  pdl_wait();
+  pdl_launch();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += stride) {
     uint4 ua = (MODE == 2 && op == RB_FILL) ? make_uint4(0, 0, 0, 0) : a[i];
@@ -121,18 +126,18 @@ int launch_pointwise(int op, const void* a, const void* b, float s, void* out, l
     const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(out);
     const long long n8 = ((bits & 15) == 0) ? n / 8 : 0;
     if (n8 > 0)
-      pointwise_bf16x8_kernel<MODE><<<ew_grid(n8), 256, 0, st>>>(op, reinterpret_cast<const uint4*>(a),
+      rbhost::launch_pdl(pointwise_bf16x8_kernel<MODE>, dim3(ew_grid(n8)), dim3(256), 0, st, 1, op, reinterpret_cast<const uint4*>(a),
                                                                  reinterpret_cast<const uint4*>(b), s,
                                                                  reinterpret_cast<uint4*>(out), n8);
     const long long done = n8 * 8;
     if (done < n) {
       auto A = reinterpret_cast<const __nv_bfloat16*>(a);
       auto B = reinterpret_cast<const __nv_bfloat16*>(b);
-      pointwise_kernel<__nv_bfloat16, MODE><<<ew_grid(n - done), 256, 0, st>>>(
+      rbhost::launch_pdl(pointwise_kernel<__nv_bfloat16, MODE>, dim3(ew_grid(n - done)), dim3(256), 0, st, 1, 
           op, A ? A + done : A, B ? B + done : B, s, reinterpret_cast<__nv_bfloat16*>(out) + done, n - done);
     }
   } else {
-    pointwise_kernel<float, MODE><<<ew_grid(n), 256, 0, st>>>(op, reinterpret_cast<const float*>(a),
+    rbhost::launch_pdl(pointwise_kernel<float, MODE>, dim3(ew_grid(n)), dim3(256), 0, st, 1, op, reinterpret_cast<const float*>(a),
                                                               reinterpret_cast<const float*>(b), s,
                                                               reinterpret_cast<float*>(out), n);
   }
@@ -154,6 +159,8 @@ constexpr int kSumDim0Slabs = 128;
 template <typename T>
 __global__ void __launch_bounds__(256)
 sum_dim0_stage1(const T* __restrict__ a, long long lda, float* __restrict__ partial, long long rows, int cols) {
+  pdl_wait();
+  pdl_launch();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int slab = blockIdx.y;
   const long long per = (rows + gridDim.y - 1) / gridDim.y;
@@ -168,6 +175,8 @@ sum_dim0_stage1(const T* __restrict__ a, long long lda, float* __restrict__ part
 // slab; the 8 row lanes of a column group are folded through shared memory in lane order (deterministic).
 __global__ void __launch_bounds__(256)
 sum_dim0_stage1_vec(const __nv_bfloat16* __restrict__ a, long long lda, float* __restrict__ partial, long long rows, int cols) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh[8][32][9];
   const int cg = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + cg) * 8;
@@ -211,6 +220,8 @@ sum_dim0_stage1_vec(const __nv_bfloat16* __restrict__ a, long long lda, float* _
 }
 __global__ void __launch_bounds__(256)
 sum_dim0_stage2(const float* __restrict__ partial, int slabs, float* __restrict__ out, int cols, int accumulate) {
+  pdl_wait();
+  pdl_launch();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
   float acc = 0.f;
@@ -238,6 +249,8 @@ sum_dim0_direct(const T* __restrict__ a, long long lda, float* __restrict__ out,
 
 template <typename T>
 __global__ void __launch_bounds__(256) sum_all_stage1(const T* __restrict__ a, long long n, float* __restrict__ scratch) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh[8];
   const long long per = (n + gridDim.x - 1) / gridDim.x;
   const long long lo = per * blockIdx.x;
@@ -254,6 +267,8 @@ __global__ void __launch_bounds__(256) sum_all_stage1(const T* __restrict__ a, l
   }
 }
 __global__ void __launch_bounds__(256) sum_all_stage2(const float* __restrict__ scratch, int nb, float* out) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh[256];
   float acc = 0.f;
   for (int i = threadIdx.x; i < nb; i += 256) acc += scratch[i];
@@ -285,6 +300,8 @@ template <typename T, bool SCATTER>
 __global__ void __launch_bounds__(256)
 rows_kernel(const T* __restrict__ a, const long long* __restrict__ idx, T* __restrict__ out, long long n_idx, int cols,
             long long limit RB_BOUNDS_PARAM) {
+  pdl_wait();
+  pdl_launch();
   const long long n = n_idx * cols;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -446,11 +463,11 @@ RB_API int rb_sum_dim0_staged(const void* a, long long lda, float* out, float* p
   int slabs = rb::kSumDim0Slabs;
   if (rows < slabs) slabs = static_cast<int>(rows);
   dim3 grid((cols + 255) / 256, slabs);
-  if (dtype == 0) rb::sum_dim0_stage1<float><<<grid, 256, 0, RB_STREAM>>>((const float*)a, lda, partial, rows, cols);
+  if (dtype == 0) rbhost::launch_pdl(rb::sum_dim0_stage1<float>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const float*)a, lda, partial, rows, cols);
   else if ((cols % 8 == 0) && (lda % 8 == 0) && (reinterpret_cast<uintptr_t>(a) % 16 == 0))
-    rb::sum_dim0_stage1_vec<<<dim3((cols + 255) / 256, slabs), 256, 0, RB_STREAM>>>((const __nv_bfloat16*)a, lda, partial, rows, cols);
-  else rb::sum_dim0_stage1<__nv_bfloat16><<<grid, 256, 0, RB_STREAM>>>((const __nv_bfloat16*)a, lda, partial, rows, cols);
-  rb::sum_dim0_stage2<<<(cols + 255) / 256, 256, 0, RB_STREAM>>>(partial, slabs, out, cols, accumulate);
+    rbhost::launch_pdl(rb::sum_dim0_stage1_vec, dim3((cols + 255) / 256, slabs), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
+  else rbhost::launch_pdl(rb::sum_dim0_stage1<__nv_bfloat16>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
+  rbhost::launch_pdl(rb::sum_dim0_stage2, dim3((cols + 255) / 256), dim3(256), 0, RB_STREAM, 1, partial, slabs, out, cols, accumulate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -458,9 +475,9 @@ RB_API int rb_sum_all(const void* a, long long n, int dtype, float* scratch, flo
   if (n <= 0 || !scratch || !out) return -1;
   long long want = (n + 4095) / 4096;
   const int nb = static_cast<int>(want < 1024 ? (want < 1 ? 1 : want) : 1024);
-  if (dtype == 0) rb::sum_all_stage1<float><<<nb, 256, 0, RB_STREAM>>>((const float*)a, n, scratch);
-  else rb::sum_all_stage1<__nv_bfloat16><<<nb, 256, 0, RB_STREAM>>>((const __nv_bfloat16*)a, n, scratch);
-  rb::sum_all_stage2<<<1, 256, 0, RB_STREAM>>>(scratch, nb, out);
+  if (dtype == 0) rbhost::launch_pdl(rb::sum_all_stage1<float>, dim3(nb), dim3(256), 0, RB_STREAM, 1, (const float*)a, n, scratch);
+  else rbhost::launch_pdl(rb::sum_all_stage1<__nv_bfloat16>, dim3(nb), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, n, scratch);
+  rbhost::launch_pdl(rb::sum_all_stage2, dim3(1), dim3(256), 0, RB_STREAM, 1, scratch, nb, out);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -474,14 +491,14 @@ RB_API int rb_transpose(const void* a, void* out, int rows, int cols, int dtype,
 RB_API int rb_gather_rows(const void* a, const long long* idx, void* out, long long n_idx, int cols, long long src_rows, int dtype, void* stream_v) {
   if (n_idx <= 0 || cols <= 0) return 0;
   const int grid = rb::ew_grid(n_idx * cols);
-  RB_BY_DTYPE((rb::rows_kernel<float, false><<<grid, 256, 0, RB_STREAM>>>((const float*)a, idx, (float*)out, n_idx, cols, src_rows RB_BOUNDS_ARG)),
-              (rb::rows_kernel<__nv_bfloat16, false><<<grid, 256, 0, RB_STREAM>>>((const __nv_bfloat16*)a, idx, (__nv_bfloat16*)out, n_idx, cols, src_rows RB_BOUNDS_ARG)))
+  RB_BY_DTYPE((rbhost::launch_pdl(rb::rows_kernel<float, false>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const float*)a, idx, (float*)out, n_idx, cols, src_rows RB_BOUNDS_ARG)),
+              (rbhost::launch_pdl(rb::rows_kernel<__nv_bfloat16, false>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, idx, (__nv_bfloat16*)out, n_idx, cols, src_rows RB_BOUNDS_ARG)))
 }
 RB_API int rb_scatter_rows(const void* a, const long long* idx, void* out, long long n_idx, int cols, long long dst_rows, int dtype, void* stream_v) {
   if (n_idx <= 0 || cols <= 0) return 0;
   const int grid = rb::ew_grid(n_idx * cols);
-  RB_BY_DTYPE((rb::rows_kernel<float, true><<<grid, 256, 0, RB_STREAM>>>((const float*)a, idx, (float*)out, n_idx, cols, dst_rows RB_BOUNDS_ARG)),
-              (rb::rows_kernel<__nv_bfloat16, true><<<grid, 256, 0, RB_STREAM>>>((const __nv_bfloat16*)a, idx, (__nv_bfloat16*)out, n_idx, cols, dst_rows RB_BOUNDS_ARG)))
+  RB_BY_DTYPE((rbhost::launch_pdl(rb::rows_kernel<float, true>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const float*)a, idx, (float*)out, n_idx, cols, dst_rows RB_BOUNDS_ARG)),
+              (rbhost::launch_pdl(rb::rows_kernel<__nv_bfloat16, true>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, idx, (__nv_bfloat16*)out, n_idx, cols, dst_rows RB_BOUNDS_ARG)))
 }
 RB_API int rb_broadcast_to(const void* a, void* out, long long arows, long long acols, long long rows, long long cols, int dtype, void* stream_v) {
   if (rows <= 0 || cols <= 0 || arows <= 0 || acols <= 0) return -1;

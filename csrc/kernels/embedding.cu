@@ -8,6 +8,7 @@
 
 #include <limits.h>
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -16,6 +17,8 @@ __global__ void __launch_bounds__(128)
 embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ wte,
                      const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out, long long tokens, int dim,
                      int seq_len, long long vocab RB_BOUNDS_PARAM) {
+  pdl_wait();
+  pdl_launch();
   const int chunks = dim / 8;
   const long long total = tokens * chunks;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -49,6 +52,8 @@ __global__ void hist_kernel(const long long* __restrict__ ids, long long tokens,
 
 // single CTA exclusive scan; offsets[vocab] = total
 __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, long long vocab) {
+  pdl_wait();
+  pdl_launch();
   __shared__ int sh[1024];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -74,6 +79,8 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ coun
 
 __global__ void fill_kernel(const long long* __restrict__ ids, long long tokens, long long vocab,
                             const int* __restrict__ offsets, int* cursor, int* __restrict__ perm) {
+  pdl_wait();
+  pdl_launch();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < tokens; t += stride) {
     const long long id = ids[t];
@@ -88,6 +95,8 @@ __global__ void fill_kernel(const long long* __restrict__ ids, long long tokens,
 __global__ void __launch_bounds__(128)
 scatter_rows_kernel(const __nv_bfloat16* __restrict__ dy, const int* __restrict__ offsets, const int* __restrict__ perm,
                     int* __restrict__ sorted, float* __restrict__ dw, int dim, long long vocab) {
+  pdl_wait();
+  pdl_launch();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= vocab) return;
@@ -129,6 +138,8 @@ scatter_rows_kernel(const __nv_bfloat16* __restrict__ dy, const int* __restrict_
 // dwpe[s, c] += sum_b dy[b*seq_len + s, c]
 __global__ void __launch_bounds__(128)
 pos_grad_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dwpe, long long tokens, int dim, int seq_len) {
+  pdl_wait();
+  pdl_launch();
   const int chunks = dim / 8;
   const long long total = static_cast<long long>(seq_len) * chunks;
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -195,7 +206,7 @@ RB_API int rb_embedding_fwd(const long long* ids, const void* wte, const void* w
   const long long total = tokens * (dim / 8);
   long long blocks = (total + 127) / 128;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
-  rb::embedding_fwd_kernel<<<static_cast<int>(blocks), 128, 0, stream>>>(
+  rbhost::launch_pdl(rb::embedding_fwd_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, stream, 1, 
       ids, reinterpret_cast<const __nv_bfloat16*>(wte), reinterpret_cast<const __nv_bfloat16*>(wpe),
       reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, seq_len < 1 ? 1 : seq_len, vocab RB_BOUNDS_ARG);
   return static_cast<int>(cudaGetLastError());
@@ -223,13 +234,13 @@ RB_API int rb_embedding_bwd(const long long* ids, const void* dy, float* dwte, f
   auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
   if (dwte) {
     rb::hist_kernel<<<tb, 256, 0, stream>>>(ids, tokens, vocab, counts);
-    rb::scan_kernel<<<1, 1024, 0, stream>>>(counts, offsets, vocab);
-    rb::fill_kernel<<<tb, 256, 0, stream>>>(ids, tokens, vocab, offsets, cursor, perm);
-    rb::scatter_rows_kernel<<<static_cast<int>((vocab + 3) / 4), 128, 0, stream>>>(DY, offsets, perm, sorted, dwte, dim, vocab);
+    rbhost::launch_pdl(rb::scan_kernel, dim3(1), dim3(1024), 0, stream, 1, counts, offsets, vocab);
+    rbhost::launch_pdl(rb::fill_kernel, dim3(tb), dim3(256), 0, stream, 1, ids, tokens, vocab, offsets, cursor, perm);
+    rbhost::launch_pdl(rb::scatter_rows_kernel, dim3(static_cast<int>((vocab + 3) / 4)), dim3(128), 0, stream, 1, DY, offsets, perm, sorted, dwte, dim, vocab);
   }
   if (dwpe) {
     const long long total = static_cast<long long>(seq_len) * (dim / 8);
-    rb::pos_grad_kernel<<<static_cast<int>((total + 127) / 128), 128, 0, stream>>>(DY, dwpe, tokens, dim, seq_len);
+    rbhost::launch_pdl(rb::pos_grad_kernel, dim3(static_cast<int>((total + 127) / 128)), dim3(128), 0, stream, 1, DY, dwpe, tokens, dim, seq_len);
   }
   return static_cast<int>(cudaGetLastError());
 }

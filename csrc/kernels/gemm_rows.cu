@@ -48,7 +48,7 @@ __device__ __forceinline__ float rows_act(int act, float v) {
 
 __global__ void __launch_bounds__(kRowsThreads)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, int M, int N, int K, int mpad,
-                 int parts, int stages, const RowsEpi ep, unsigned int* status) {
+                 int parts, int stages, int w_constant, const RowsEpi ep, unsigned int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t base = smem_u32(smem);
@@ -82,13 +82,21 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   if (warp == 0) {
     if (elect_one()) {
+      // W of the first stages is on its way before the kernel in front has ended, X follows when it has
+      const int ahead = w_constant ? min(stages, kb1 - kb0) : 0;
+      for (int it = 0; it < ahead; ++it) {
+        mbar_arrive_expect_tx(bar_full + 8 * it, stage_bytes);
+        tma_load_2d(base + it * stage_bytes, &tmW, (kb0 + it) * 64, tile * kRowsTile, bar_full + 8 * it);
+      }
       pdl_wait();
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int it = kb - kb0, s = it % stages;
-        if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag, status, 81)) break;
-        mbar_arrive_expect_tx(bar_full + 8 * s, stage_bytes);
-        tma_load_2d(base + s * stage_bytes, &tmW, kb * 64, tile * kRowsTile, bar_full + 8 * s);
-        tma_load_2d(base + s * stage_bytes + kRowsWBytes, &tmX, kb * 64, 0, bar_full + 8 * s);
+      for (int it = 0; it < kb1 - kb0; ++it) {
+        const int s = it % stages;
+        if (it >= ahead) {
+          if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag, status, 81)) break;
+          mbar_arrive_expect_tx(bar_full + 8 * s, stage_bytes);
+          tma_load_2d(base + s * stage_bytes, &tmW, (kb0 + it) * 64, tile * kRowsTile, bar_full + 8 * s);
+        }
+        tma_load_2d(base + s * stage_bytes + kRowsWBytes, &tmX, (kb0 + it) * 64, 0, bar_full + 8 * s);
       }
     }
   } else if (warp == 1) {
@@ -237,7 +245,7 @@ int gemm_rows(const RbGemmArgs& g, cudaStream_t stream) {
   ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual); ep.ldr = g.ldr;
   ep.act = g.act; ep.out_f32 = g.out_f32; ep.alpha = g.alpha;
   return static_cast<int>(launch_pdl(rb::gemm_rows_kernel, dim3(tiles * parts), dim3(rb::kRowsThreads), smem, stream, parts, *tw, *tx,
-                                     g.M, g.N, g.K, mpad, parts, stages, ep, status_ptr()));
+                                     g.M, g.N, g.K, mpad, parts, stages, g.b_constant, ep, status_ptr()));
 }
 
 }  // namespace rbhost

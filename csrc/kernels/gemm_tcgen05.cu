@@ -23,6 +23,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -370,6 +371,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();            // barriers, TMEM and descriptors were set up under the kernel in front
+  // A kernel that waits for other kernels' stores must not let its successor's blocks take the room that those kernels need.
+  if (peer.mode == 0 && grp.tile_arrived == nullptr) pdl_launch();
 
   int num_m = (M + kBlockM - 1) / kBlockM;
   if (grp.mode == 1) num_m = min(num_m, __ldg(grp.num_m_tiles));
@@ -869,6 +873,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync_all();                                 // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();            // barriers, TMEM and descriptors were set up under the kernel in front
+  pdl_launch();
 
   const int num_m = (M + kPairM - 1) / kPairM;
   const int num_n = (N + BLOCK_N - 1) / BLOCK_N;
@@ -1178,6 +1184,8 @@ __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slab, void* d, long long ldd, int M, int N,
                      int out_f32, int accumulate, const __nv_bfloat16* __restrict__ bias,
                      const __nv_bfloat16* __restrict__ residual, long long ldr) {
+  pdl_wait();
+  pdl_launch();
   const long long n4 = static_cast<long long>(M) * N / 4;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -1314,13 +1322,13 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
     peer.a_peer[r] = reinterpret_cast<const __nv_bfloat16*>(g.peer_ptrs[r]);
     peer.d_peer[r] = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(g.peer_ptrs[r]));
   }
-  kern<<<grid, rb::kNumThreads, smem, stream>>>(*ta, *tb, *td, *tx, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
+  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kNumThreads), smem, stream, 1, *ta, *tb, *td, *tx, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
                                                 rbhost::status_ptr());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
   const long long n4 = slab / 4;
   int rgrid = static_cast<int>((n4 + 255) / 256 < 148 * 8 ? (n4 + 255) / 256 : 148 * 8);
-  rb::splitk_reduce_kernel<<<rgrid, 256, 0, stream>>>(reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
+  rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
                                                       reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);
@@ -1394,23 +1402,12 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
     ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
     ep.bias = nullptr; ep.residual = nullptr;
   }
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(rb::kNumThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *ta, *tb_half, *td, *tx, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep,
-                                     rbhost::status_ptr());
+  const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(rb::kNumThreads), smem, stream, 2, *ta, *tb_half, *td, *tx, g.M, g.N,
+                                           k_units, group_m, splits, kb_per, slab, ep, rbhost::status_ptr());
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
   const long long n4 = slab / 4;
   int rgrid = static_cast<int>((n4 + 255) / 256 < 148 * 8 ? (n4 + 255) / 256 : 148 * 8);
-  rb::splitk_reduce_kernel<<<rgrid, 256, 0, stream>>>(reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
+  rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
                                                       reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);

@@ -66,6 +66,8 @@ typedef struct RbGemmArgs {
   int ab_fp8;                  // 0: bf16 operands; 1: a and b e4m3; 2: a e4m3, b e5m2
   const void* a_scale;         // fp32 [M] or NULL: one scale per row of A (per token)
   const void* b_scale;         // fp32 [N] or NULL: one scale per row of B (per output channel)
+  int b_constant;              // 1: the kernel in front of this call in its stream does not write B (a served model's weights), so
+                               // that B may be read while that kernel still runs
 } RbGemmArgs;
 
 // Returns 0 on success, a negative code for rejected arguments, a positive cudaError otherwise.

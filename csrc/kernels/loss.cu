@@ -10,6 +10,7 @@
 
 #include <float.h>
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -54,6 +55,8 @@ __global__ void __launch_bounds__(kCeThreads)
 cross_entropy_kernel(const __nv_bfloat16* logits, long long ld, const long long* __restrict__ targets,
                      float* __restrict__ loss, float* __restrict__ lse_out, __nv_bfloat16* dlogits, long long ldd,
                      int n_valid, int n_pad, float grad_scale, long long ignore_index RB_BOUNDS_PARAM) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh_m[32], sh_s[32];
   const long long row = blockIdx.x;
   const __nv_bfloat16* x = logits + row * ld;
@@ -232,7 +235,7 @@ RB_API int rb_cross_entropy(const void* logits, long long ld, const long long* t
                             long long ignore_index, void* stream_v) {
   if (rows <= 0 || n_valid <= 0 || n_pad < n_valid || !logits || !targets || !loss) return -1;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  rb::cross_entropy_kernel<<<rows, rb::kCeThreads, 0, stream>>>(
+  rbhost::launch_pdl(rb::cross_entropy_kernel, dim3(rows), dim3(rb::kCeThreads), 0, stream, 1, 
       reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, loss, lse, reinterpret_cast<__nv_bfloat16*>(dlogits),
       ldd, n_valid, n_pad, grad_scale, ignore_index RB_BOUNDS_ARG);
   return static_cast<int>(cudaGetLastError());

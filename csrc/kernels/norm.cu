@@ -9,6 +9,7 @@
 // root (crates/nn/src/normalization.rs:87-158; backward crates/autodiff/src/lib.rs:1167-1214).
 #include "norm.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -67,6 +68,8 @@ __global__ void __launch_bounds__(kNormWarps * 32)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, long long ldy,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int n, float eps) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float red[kNormWarps];
   constexpr int RPB = kNormWarps / WPR;
   const int lane = threadIdx.x & 31;
@@ -135,6 +138,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
                 long long ldx, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres, long long lddres,
                 __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ partial, int rows, int n) {
+  pdl_wait();
+  pdl_launch();
   extern __shared__ float sm[];   // [RPB][2][n_pad]
   __shared__ float red[kNormWarps];
   constexpr int RPB = kNormWarps / WPR;
@@ -264,6 +269,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
 __global__ void __launch_bounds__(256)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int num_partials, int n, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, int accumulate) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sa[8][33], sb[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + tx;
@@ -349,9 +356,9 @@ RB_API int rb_norm_fwd(const void* x, long long ldx, const void* gamma, const vo
   auto B = reinterpret_cast<const __nv_bfloat16*>(beta);
   auto Y = reinterpret_cast<__nv_bfloat16*>(y);
 #define RB_LAUNCH(C, W)                                                                                           \
-  if (rms) rb::norm_fwd_kernel<C, W, true><<<grid, rb::kNormWarps * 32, 0, stream>>>(X, ldx, G, nullptr, Y, ldy,  \
+  if (rms) rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, true>, dim3(grid), dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, nullptr, Y, ldy,  \
                                                                                      nullptr, rstd, rows, n, eps);\
-  else rb::norm_fwd_kernel<C, W, false><<<grid, rb::kNormWarps * 32, 0, stream>>>(X, ldx, G, B, Y, ldy, mean,     \
+  else rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, false>, dim3(grid), dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, B, Y, ldy, mean,     \
                                                                                   rstd, rows, n, eps);
   RB_NORM_DISPATCH(n, RB_LAUNCH)
 #undef RB_LAUNCH
@@ -382,12 +389,12 @@ RB_API int rb_norm_bwd(const void* dy, long long lddy, const void* x, long long 
     if (rms) {                                                                                                     \
       auto k = rb::norm_bwd_kernel<C, W, true>;                                                                    \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-      k<<<grid, rb::kNormWarps * 32, smem, stream>>>(DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
+      rbhost::launch_pdl(k, dim3(grid), dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
                                                      partial, rows, n);                                            \
     } else {                                                                                                       \
       auto k = rb::norm_bwd_kernel<C, W, false>;                                                                   \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-      k<<<grid, rb::kNormWarps * 32, smem, stream>>>(DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
+      rbhost::launch_pdl(k, dim3(grid), dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
                                                      partial, rows, n);                                            \
     }                                                                                                              \
   }
@@ -395,7 +402,7 @@ RB_API int rb_norm_bwd(const void* dy, long long lddy, const void* x, long long 
 #undef RB_LAUNCH
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  rb::norm_bwd_reduce_kernel<<<(n + 31) / 32, 256, 0, stream>>>(partial, grid, n, dgamma, rms ? nullptr : dbeta,
+  rbhost::launch_pdl(rb::norm_bwd_reduce_kernel, dim3((n + 31) / 32), dim3(256), 0, stream, 1, partial, grid, n, dgamma, rms ? nullptr : dbeta,
                                                                  accumulate);
   return static_cast<int>(cudaGetLastError());
 }

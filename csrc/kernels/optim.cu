@@ -8,6 +8,7 @@
 // (crates/optim/src/lib.rs:464-470,604) and that behaviour is available with decoupled = 0.
 #include "optim.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -17,6 +18,8 @@ __global__ void __launch_bounds__(256)
 adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, const void* __restrict__ g_v,
             __nv_bfloat16* __restrict__ p_bf16, long long n, RbAdamArgs a, const float* __restrict__ grad_norm,
             const int* __restrict__ found_inf) {
+  pdl_wait();
+  pdl_launch();
   if (found_inf != nullptr && *found_inf != 0) return;   // overflow: skip the whole step
   float gscale = a.grad_scale;
   if (a.max_grad_norm > 0.f && grad_norm != nullptr) {
@@ -107,6 +110,8 @@ constexpr int kSumsqBlocks = 1024;
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 sumsq_stage1(const void* __restrict__ x_v, long long n, float* __restrict__ scratch, int* __restrict__ found_inf) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh[8];
   float acc = 0.f;
   bool bad = false;
@@ -131,6 +136,8 @@ sumsq_stage1(const void* __restrict__ x_v, long long n, float* __restrict__ scra
   }
 }
 __global__ void __launch_bounds__(256) sumsq_stage2(const float* __restrict__ scratch, int nblocks, float* out, int accumulate) {
+  pdl_wait();
+  pdl_launch();
   __shared__ float sh[256];
   float acc = 0.f;
   for (int i = threadIdx.x; i < nblocks; i += 256) acc += scratch[i];
@@ -142,7 +149,9 @@ __global__ void __launch_bounds__(256) sumsq_stage2(const float* __restrict__ sc
   }
   if (threadIdx.x == 0) out[0] = accumulate ? out[0] + sh[0] : sh[0];
 }
-__global__ void sqrt_scalar_kernel(const float* in, float* out) { out[0] = sqrtf(in[0]); }
+__global__ void sqrt_scalar_kernel(const float* in, float* out) {
+  pdl_wait();
+  pdl_launch(); out[0] = sqrtf(in[0]); }
 
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ d, long long n) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * 4;
@@ -185,10 +194,10 @@ RB_API int rb_adam_step(float* p, float* m, float* v, const void* g, int g_bf16,
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   const int grid = rb::grid_for(n, 4);
   if (g_bf16)
-    rb::adam_kernel<true><<<grid, 256, 0, stream>>>(p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
+    rbhost::launch_pdl(rb::adam_kernel<true>, dim3(grid), dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
                                                     grad_norm, found_inf);
   else
-    rb::adam_kernel<false><<<grid, 256, 0, stream>>>(p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
+    rbhost::launch_pdl(rb::adam_kernel<false>, dim3(grid), dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
                                                      grad_norm, found_inf);
   return static_cast<int>(cudaGetLastError());
 }
@@ -216,14 +225,14 @@ RB_API int rb_sumsq(const void* x, int is_bf16, long long n, float* scratch, flo
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   long long want = (n + 4095) / 4096;
   const int blocks = static_cast<int>(want < rb::kSumsqBlocks ? (want < 1 ? 1 : want) : rb::kSumsqBlocks);
-  if (is_bf16) rb::sumsq_stage1<true><<<blocks, 256, 0, stream>>>(x, n, scratch, found_inf);
-  else rb::sumsq_stage1<false><<<blocks, 256, 0, stream>>>(x, n, scratch, found_inf);
-  rb::sumsq_stage2<<<1, 256, 0, stream>>>(scratch, blocks, out, accumulate);
+  if (is_bf16) rbhost::launch_pdl(rb::sumsq_stage1<true>, dim3(blocks), dim3(256), 0, stream, 1, x, n, scratch, found_inf);
+  else rbhost::launch_pdl(rb::sumsq_stage1<false>, dim3(blocks), dim3(256), 0, stream, 1, x, n, scratch, found_inf);
+  rbhost::launch_pdl(rb::sumsq_stage2, dim3(1), dim3(256), 0, stream, 1, scratch, blocks, out, accumulate);
   return static_cast<int>(cudaGetLastError());
 }
 
 RB_API int rb_sqrt_scalar(const float* in, float* out, void* stream_v) {
-  rb::sqrt_scalar_kernel<<<1, 1, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(in, out);
+  rbhost::launch_pdl(rb::sqrt_scalar_kernel, dim3(1), dim3(1), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, in, out);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -12,6 +12,7 @@
 
 #include <float.h>
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -20,6 +21,8 @@ __global__ void __launch_bounds__(128)
 kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, long long ld_k, const __nv_bfloat16* __restrict__ v_new,
                  long long ld_v, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                  const long long* __restrict__ slots, long long tokens, int row_elems, long long num_slots RB_BOUNDS_PARAM) {
+  pdl_wait();
+  pdl_launch();
   const int chunks = row_elems / 8;
   const long long total = tokens * chunks;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -123,6 +126,8 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
                           int block_size, long long num_blocks, float scale, int g0, int gcount, float* __restrict__ partial,
                           int nsplit, __nv_bfloat16* __restrict__ direct_out, long long ld_o, const PaRule rule
                           RB_BOUNDS_PARAM) {
+  pdl_wait();
+  pdl_launch();
   constexpr int LPK = DK / 8, LPV = DV / 8;  // 16-byte pieces per K / V row = copies per lane for a 32-row tile
   constexpr int KROW = DK + 8, VROW = DV + 8;  // padded rows (elements): ldmatrix rows 272 (144) bytes apart hit distinct banks
   constexpr int NT = DV / 8;                 // n-tiles of the output accumulator
@@ -370,6 +375,8 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
 __global__ void __launch_bounds__(128)
 paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restrict__ context_lens, int heads, int dv,
                           int nsplit, __nv_bfloat16* __restrict__ out, long long ld_o, const PaRule rule) {
+  pdl_wait();
+  pdl_launch();
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   if (d >= dv) return;
   const int ctx = context_lens[b];
@@ -511,7 +518,7 @@ RB_API int rb_kv_append(const void* k_new, long long ld_k, const void* v_new, lo
   const long long total = tokens * (row / 8);
   long long blocks = (total + 127) / 128;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  rb::kv_append_kernel<<<static_cast<int>(blocks), 128, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  rbhost::launch_pdl(rb::kv_append_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
       reinterpret_cast<const __nv_bfloat16*>(k_new), ld_k, reinterpret_cast<const __nv_bfloat16*>(v_new), ld_v,
       reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), slot_mapping, tokens, row,
       num_slots RB_BOUNDS_ARG);
@@ -547,13 +554,13 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
                            a.window, a.keep_first, a.sink, a.log_amount, a.log_rate, a.out_scale};
   const dim3 grid(a.batch, a.kv_heads, nsplit);
   for (int g0 = 0; g0 < group; g0 += rb::kMaxGroup)       // groups wider than 16 heads take several passes
-    kern<<<grid, rb::kPaWarps * 32, smem, stream>>>(
+    rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kPaWarps * 32), smem, stream, 1, 
         reinterpret_cast<const __nv_bfloat16*>(a.q), a.ld_q, reinterpret_cast<const __nv_bfloat16*>(a.k_cache),
         reinterpret_cast<const __nv_bfloat16*>(a.v_cache), a.block_tables, a.max_blocks, a.context_lens, a.heads, a.kv_heads,
         a.dk, a.dv, a.block_size, a.num_blocks, a.scale, g0, group - g0 < rb::kMaxGroup ? group - g0 : rb::kMaxGroup,
         a.scratch, nsplit, nsplit == 1 ? O : nullptr, a.ld_o, rule RB_BOUNDS_ARG);
   if (nsplit > 1)
-    rb::paged_decode_merge_kernel<<<dim3(a.batch, a.heads), 128, 0, stream>>>(a.scratch, a.context_lens, a.heads, a.dv, nsplit,
+    rbhost::launch_pdl(rb::paged_decode_merge_kernel, dim3(a.batch, a.heads), dim3(128), 0, stream, 1, a.scratch, a.context_lens, a.heads, a.dv, nsplit,
                                                                               O, a.ld_o, rule);
   return static_cast<int>(cudaGetLastError());
 }

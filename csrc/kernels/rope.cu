@@ -4,6 +4,7 @@
 // crates/nn/src/shared_expert.rs:143-169); they are required by its Llama-shaped benchmark config.
 #include "rope.h"
 
+#include "pdl.cuh"
 #include "rb_common.cuh"
 
 namespace rb {
@@ -12,6 +13,8 @@ namespace rb {
 __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __restrict__ positions, long long tokens,
             int heads, int head_dim, int seq_len, long long pos_offset, float log2_theta, int inverse) {
+  pdl_wait();
+  pdl_launch();
   const int half = head_dim / 2;
   const int groups = half / 8;
   const long long total = tokens * heads * groups;
@@ -102,6 +105,8 @@ rotate_pairs_kernel(T* __restrict__ x, long long ld, const float2* __restrict__ 
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, long long ld_gu, __nv_bfloat16* __restrict__ h, long long ld_h,
                   long long tokens, int F) {
+  pdl_wait();
+  pdl_launch();
   const int chunks = F / 8;
   const long long total = tokens * chunks;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -126,6 +131,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, long long ld_gu, __nv_bf
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, long long ld_dh, const __nv_bfloat16* __restrict__ gu,
                   long long ld_gu, __nv_bfloat16* __restrict__ dgu, long long ld_dgu, long long tokens, int F) {
+  pdl_wait();
+  pdl_launch();
   const int chunks = F / 8;
   const long long total = tokens * chunks;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -165,7 +172,7 @@ RB_API int rb_rope(void* x, long long ld, const long long* positions, long long 
   if (tokens <= 0 || heads <= 0 || head_dim <= 0 || (head_dim % 16) || (ld % 8) || theta <= 0.f) return -1;
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (!positions && seq_len <= 0)) return -2;
   const long long total = tokens * heads * (head_dim / 16);
-  rb::rope_kernel<<<rb::grid1d(total), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  rbhost::launch_pdl(rb::rope_kernel, dim3(rb::grid1d(total)), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
       reinterpret_cast<__nv_bfloat16*>(x), ld, positions, tokens, heads, head_dim, seq_len < 1 ? 1 : seq_len, pos_offset,
       log2f(theta), inverse);
   return static_cast<int>(cudaGetLastError());
@@ -195,7 +202,7 @@ RB_API int rb_rotate_pairs(void* x, long long ld, const float* table, long long 
 RB_API int rb_swiglu_fwd(const void* gu, long long ld_gu, void* h, long long ld_h, long long tokens, int F, void* stream_v) {
   if (tokens <= 0 || F <= 0 || (F % 8) || (ld_gu % 8) || (ld_h % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(h)) & 15) return -2;
-  rb::swiglu_fwd_kernel<<<rb::grid1d(tokens * (F / 8)), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  rbhost::launch_pdl(rb::swiglu_fwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
       reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(h), ld_h, tokens, F);
   return static_cast<int>(cudaGetLastError());
 }
@@ -204,7 +211,7 @@ RB_API int rb_swiglu_bwd(const void* dh, long long ld_dh, const void* gu, long l
                          long long tokens, int F, void* stream_v) {
   if (tokens <= 0 || F <= 0 || (F % 8) || (ld_gu % 8) || (ld_dh % 8) || (ld_dgu % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(dh) | reinterpret_cast<uintptr_t>(dgu)) & 15) return -2;
-  rb::swiglu_bwd_kernel<<<rb::grid1d(tokens * (F / 8)), 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(
+  rbhost::launch_pdl(rb::swiglu_bwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
       reinterpret_cast<const __nv_bfloat16*>(dh), ld_dh, reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu,
       reinterpret_cast<__nv_bfloat16*>(dgu), ld_dgu, tokens, F);
   return static_cast<int>(cudaGetLastError());

@@ -206,8 +206,9 @@ def _gemm_f32(a, b, out, alpha, tile_expert=None, num_tiles=None, expert_stride=
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, aux_out=None, out=None, out_dtype=None, accumulate: bool = False,
          alpha: float = 1.0, block_n: int = 0, group_m: int = 0, max_ctas: int = 0, splits: int = 0,
-         peer: dict | None = None, row_scale=None, col_scale=None) -> torch.Tensor:
-    """`row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
+         peer: dict | None = None, row_scale=None, col_scale=None, b_constant: bool = False) -> torch.Tensor:
+    """`b_constant`: the kernel in front of this call in its stream does not write `b` (a served model's weights), so reading `b` may
+    begin while that kernel still runs.  `row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
     scales of quantised layers).  `peer` selects the tensor-parallel modes of the kernel (see parallel/fused_tp.py): a dict with `mode`
     (1: remote row blocks of A are pulled from the peers' shards inside the kernel; 2: output row blocks are
     stored into their owner's receive slot), `world`, `rank`, `rows_per_rank`, `epoch`, `ready_flags` (pointer,
@@ -277,7 +278,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         # three addresses (and the split-K workspace), which halves the Python time of a small launch.
         cache = _plain_args()
         key = (M, Nn, K, a_mn, b_mn, act, out.dtype, accumulate, alpha, block_n, group_m, max_ctas, splits,
-               a.stride(0), b.stride(0), out.stride(0))
+               a.stride(0), b.stride(0), out.stride(0), b_constant)
         g = cache.get(key)
         if g is None:
             if len(cache) > 4096:
@@ -291,6 +292,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.accumulate = int(accumulate)
             g.alpha = alpha
             g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
+            g.b_constant = int(b_constant)
             cache[key] = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
         if splits != 1 and K >= 2048 and act == "none":
@@ -318,6 +320,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     g.accumulate = int(accumulate)
     g.alpha = alpha
     g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
+    g.b_constant = int(b_constant)
     for t, n_, nm in ((row_scale, M, "row_scale"), (col_scale, Nn, "col_scale")):
         if t is not None and (t.dtype != torch.float32 or t.numel() != n_ or not t.is_contiguous() or t.device != a.device):
             raise TypeError(f"gemm: {nm} must be a contiguous fp32 vector of {n_} elements on the operands' device")

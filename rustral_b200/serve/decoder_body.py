@@ -28,6 +28,11 @@ from .kv_cache import CacheLayer
 from .weights import latent_columns, mixer_columns, packed_columns
 
 
+def _product(a, w, **kw):
+    """a @ w^T for a weight of the model: no kernel of a step writes it."""
+    return gemm(a, w, b_constant=True, **kw)
+
+
 class GPTBody:
     """GPT-2 style and Llama style decoders (pre-norm, residual stream in the activation dtype)."""
 
@@ -49,9 +54,9 @@ class GPTBody:
         """a @ w^T (+ bias) + residual; with tensor parallelism the partial products are summed over the ranks."""
         tp = self.r.tp
         if tp is None:
-            return gemm(a, w, bias=bias, residual=residual)
+            return _product(a, w, bias=bias, residual=residual)
         rows = a.shape[0]
-        gemm(a, w, out=tp.staging(rows, w.shape[0]))
+        _product(a, w, out=tp.staging(rows, w.shape[0]))
         return tp.all_reduce(rows, w.shape[0], residual=residual)
 
     def embed(self, sb):
@@ -66,7 +71,7 @@ class GPTBody:
         H, Hk, D = r.n_head, r.n_kv_head, self.cfg.head_dim
         p = f"layers.{l}."
         h = self._norm(x, p + "ln1")
-        qkv = gemm(h, P.w(p + "attn.wqkv.weight"), bias=None if rms else P.w(p + "attn.wqkv.bias"))
+        qkv = _product(h, P.w(p + "attn.wqkv.weight"), bias=None if rms else P.w(p + "attn.wqkv.bias"))
         if rms:
             rope_ops.rope_(qkv, H + Hk, D, positions=sb.pos, theta=self.cfg.rope_theta)
         k2, v2 = qkv[:, H * D:(H + Hk) * D], qkv[:, (H + Hk) * D:]
@@ -75,10 +80,10 @@ class GPTBody:
         x = self._row_parallel(a, P.w(p + "attn.wo.weight"), None if rms else P.w(p + "attn.wo.bias"), x)
         h = self._norm(x, p + "ln2")
         if rms:
-            gu = gemm(h, P.w(p + "ffn.gate_up.weight"))
+            gu = _product(h, P.w(p + "ffn.gate_up.weight"))
             return self._row_parallel(rope_ops.swiglu_forward(gu), P.w(p + "ffn.down.weight"), None, x)
-        h = gemm(h, P.w(p + "ffn.fc1.weight"), bias=P.w(p + "ffn.fc1.bias"), act="gelu")
-        return gemm(h, P.w(p + "ffn.fc2.weight"), bias=P.w(p + "ffn.fc2.bias"), residual=x)
+        h = _product(h, P.w(p + "ffn.fc1.weight"), bias=P.w(p + "ffn.fc1.bias"), act="gelu")
+        return _product(h, P.w(p + "ffn.fc2.weight"), bias=P.w(p + "ffn.fc2.bias"), residual=x)
 
     def head(self, x, rows):
         P, cfg, tp = self.r.params, self.cfg, self.r.tp
@@ -87,9 +92,9 @@ class GPTBody:
         xf = self._norm(x.contiguous(), "final_norm")
         if tp is not None:
             w = P.w("head.weight")
-            gemm(xf, w, out=tp.staging(xf.shape[0], w.shape[0]))
+            _product(xf, w, out=tp.staging(xf.shape[0], w.shape[0]))
             return tp.all_gather_cols(xf.shape[0], w.shape[0])
-        return gemm(xf, P.w("tok_embed.embed" if cfg.tie_embeddings else "head.weight"))
+        return _product(xf, P.w("tok_embed.embed" if cfg.tie_embeddings else "head.weight"))
 
 
 class Stream:
@@ -139,7 +144,7 @@ class LayeredBody:
         r, P, s = self.r, self.r.params, self.cfg.layers[l]
         a, p = s.mixer, f"l{l}."
         H, G, dk, dv = a.heads, a.kv_heads, a.dim, a.vdim
-        z = gemm(st.h, P.w(p + "attn.in"))
+        z = _product(st.h, P.w(p + "attn.in"))
         ov = (H + G) * dk
         k2, v2, gate = z[:, H * dk:ov], z[:, ov:ov + G * dv], z[:, ov + G * dv:]
         mixed = a.v_mix and l != self.cfg.first_mix
@@ -149,28 +154,28 @@ class LayeredBody:
         if l == self.cfg.first_mix:
             st.v_first = v2                            # a view: this layer's projection buffer stays alive
         o = r.attend(l, z[:, :H * dk], k2, v2, sb, a.scale, self.rules[l], gate)
-        self._add_norm(st, gemm(o, P.w(p + "attn.out"), out_dtype=torch.float32), p + "norm1")
+        self._add_norm(st, _product(o, P.w(p + "attn.out"), out_dtype=torch.float32), p + "norm1")
         if s.mlp is not None:
             self._experts(st, s.mlp, p)
         return st
 
     def _experts(self, st, m, p):
         P, h = self.r.params, st.h
-        logits = gemm(h, P.w(p + "moe.router"), out_dtype=torch.float32)
+        logits = _product(h, P.w(p + "moe.router"), out_dtype=torch.float32)
         idx, w = moe_ops.route_groups(logits, m.top, m.groups, m.keep)
         pl = moe_ops.plan(idx, m.experts)
         gu = moe_ops.grouped_gemm(moe_ops.scatter_tokens(h, pl), P.w(p + "moe.w1"), pl)
         y = moe_ops.grouped_gemm(moe_ops.swiglu_rows(gu, pl), P.w(p + "moe.w2"), pl)
         shared = None
         if m.shared_ff:
-            shared = gemm(moe_ops.swiglu_rows(gemm(h, P.w(p + "shared.in"))), P.w(p + "shared.out"))
+            shared = _product(moe_ops.swiglu_rows(_product(h, P.w(p + "shared.in"))), P.w(p + "shared.out"))
         self._add_norm(st, y, p + "norm2", routed=(pl.slot_pos, w), add=shared)
 
     def head(self, st, rows):
         P, cfg = self.r.params, self.cfg
         x = st.x if rows is None else ops.gather_rows(st.x, rows)
         h = norm_ops.residual_norm(x, P.w("final.norm"), P.w("final.norm.b"), cfg.norm_eps, h=torch.empty_like(x, dtype=self.r.dtype))
-        logits = gemm(h, P.w("head"), out_dtype=torch.float32)
+        logits = _product(h, P.w("head"), out_dtype=torch.float32)
         return ops.scale_softcap_(logits, cfg.logit_scale, cfg.logit_softcap)
 
 
@@ -231,8 +236,8 @@ class ParallelBody:
     def layer(self, l, st, sb):
         P, p, s = self.r.params, self.prefix[l], self.cfg.layers[l]
         cols, gates = self.columns[l]
-        z = gemm(st.h, P.w(p + "in"))
-        small = gemm(st.h, P.w(p + "gates"), out_dtype=torch.float32)
+        z = _product(st.h, P.w(p + "in"))
+        small = _product(st.h, P.w(p + "gates"), out_dtype=torch.float32)
         run = self._parallel if isinstance(s.mixer, ParallelSpec) else self._delta
         return run(l, st, sb, s, p, lambda c: z[:, cols[c][0]:cols[c][0] + cols[c][1]], lambda c: small[:, gates[c][0]:gates[c][0] + gates[c][1]],
                    z)
@@ -252,10 +257,10 @@ class ParallelBody:
         y = rc_ops.state_space(xbc, gate("dt"), dt_bias=P.w(p + "dt_bias"), a_log=P.w(p + "A_log"), D=P.w(p + "D"), state=state["state"],
                                heads=m.heads, groups=m.groups, vdim=m.vdim, n=m.state, seg=sb.segments)
         y = rc_ops.gated_norm(y, col("z"), P.w(p + "norm"), m.norm_groups, cfg.norm_eps, gate_first=True, out=y)
-        out = dict(a=gemm(o, P.w(p + "left.o")), wa=P.w(p + "left.out"),
-                   b=gemm(y, P.w(p + "right.o")), wb=P.w(p + "right.out"), normed=0.5)
+        out = dict(a=_product(o, P.w(p + "left.o")), wa=P.w(p + "left.out"),
+                   b=_product(y, P.w(p + "right.o")), wb=P.w(p + "right.out"), normed=0.5)
         if s.mlp is not None:
-            out["c"] = gemm(self._feed_forward(l, s, z), P.w(p + "down"))
+            out["c"] = _product(self._feed_forward(l, s, z), P.w(p + "down"))
         return self._update(st, l, **out)
 
     def _delta(self, l, st, sb, s, p, col, gate, z):
@@ -271,13 +276,13 @@ class ParallelBody:
         rc_ops.gated_norm(o, col("z"), P.w(p + "norm"), m.heads, self.cfg.norm_eps, gate_first=False, out=o)
         if s.mlp is not None:
             self._feed_forward(l, s, z, out=joined[:, up8(n):])
-        return self._update(st, l, c=gemm(joined, w_out))
+        return self._update(st, l, c=_product(joined, w_out))
 
     def head(self, st, rows):
         P = self.r.params
         x = st.x if rows is None else ops.gather_rows(st.x, rows)
         h = norm_ops.stream_update(x, dyt=self._norm("final.norm"), h=torch.empty(x.shape, dtype=self.r.dtype, device=x.device))
-        logits = gemm(h, P.w("head"), out_dtype=torch.float32)
+        logits = _product(h, P.w("head"), out_dtype=torch.float32)
         if self.cfg.logit_scale != 1.0 or self.cfg.logit_softcap:
             ops.scale_softcap_(logits, self.cfg.logit_scale, self.cfg.logit_softcap)
         return logits
@@ -296,7 +301,7 @@ def _rotation(sb, rot, freqs):
 def _experts(P, h, m, p):
     """Routed feed-forward `m` (models.layered.MoESpec) over rows h: (expert rows, (their places, weights or None)) for the sum that
     ops.norm.residual_norm takes."""
-    logits = gemm(h, P.w(p + "moe.router"), out_dtype=torch.float32)
+    logits = _product(h, P.w(p + "moe.router"), out_dtype=torch.float32)
     if m.score == "sigmoid":
         idx, w = moe_ops.route_sigmoid(logits, m.top, m.groups, m.keep, P.w(p + "moe.correction") if m.correction else None,
                                        m.group_best, m.renorm)
@@ -351,7 +356,7 @@ class SandwichBody:
             left = st.pair[:, :self.cfg.d_model]
             if y is not None:
                 norm_ops.residual_norm(y, P.w(name), None, eps, True, x=st.x, h=left, **kw)
-            st.x = gemm(st.pair, P.w("loop.in"), bias=P.w("loop.step")[opens], out_dtype=torch.float32)
+            st.x = _product(st.pair, P.w("loop.in"), bias=P.w("loop.step")[opens], out_dtype=torch.float32)
             y = None
         if i is None:
             norm_ops.residual_norm(y, P.w(name), None, eps, True, x=st.x, **kw)
@@ -379,12 +384,12 @@ class SandwichBody:
         i, _ = self.runs[run]
         s, p = self.cfg.layers[i], f"l{i}."
         o = (self._latent if isinstance(s.mixer, LatentSpec) else self._attention)(run, i, s.mixer, p, st.h, sb)
-        y = gemm(o, P.w(p + "attn.out"), out_dtype=torch.float32)
+        y = _product(o, P.w(p + "attn.out"), out_dtype=torch.float32)
         if s.mlp is None:
             return self._start(st, run + 1, y, p + "norm1b")
         norm_ops.residual_norm(y, P.w(p + "norm1b"), None, self.cfg.norm_eps, True, x=st.x, h=st.h, next_gamma=P.w(p + "norm2"))
         if isinstance(s.mlp, DenseSpec):
-            y = gemm(gemm(st.h, P.w(p + "up"), act=s.mlp.act), P.w(p + "down"), out_dtype=torch.float32)
+            y = _product(_product(st.h, P.w(p + "up"), act=s.mlp.act), P.w(p + "down"), out_dtype=torch.float32)
             return self._start(st, run + 1, y, p + "norm2b")
         y, routed = _experts(P, st.h, s.mlp, p)
         return self._start(st, run + 1, y, p + "norm2b", routed=routed)
@@ -392,26 +397,26 @@ class SandwichBody:
     def _attention(self, run, i, a, p, h, sb):
         r, P = self.r, self.r.params
         H, G, dk, dv = a.heads, a.kv_heads, a.dim, a.vdim
-        z = gemm(h, P.w(p + "attn.in"), bias=P.w(p + "attn.in.b") if a.bias else None)
+        z = _product(h, P.w(p + "attn.in"), bias=P.w(p + "attn.in.b") if a.bias else None)
         ov = (H + G) * dk
         head_prep_(z, H, G, dk, dv, k_cache=r.cache.k[run], v_cache=r.cache.v[run], slots=sb.slots, rot=_rotation(sb, a.rot, self.freqs))
         return r.attend(run, z[:, :H * dk], z[:, H * dk:ov], z[:, ov:], sb, a.scale, self.rules[i])
 
     def _latent(self, run, i, m, p, h, sb):
         r, P, cols = self.r, self.r.params, self.columns[i]
-        z = gemm(h, P.w(p + "attn.in"))
+        z = _product(h, P.w(p + "attn.in"))
         part = lambda c: z[:, cols[c][0]:cols[c][0] + cols[c][1]]
         table = _rotation(sb, m.rot, self.freqs)
         latent_ops.latent_prep_(z, cols["q"][0], m.q_rank, cols["kv"][0], m.kv_rank, m.rot_dim, q_gamma=P.w(p + "attn.q_norm"),
                                 kv_gamma=P.w(p + "attn.kv_norm"), eps=self.cfg.norm_eps, table=table, cache=r.cache.k[run], slots=sb.slots)
-        q = gemm(part("q"), P.w(p + "attn.uq"))
+        q = _product(part("q"), P.w(p + "attn.uq"))
         return r.attend_latent(run, q, part("kv"), sb, m, P.w(p + "attn.ukv"), table, part("g") if "g" in cols else None)
 
     def head(self, st, rows):
         P, cfg = self.r.params, self.cfg
         x = st.x if rows is None else ops.gather_rows(st.x, rows)
         h = norm_ops.residual_norm(x, P.w("final.norm"), None, cfg.norm_eps, True, h=torch.empty_like(x, dtype=self.r.dtype))
-        logits = gemm(h, P.w("head"), out_dtype=torch.float32)
+        logits = _product(h, P.w("head"), out_dtype=torch.float32)
         if cfg.logit_scale != 1.0 or cfg.logit_softcap:
             ops.scale_softcap_(logits, cfg.logit_scale, cfg.logit_softcap)
         return logits
@@ -483,12 +488,12 @@ class PreNormBody:
         m = s.mixer
         mix = self._attention if isinstance(m, AttentionSpec) else self._retention if isinstance(m, RetentionSpec) else self._parallel
         o = mix(l, m, p, st, sb)
-        y = gemm(o, P.w(p + "attn.out"), bias=P.w(p + "attn.out.b") if getattr(m, "out_bias", False) else None, out_dtype=torch.float32)
+        y = _product(o, P.w(p + "attn.out"), bias=P.w(p + "attn.out.b") if getattr(m, "out_bias", False) else None, out_dtype=torch.float32)
         if s.mlp is None:
             return self._start(st, l + 1, y)
         self._add(st, P.w(p + "norm2"), y)
         if isinstance(s.mlp, DenseSpec):
-            return self._start(st, l + 1, gemm(gemm(st.h, P.w(p + "up"), act=s.mlp.act), P.w(p + "down"), out_dtype=torch.float32))
+            return self._start(st, l + 1, _product(_product(st.h, P.w(p + "up"), act=s.mlp.act), P.w(p + "down"), out_dtype=torch.float32))
         y, routed = _experts(P, st.h, s.mlp, p)
         return self._start(st, l + 1, y, routed=routed)
 
@@ -496,7 +501,7 @@ class PreNormBody:
         r, P = self.r, self.r.params
         H, dk, dv, own = a.heads, a.dim, a.vdim, a.kv_from is None
         G = a.kv_heads if own else 0
-        z = gemm(st.h, P.w(p + "attn.in"), bias=P.w(p + "attn.in.b") if a.bias else None)
+        z = _product(st.h, P.w(p + "attn.in"), bias=P.w(p + "attn.in.b") if a.bias else None)
         if a.conv:
             z = rc_ops.short_conv(z, P.w(p + "attn.conv"), None, r.cache.state[l]["conv"], sb.segments, silu=False)
         row_prep_(z, H, G, dk, dv, q_gamma=P.w(p + "attn.q_norm"), k_gamma=P.w(p + "attn.k_norm") if own else None, eps=self.cfg.norm_eps,
@@ -509,7 +514,7 @@ class PreNormBody:
 
     def _retention(self, l, m, p, st, sb):
         P, cols, H = self.r.params, self.columns[l], m.heads
-        z = gemm(st.h, P.w(p + "attn.in"))
+        z = _product(st.h, P.w(p + "attn.in"))
         head_prep_(z, H, H, m.dim, m.dim, rot=_rotation(sb, m.rot, self.freqs), half=True, k_scale=m.dim ** -0.5, q_col=cols["q"][0],
                    k_col=cols["k"][0])
         o = rc_ops.state_space(z[:, :H * (m.vdim + 2 * m.dim)], decay=P.w(p + "attn.decay"), state=self.r.cache.state[l]["state"], heads=H,
@@ -522,7 +527,7 @@ class PreNormBody:
         a, s = m.left, m.right
         w_in, (lo, n) = P.w(p + "attn.in"), cols["v"]
         z = torch.empty((sb.rows, up8(lo + n)), dtype=r.dtype, device=r.device)
-        gemm(st.h, w_in, out=z[:, :cols["end"][0]])
+        _product(st.h, w_in, out=z[:, :cols["end"][0]])
         part = lambda c: z[:, cols[c][0]:cols[c][0] + cols[c][1]]
         head_prep_(z, a.heads, a.kv_heads, a.dim, a.vdim, q_gamma=P.w(p + "attn.q_norm"), k_gamma=P.w(p + "attn.k_norm"), eps=self.cfg.norm_eps,
                    rot=_rotation(sb, a.rot, self.freqs), half=True, k_cache=r.cache.k[l], v_cache=r.cache.v[l], slots=sb.slots, v_col=lo,
@@ -534,9 +539,9 @@ class PreNormBody:
                 joined[:, edge:room] = 0
         r.attend(l, part("q"), part("k"), part("v"), sb, a.scale, self.rules[l], out=joined[:, :n])
         x = rc_ops.short_conv(part("conv"), P.w(p + "scan.conv"), P.w(p + "scan.conv.b"), state["conv"], sb.segments)
-        low = gemm(x, P.w(p + "scan.x"))
+        low = _product(x, P.w(p + "scan.x"))
         r8, ns = up8(s.dt_rank), s.state
-        dt = gemm(low[:, :r8], P.w(p + "scan.dt"), out_dtype=torch.float32)
+        dt = _product(low[:, :r8], P.w(p + "scan.dt"), out_dtype=torch.float32)
         rc_ops.selective_scan(x, dt, low[:, r8:r8 + ns], low[:, r8 + ns:r8 + 2 * ns], part("z"), A=P.w(p + "scan.A"), D=P.w(p + "scan.D"),
                               dt_bias=P.w(p + "scan.dt.b"), state=state["state"], seg=sb.segments, scale=m.scales[1],
                               out=joined[:, up8(n):up8(n) + s.inner])
@@ -546,7 +551,7 @@ class PreNormBody:
         P = self.r.params
         x = st.x if rows is None else ops.gather_rows(st.x, rows)
         h = norm_ops.residual_norm(x, P.w("final.norm"), None, self.cfg.norm_eps, True, h=torch.empty_like(x, dtype=self.r.dtype))
-        logits = gemm(h, P.w("head"), out_dtype=torch.float32)
+        logits = _product(h, P.w("head"), out_dtype=torch.float32)
         if self.cfg.logit_scale != 1.0 or self.cfg.logit_softcap:
             ops.scale_softcap_(logits, self.cfg.logit_scale, self.cfg.logit_softcap)
         return logits
