@@ -50,7 +50,9 @@ struct EpiParams {
   int accumulate;
   float alpha;
   int staged;   // 1: bf16 output goes through a per-warp shared-memory tile and leaves as whole 128/256-byte row segments;
-                // 2: the same tile leaves through a TMA store (tensor maps tmD / tmAux; 64-column tiles only)
+                // 2: 64-column tiles that leave through TMA stores (tensor maps tmD / tmAux; 256- and 128-wide tiles only);
+                // 3: fp32 output in 32-column tiles through TMA stores; 4: the same, added to d by TMA reductions
+  int side;     // staged == 2: what TMA loads into the tiles before the accumulator is complete: 0 nothing, 1 residual, 2 aux_in
   const float* row_scale;   // fp32 [M] or nullptr: multiplies row i of the accumulator (8-bit operands: per-token scale)
   const float* col_scale;   // fp32 [N] or nullptr: multiplies column j (per-output-channel weight scale)
   int fp8_b_format;         // 8-bit operands: format of B in the instruction descriptor (0 = e4m3, 1 = e5m2); A is e4m3
@@ -122,12 +124,15 @@ struct SmemLayout {
   static constexpr int kBBytes = BLOCK_N * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarOffset = STAGES * kStageBytes;
-  // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], tmem ptr, abort flag
-  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4) * 8 + 16;
-  // optional output staging (EpiParams::staged): per epilogue warp 32 rows x kStageCols bf16
+  // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], side[warps][2], tmem ptr, abort flag
+  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  // optional output staging (EpiParams::staged): per epilogue warp kSlots tiles of 32 rows x kStageCols bf16 (4 KB: or 32 x 32 fp32)
   static constexpr int kStageCols = (BLOCK_N % 128 == 0) ? 64 : 32;
+  static constexpr int kSlots = BLOCK_N == 128 ? 2 : 1;
+  static constexpr bool kTma = BLOCK_N % 128 == 0;                 // tiles of 128-byte rows: TMA can move them
+  static constexpr bool kSide = kSlots * 64 >= BLOCK_N / 2;        // a tile for each of a warp's column blocks
   static constexpr int kStagingOffset = (kTotal + 1023) & ~1023;   // 1024-byte aligned: the tiles are also TMA-store sources (128B swizzle)
-  static constexpr int kStagingBytesPerWarp = 32 * kStageCols * 2;
+  static constexpr int kStagingBytesPerWarp = kSlots * 32 * kStageCols * 2;
   static constexpr int kTotalStaged = kStagingOffset + kNumEpilogueWarps * kStagingBytesPerWarp;
 };
 
@@ -322,13 +327,232 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams& ep, uint32_t (&r
   epilogue_store(ep, v, row, col0, N);
 }
 
+__device__ __forceinline__ uint32_t stage_addr(uint32_t slot, int lane, int chunk) {
+  return slot + lane * 128 + ((chunk ^ (lane & 7)) << 4);
+}
+__device__ __forceinline__ void stage_put(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Epilogue of one warp through tiles of 32 rows x 128 bytes in shared memory that TMA moves: bf16 in 64-column blocks (staged 2), fp32 in
+// 32-column blocks (3; 4 adds to d: every element is added to by one warp once, so the sum does not depend on any order).  With two tiles
+// per warp (SLOTS) one is filled while the other is stored.  With `side`, TMA has loaded the residual or aux_in into the tiles (`epilogue_side_load`,
+// issued before the accumulator is waited for); results replace it in place.  Reading those through the SM's own loads instead, each
+// lane 64 bytes of its row, cost more than the products at K = 768: 32768 x 3072 with gelu'(aux_in) 292 us, residual 32768 x 768 61 us.
+// `arrive` hands the accumulator back; `row0` is the warp's first row, `col` the first of its COLS columns.
+template <int COLS>
+__device__ __forceinline__ void epilogue_side_load(const EpiParams& ep, const CUtensorMap* tmSide, uint32_t stg, uint32_t bar_side, int row0,
+                                                   int col, int lane) {
+  if (lane == 0) {
+    tma_store_wait_read<0>();                              // the tiles' last contents have been read out
+#pragma unroll
+    for (int h = 0; h < COLS / 64; ++h) {
+      mbar_arrive_expect_tx(bar_side + 8 * h, 4096);
+      tma_load_2d(stg + h * 4096, tmSide, col + h * 64, row0, bar_side + 8 * h);
+    }
+  }
+  __syncwarp();
+}
+
+// Pairs of neighbouring columns, for the packed fp32 instructions.
+struct Pair {
+  unsigned long long v;
+};
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ float2 floats(Pair p) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p.v));
+  return f;
+}
+__device__ __forceinline__ Pair pair_of(uint32_t bf16x2) {
+  const float2 f = unpack_bf16x2(bf16x2);
+  return pair_of(f.x, f.y);
+}
+__device__ __forceinline__ uint32_t packed(Pair p) {
+  const float2 f = floats(p);
+  return pack_bf16x2(f.x, f.y);
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+  Pair d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ Pair gelu2(Pair x) {
+  constexpr float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float2 u = floats(mul2(x, fma2(pair_of(k0 * k1, k0 * k1), mul2(x, x), pair_of(k0, k0))));
+  const Pair h = mul2(x, pair_of(0.5f, 0.5f));
+  return fma2(h, pair_of(tanh_fast(u.x), tanh_fast(u.y)), h);
+}
+__device__ __forceinline__ Pair gelu_grad2(Pair x) {
+  constexpr float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const Pair x2 = mul2(x, x), half = pair_of(0.5f, 0.5f);
+  const float2 u = floats(mul2(x, fma2(pair_of(k0 * k1, k0 * k1), x2, pair_of(k0, k0))));
+  const Pair t = pair_of(tanh_fast(u.x), tanh_fast(u.y));
+  const Pair du = fma2(pair_of(3.f * k0 * k1, 3.f * k0 * k1), x2, pair_of(k0, k0));
+  const Pair one_t2 = fma2(mul2(t, pair_of(-1.f, -1.f)), t, pair_of(1.f, 1.f));
+  return fma2(mul2(mul2(x, half), one_t2), du, fma2(half, t, half));
+}
+
+// Accumulator -> pre-activation of 32 columns (scales, bias).  N is a multiple of 4.
+__device__ __forceinline__ void tile_pre(const EpiParams& ep, const uint32_t (&r)[32], long long row, int col0, int N, Pair (&v)[16]) {
+  const Pair alpha = pair_of(ep.alpha, ep.alpha);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = mul2(pair_of(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), alpha);
+  if (ep.row_scale != nullptr) {
+    const float rs = __ldg(ep.row_scale + row);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = mul2(v[j], pair_of(rs, rs));
+  }
+  if (ep.col_scale != nullptr) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (col0 + 4 * q >= N) break;
+      const float4 c = __ldg(reinterpret_cast<const float4*>(ep.col_scale + col0) + q);
+      v[2 * q] = mul2(v[2 * q], pair_of(c.x, c.y));
+      v[2 * q + 1] = mul2(v[2 * q + 1], pair_of(c.z, c.w));
+    }
+  }
+  if (ep.bias != nullptr) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (col0 + 4 * q >= N) break;
+      const uint2 b = __ldg(reinterpret_cast<const uint2*>(ep.bias + col0) + q);
+      v[2 * q] = add2(v[2 * q], pair_of(b.x));
+      v[2 * q + 1] = add2(v[2 * q + 1], pair_of(b.y));
+    }
+  }
+}
+__device__ __forceinline__ void tile_act(const EpiParams& ep, const uint32_t (&side)[16], Pair (&v)[16]) {
+  if (ep.act == RB_ACT_GELU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = gelu2(v[j]);
+  } else if (ep.act == RB_ACT_DGELU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = mul2(v[j], gelu_grad2(pair_of(side[j])));
+  } else if (ep.act != RB_ACT_NONE) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      float2 f = floats(v[j]);
+      const float2 a = unpack_bf16x2(side[j]);
+      if (ep.act == RB_ACT_SILU) { f.x = silu(f.x); f.y = silu(f.y); }
+      else if (ep.act == RB_ACT_MUL) { f.x *= a.x; f.y *= a.y; }
+      else if (ep.act == RB_ACT_DSILU) { f.x *= silu_grad(a.x); f.y *= silu_grad(a.y); }
+      else if (ep.act == RB_ACT_DRELU) { f.x = a.x > 0.f ? f.x : 0.f; f.y = a.y > 0.f ? f.y : 0.f; }
+      else {
+        f.x = fmaxf(f.x, 0.f); f.y = fmaxf(f.y, 0.f);
+        if (ep.act == RB_ACT_RELU2) { f.x *= f.x; f.y *= f.y; }
+      }
+      v[j] = pair_of(f.x, f.y);
+    }
+  }
+}
+
+template <int COLS, int SLOTS, class Arrive>
+__device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensorMap* tmD, const CUtensorMap* tmAux, uint32_t stg,
+                                             uint32_t bar_side, uint32_t side_parity, uint32_t taddr, int row0, int drow, int col, int M, int N,
+                                             int lane, bool empty_k, volatile int* abort_flag, unsigned int* status, Arrive arrive) {
+  // rows behind the matrix are computed like the others (on what the accumulator holds for them) and clipped by the stores
+  const long long row = min(row0 + lane, M - 1);
+  const bool two = ep.aux_out != nullptr && (ep.act == RB_ACT_GELU || ep.act == RB_ACT_RELU || ep.act == RB_ACT_SILU);
+  const int cols = ep.staged >= 3 ? 32 : 64;                 // columns of a tile
+#pragma unroll 1
+  for (int c = 0; c < COLS; c += 32) {
+    // 32 columns at a time; `half`: which part of a 64-column tile they are
+    const int block = c / cols, half = (c & (cols - 1)) >> 5;
+    const uint32_t slot = stg + (two ? 0 : block % SLOTS) * 4096;
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c, r);
+    uint32_t side[16];
+    if (ep.side != 0) {
+      if (half == 0 && !mbar_wait(bar_side + 8 * block, side_parity, abort_flag, status, 7)) return;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(side[4 * q]), "=r"(side[4 * q + 1]), "=r"(side[4 * q + 2]),
+                     "=r"(side[4 * q + 3]) : "r"(stage_addr(slot, lane, half * 4 + q)));
+    } else if (half == 0) {
+      // with two results the first tile may be filled again while the second one, stored later, still leaves
+      if (lane == 0) tma_store_wait_read<SLOTS - 1>();
+      __syncwarp();
+    }
+    tmem_ld_wait();
+    if (c == COLS - 32) arrive();
+    if (empty_k) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = 0u;
+    }
+    Pair v[16];
+    tile_pre(ep, r, row, col + c, N, v);
+    if (ep.staged >= 3) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float2 a = floats(v[2 * q]), b = floats(v[2 * q + 1]);
+        stage_put(stage_addr(slot, lane, q), __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+      }
+    } else {
+      if (!two) {
+        tile_act(ep, side, v);
+        if (ep.side == 1) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = add2(v[j], pair_of(side[j]));
+        }
+      }
+      uint32_t o[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) o[j] = packed(v[j]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) stage_put(stage_addr(slot, lane, half * 4 + q), o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+      if (two) {
+        // the result is formed from the rounded pre-activation, in the second tile
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = pair_of(o[j]);
+        tile_act(ep, side, v);
+        if (half == 0) {
+          if (lane == 0) tma_store_wait_read<0>();
+          __syncwarp();
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          stage_put(stage_addr(slot + 4096, lane, half * 4 + q), packed(v[4 * q]), packed(v[4 * q + 1]), packed(v[4 * q + 2]), packed(v[4 * q + 3]));
+      }
+      if (half == 0) continue;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      const int x = col + c - half * 32;
+      if (ep.staged == 4) { if (row0 < M) tma_reduce_add_2d(tmD, slot, x, drow); }
+      else if (ep.staged == 3) { if (row0 < M) tma_store_2d(tmD, slot, x, drow); }
+      else tma_store_2d(two ? tmAux : tmD, slot, x, drow);
+      tma_store_commit();
+      if (two) {
+        tma_store_2d(tmD, slot + 4096, x, drow);
+        tma_store_commit();
+      }
+    }
+  }
+}
+
 // FP8 = 1: both operands hold e4m3 bytes (K-major only).  A 128-byte swizzle row then carries 128 elements, so K, lda
 // and ldb arrive halved (in units of two bytes) and only the TMA coordinates, which count elements, are doubled back.
 template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, int M, int N,
-                 int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
+                 const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
+                 const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
                  GroupInfo grp, PeerInfo peer, unsigned int* status) {
   using L = SmemLayout<BLOCK_N, STAGES>;
   extern __shared__ uint8_t smem_raw[];
@@ -340,7 +564,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t bar_empty = smem_u32(bars + STAGES);
   const uint32_t bar_tfull = smem_u32(bars + 2 * STAGES);
   const uint32_t bar_tempty = smem_u32(bars + 2 * STAGES + 2);
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  const uint32_t bar_side = smem_u32(bars + 2 * STAGES + 4);
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + 2 * kNumEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -358,6 +583,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(bar_tfull + 8 * a, 1);
       mbar_init(bar_tempty + 8 * a, kNumEpilogueWarps);
     }
+    for (int w = 0; w < 2 * kNumEpilogueWarps; ++w) mbar_init(bar_side + 8 * w, 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
@@ -418,7 +644,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    // elect.sync, not lane 0: the compiler then knows that one lane runs this and keeps what it issues in uniform registers
+    if (elect_one()) {
       // ------------------------------------------------------------------ TMA producer
       uint32_t it = 0;
       bool ok = true;
@@ -494,10 +721,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------------------------------------------ MMA issuer
       const uint32_t idesc = FP8 ? (umma_idesc_e4m3(kBlockM, BLOCK_N) | (static_cast<uint32_t>(ep.fp8_b_format) << 10))
                                  : umma_idesc_bf16(kBlockM, BLOCK_N, A_MN, B_MN);
+      // K-major: 32 bytes per step of 16 inside the swizzle row, 8-row groups 1024 bytes apart.  MN-major: 16 k-rows of 128 bytes per
+      // step, 64-wide MN atoms kBlockK * 128 bytes apart.  An offset of o bytes is o / 16 in the address field.
+      const uint64_t desc_a = A_MN ? umma_smem_desc_sw128(smem_base, kBlockK * 128, 1024) : umma_smem_desc_sw128(smem_base, 16, 1024);
+      const uint64_t desc_b = B_MN ? umma_smem_desc_sw128(smem_base + L::kABytes, kBlockK * 128, 1024) : umma_smem_desc_sw128(smem_base + L::kABytes, 16, 1024);
+      constexpr int kStepA = A_MN ? kUmmaK * 8 : kUmmaK / 8, kStepB = B_MN ? kUmmaK * 8 : kUmmaK / 8;
       uint32_t it = 0, t = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_units && ok; tile += gridDim.x, ++t) {
@@ -511,18 +743,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, status, 3)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_base + s * L::kStageBytes;
-          const uint32_t sb = sa + L::kABytes;
+          const uint64_t da = desc_a + s * (L::kStageBytes / 16), db = desc_b + s * (L::kStageBytes / 16);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            // K-major: 32 bytes per UMMA_K step inside the swizzle row; 8-row groups 1024 B apart.
-            // MN-major: 16 k-rows of 128 B per step; 64-wide MN atoms kBlockK*128 B apart.
-            const uint64_t da = A_MN ? umma_smem_desc_sw128(sa + k * (kUmmaK * 128), kBlockK * 128, 1024)
-                                     : umma_smem_desc_sw128(sa + k * (kUmmaK * 2), 16, 1024);
-            const uint64_t db = B_MN ? umma_smem_desc_sw128(sb + k * (kUmmaK * 128), kBlockK * 128, 1024)
-                                     : umma_smem_desc_sw128(sb + k * (kUmmaK * 2), 16, 1024);
-            if (FP8) umma_f8_ss(tmem_d, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-            else umma_bf16_ss(tmem_d, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            if (FP8) umma_f8_ss(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            else umma_bf16_ss(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
           }
           umma_commit(bar_empty + 8 * s);   // frees the smem stage once these MMAs have read it
         }
@@ -534,7 +759,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;   // TMEM lane quarter this warp may read
     const int ew = warp - 2;  // 0..7
     const int cgrp = ew >> 2; // which half of the tile's columns this warp handles
-    bool store_pending = false;   // a bulk tensor store of this warp's staging tile may still be reading it
     // ---- all-gather duty (peer modes 1 and 3): every epilogue warp of every CTA owns a strided share of the 16-row
     // pieces of the remote rows, in the order the tiles consume them.  A warp pulls pieces whenever its next
     // accumulator is not ready yet, and finishes its share after its last tile; nothing a piece needs ever waits.
@@ -576,6 +800,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int tile = blockIdx.x; tile < num_units; tile += gridDim.x, ++t) {
       int m_blk, n_blk, kb0, kb1, outer;
       decode_tile(tile, m_blk, n_blk, kb0, kb1, outer);
+      const bool empty_k = kb1 <= kb0;     // an expert without tokens: the accumulator was never written
+      const uint32_t acc = t & 1, acc_ph = (t >> 1) & 1;
+      const uint32_t stg = smem_base + L::kStagingOffset + ew * L::kStagingBytesPerWarp;
+      const uint32_t side_bars = bar_side + 16 * ew;
+      const int row0 = m_blk * kBlockM + q * 32, colg = n_blk * BLOCK_N + cgrp * (BLOCK_N / 2);
+      if (L::kSide && ep.side != 0) epilogue_side_load<BLOCK_N / 2>(ep, &tmSide, stg, side_bars, row0, colg, lane);
+      while (next_item < remote_items && !mbar_test(bar_tfull + 8 * acc, acc_ph)) copy_one();
+      if (!mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag, status, 4)) break;
+      tc_fence_after();
+      const long long row = row0 + lane;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BLOCK_N;
+      auto arrive = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+      };
+      if (L::kTma && ep.staged >= 2) {
+        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t & 1, taddr + cgrp * (BLOCK_N / 2), row0,
+                                  num_splits > 1 ? outer * M + row0 : row0, colg, M, N, lane, empty_k, abort_flag, status, arrive);
+        continue;
+      }
       EpiParams epu = ep;
       if (num_splits > 1)
         epu.d = reinterpret_cast<float*>(ep.d) + static_cast<long long>(outer) * d_split_stride;
@@ -588,106 +833,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int owner = (m_blk * kBlockM) / peer.rows_per_rank;
         epu.d = peer.d_peer[owner] + (static_cast<long long>(peer.rank) - owner) * peer.rows_per_rank * ep.ldd;
       }
-      const bool empty_k = kb1 <= kb0;     // an expert without tokens: the accumulator was never written
-      const uint32_t acc = t & 1, acc_ph = (t >> 1) & 1;
-      while (next_item < remote_items && !mbar_test(bar_tfull + 8 * acc, acc_ph)) copy_one();
-      if (!mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag, status, 4)) break;
-      tc_fence_after();
-      const long long row = static_cast<long long>(m_blk) * kBlockM + q * 32 + lane;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BLOCK_N;
       if (epu.staged) {
         // registers -> swizzled per-warp tile in shared memory -> whole row segments to global / peer memory
         constexpr int SC = L::kStageCols, CPR = SC / 8;           // staged columns, 16-byte chunks per row
-        const uint32_t stg = smem_base + L::kStagingOffset + ew * L::kStagingBytesPerWarp;
         constexpr int NB = (BLOCK_N / 2) / SC;                    // column blocks per warp group
         const bool two_pass = epu.aux_out != nullptr &&
                               (epu.act == RB_ACT_GELU || epu.act == RB_ACT_RELU || epu.act == RB_ACT_SILU);
-        if (SC == 64 && epu.staged == 2 && two_pass) {
-          // One pass over the accumulator: the pre-activation is rounded to bf16, kept packed in registers for the 64
-          // columns of a block and sent to aux_out by a bulk store; the activation is computed from the rounded values
-          // while that store reads the tile, and follows through the same tile to d.
-#pragma unroll 1
-          for (int h = 0; h < NB; ++h) {
-            uint32_t keep[2][16];
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-              const int c = cgrp * (BLOCK_N / 64) + h * 2 + cc;
-              uint32_t r[32];
-              tmem_ld_32x32(taddr + c * 32, r);
-              if (cc == 0 && store_pending) {
-                if (lane == 0) tma_store_wait_read<0>();
-                __syncwarp();
-                store_pending = false;
-              }
-              tmem_ld_wait();
-              if (h == NB - 1 && cc == 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-              }
-              const int col0 = n_blk * BLOCK_N + c * 32;
-              float v[32];
-              if (empty_k) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = 0u;
-              }
-              if (row < M && col0 < N) {
-                epilogue_math<false, true>(epu, r, row, col0, N, v);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = 0.f;
-              }
-#pragma unroll
-              for (int i = 0; i < 16; ++i) keep[cc][i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) {
-                const uint32_t addr = stg + lane * (SC * 2) + (((cc * 4 + qq) ^ (lane & (CPR - 1))) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(keep[cc][qq * 4 + 0]), "r"(keep[cc][qq * 4 + 1]),
-                             "r"(keep[cc][qq * 4 + 2]), "r"(keep[cc][qq * 4 + 3]) : "memory");
-              }
-            }
-            const int colb = n_blk * BLOCK_N + cgrp * (BLOCK_N / 2) + h * SC;
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmAux, stg, colb, static_cast<int>((static_cast<long long>(m_blk) * kBlockM + q * 32)));
-              tma_store_commit();
-            }
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-              const int col0 = colb + cc * 32;
-              float v[32];
-              uint32_t dummy[32];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float2 f = unpack_bf16x2(keep[cc][i]);
-                v[2 * i] = f.x; v[2 * i + 1] = f.y;
-              }
-              if (row < M && col0 < N) epilogue_math<false, false, true>(epu, dummy, row, col0, N, v);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) keep[cc][i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-            }
-            if (lane == 0) tma_store_wait_read<0>();       // the pre-activation tile has been read out
-            __syncwarp();
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) {
-                const uint32_t addr = stg + lane * (SC * 2) + (((cc * 4 + qq) ^ (lane & (CPR - 1))) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(keep[cc][qq * 4 + 0]), "r"(keep[cc][qq * 4 + 1]),
-                             "r"(keep[cc][qq * 4 + 2]), "r"(keep[cc][qq * 4 + 3]) : "memory");
-              }
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmD, stg, colb, static_cast<int>((static_cast<long long>(m_blk) * kBlockM + q * 32)));
-              tma_store_commit();
-            }
-            store_pending = true;
-          }
-          continue;
-        }
         const int num_pass = two_pass ? 2 : 1;
 #pragma unroll 1
         for (int hp = 0; hp < NB * num_pass; ++hp) {
@@ -703,18 +854,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int c = cgrp * (BLOCK_N / 64) + h * (SC / 32) + cc;
             uint32_t r[32];
             tmem_ld_32x32(taddr + c * 32, r);
-            if (cc == 0 && store_pending) {
-              // the bulk store issued for the previous block has to be done reading the tile before it is overwritten
-              if (lane == 0) tma_store_wait_read<0>();
-              __syncwarp();
-              store_pending = false;
-            }
             tmem_ld_wait();
-            if (last_pass && cc == SC / 32 - 1) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-            }
+            if (last_pass && cc == SC / 32 - 1) arrive();
             const int col0 = n_blk * BLOCK_N + c * 32;
             float v[32];
             if (empty_k) {
@@ -737,18 +878,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                            "r"(pack_bf16x2(v[qq * 8 + 4], v[qq * 8 + 5])), "r"(pack_bf16x2(v[qq * 8 + 6], v[qq * 8 + 7]))
                            : "memory");
             }
-          }
-          if (SC == 64 && epu.staged == 2) {
-            // the tile leaves through a bulk tensor store; rows and columns past the matrix are clipped by the copy
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(pre_pass ? &tmAux : &tmD, stg, n_blk * BLOCK_N + cgrp * (BLOCK_N / 2) + h * SC,
-                           static_cast<int>(static_cast<long long>(m_blk) * kBlockM + q * 32));
-              tma_store_commit();
-            }
-            store_pending = true;
-            continue;
           }
           __syncwarp();
           constexpr int RPI = 32 / CPR;                            // rows written per warp instruction
@@ -776,12 +905,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
-        if (c == (cgrp + 1) * (BLOCK_N / 64) - 1) {
-          // all of this warp's accumulator reads are done: hand the buffer back to the MMA warp
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-        }
+        // all of this warp's accumulator reads are done: hand the buffer back to the MMA warp
+        if (c == (cgrp + 1) * (BLOCK_N / 64) - 1) arrive();
         const int col0 = n_blk * BLOCK_N + c * 32;
         if (row < M && col0 < N) epilogue_chunk(epu, r, row, col0, N);
       }
@@ -817,18 +942,20 @@ struct SmemLayoutPair {
   static constexpr int kBBytes = (BLOCK_N / 2) * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarOffset = STAGES * kStageBytes;
-  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4) * 8 + 16;
-  static constexpr int kStageCols = (BLOCK_N % 128 == 0) ? 64 : 32;
+  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  static constexpr int kStageCols = 64;
+  static constexpr int kSlots = 2;
+  static constexpr bool kTma = true, kSide = true;
   static constexpr int kStagingOffset = (kTotal + 1023) & ~1023;   // 1024-byte aligned: the tiles are also TMA-store sources (128B swizzle)
-  static constexpr int kStagingBytesPerWarp = 32 * kStageCols * 2;
+  static constexpr int kStagingBytesPerWarp = kSlots * 32 * kStageCols * 2;
   static constexpr int kTotalStaged = kStagingOffset + kNumEpilogueWarps * kStagingBytesPerWarp;
 };
 
 template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, int M, int N,
-                      int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
+                      const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
+                      const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
                       unsigned int* status) {
   using L = SmemLayoutPair<BLOCK_N, STAGES>;
   extern __shared__ uint8_t smem_raw[];
@@ -839,7 +966,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t bar_empty = smem_u32(bars + STAGES);
   const uint32_t bar_tfull = smem_u32(bars + 2 * STAGES);
   const uint32_t bar_tempty = smem_u32(bars + 2 * STAGES + 2);
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  const uint32_t bar_side = smem_u32(bars + 2 * STAGES + 4);
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + 2 * kNumEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -859,6 +987,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(bar_tfull + 8 * a, 1);
       mbar_init(bar_tempty + 8 * a, 2 * kNumEpilogueWarps);   // leader: the epilogue warps of both CTAs
     }
+    for (int w = 0; w < 2 * kNumEpilogueWarps; ++w) mbar_init(bar_side + 8 * w, 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
@@ -897,7 +1026,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------------------------------------------ TMA producer (both CTAs)
       uint32_t it = 0;
       bool ok = true;
@@ -932,10 +1061,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       // ------------------------------------------------------------------ MMA issuer (leader CTA only)
       const uint32_t idesc = FP8 ? (umma_idesc_e4m3(kPairM, BLOCK_N) | (static_cast<uint32_t>(ep.fp8_b_format) << 10))
                                  : umma_idesc_bf16(kPairM, BLOCK_N, A_MN, B_MN);
+      // K-major: 32 bytes per step of 16 inside the swizzle row, 8-row groups 1024 bytes apart.  MN-major: 16 k-rows of 128 bytes per
+      // step, 64-wide MN atoms kBlockK * 128 bytes apart.  An offset of o bytes is o / 16 in the address field.
+      const uint64_t desc_a = A_MN ? umma_smem_desc_sw128(smem_base, kBlockK * 128, 1024) : umma_smem_desc_sw128(smem_base, 16, 1024);
+      const uint64_t desc_b = B_MN ? umma_smem_desc_sw128(smem_base + L::kABytes, kBlockK * 128, 1024) : umma_smem_desc_sw128(smem_base + L::kABytes, 16, 1024);
+      constexpr int kStepA = A_MN ? kUmmaK * 8 : kUmmaK / 8, kStepB = B_MN ? kUmmaK * 8 : kUmmaK / 8;
       uint32_t it = 0, t = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < num_units && ok; tile += num_clusters, ++t) {
@@ -949,16 +1083,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, status, 13)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_base + s * L::kStageBytes;
-          const uint32_t sb = sa + L::kABytes;
+          const uint64_t da = desc_a + s * (L::kStageBytes / 16), db = desc_b + s * (L::kStageBytes / 16);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            const uint64_t da = A_MN ? umma_smem_desc_sw128(sa + k * (kUmmaK * 128), kBlockK * 128, 1024)
-                                     : umma_smem_desc_sw128(sa + k * (kUmmaK * 2), 16, 1024);
-            const uint64_t db = B_MN ? umma_smem_desc_sw128(sb + k * (kUmmaK * 128), kBlockK * 128, 1024)
-                                     : umma_smem_desc_sw128(sb + k * (kUmmaK * 2), 16, 1024);
-            if (FP8) umma_f8_ss_pair(tmem_d, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-            else umma_bf16_ss_pair(tmem_d, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            if (FP8) umma_f8_ss_pair(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            else umma_bf16_ss_pair(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
           }
           umma_commit_pair(bar_empty + 8 * s, 3);     // both CTAs may refill this stage
         }
@@ -970,194 +1099,39 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;
     const int ew = warp - 2;
     const int cgrp = ew >> 2;
-    bool store_pending = false;
     uint32_t t = 0;
     for (int tile = cluster_id; tile < num_units; tile += num_clusters, ++t) {
       int m_blk, n_blk, kb0, kb1, split;
       decode_tile(tile, m_blk, n_blk, kb0, kb1, split);
-      EpiParams epu = ep;
-      if (num_splits > 1)
-        epu.d = reinterpret_cast<float*>(ep.d) + static_cast<long long>(split) * d_split_stride;
       const uint32_t acc = t & 1, acc_ph = (t >> 1) & 1;
+      const uint32_t stg = smem_base + L::kStagingOffset + ew * L::kStagingBytesPerWarp;
+      const uint32_t side_bars = bar_side + 16 * ew;
+      const int row0 = m_blk * kPairM + static_cast<int>(cta_rank) * kBlockM + q * 32, colg = n_blk * BLOCK_N + cgrp * (BLOCK_N / 2);
+      if (ep.side != 0) epilogue_side_load<BLOCK_N / 2>(ep, &tmSide, stg, side_bars, row0, colg, lane);
       if (!mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag, status, 14)) break;
       tc_fence_after();
-      const long long row0 = static_cast<long long>(m_blk) * kPairM + static_cast<long long>(cta_rank) * kBlockM + q * 32;
       const long long row = row0 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BLOCK_N;
       const uint32_t tempty_leader = mapa_shared(bar_tempty + 8 * acc, 0);
-      if (epu.staged) {
-        constexpr int SC = L::kStageCols, CPR = SC / 8;
-        const uint32_t stg = smem_base + L::kStagingOffset + ew * L::kStagingBytesPerWarp;
-        constexpr int NB = (BLOCK_N / 2) / SC;
-        const bool two_pass = epu.aux_out != nullptr &&
-                              (epu.act == RB_ACT_GELU || epu.act == RB_ACT_RELU || epu.act == RB_ACT_SILU);
-        if (SC == 64 && epu.staged == 2 && two_pass) {
-          // One pass over the accumulator: the pre-activation is rounded to bf16, kept packed in registers for the 64
-          // columns of a block and sent to aux_out by a bulk store; the activation is computed from the rounded values
-          // while that store reads the tile, and follows through the same tile to d.
-#pragma unroll 1
-          for (int h = 0; h < NB; ++h) {
-            uint32_t keep[2][16];
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-              const int c = cgrp * (BLOCK_N / 64) + h * 2 + cc;
-              uint32_t r[32];
-              tmem_ld_32x32(taddr + c * 32, r);
-              if (cc == 0 && store_pending) {
-                if (lane == 0) tma_store_wait_read<0>();
-                __syncwarp();
-                store_pending = false;
-              }
-              tmem_ld_wait();
-              if (h == NB - 1 && cc == 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(tempty_leader);
-              }
-              const int col0 = n_blk * BLOCK_N + c * 32;
-              float v[32];
-              if (false) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = 0u;
-              }
-              if (row < M && col0 < N) {
-                epilogue_math<false, true>(epu, r, row, col0, N, v);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = 0.f;
-              }
-#pragma unroll
-              for (int i = 0; i < 16; ++i) keep[cc][i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) {
-                const uint32_t addr = stg + lane * (SC * 2) + (((cc * 4 + qq) ^ (lane & (CPR - 1))) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(keep[cc][qq * 4 + 0]), "r"(keep[cc][qq * 4 + 1]),
-                             "r"(keep[cc][qq * 4 + 2]), "r"(keep[cc][qq * 4 + 3]) : "memory");
-              }
-            }
-            const int colb = n_blk * BLOCK_N + cgrp * (BLOCK_N / 2) + h * SC;
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmAux, stg, colb, static_cast<int>(row0));
-              tma_store_commit();
-            }
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-              const int col0 = colb + cc * 32;
-              float v[32];
-              uint32_t dummy[32];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float2 f = unpack_bf16x2(keep[cc][i]);
-                v[2 * i] = f.x; v[2 * i + 1] = f.y;
-              }
-              if (row < M && col0 < N) epilogue_math<false, false, true>(epu, dummy, row, col0, N, v);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) keep[cc][i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-            }
-            if (lane == 0) tma_store_wait_read<0>();       // the pre-activation tile has been read out
-            __syncwarp();
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) {
-                const uint32_t addr = stg + lane * (SC * 2) + (((cc * 4 + qq) ^ (lane & (CPR - 1))) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(keep[cc][qq * 4 + 0]), "r"(keep[cc][qq * 4 + 1]),
-                             "r"(keep[cc][qq * 4 + 2]), "r"(keep[cc][qq * 4 + 3]) : "memory");
-              }
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmD, stg, colb, static_cast<int>(row0));
-              tma_store_commit();
-            }
-            store_pending = true;
-          }
-          continue;
-        }
-        const int num_pass = two_pass ? 2 : 1;
-#pragma unroll 1
-        for (int hp = 0; hp < NB * num_pass; ++hp) {
-          const int h = hp / num_pass;
-          const bool pre_pass = two_pass && (hp - h * num_pass) == 0;
-          const bool last_pass = hp == NB * num_pass - 1;
-          __nv_bfloat16* dbase = pre_pass ? epu.aux_out : reinterpret_cast<__nv_bfloat16*>(epu.d);
-          const long long dld = pre_pass ? epu.ld_aux_out : epu.ldd;
-#pragma unroll 1
-          for (int cc = 0; cc < SC / 32; ++cc) {
-            const int c = cgrp * (BLOCK_N / 64) + h * (SC / 32) + cc;
-            uint32_t r[32];
-            tmem_ld_32x32(taddr + c * 32, r);
-            if (cc == 0 && store_pending) {
-              // the bulk store issued for the previous block has to be done reading the tile before it is overwritten
-              if (lane == 0) tma_store_wait_read<0>();
-              __syncwarp();
-              store_pending = false;
-            }
-            tmem_ld_wait();
-            if (last_pass && cc == SC / 32 - 1) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster(tempty_leader);
-            }
-            const int col0 = n_blk * BLOCK_N + c * 32;
-            float v[32];
-            if (row < M && col0 < N) {
-              if (pre_pass) epilogue_math<false, true>(epu, r, row, col0, N, v);
-              else epilogue_math<false, false>(epu, r, row, col0, N, v);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = 0.f;
-            }
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-              const int chunk = cc * 4 + qq;
-              const uint32_t addr = stg + lane * (SC * 2) + ((chunk ^ (lane & (CPR - 1))) << 4);
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
-                           "r"(pack_bf16x2(v[qq * 8 + 0], v[qq * 8 + 1])), "r"(pack_bf16x2(v[qq * 8 + 2], v[qq * 8 + 3])),
-                           "r"(pack_bf16x2(v[qq * 8 + 4], v[qq * 8 + 5])), "r"(pack_bf16x2(v[qq * 8 + 6], v[qq * 8 + 7]))
-                           : "memory");
-            }
-          }
-          if (SC == 64 && epu.staged == 2) {
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(pre_pass ? &tmAux : &tmD, stg, n_blk * BLOCK_N + cgrp * (BLOCK_N / 2) + h * SC, static_cast<int>(row0));
-              tma_store_commit();
-            }
-            store_pending = true;
-            continue;
-          }
-          __syncwarp();
-          constexpr int RPI = 32 / CPR;
-          const int ch = lane % CPR, rsub = lane / CPR;
-          const int colg = n_blk * BLOCK_N + cgrp * (BLOCK_N / 2) + h * SC + ch * 8;
-#pragma unroll 4
-          for (int r0 = 0; r0 < 32; r0 += RPI) {
-            const int rl = r0 + rsub;
-            const long long rg = row0 + rl;
-            uint4 val;
-            const uint32_t addr = stg + rl * (SC * 2) + ((ch ^ (rl & (CPR - 1))) << 4);
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(val.x), "=r"(val.y), "=r"(val.z), "=r"(val.w) : "r"(addr));
-            if (rg < M && colg < N) *reinterpret_cast<uint4*>(dbase + rg * dld + colg) = val;
-          }
-          __syncwarp();
-        }
+      auto arrive = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty_leader);
+      };
+      if (ep.staged >= 2) {
+        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t & 1, taddr + cgrp * (BLOCK_N / 2), row0,
+                                  num_splits > 1 ? split * M + row0 : row0, colg, M, N, lane, false, abort_flag, status, arrive);
         continue;
       }
+      EpiParams epu = ep;
+      if (num_splits > 1)
+        epu.d = reinterpret_cast<float*>(ep.d) + static_cast<long long>(split) * d_split_stride;
 #pragma unroll 1
       for (int c = cgrp * (BLOCK_N / 64); c < (cgrp + 1) * (BLOCK_N / 64); ++c) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
-        if (c == (cgrp + 1) * (BLOCK_N / 64) - 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(tempty_leader);
-        }
+        if (c == (cgrp + 1) * (BLOCK_N / 64) - 1) arrive();
         const int col0 = n_blk * BLOCK_N + c * 32;
         if (row < M && col0 < N) epilogue_chunk(epu, r, row, col0, N);
       }
@@ -1255,43 +1229,58 @@ bool tma_store_default() {
   return v == 1;
 }
 
-template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
-int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, int grid, int splits, cudaStream_t stream) {
-  using L = rb::SmemLayout<BLOCK_N, STAGES>;
-  const CUtensorMap* td = ta;        // placeholders unless the bulk-store epilogue is chosen below
-  const CUtensorMap* tx = ta;
-  auto kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8>;
-  // Staged (coalesced) stores: plain bf16 outputs whose rows are whole 16-byte chunks.  Always on for peer stores.
-  const bool can_stage = !g.out_f32 && !g.accumulate && splits <= 1 && (g.N % 8 == 0) && g.group_mode != 2 &&
-                         L::kTotalStaged + 1024 <= 232448;
-  const bool staged = can_stage && (g.peer_mode == 2 || staged_store_default());
-  if (g.peer_mode == 2 && !staged) return -11;
-  const int smem = (staged ? L::kTotalStaged : L::kTotal) + 1024;
-  static int configured_dev[64] = {0};   // per instantiation and device: largest size set so far
-  int& configured = configured_dev[rbhost::device_slot()];
-  if (configured < smem) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = smem;
-  }
-  rb::EpiParams ep;
+// Fills the epilogue's parameters and the tensor maps of what TMA moves for it.  Returns the shared memory to ask for.
+template <class L>
+int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUtensorMap*& td, const CUtensorMap*& tx,
+                  const CUtensorMap*& ts) {
   ep.d = g.d; ep.ldd = g.ldd;
   ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
   ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual); ep.ldr = g.ldr;
   ep.aux_in = reinterpret_cast<const __nv_bfloat16*>(g.aux_in); ep.ld_aux_in = g.ld_aux_in;
   ep.aux_out = reinterpret_cast<__nv_bfloat16*>(g.aux_out); ep.ld_aux_out = g.ld_aux_out;
   ep.act = g.act; ep.out_f32 = g.out_f32; ep.accumulate = g.accumulate; ep.alpha = g.alpha;
-  ep.staged = staged ? 1 : 0;
-  if (staged && g.peer_mode == 0 && L::kStageCols == 64 && tma_store_default()) {
-    int err = 0;
-    td = rbhost::get_tmap_2d(g.d, 2, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ldd, 64, 32, 1, &err);
-    tx = g.aux_out ? rbhost::get_tmap_2d(g.aux_out, 2, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ld_aux_out, 64, 32, 1, &err) : td;
-    if (td && tx) ep.staged = 2;
-    else { td = ta; tx = ta; }
-  }
   ep.row_scale = reinterpret_cast<const float*>(g.a_scale);
   ep.col_scale = reinterpret_cast<const float*>(g.b_scale);
   ep.fp8_b_format = g.ab_fp8 == 2 ? 1 : 0;
+  ep.staged = 0; ep.side = 0;
+  if (splits > 1) {
+    ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
+    ep.bias = nullptr; ep.residual = nullptr;          // applied once, by the kernel that folds the slabs
+  }
+  if (L::kTotalStaged + 1024 > 232448) return L::kTotal + 1024;
+  const bool tma = L::kTma && g.peer_mode == 0 && tma_store_default() && staged_store_default();
+  int err = 0;
+  if (!ep.out_f32) {
+    if (g.accumulate || (g.N % 8) || g.group_mode == 2) return L::kTotal + 1024;
+    if (g.peer_mode != 2 && !staged_store_default()) return L::kTotal + 1024;
+    ep.staged = 1;
+    const bool reads = g.aux_in || g.residual;
+    if (tma && (L::kSide ? !(g.aux_in && g.residual) && !(reads && g.aux_out) : !reads && !g.aux_out)) {
+      const uint64_t n = g.N, m = g.M;
+      const CUtensorMap* d = rbhost::get_tmap_2d(g.d, 2, n, m, (uint64_t)g.ldd, 64, 32, 1, &err);
+      const CUtensorMap* x = g.aux_out ? rbhost::get_tmap_2d(g.aux_out, 2, n, m, (uint64_t)g.ld_aux_out, 64, 32, 1, &err) : d;
+      const CUtensorMap* side = nullptr;
+      if (reads) {
+        if (g.aux_in) side = rbhost::get_tmap_2d(g.aux_in, 2, n, m, (uint64_t)g.ld_aux_in, 64, 32, 1, &err);
+        else if (g.residual) side = rbhost::get_tmap_2d(g.residual, 2, n, m, (uint64_t)g.ldr, 64, 32, 1, &err);
+      }
+      if (d && x && (side || !reads)) {
+        ep.staged = 2; td = d; tx = x;
+        if (side) { ts = side; ep.side = g.aux_in ? 2 : 1; }
+      }
+    }
+  } else if (tma && g.group_mode != 2 && (splits <= 1 || g.M % 32 == 0) && ep.ldd % 4 == 0 && g.N % 4 == 0 && g.act == RB_ACT_NONE &&
+             !ep.residual) {
+    // slabs of a split contraction lie below one another: whole 32-row tiles keep each in its own
+    const CUtensorMap* d = rbhost::get_tmap_2d(ep.d, 4, (uint64_t)g.N, (uint64_t)g.M * (splits > 1 ? splits : 1), (uint64_t)ep.ldd, 32, 32, 1, &err);
+    if (d) { ep.staged = ep.accumulate ? 4 : 3; td = d; ep.accumulate = 0; }
+  }
+  return (ep.staged ? L::kTotalStaged : L::kTotal) + 1024;
+}
+
+template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
+int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, int grid, int splits, cudaStream_t stream) {
+  using L = rb::SmemLayout<BLOCK_N, STAGES>;
   const int group_m = g.group_m > 0 ? g.group_m : 8;
   const int k_units = FP8 ? (g.K + 1) / 2 : g.K;          // the kernel counts K in two-byte units
   const int num_kb = (k_units + rb::kBlockK - 1) / rb::kBlockK;
@@ -1301,8 +1290,18 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
     kb_per = (num_kb + splits - 1) / splits;
     splits = (num_kb + kb_per - 1) / kb_per;   // no split may end up with an empty K range
     slab = static_cast<long long>(g.M) * g.N;
-    ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
-    ep.bias = nullptr; ep.residual = nullptr;          // applied once, by the kernel that folds the slabs
+  }
+  const CUtensorMap *td = ta, *tx = ta, *ts = ta;         // placeholders unless TMA moves the results
+  auto kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8>;
+  rb::EpiParams ep;
+  const int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts);
+  if (g.peer_mode == 2 && !ep.staged) return -11;
+  static int configured_dev[64] = {0};   // per instantiation and device: largest size set so far
+  int& configured = configured_dev[rbhost::device_slot()];
+  if (configured < smem) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = smem;
   }
   rb::GroupInfo grp;
   grp.mode = g.group_mode; grp.num_experts = g.num_experts;
@@ -1322,7 +1321,7 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
     peer.a_peer[r] = reinterpret_cast<const __nv_bfloat16*>(g.peer_ptrs[r]);
     peer.d_peer[r] = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(g.peer_ptrs[r]));
   }
-  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kNumThreads), smem, stream, 1, *ta, *tb, *td, *tx, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
+  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kNumThreads), smem, stream, 1, *ta, *tb, *td, *tx, *ts, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
                                                 rbhost::status_ptr());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
@@ -1357,39 +1356,9 @@ bool pair_kernel_enabled() {
 template <int A_MN, int B_MN, int FP8 = 0>
 int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb_half, int clusters, int splits,
                 cudaStream_t stream) {
-  constexpr int BLOCK_N = 256, STAGES = 6;
+  constexpr int BLOCK_N = 256, STAGES = 5;
   using L = rb::SmemLayoutPair<BLOCK_N, STAGES>;
   auto kern = rb::gemm_bf16_pair_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8>;
-  const bool staged = !g.out_f32 && !g.accumulate && splits <= 1 && (g.N % 8 == 0) && staged_store_default() &&
-                      L::kTotalStaged + 1024 <= 232448;
-  const int smem = (staged ? L::kTotalStaged : L::kTotal) + 1024;
-  static int configured_dev[64] = {0};
-  int& configured = configured_dev[rbhost::device_slot()];
-  if (configured < smem) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = smem;
-  }
-  rb::EpiParams ep;
-  ep.d = g.d; ep.ldd = g.ldd;
-  ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
-  ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual); ep.ldr = g.ldr;
-  ep.aux_in = reinterpret_cast<const __nv_bfloat16*>(g.aux_in); ep.ld_aux_in = g.ld_aux_in;
-  ep.aux_out = reinterpret_cast<__nv_bfloat16*>(g.aux_out); ep.ld_aux_out = g.ld_aux_out;
-  ep.act = g.act; ep.out_f32 = g.out_f32; ep.accumulate = g.accumulate; ep.alpha = g.alpha;
-  ep.staged = staged ? 1 : 0;
-  const CUtensorMap* td = ta;
-  const CUtensorMap* tx = ta;
-  if (staged && tma_store_default()) {
-    int err = 0;
-    td = rbhost::get_tmap_2d(g.d, 2, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ldd, 64, 32, 1, &err);
-    tx = g.aux_out ? rbhost::get_tmap_2d(g.aux_out, 2, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ld_aux_out, 64, 32, 1, &err) : td;
-    if (td && tx) ep.staged = 2;
-    else { td = ta; tx = ta; }
-  }
-  ep.row_scale = reinterpret_cast<const float*>(g.a_scale);
-  ep.col_scale = reinterpret_cast<const float*>(g.b_scale);
-  ep.fp8_b_format = g.ab_fp8 == 2 ? 1 : 0;
   const int group_m = g.group_m > 0 ? g.group_m : 4;      // in 256-row units
   const int k_units = FP8 ? (g.K + 1) / 2 : g.K;
   const int num_kb = (k_units + rb::kBlockK - 1) / rb::kBlockK;
@@ -1399,10 +1368,19 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
     kb_per = (num_kb + splits - 1) / splits;
     splits = (num_kb + kb_per - 1) / kb_per;
     slab = static_cast<long long>(g.M) * g.N;
-    ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
-    ep.bias = nullptr; ep.residual = nullptr;
   }
-  const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(rb::kNumThreads), smem, stream, 2, *ta, *tb_half, *td, *tx, g.M, g.N,
+  const CUtensorMap *td = ta, *tx = ta, *ts = ta;
+  rb::EpiParams ep;
+  int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts);
+  if (ep.staged == 1) ep.staged = 0, smem = L::kTotal + 1024;       // this kernel stores through TMA or straight from registers
+  static int configured_dev[64] = {0};
+  int& configured = configured_dev[rbhost::device_slot()];
+  if (configured < smem) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = smem;
+  }
+  const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(rb::kNumThreads), smem, stream, 2, *ta, *tb_half, *td, *tx, *ts, g.M, g.N,
                                            k_units, group_m, splits, kb_per, slab, ep, rbhost::status_ptr());
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
   const long long n4 = slab / 4;
