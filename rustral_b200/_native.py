@@ -377,6 +377,18 @@ def stream_key(device) -> tuple:
     return (device, torch.cuda.current_stream(device).cuda_stream)
 
 
+def scratch(cache: dict, device, n: int, dtype, least: int = 0) -> torch.Tensor:
+    """`n` elements of scratch memory from the grow-only `cache`, one buffer per device and stream.  While a graph is being captured the
+    buffer is the capture's own instead: a buffer that grows later would be freed under the graph that still names it."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(n, dtype=dtype, device=device)
+    key = stream_key(device)
+    buf = cache.get(key)
+    if buf is None or buf.numel() < n:
+        buf = cache[key] = torch.empty(max(n, least), dtype=dtype, device=device)
+    return buf
+
+
 def wants_grad(*tensors) -> bool:
     """True when autograd would record an op on these inputs; wrappers skip their autograd.Function otherwise (its
     `apply` alone costs several microseconds per call)."""

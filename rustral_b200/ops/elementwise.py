@@ -20,12 +20,7 @@ _scratch: dict = {}
 
 
 def _f32_scratch(device, n: int) -> torch.Tensor:
-    key = N.stream_key(device)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.empty(max(n, 4096), dtype=torch.float32, device=device)
-        _scratch[key] = buf
-    return buf
+    return N.scratch(_scratch, device, n, torch.float32, 4096)
 
 
 def _dt(t: torch.Tensor) -> int:

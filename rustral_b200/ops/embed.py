@@ -9,12 +9,7 @@ _scratch: dict = {}
 
 
 def _int_scratch(device, n: int) -> torch.Tensor:
-    key = N.stream_key(device)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.empty(n, dtype=torch.int32, device=device)
-        _scratch[key] = buf
-    return buf
+    return N.scratch(_scratch, device, n, torch.int32, 0)
 
 
 def embedding_forward(ids: torch.Tensor, wte: torch.Tensor, wpe=None, seq_len: int = 0, out=None) -> torch.Tensor:

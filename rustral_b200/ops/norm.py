@@ -10,12 +10,7 @@ _scratch: dict = {}
 
 def _partial_scratch(device, numel: int) -> torch.Tensor:
     """Grow-only fp32 scratch for the parameter-gradient partials, one per device and stream."""
-    key = N.stream_key(device)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < numel:
-        buf = torch.empty(max(numel, 1 << 16), dtype=torch.float32, device=device)
-        _scratch[key] = buf
-    return buf
+    return N.scratch(_scratch, device, numel, torch.float32, 1 << 16)
 
 
 def norm_forward(x2: torch.Tensor, gamma: torch.Tensor, beta, eps: float, rms: bool, out=None, want_stats: bool = True):

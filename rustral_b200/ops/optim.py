@@ -11,12 +11,7 @@ _scratch: dict = {}
 
 
 def _f32_scratch(device, n: int) -> torch.Tensor:
-    key = N.stream_key(device)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.empty(n, dtype=torch.float32, device=device)
-        _scratch[key] = buf
-    return buf
+    return N.scratch(_scratch, device, n, torch.float32, 0)
 
 
 def adam_step(p, m, v, g, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, step: int, decoupled=True,

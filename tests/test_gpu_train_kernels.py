@@ -135,3 +135,23 @@ def test_max_pool2d_forward_and_backward(H, W, k, stride, dtype, cuda_status):
     assert torch.allclose(xd.grad.float().cpu(), xr.grad, atol=2e-2 if dtype is torch.bfloat16 else 1e-6)
     if H == W:
         assert torch.equal(global_max_pool2d(x.cuda()).float().cpu(), x.float().amax((2, 3)))
+
+
+def test_a_captured_graph_owns_its_scratch(cuda_status):
+    """Scratch that a graph names must not be in the grow-only buffers: those are freed when a later call needs more, and the graph would
+    read and write what is not its own any more."""
+    from rustral_b200 import ops
+    from rustral_b200.ops import elementwise, embed, norm, optim
+    a = torch.randn(500, 256, device="cuda").bfloat16()
+    wide = torch.randn(64, 40000, device="cuda").bfloat16()
+    want, want_wide = ops.sum_dim0(a), ops.sum_dim0(wide)
+    caches = [m._scratch for m in (elementwise, embed, norm, optim)]
+    before = [{k: v.data_ptr() for k, v in c.items()} for c in caches]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, total = ops.sum_dim0(a), ops.sum_all(a)
+        got_wide = ops.sum_dim0(wide)
+    assert [{k: v.data_ptr() for k, v in c.items()} for c in caches] == before
+    torch.cuda.empty_cache()
+    graph.replay()
+    assert torch.equal(got, want) and torch.equal(got_wide, want_wide) and torch.isfinite(total)
