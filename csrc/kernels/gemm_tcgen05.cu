@@ -534,12 +534,12 @@ __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensor
     __syncwarp();
     if (lane == 0) {
       const int x = col + c - half * 32;
-      if (ep.staged == 4) { if (row0 < M) tma_reduce_add_2d(tmD, slot, x, drow); }
-      else if (ep.staged == 3) { if (row0 < M) tma_store_2d(tmD, slot, x, drow); }
+      if (row0 >= M) {}                        // nothing of the matrix; with stacked results these are another one's rows
+      else if (ep.staged == 4) tma_reduce_add_2d(tmD, slot, x, drow);
       else tma_store_2d(two ? tmAux : tmD, slot, x, drow);
       tma_store_commit();
       if (two) {
-        tma_store_2d(tmD, slot + 4096, x, drow);
+        if (row0 < M) tma_store_2d(tmD, slot + 4096, x, drow);
         tma_store_commit();
       }
     }
@@ -818,7 +818,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       };
       if (L::kTma && ep.staged >= 2) {
         epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t & 1, taddr + cgrp * (BLOCK_N / 2), row0,
-                                  num_splits > 1 ? outer * M + row0 : row0, colg, M, N, lane, empty_k, abort_flag, status, arrive);
+                                  num_splits > 1 || grp.mode == 2 ? outer * M + row0 : row0, colg, M, N, lane, empty_k, abort_flag, status, arrive);
         continue;
       }
       EpiParams epu = ep;
@@ -1249,14 +1249,17 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
   }
   if (L::kTotalStaged + 1024 > 232448) return L::kTotal + 1024;
   const bool tma = L::kTma && g.peer_mode == 0 && tma_store_default() && staged_store_default();
+  // slabs of a split contraction and the experts' results (grouped mode 2) lie below one another: whole 32-row tiles keep each in its own
+  const bool stacked = g.M % 32 == 0 && (splits > 1 || (tma && g.d_expert_stride == static_cast<long long>(g.M) * g.ldd));
+  const uint64_t stack = splits > 1 ? splits : g.group_mode == 2 ? g.num_experts : 1;
   int err = 0;
   if (!ep.out_f32) {
-    if (g.accumulate || (g.N % 8) || g.group_mode == 2) return L::kTotal + 1024;
+    if (g.accumulate || (g.N % 8) || (g.group_mode == 2 && !stacked)) return L::kTotal + 1024;
     if (g.peer_mode != 2 && !staged_store_default()) return L::kTotal + 1024;
     ep.staged = 1;
     const bool reads = g.aux_in || g.residual;
     if (tma && (L::kSide ? !(g.aux_in && g.residual) && !(reads && g.aux_out) : !reads && !g.aux_out)) {
-      const uint64_t n = g.N, m = g.M;
+      const uint64_t n = g.N, m = g.M * stack;
       const CUtensorMap* d = rbhost::get_tmap_2d(g.d, 2, n, m, (uint64_t)g.ldd, 64, 32, 1, &err);
       const CUtensorMap* x = g.aux_out ? rbhost::get_tmap_2d(g.aux_out, 2, n, m, (uint64_t)g.ld_aux_out, 64, 32, 1, &err) : d;
       const CUtensorMap* side = nullptr;
@@ -1269,10 +1272,9 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
         if (side) { ts = side; ep.side = g.aux_in ? 2 : 1; }
       }
     }
-  } else if (tma && g.group_mode != 2 && (splits <= 1 || g.M % 32 == 0) && ep.ldd % 4 == 0 && g.N % 4 == 0 && g.act == RB_ACT_NONE &&
+  } else if (tma && (stack == 1 || stacked) && ep.ldd % 4 == 0 && g.N % 4 == 0 && g.act == RB_ACT_NONE &&
              !ep.residual) {
-    // slabs of a split contraction lie below one another: whole 32-row tiles keep each in its own
-    const CUtensorMap* d = rbhost::get_tmap_2d(ep.d, 4, (uint64_t)g.N, (uint64_t)g.M * (splits > 1 ? splits : 1), (uint64_t)ep.ldd, 32, 32, 1, &err);
+    const CUtensorMap* d = rbhost::get_tmap_2d(ep.d, 4, (uint64_t)g.N, (uint64_t)g.M * stack, (uint64_t)ep.ldd, 32, 32, 1, &err);
     if (d) { ep.staged = ep.accumulate ? 4 : 3; td = d; ep.accumulate = 0; }
   }
   return (ep.staged ? L::kTotalStaged : L::kTotal) + 1024;

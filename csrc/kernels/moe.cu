@@ -67,12 +67,13 @@ moe_route_kernel(const float* __restrict__ logits, int T, int E, int k, int reno
 __global__ void __launch_bounds__(128)
 moe_route_bwd_kernel(const float* __restrict__ probs, const int* __restrict__ idx, const float* __restrict__ w,
                      const float* __restrict__ dw, const int* __restrict__ counts, int T, int E, int k, int renorm,
-                     float aux_grad_scale, float* __restrict__ dlogits) {
+                     const float* __restrict__ aux_grad_scale, float* __restrict__ dlogits) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
   const float* p = probs + static_cast<long long>(t) * E;
   float dp[2] = {0.f, 0.f};
+  const float aux_scale = aux_grad_scale ? *aux_grad_scale : 0.f;
   // gradient through the (renormalised) selected weights
   float S = 0.f, dot = 0.f;
   for (int j = 0; j < k; ++j) {
@@ -92,7 +93,7 @@ moe_route_bwd_kernel(const float* __restrict__ probs, const int* __restrict__ id
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int e = lane + 32 * h;
-    if (e < E) dp[h] += aux_grad_scale * static_cast<float>(E) * (static_cast<float>(counts[e]) / denom) / static_cast<float>(T);
+    if (e < E) dp[h] += aux_scale * static_cast<float>(E) * (static_cast<float>(counts[e]) / denom) / static_cast<float>(T);
   }
   // softmax backward
   const float pv0 = lane < E ? p[lane] : 0.f, pv1 = lane + 32 < E ? p[lane + 32] : 0.f;
@@ -572,7 +573,7 @@ RB_API int rb_moe_scatter(const void* x, const int* slot_pos, void* xp, int slot
   return static_cast<int>(cudaGetLastError());
 }
 RB_API int rb_moe_route_bwd(const float* probs, const int* idx, const float* w, const float* dw, const int* counts, int T,
-                            int E, int k, int renorm, float aux_grad_scale, float* dlogits, void* stream_v) {
+                            int E, int k, int renorm, const float* aux_grad_scale, float* dlogits, void* stream_v) {
   if (T <= 0 || E <= 0 || E > 64 || k <= 0 || k > rb::kMaxK) return -1;
   rb::moe_route_bwd_kernel<<<(T + 3) / 4, 128, 0, RB_ST>>>(probs, idx, w, dw, counts, T, E, k, renorm, aux_grad_scale, dlogits);
   return static_cast<int>(cudaGetLastError());

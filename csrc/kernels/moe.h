@@ -11,9 +11,9 @@ extern "C" {
 int rb_moe_route(const float* logits, int T, int E, int k, int renorm, int* idx, float* w, float* probs_out, void* stream);
 // Backward of the router: dlogits [T, E] fp32 from dw [T, k] and the load-balancing loss
 //   aux = E * sum_e f_e * P_e,  f_e = (tokens routed to e) / (T k),  P_e = mean_t probs[t, e]
-// aux_grad_scale multiplies d aux (pass coefficient * upstream gradient).  counts: int32 [E] tokens per expert.
+// *aux_grad_scale (device memory; NULL: 0) multiplies d aux: coefficient * upstream gradient.  counts: int32 [E] tokens per expert.
 int rb_moe_route_bwd(const float* probs, const int* idx, const float* w, const float* dw, const int* counts, int T, int E,
-                     int k, int renorm, float aux_grad_scale, float* dlogits, void* stream);
+                     int k, int renorm, const float* aux_grad_scale, float* dlogits, void* stream);
 // Grouped-limited router (inference): scores = softmax(logits[T, E]) in fp32; the experts form `groups` equal groups of
 // neighbours, a group counts as its largest score, and only experts of the best `keep` groups can be chosen; the k largest
 // scores are taken (ties to the lower index) and divided by (their sum + eps) when renorm != 0.  groups <= 1: no limit.

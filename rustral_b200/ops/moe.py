@@ -17,7 +17,7 @@ from .matmul import gemm, _gemm_f32, act_reference, act_grad_reference
 
 P, I, F, LL = N.c_void_p, N.c_int, N.c_float, N.c_ll
 N.optional_sig("rb_moe_route", [P, I, I, I, I, P, P, P, P])
-N.optional_sig("rb_moe_route_bwd", [P, P, P, P, P, I, I, I, I, F, P, P])
+N.optional_sig("rb_moe_route_bwd", [P, P, P, P, P, I, I, I, I, P, P, P])
 N.optional_sig("rb_moe_route_groups", [P, I, I, I, I, I, I, F, P, P, P])
 N.optional_sig("rb_moe_route_sigmoid", [P, P, I, I, I, I, I, I, I, F, P, P, P])
 N.optional_sig("rb_swiglu_slots", [P, LL, P, LL, I, I, I, P, P, I, F, P])
@@ -148,8 +148,9 @@ def scatter_tokens(x: torch.Tensor, pl: MoEPlan) -> torch.Tensor:
     return xp
 
 
-def route_backward(probs, idx, w, dw, counts, renorm: bool, aux_grad_scale: float):
-    """dlogits fp32 [T, E] from dw [T, k] and the load-balancing loss E * sum_e f_e P_e scaled by aux_grad_scale."""
+def route_backward(probs, idx, w, dw, counts, renorm: bool, aux_grad_scale):
+    """dlogits fp32 [T, E] from dw [T, k] and the load-balancing loss E * sum_e f_e P_e scaled by aux_grad_scale (a number, or a tensor of
+    one element: on a GPU it is then read there, without waiting for it on the host)."""
     T, E = probs.shape
     k = idx.shape[1]
     if not probs.is_cuda:
@@ -164,8 +165,9 @@ def route_backward(probs, idx, w, dw, counts, renorm: bool, aux_grad_scale: floa
         dp = dp + aux_grad_scale * E * (counts.float() / (T * k))[None, :] / T
         return probs * (dp - (dp * probs).sum(-1, keepdim=True))
     out = torch.empty_like(probs)
+    scale = torch.as_tensor(aux_grad_scale, dtype=torch.float32, device=probs.device)
     N.check(N.kernels().rb_moe_route_bwd(probs.data_ptr(), idx.data_ptr(), w.data_ptr(), dw.contiguous().data_ptr(),
-                                         counts.data_ptr(), T, E, k, int(renorm), float(aux_grad_scale), out.data_ptr(),
+                                         counts.data_ptr(), T, E, k, int(renorm), scale.data_ptr(), out.data_ptr(),
                                          N.stream_ptr()), "rb_moe_route_bwd")
     return out
 
@@ -308,12 +310,12 @@ def grouped_gemm(xp: torch.Tensor, W: torch.Tensor, pl: MoEPlan, *, b_mn: bool =
 
 
 def grouped_wgrad(dyp: torch.Tensor, xp: torch.Tensor, pl: MoEPlan, out: torch.Tensor | None = None,
-                  accumulate: bool = False) -> torch.Tensor:
-    """dW[e] = dyp[seg_e]^T @ xp[seg_e]  ->  [E, N, K] (fp32 or the dtype of `out`)."""
+                  accumulate: bool = False, dtype=torch.float32) -> torch.Tensor:
+    """dW[e] = dyp[seg_e]^T @ xp[seg_e]  ->  [E, N, K] in `dtype` (fp32 sums, rounded once) or in the dtype of `out`."""
     E = pl.num_experts
     Nn, K = dyp.shape[1], xp.shape[1]
     if out is None:
-        out = torch.zeros((E, Nn, K), dtype=torch.float32, device=xp.device)
+        out = torch.empty((E, Nn, K), dtype=dtype, device=xp.device)           # experts without tokens are written as zeros
         accumulate = False
     if not xp.is_cuda:
         for e, (o, c) in enumerate(_segments(pl)):
@@ -370,17 +372,17 @@ class _MoEMlpFn(torch.autograd.Function):
         dy = dy.contiguous()
         dw = weight_grad(dy, yp, pl)                                   # [T, k]
         dyp = gather(dy, pl, slot_scale=w.reshape(-1).contiguous())      # w_j * dy at every slot
-        dw2 = grouped_wgrad(dyp, h, pl)
+        dw2 = grouped_wgrad(dyp, h, pl, dtype=w2.dtype)
         dh = grouped_gemm(dyp, w2, pl, b_mn=True)
         if kind == "swiglu":
             dpre = rotary.swiglu_backward(dh, pre)
         else:
             from .elementwise import unary_bwd
             dpre = unary_bwd("gelu", pre, dh)
-        dw1 = grouped_wgrad(dpre, xp, pl)
+        dw1 = grouped_wgrad(dpre, xp, pl, dtype=w1.dtype)
         dxp = grouped_gemm(dpre, w1, pl, b_mn=True)
         dx_experts = combine(dxp, pl, None)
-        aux_scale = float(daux) if daux is not None else 0.0
+        aux_scale = daux if daux is not None else 0.0
         dlogits = route_backward(probs, idx, w, dw, pl.counts, ctx.renorm, aux_scale)
         dl = dlogits.to(x.dtype)
         dx = gemm(dl, router_w, b_mn=True, out_dtype=x.dtype) if dl.shape[1] % 8 == 0 and x.is_cuda else \
@@ -389,7 +391,7 @@ class _MoEMlpFn(torch.autograd.Function):
         dx = binary("add", dx.contiguous(), dx_experts)
         drw = (dlogits.t() @ x.float()).to(router_w.dtype) if not x.is_cuda or dl.shape[1] % 8 else \
             gemm(dl, x, a_mn=True, b_mn=True, out_dtype=router_w.dtype)
-        return dx, drw, dw1.to(w1.dtype), dw2.to(w2.dtype), None, None, None
+        return dx, drw, dw1, dw2, None, None, None
 
 
 def moe_mlp(x, router_w, w1, w2, k: int = 2, kind: str = "swiglu", renorm: bool = True):
