@@ -218,23 +218,25 @@ sum_dim0_stage1_vec(const __nv_bfloat16* __restrict__ a, long long lda, float* _
     partial[static_cast<long long>(slab) * cols + c2] = t;
   }
 }
-__global__ void __launch_bounds__(256)
+// 32 columns per block, 32 lanes share a column's slabs: with one thread per column the fold was 16 rounds of loads, 5.3 us for any size.
+__global__ void __launch_bounds__(1024)
 sum_dim0_stage2(const float* __restrict__ partial, int slabs, float* __restrict__ out, int cols, int accumulate) {
   pdl_wait();
   pdl_launch();
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= cols) return;
-  float acc = 0.f;
-  int s = 0;
-  for (; s + 7 < slabs; s += 8) {          // the loads of eight slabs are requested together, then added in slab order
-    float v[8];
+  __shared__ float sh[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + tx;
+  float t = 0.f;
+  if (col < cols)
+    for (int s = ty; s < slabs; s += 32) t += partial[static_cast<long long>(s) * cols + col];
+  sh[ty][tx] = t;
+  __syncthreads();
+  if (ty == 0 && col < cols) {
+    t = 0.f;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = partial[static_cast<long long>(s + u) * cols + col];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc += v[u];
+    for (int y = 0; y < 32; ++y) t += sh[y][tx];
+    out[col] = accumulate ? out[col] + t : t;
   }
-  for (; s < slabs; ++s) acc += partial[static_cast<long long>(s) * cols + col];
-  out[col] = accumulate ? out[col] + acc : acc;
 }
 // Single-kernel variant for when no scratch is available: one thread per column walks all rows.
 template <typename T>
@@ -461,13 +463,14 @@ RB_API int rb_sum_dim0_staged(const void* a, long long lda, float* out, float* p
   if (rows <= 0 || cols <= 0) return 0;
   if (!partial) return -1;
   int slabs = rb::kSumDim0Slabs;
-  if (rows < slabs) slabs = static_cast<int>(rows);
+  // 64 rows or more per slab: each of the 8 row lanes of a block then has its 8 loads in flight
+  if ((rows + 63) / 64 < slabs) slabs = static_cast<int>((rows + 63) / 64);
   dim3 grid((cols + 255) / 256, slabs);
   if (dtype == 0) rbhost::launch_pdl(rb::sum_dim0_stage1<float>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const float*)a, lda, partial, rows, cols);
   else if ((cols % 8 == 0) && (lda % 8 == 0) && (reinterpret_cast<uintptr_t>(a) % 16 == 0))
     rbhost::launch_pdl(rb::sum_dim0_stage1_vec, dim3((cols + 255) / 256, slabs), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
   else rbhost::launch_pdl(rb::sum_dim0_stage1<__nv_bfloat16>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
-  rbhost::launch_pdl(rb::sum_dim0_stage2, dim3((cols + 255) / 256), dim3(256), 0, RB_STREAM, 1, partial, slabs, out, cols, accumulate);
+  rbhost::launch_pdl(rb::sum_dim0_stage2, dim3((cols + 31) / 32), dim3(1024), 0, RB_STREAM, 1, partial, slabs, out, cols, accumulate);
   return static_cast<int>(cudaGetLastError());
 }
 

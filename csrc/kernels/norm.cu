@@ -266,30 +266,19 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
 
 // out[col] (+)= sum_p partial[p][col].  Eight row groups per CTA each sum every eighth partial, then the
 // groups are folded in index order: parallel enough to hide latency, and the order is fixed.
-__global__ void __launch_bounds__(256)
+// 32 columns per block, 32 lanes share a column's partials and add theirs in order: with 8 lanes a fold took 5 us for rows of any length.
+__global__ void __launch_bounds__(1024)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int num_partials, int n, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, int accumulate) {
   pdl_wait();
   pdl_launch();
-  __shared__ float sa[8][33], sb[8][33];
+  __shared__ float sa[32][33], sb[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + tx;
   float a = 0.f, b = 0.f;
   if (col < n) {
-    // eight independent loads per array are requested before they are added (in the same order as a plain loop):
-    // the fold is a chain of dependent additions, but its loads need not wait for one another
-    int p = ty;
-    for (; p + 56 < num_partials; p += 64) {
-      float va[8], vb[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        va[u] = partial[static_cast<long long>(p + 8 * u) * n + col];
-        vb[u] = dbeta ? partial[static_cast<long long>(num_partials + p + 8 * u) * n + col] : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) { a += va[u]; b += vb[u]; }
-    }
-    for (; p < num_partials; p += 8) {
+#pragma unroll 4
+    for (int p = ty; p < num_partials; p += 32) {
       a += partial[static_cast<long long>(p) * n + col];
       if (dbeta) b += partial[static_cast<long long>(num_partials + p) * n + col];
     }
@@ -297,12 +286,13 @@ norm_bwd_reduce_kernel(const float* __restrict__ partial, int num_partials, int 
   sa[ty][tx] = a;
   sb[ty][tx] = b;
   __syncthreads();
-  if (ty == 0 && col < n) {
-    float ta = 0.f, tb = 0.f;
+  if (ty < 2 && col < n) {
+    float (*sh)[33] = ty == 0 ? sa : sb;
+    float* out = ty == 0 ? dgamma : dbeta;
+    float t = 0.f;
 #pragma unroll
-    for (int g = 0; g < 8; ++g) { ta += sa[g][tx]; tb += sb[g][tx]; }
-    dgamma[col] = accumulate ? dgamma[col] + ta : ta;
-    if (dbeta) dbeta[col] = accumulate ? dbeta[col] + tb : tb;
+    for (int y = 0; y < 32; ++y) t += sh[y][tx];
+    if (out) out[col] = accumulate ? out[col] + t : t;
   }
 }
 
@@ -402,7 +392,7 @@ RB_API int rb_norm_bwd(const void* dy, long long lddy, const void* x, long long 
 #undef RB_LAUNCH
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  rbhost::launch_pdl(rb::norm_bwd_reduce_kernel, dim3((n + 31) / 32), dim3(256), 0, stream, 1, partial, grid, n, dgamma, rms ? nullptr : dbeta,
+  rbhost::launch_pdl(rb::norm_bwd_reduce_kernel, dim3((n + 31) / 32), dim3(1024), 0, stream, 1, partial, grid, n, dgamma, rms ? nullptr : dbeta,
                                                                  accumulate);
   return static_cast<int>(cudaGetLastError());
 }
