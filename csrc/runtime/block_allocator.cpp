@@ -118,6 +118,37 @@ int rb_ba_table(const RbBlockAllocator* a, int64_t seq_id, int32_t* out, int max
   return n;
 }
 
+// Block tables of `n` sequences, one row of `width` entries each (zeros behind a table's end and for
+// unknown sequences).  Returns 0, or -1 when a table is longer than that.
+int rb_ba_tables(const RbBlockAllocator* a, const int64_t* seq_ids, int n, int width, int32_t* out) {
+  std::lock_guard<std::mutex> l(a->mu);
+  int rc = 0;
+  for (int i = 0; i < n; ++i) {
+    int32_t* row = out + (int64_t)i * width;
+    int m = 0;
+    auto it = a->tables.find(seq_ids[i]);
+    if (it != a->tables.end()) {
+      if ((int)it->second.size() > width) rc = -1;
+      for (m = 0; m < width && m < (int)it->second.size(); ++m) row[m] = it->second[m];
+    }
+    for (; m < width; ++m) row[m] = 0;
+  }
+  return rc;
+}
+
+// Positions start .. start + n - 1 of a sequence and their cache slots.  Returns 0, or -1 when one of them has no block.
+int rb_ba_slots(const RbBlockAllocator* a, int64_t seq_id, int64_t start, int64_t n, int64_t* pos, int64_t* slots) {
+  std::lock_guard<std::mutex> l(a->mu);
+  auto it = a->tables.find(seq_id);
+  if (it == a->tables.end() || start < 0 || start + n > (int64_t)it->second.size() * a->block_size) return -1;
+  for (int64_t i = 0; i < n; ++i) {
+    const int64_t p = start + i;
+    pos[i] = p;
+    slots[i] = (int64_t)it->second[p / a->block_size] * a->block_size + p % a->block_size;
+  }
+  return 0;
+}
+
 int64_t rb_ba_slot(const RbBlockAllocator* a, int64_t seq_id, int token_index) {
   std::lock_guard<std::mutex> l(a->mu);
   auto it = a->tables.find(seq_id);

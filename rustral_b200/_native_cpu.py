@@ -38,6 +38,8 @@ def declare_runtime(lib) -> None:
     _sig(lib, "rb_ba_free", [P, LL], I)
     _sig(lib, "rb_ba_table_len", [P, LL], I)
     _sig(lib, "rb_ba_table", [P, LL, P, I], I)
+    _sig(lib, "rb_ba_tables", [P, P, I, I, P], I)
+    _sig(lib, "rb_ba_slots", [P, LL, LL, LL, P, P], I)
     _sig(lib, "rb_ba_slot", [P, LL, I], LL)
     _sig(lib, "rb_ba_set_state_slots", [P, I], I)
     _sig(lib, "rb_ba_state_slot", [P, LL], I)

@@ -251,6 +251,17 @@ class PagedCache:
         self._lib.rb_ba_table(self._h, seq_id, buf, n)
         return list(buf[:n])
 
+    def fill_tables(self, seq_ids: list, out: torch.Tensor) -> None:
+        """Block tables of `seq_ids` into `out` (int32 on the host, contiguous, one row per sequence), zeros behind each."""
+        ids = (C.c_int64 * max(len(seq_ids), 1))(*seq_ids)
+        if self._lib.rb_ba_tables(self._h, ids, len(seq_ids), out.shape[1], out.data_ptr()) < 0:
+            raise RuntimeError("a sequence has more blocks than the table has columns")
+
+    def fill_slots(self, seq_id: int, start: int, n: int, pos: int, slots: int) -> None:
+        """Positions start .. start + n - 1 and their cache slots, as int64 to the host addresses `pos` and `slots`."""
+        if n and self._lib.rb_ba_slots(self._h, seq_id, start, n, pos, slots) < 0:
+            raise IndexError(f"positions {start} to {start + n - 1} of sequence {seq_id} have no blocks")
+
     def slot(self, seq_id: int, token_index: int) -> int:
         return int(self._lib.rb_ba_slot(self._h, seq_id, token_index))
 

@@ -226,27 +226,26 @@ class ModelRunner:
         [len(dec_ids), vocab_padded] or None).
         (Batched and chunked prefill of the reference's scheduler: crates/nn/src/continuous_batching.rs:248-295.)"""
         dev, bs = self.device, self.block_size
-        ids_h, pos_h, slot_h, spans, tables = [], [], [], [], []
+        rd = sum(len(c[1]) for c in chunks)
+        T = rd + len(dec_ids)
+        host = self._host((3, T), torch.int64)                       # token ids, positions, cache slots
+        ids_h, at_pos, at_slots = host[0].numpy(), host[1].data_ptr(), host[2].data_ptr()
+        spans, tables, r0 = [], [], 0
         for seq_id, tokens, start, _ in chunks:
-            table = self.cache.block_table(seq_id)
-            L = len(tokens)
-            spans.append((len(ids_h), len(ids_h) + L, start))
-            tables.append(table)
-            ids_h += list(tokens)
-            pos_h += list(range(start, start + L))
-            slot_h += [table[p_ // bs] * bs + p_ % bs for p_ in range(start, start + L)]
-        rd = len(ids_h)
-        for seq_id, tok, n in zip(dec_ids, dec_tok, dec_len):
-            table = self.cache.block_table(seq_id)
-            ids_h.append(tok)
-            pos_h.append(n - 1)
-            slot_h.append(table[(n - 1) // bs] * bs + (n - 1) % bs)
-        T = len(ids_h)
-        host = torch.tensor([ids_h, pos_h, slot_h], dtype=torch.int64).to(dev)
+            r1 = r0 + len(tokens)
+            spans.append((r0, r1, start))
+            tables.append(self.cache.block_table(seq_id))
+            ids_h[r0:r1] = tokens
+            self.cache.fill_slots(seq_id, start, r1 - r0, at_pos + 8 * r0, at_slots + 8 * r0)
+            r0 = r1
+        for r, (seq_id, tok, n) in enumerate(zip(dec_ids, dec_tok, dec_len), rd):
+            ids_h[r] = tok
+            self.cache.fill_slots(seq_id, n - 1, 1, at_pos + 8 * r, at_slots + 8 * r)
+        host = host.to(dev, non_blocking=True)
         bt = ctx = None
         if dec_ids:
             width = max(len(self.cache.block_table(s_)) for s_ in dec_ids)
-            bt = self._fill_tables(dec_ids, width).to(dev)
+            bt = self._fill_tables(dec_ids, width).to(dev, non_blocking=True)
             ctx = torch.tensor(dec_len, dtype=torch.int32, device=dev)
         segments = None
         if self.recurrent:
@@ -289,11 +288,13 @@ class ModelRunner:
         slots = bt.gather(1, (pos // bs).view(B, 1)).view(B).to(torch.int64) * bs + pos % bs
         return self._run(StepBatch(ids, pos, slots, [], 0, [], bt, ctx, bs, segments), None)
 
+    def _host(self, shape, dtype) -> torch.Tensor:
+        """Host memory for a step's inputs; pinned for a GPU, so that their copies need not be waited for."""
+        return torch.empty(shape, dtype=dtype, pin_memory=self.device.type == "cuda")
+
     def _fill_tables(self, seq_ids, width: int) -> torch.Tensor:
-        tables = [self.cache.block_table(s) for s in seq_ids]
-        bt_host = torch.zeros((len(seq_ids), width), dtype=torch.int32)
-        for i, t in enumerate(tables):
-            bt_host[i, :len(t)] = torch.tensor(t, dtype=torch.int32)
+        bt_host = self._host((len(seq_ids), width), torch.int32)
+        self.cache.fill_tables(seq_ids, bt_host)
         return bt_host
 
     @torch.no_grad()
@@ -319,6 +320,11 @@ class ModelRunner:
         need = (max(context_lens) + self.block_size - 1) // self.block_size
         return min(full, max(64, 1 << (need - 1).bit_length()))
 
+    @staticmethod
+    def _step_views(buf: torch.Tensor, B: int, width: int) -> dict:
+        return {"ids": buf[:8 * B].view(torch.int64), "ctx": buf[8 * B:12 * B].view(torch.int32),
+                "bt": buf[12 * B:].view(torch.int32).view(B, width)}
+
     def _decode_graphed(self, seq_ids, last_tokens, context_lens) -> torch.Tensor:
         """Replays one captured CUDA graph per batch size: the 10 to 20 launches per layer of a decode step are
         launch-bound from Python, the graph submits them in one call.  Inputs live in static device tensors that
@@ -328,16 +334,18 @@ class ModelRunner:
         width = self._table_width(context_lens)
         g = self._graphs.get((B, width))
         if g is None:
-            ids = torch.zeros(B, dtype=torch.int64, device=dev)
-            ctx = torch.ones(B, dtype=torch.int32, device=dev)
-            bt = torch.zeros((B, width), dtype=torch.int32, device=dev)
-            g = {"ids": ids, "ctx": ctx, "bt": bt, "seg": None, "graph": None, "out": None}
+            # ids (int64), context lengths and block tables (int32) behind one another: one copy refreshes all three
+            buf = torch.zeros(12 * B + 4 * B * width, dtype=torch.uint8, device=dev)
+            g = {"buf": buf, "seg": None, "graph": None, "out": None, **self._step_views(buf, B, width)}
             if self.recurrent:
                 g["seg"] = Segments(torch.zeros((B, 4), dtype=torch.int32, device=dev), None)
             self._graphs[(B, width)] = g
-        g["ids"].copy_(torch.tensor(last_tokens, dtype=torch.int64), non_blocking=True)
-        g["ctx"].copy_(torch.tensor(context_lens, dtype=torch.int32), non_blocking=True)
-        g["bt"].copy_(self._fill_tables(seq_ids, width), non_blocking=True)
+        host = self._host(g["buf"].shape, torch.uint8)
+        view = self._step_views(host, B, width)
+        view["ids"].numpy()[:] = last_tokens
+        view["ctx"].numpy()[:] = context_lens
+        self.cache.fill_tables(seq_ids, view["bt"])
+        g["buf"].copy_(host, non_blocking=True)
         if g["seg"] is not None:
             g["seg"].table.copy_(torch.tensor(self._decode_segments(seq_ids, context_lens), dtype=torch.int32), non_blocking=True)
         if g["graph"] is None:
