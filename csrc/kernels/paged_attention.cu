@@ -39,7 +39,11 @@ kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, long long ld_k, const 
 
 constexpr int kMaxGroup = 16;    // query heads per KV head served by one CTA pass (the M of the mma tile)
 constexpr int kPaWarps = 4;
-constexpr int kSplitTokens = 256;          // cached tokens per CTA (split-KV): 2 passes of 32 tokens per warp
+constexpr int kSplitTokens = 256;          // least tokens of a slice (split-KV): 2 passes of 32 tokens per warp
+// Tokens per slice of a sequence with `count` visible tokens when a launch has room for `nsplit` slices of each sequence.
+__device__ __forceinline__ int pa_slice(int count, int nsplit) {
+  return max(kSplitTokens, ((count + nsplit - 1) / nsplit + kPaWarps * 32 - 1) / (kPaWarps * 32) * (kPaWarps * 32));
+}
 
 __device__ __forceinline__ void pa_ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -142,9 +146,10 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
   const int group = heads / kv_heads;
   const int ctx = context_lens[b];
   const PaVisible vis = RULE ? pa_visible(ctx, rule) : PaVisible{0, 0, ctx};
-  const int t_begin = sp * kSplitTokens;
+  const int slice = pa_slice(vis.count, nsplit);
+  const int t_begin = sp * slice;
   if (t_begin >= vis.count) return;
-  const int t_end = min(vis.count, t_begin + kSplitTokens);
+  const int t_end = min(vis.count, t_begin + slice);
   const int h_base = hk * group + g0;        // first query head of this pass
   const uint32_t kt_u32 = smem_u32(reinterpret_cast<__nv_bfloat16*>(big) + warp * (kKTile + kVTile));
   const uint32_t vt_u32 = kt_u32 + kKTile * 2;
@@ -380,7 +385,8 @@ paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restri
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   if (d >= dv) return;
   const int ctx = context_lens[b];
-  const int n = min(nsplit, (pa_visible(ctx, rule).count + kSplitTokens - 1) / kSplitTokens);
+  const int count = pa_visible(ctx, rule).count, slice = pa_slice(count, nsplit);
+  const int n = (count + slice - 1) / slice;
   const float* base = partial + (static_cast<long long>(b) * heads + h) * nsplit * (dv + 2);
   float mx = -INFINITY;
   for (int s = 0; s < n; ++s) mx = fmaxf(mx, base[s * (dv + 2)]);
@@ -537,7 +543,12 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
   long long span = static_cast<long long>(a.max_blocks) * a.block_size;      // most keys a row can see
   if (a.chunk > 0 && a.chunk < span) span = a.chunk;
   if (a.window > 0 && static_cast<long long>(a.window) + a.keep_first < span) span = a.window + a.keep_first;
-  const int nsplit = static_cast<int>((span + rb::kSplitTokens - 1) / rb::kSplitTokens);
+  // About four CTAs for each of the 148 x 3 that fit at a time.  The tables are as wide as the model's context, so slices of 256 tokens for
+  // all of it were mostly CTAs without a token, each of which still takes its turn: 64 sequences of 100 to 4000 tokens in tables for
+  // 16384, 4 KV heads of 128: 74.5 us as 16384 CTAs, 64.9 us (4.1 TB/s) with 7 slices of each sequence, merges included.
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads, most = (span + rb::kSplitTokens - 1) / rb::kSplitTokens;
+  const long long wanted = (148 * 3 * 4 + pairs - 1) / pairs;
+  const int nsplit = static_cast<int>(wanted < most ? wanted : most);
   // dynamic shared memory: per warp a K and a V tile of 32 padded rows, plus the 16 padded query rows
   const int smem = (rb::kPaWarps * 32 * (DK + 8 + DV + 8) + rb::kMaxGroup * (DK + 8)) * 2;
   auto kern = rb::paged_decode_split_kernel<DK, DV, RULE>;
