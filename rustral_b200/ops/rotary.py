@@ -43,6 +43,27 @@ def rope_(x2: torch.Tensor, heads: int, head_dim: int, seq_len: int = 0, positio
     return x2
 
 
+N.optional_sig("rb_rope_append", [N.c_void_p, N.c_ll, N.c_void_p, N.c_ll, N.c_int, N.c_int, N.c_int, N.c_float, N.c_void_p, N.c_void_p,
+                                  N.c_void_p, N.c_ll, N.c_void_p])
+
+
+def rope_append_(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, positions, theta: float, k_cache, v_cache, slots) -> torch.Tensor:
+    """Rotates the query and key heads of qkv [tokens, (heads + 2 kv_heads) * head_dim] in place and stores keys and values in their cache
+    slots (int64, negative: not stored): `rope_` and `paged.kv_append` in one launch."""
+    nb, bs, hk, d = k_cache.shape
+    if not qkv.is_cuda:
+        from . import paged
+        rope_(qkv, heads + kv_heads, head_dim, positions=positions, theta=theta)
+        paged.kv_append(qkv[:, heads * head_dim:(heads + kv_heads) * head_dim], qkv[:, (heads + kv_heads) * head_dim:], k_cache, v_cache, slots)
+        return qkv
+    if qkv.dtype != torch.bfloat16 or qkv.stride(1) != 1 or (hk, d) != (kv_heads, head_dim) or v_cache.shape != k_cache.shape:
+        raise TypeError("rope_append: bf16 rows with a contiguous last dimension and a cache of the same heads are required")
+    N.check(N.kernels().rb_rope_append(qkv.data_ptr(), qkv.stride(0), positions.to(torch.int64).contiguous().data_ptr(), qkv.shape[0], heads, kv_heads,
+                                       head_dim, theta, k_cache.data_ptr(), v_cache.data_ptr(), slots.data_ptr(), nb * bs, N.stream_ptr()),
+            "rb_rope_append")
+    return qkv
+
+
 N.optional_sig("rb_rotary_table", [N.c_void_p, N.c_void_p, N.c_float, N.c_void_p, N.c_ll, N.c_int, N.c_void_p])
 N.optional_sig("rb_rotate_pairs", [N.c_void_p, N.c_ll, N.c_void_p, N.c_ll, N.c_int, N.c_ll, N.c_int, N.c_int, N.c_void_p])
 

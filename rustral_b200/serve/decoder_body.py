@@ -72,10 +72,11 @@ class GPTBody:
         p = f"layers.{l}."
         h = self._norm(x, p + "ln1")
         qkv = _product(h, P.w(p + "attn.wqkv.weight"), bias=None if rms else P.w(p + "attn.wqkv.bias"))
-        if rms:
-            rope_ops.rope_(qkv, H + Hk, D, positions=sb.pos, theta=self.cfg.rope_theta)
         k2, v2 = qkv[:, H * D:(H + Hk) * D], qkv[:, (H + Hk) * D:]
-        paged_ops.kv_append(k2, v2, r.cache.k[l], r.cache.v[l], sb.slots)
+        if rms:
+            rope_ops.rope_append_(qkv, H, Hk, D, sb.pos, self.cfg.rope_theta, r.cache.k[l], r.cache.v[l], sb.slots)
+        else:
+            paged_ops.kv_append(k2, v2, r.cache.k[l], r.cache.v[l], sb.slots)
         a = r.attend(l, qkv[:, :H * D], k2, v2, sb, self.scale)
         x = self._row_parallel(a, P.w(p + "attn.wo.weight"), None if rms else P.w(p + "attn.wo.bias"), x)
         h = self._norm(x, p + "ln2")

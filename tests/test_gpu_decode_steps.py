@@ -1,10 +1,37 @@
-"""Decoding kernels at the edges of their work splits: slices of the cached tokens."""
+"""Decoding kernels at the edges of their work splits: rotation with append, slices of the cached tokens."""
 import pytest
 import torch
 
 from rustral_b200.ops import paged
+from rustral_b200.ops import rotary
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,heads,kv,dim", [(1, 4, 1, 64), (7, 6, 2, 80), (33, 16, 4, 128), (9000, 30, 5, 64)])
+def test_rope_append_is_rope_and_append(tokens, heads, kv, dim, cuda_status):
+    """One head per thread and four (the last case, with a count of heads that four does not divide); skipped tokens; wide rows."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    cols = (heads + 2 * kv) * dim
+    qkv = torch.randn(tokens, cols + 8, device="cuda", generator=g).bfloat16()[:, :cols]
+    other = qkv.clone()
+    pos = torch.randint(0, 20000, (tokens,), device="cuda", generator=g)
+    slots = torch.randperm(tokens + 32, device="cuda", generator=g)[:tokens]
+    slots[::5] = -1
+    kc, vc = (torch.zeros((tokens + 47) // 16, 16, kv, dim, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    kc2, vc2 = kc.clone(), vc.clone()
+    rotary.rope_append_(qkv, heads, kv, dim, pos, 10000.0, kc, vc, slots)
+    rotary.rope_(other, heads + kv, dim, positions=pos, theta=10000.0)
+    paged.kv_append(other[:, heads * dim:(heads + kv) * dim], other[:, (heads + kv) * dim:], kc2, vc2, slots)
+    assert torch.equal(qkv, other) and torch.equal(kc, kc2) and torch.equal(vc, vc2)
+    # against 64 bits: bf16 result, fp32 angles up to 20000 (2^-24 of them)
+    x = torch.randn(tokens, heads * dim, device="cuda", generator=g).bfloat16()
+    freq = 10000.0 ** (-torch.arange(dim // 2, device="cuda").double() * 2 / dim)
+    a = pos.double()[:, None] * freq
+    u, v = x.double().view(tokens, heads, dim).split(dim // 2, -1)
+    want = torch.cat([u * a.cos()[:, None] - v * a.sin()[:, None], v * a.cos()[:, None] + u * a.sin()[:, None]], -1)
+    got = rotary.rope_(x.clone(), heads, dim, positions=pos, theta=10000.0).view(tokens, heads, dim).double()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 20000 * 2.0 ** -22 * (u.abs() + v.abs()).repeat(1, 1, 2)).all()
 
 
 @pytest.mark.parametrize("batch,heads,kv,dim,longest,width", [(1, 8, 2, 128, 2500, 400), (64, 8, 4, 128, 1300, 1024), (120, 32, 16, 64, 700, 64),
