@@ -76,6 +76,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
+  // swiglu: a tile is 64 gate rows and the 64 up rows of the same columns
+  const bool glu = ep.act == RB_ACT_SWIGLU;
+  const int tile_n = glu ? kRowsTile / 2 : kRowsTile;
   const int num_kb = (K + 63) / 64;
   const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * part / parts);
   const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (part + 1) / parts);
@@ -83,10 +86,15 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   if (warp == 0) {
     if (elect_one()) {
       // W of the first stages is on its way before the kernel in front has ended, X follows when it has
+      auto load_w = [&](int it, int s) {
+        const uint32_t dst = base + s * stage_bytes;
+        tma_load_2d(dst, &tmW, (kb0 + it) * 64, tile * tile_n, bar_full + 8 * s);
+        if (glu) tma_load_2d(dst + kRowsWBytes / 2, &tmW, (kb0 + it) * 64, N + tile * tile_n, bar_full + 8 * s);
+      };
       const int ahead = w_constant ? min(stages, kb1 - kb0) : 0;
       for (int it = 0; it < ahead; ++it) {
         mbar_arrive_expect_tx(bar_full + 8 * it, stage_bytes);
-        tma_load_2d(base + it * stage_bytes, &tmW, (kb0 + it) * 64, tile * kRowsTile, bar_full + 8 * it);
+        load_w(it, it);
       }
       pdl_wait();
       for (int it = 0; it < kb1 - kb0; ++it) {
@@ -94,7 +102,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (it >= ahead) {
           if (!mbar_wait(bar_empty + 8 * s, ((it / stages) & 1) ^ 1, abort_flag, status, 81)) break;
           mbar_arrive_expect_tx(bar_full + 8 * s, stage_bytes);
-          tma_load_2d(base + s * stage_bytes, &tmW, (kb0 + it) * 64, tile * kRowsTile, bar_full + 8 * s);
+          load_w(it, s);
         }
         tma_load_2d(base + s * stage_bytes + kRowsWBytes, &tmX, (kb0 + it) * 64, 0, bar_full + 8 * s);
       }
@@ -141,19 +149,23 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   // ---- results: four neighbouring columns per item, items dealt to the CTAs of the cluster
   if (!*abort_flag) {
-    for (int i = part * kRowsThreads + threadIdx.x; i < M * (kRowsTile / 4); i += parts * kRowsThreads) {
-      const int m = i >> 5, n = (i & 31) * 4, col = tile * kRowsTile + n;
+    const int per_row = tile_n / 4;
+    for (int i = part * kRowsThreads + threadIdx.x; i < M * per_row; i += parts * kRowsThreads) {
+      const int m = i / per_row, n = (i - m * per_row) * 4, col = tile * tile_n + n;
       if (col >= N) continue;
-      const uint32_t off = base + (m * kRowsTile + n) * 4;
-      float4 a;
-      if (parts > 1) {
-        a = ld_cluster_f4(mapa_shared(off, 0));
+      auto sum = [&](int at) {
+        if (parts == 1) return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem) + at);
+        float4 a = ld_cluster_f4(mapa_shared(base + at * 4, 0));
         for (int s = 1; s < parts; ++s) {
-          const float4 b = ld_cluster_f4(mapa_shared(off, s));
+          const float4 b = ld_cluster_f4(mapa_shared(base + at * 4, s));
           a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
-      } else {
-        a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem) + m * kRowsTile + n);
+        return a;
+      };
+      float4 a = sum(m * kRowsTile + n);
+      if (glu) {
+        const float4 b = sum(m * kRowsTile + tile_n + n);
+        a.x = silu(a.x) * b.x; a.y = silu(a.y) * b.y; a.z = silu(a.z) * b.z; a.w = silu(a.w) * b.w;
       }
       float v[4] = {a.x * ep.alpha, a.y * ep.alpha, a.z * ep.alpha, a.w * ep.alpha};
       const bool full = col + 4 <= N;
@@ -162,7 +174,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         for (int j = 0; j < 4; ++j)
           if (full || col + j < N) v[j] += __bfloat162float(__ldg(ep.bias + col + j));
       }
-      if (ep.act != RB_ACT_NONE) {
+      if (ep.act != RB_ACT_NONE && !glu) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = rows_act(ep.act, v[j]);
       }
@@ -209,14 +221,16 @@ namespace rbhost {
 // cross (2048 x 8192 16.3 / 17.1).  From 49 rows on a short contraction under many tiles is all results and little reading: 50304 x 768
 // with 64 rows 20.8 / 24.8, with 24 rows 21.5 / 20.0.
 bool gemm_rows_takes(const RbGemmArgs& g) {
-  if (g.M > 96 || (g.M > 48 && g.K < 1024 && g.N > 148 * rb::kRowsTile)) return false;
+  if (g.M > 96 || (g.M > 48 && g.K < 1024 && g.N > 148 * rb::kRowsTile / (g.act == RB_ACT_SWIGLU ? 2 : 1))) return false;
   return !g.a_mn_major && !g.b_mn_major && !g.accumulate && !g.aux_out && !g.aux_in && g.group_mode == 0 && g.peer_mode == 0 && !g.ab_fp8 &&
          !g.a_scale && !g.b_scale && g.block_n == 0 && g.group_m == 0 && g.max_ctas == 0 && g.splits <= 1;
 }
 
 int gemm_rows(const RbGemmArgs& g, cudaStream_t stream) {
   const int mpad = (g.M + 15) / 16 * 16;
-  const int tiles = (g.N + rb::kRowsTile - 1) / rb::kRowsTile, num_kb = (g.K + 63) / 64;
+  const bool glu = g.act == RB_ACT_SWIGLU;
+  const int tile_n = glu ? rb::kRowsTile / 2 : rb::kRowsTile;
+  const int tiles = (g.N + tile_n - 1) / tile_n, num_kb = (g.K + 63) / 64;
   // About 100 CTAs or more read at the memory's rate; each further part of K costs another CTA's partial sums.  One row, us per product
   // in a captured chain with 1 / 2 / 4 / 8 parts: 768 x 768 5.7 / 4.6 / 4.0 / 3.9, 2048 x 8192 36.9 / 20.6 / 12.5 / 9.6, 16384 x 2048
   // 14.1 / 14.2 / 17.9 / 25.0.
@@ -227,7 +241,7 @@ int gemm_rows(const RbGemmArgs& g, cudaStream_t stream) {
   const int stage_bytes = rb::kRowsWBytes + mpad * 128;
   const int stages = (111 * 1024) / stage_bytes < 6 ? (111 * 1024) / stage_bytes : 6;
   int err = 0;
-  const CUtensorMap* tw = get_tmap_2d(g.b, 2, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb, 64, rb::kRowsTile, 1, &err);
+  const CUtensorMap* tw = get_tmap_2d(g.b, 2, (uint64_t)g.K, (uint64_t)g.N * (glu ? 2 : 1), (uint64_t)g.ldb, 64, (uint32_t)tile_n, 1, &err);
   if (!tw) return err ? err : -5;
   const CUtensorMap* tx = get_tmap_2d(g.a, 2, (uint64_t)g.K, (uint64_t)g.M, (uint64_t)g.lda, 64, (uint32_t)mpad, 1, &err);
   if (!tx) return err ? err : -5;

@@ -14,7 +14,9 @@ enum RbAct {
   RB_ACT_DRELU = 5,   // zero the result where aux_in <= 0
   RB_ACT_DSILU = 6,   // multiply the result by silu'(aux_in)
   RB_ACT_MUL = 7,     // multiply the result by aux_in
-  RB_ACT_RELU2 = 8    // the square of relu (inference: no pre-activation is kept)
+  RB_ACT_RELU2 = 8,   // the square of relu (inference: no pre-activation is kept)
+  RB_ACT_SWIGLU = 9   // B holds 2 N rows, gates over ups: d = silu(A gate^T) * (A up^T).  K-major bf16 operands and result, no other
+                      // epilogue, at most 96 or more than 128 rows; what is not taken is refused with -9
 };
 
 typedef struct RbGemmArgs {

@@ -194,3 +194,24 @@ class _SwigluFn(torch.autograd.Function):
 def swiglu(gu):
     """``silu(gate) * up`` for ``gu = [gate | up]`` along the last dimension."""
     return _SwigluFn.apply(gu)
+
+
+def swiglu_product(a: torch.Tensor, w: torch.Tensor, b_constant: bool = False) -> torch.Tensor:
+    """silu(a @ gate^T) * (a @ up^T) for w = [gate; up] ([2 F, K]), for inference: one launch where the product kernels take it (bf16,
+    aligned rows, up to 96 or more than 128 of them), else product and `swiglu_forward`.  The fused form does not round the two products."""
+    from . import matmul
+    M, K = a.shape
+    F = w.shape[0] // 2
+    if a.is_cuda and a.dtype == w.dtype == torch.bfloat16 and M and F % 8 == 0 and K == w.shape[1] and a.stride(1) == 1 and w.stride(1) == 1 and \
+            not (a.stride(0) | w.stride(0) | K) & 7 and not (a.data_ptr() | w.data_ptr()) & 15:
+        out = torch.empty((M, F), dtype=a.dtype, device=a.device)
+        g = N.RbGemmArgs()
+        g.a, g.b, g.d = a.data_ptr(), w.data_ptr(), out.data_ptr()
+        g.lda, g.ldb, g.ldd = a.stride(0), w.stride(0), F
+        g.M, g.N, g.K = M, F, K
+        g.act, g.alpha, g.b_constant = 9, 1.0, int(b_constant)              # RB_ACT_SWIGLU
+        rc = N.kernels().rb_gemm_bf16(g, N.stream_ptr())
+        if rc != -9:
+            N.check(rc, "rb_gemm_bf16[swiglu]")
+            return out
+    return swiglu_forward(matmul.gemm(a, w, b_constant=b_constant))

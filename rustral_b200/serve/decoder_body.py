@@ -81,8 +81,7 @@ class GPTBody:
         x = self._row_parallel(a, P.w(p + "attn.wo.weight"), None if rms else P.w(p + "attn.wo.bias"), x)
         h = self._norm(x, p + "ln2")
         if rms:
-            gu = _product(h, P.w(p + "ffn.gate_up.weight"))
-            return self._row_parallel(rope_ops.swiglu_forward(gu), P.w(p + "ffn.down.weight"), None, x)
+            return self._row_parallel(rope_ops.swiglu_product(h, P.w(p + "ffn.gate_up.weight"), b_constant=True), P.w(p + "ffn.down.weight"), None, x)
         h = _product(h, P.w(p + "ffn.fc1.weight"), bias=P.w(p + "ffn.fc1.bias"), act="gelu")
         return _product(h, P.w(p + "ffn.fc2.weight"), bias=P.w(p + "ffn.fc2.bias"), residual=x)
 

@@ -58,3 +58,20 @@ def test_residual_in_place_and_graph_replay(cuda_status):
     r.copy_(r0)
     graph.replay()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [1, 17, 96, 97, 129, 300, 513])
+@pytest.mark.parametrize("F,K", [(8, 64), (64, 72), (72, 768), (200, 2048), (1000, 264)])
+def test_swiglu_product(M, F, K, cuda_status):
+    """Gates and ups of one result column come from two places of the weight: edges of 64- and 128-column tiles, rows of both kernels and of
+    neither, and a weight whose rows behind the gates are the ups (a tile that ends in the middle reads into them)."""
+    from rustral_b200.ops.rotary import swiglu_product
+    x, w, _, _ = _operands(M, 2 * F, K)
+    w = (w.float() * K ** -0.5).bfloat16()
+    g, u = (x.double() @ w.double().T).split(F, -1)
+    want = torch.nn.functional.silu(g) * u
+    got = swiglu_product(x, w)
+    # bf16 result (2^-8); where the two products are rounded first: 2^-8 of each, the gate's through silu's slope (at most 1.1)
+    bound = 2.0 ** -7 * want.abs() + 2.0 ** -7 * 1.1 * (g * u).abs() + 1e-5
+    assert ((got.double() - want).abs() <= bound).all()
+    assert torch.equal(got, swiglu_product(x, w, b_constant=True))
