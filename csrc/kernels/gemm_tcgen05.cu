@@ -1444,13 +1444,18 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
 // memory more often per MMA (measured on B200: 128-wide runs ~1.3x, 64-wide ~2.3x slower than 256-wide).
 int width_cost(int bn) { return bn == 256 ? 100 : bn == 192 ? 104 : bn == 128 ? 132 : 235; }
 
-long long plan_cost(int M, int N, int bn, int splits, int sms, bool pair_ok) {
+// Microseconds of a plan: waves of tiles at the measured rate (6.5 ns per unit of K for a 128 x 256 tile), the last tile's results, and
+// for a split contraction a second launch and the slabs' way through memory.  Leaving the slabs out of the sum had wide results split
+// that should not be (measured, split / whole): 2048 x 8192 x 4096 135 / 101 us, 4096 x 2048 x 8192 131 / 98, 2704 x 2048 x 2048 42 / 25.
+double plan_cost(int M, int N, int K, int bn, int splits, int sms, bool pair_ok) {
   const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn) * splits;
   const long long waves = (tiles + sms - 1) / sms;
   // 256-wide plans of plain problems run on the two-CTA kernel, measured about 10 % faster per tile
   const int wc = (bn == 256 && pair_ok) ? 88 : width_cost(bn);
-  // per-unit time ~ bn * K/splits (+ a fixed prologue/epilogue share that split-K multiplies)
-  return waves * bn * wc * (1000 / splits + 40);
+  const double width = bn / 256.0;
+  double us = waves * width * (wc / 100.0) * (static_cast<double>(K) / splits) * 0.0065 + 1.5 * width;
+  if (splits > 1) us += 2.0 + (2.0 * splits + 1.0) * M * static_cast<double>(N) * 4.0 / 5.0e6;
+  return us;
 }
 
 void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
@@ -1460,7 +1465,7 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
                          !g.a_scale && !g.b_scale && !g.ab_fp8 &&
                          (g.N % 4 == 0) && (static_cast<long long>(g.M) * g.N % 4 == 0) && (!g.residual || (g.ldr % 4 == 0));
   const bool pair_ok = g.peer_mode == 0 && g.group_mode == 0 && g.M > 128 && g.max_ctas == 0 && pair_kernel_enabled();
-  long long best = -1;
+  double best = -1.0;
   bn_out = 128; splits_out = 1;
   for (int c = 0; c < 4; ++c) {
     const int bn = cands[c];
@@ -1471,11 +1476,11 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
       if (g.splits > 0 && sp != g.splits) continue;
       if (sp > 1) {
         if (!can_split) continue;
-        if (g.splits <= 0 && g.K / sp < 1024) continue;
+        if (g.splits <= 0 && g.K / sp < 768) continue;
         if (static_cast<long long>(sp) * g.M * g.N * 4 > g.workspace_bytes) continue;
       }
-      const long long cost = plan_cost(g.M, g.N, bn, sp, sms, pair_ok);
-      if (best < 0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
+      const double cost = plan_cost(g.M, g.N, g.K, bn, sp, sms, pair_ok);
+      if (best < 0.0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
     }
   }
 }
