@@ -1292,7 +1292,7 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
     ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
     ep.bias = nullptr; ep.residual = nullptr;          // applied once, by the kernel that folds the slabs
   }
-  if (L::kTotalStaged + 1024 > 232448) return L::kTotal + 1024;
+  static_assert(L::kTotalStaged + 1024 <= 232448, "the ring and the result tiles share an SM's memory");
   const bool tma = L::kTma && g.peer_mode == 0 && tma_store_default() && staged_store_default();
   // slabs of a split contraction and the experts' results (grouped mode 2) lie below one another: whole 32-row tiles keep each in its own
   const bool stacked = g.M % 32 == 0 && (splits > 1 || (tma && g.d_expert_stride == static_cast<long long>(g.M) * g.ldd));
@@ -1525,7 +1525,7 @@ int gemm_fp8(const RbGemmArgs& g, int sms, int bn, int splits, cudaStream_t stre
   switch (bn) {
     case 256: return launch<0, 0, 256, 4, 1>(g, ta, tb, grid, splits, stream);
     case 192: return launch<0, 0, 192, 5, 1>(g, ta, tb, grid, splits, stream);
-    case 128: return launch<0, 0, 128, 6, 1>(g, ta, tb, grid, splits, stream);
+    case 128: return launch<0, 0, 128, 5, 1>(g, ta, tb, grid, splits, stream);
     default: return launch<0, 0, 64, 8, 1>(g, ta, tb, grid, splits, stream);
   }
 }
@@ -1621,7 +1621,7 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
   switch (bn) {
     case 256: return dispatch_major<256, 4>(g, ta, tb, grid, splits, stream);
     case 192: return dispatch_major<192, 5>(g, ta, tb, grid, splits, stream);
-    case 128: return dispatch_major<128, 6>(g, ta, tb, grid, splits, stream);
+    case 128: return dispatch_major<128, 5>(g, ta, tb, grid, splits, stream);
     default: return dispatch_major<64, 8>(g, ta, tb, grid, splits, stream);
   }
 }
