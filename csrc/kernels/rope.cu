@@ -210,8 +210,8 @@ void rope_launch(__nv_bfloat16* x, long long ld, const long long* positions, lon
   const int len = seq_len < 1 ? 1 : seq_len;
   const long long copies = cache.slots ? cache.kv_heads * head_dim / 8 : 0, groups = head_dim / 16;
   // Four heads per thread where that still leaves a thread for every lane of the GPU: 40 heads of 128, rotation and append of 8192 tokens
-  // 65.0 us with one head per thread in two launches, 53.3 in one with four (64 tokens, one head per thread: 5.2 and 3.3).  32-bit divisions
-  // where the counts allow.
+  // 65.0 us with one head per thread, 47.0 with four (64 tokens, one head per thread, one launch: 3.3 instead of 4.6).  32-bit divisions where the
+  // counts allow.
   const bool wide = tokens * ((heads + 3) / 4 * groups + copies) >= 148 * 2048;
   const long long total = tokens * ((wide ? (heads + 3) / 4 : heads) * groups + copies);
   auto kern = total >= (1ll << 31) ? rb::rope_kernel<4, unsigned long long>

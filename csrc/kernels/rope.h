@@ -9,6 +9,10 @@ extern "C" {
 // transposed rotation, which is the backward pass.
 int rb_rope(void* x, long long ld, const long long* positions, long long tokens, int heads, int head_dim, int seq_len,
             long long pos_offset, float theta, int inverse, void* stream);
+// Rotates the first heads + kv_heads heads of rows [heads | kv_heads keys | kv_heads values] in place and stores keys and values in the
+// cache slots (int64; negative: not stored).
+int rb_rope_append(void* x, long long ld, const long long* positions, long long tokens, int heads, int kv_heads, int head_dim,
+                   float theta, void* k_cache, void* v_cache, const long long* slots, long long num_slots, void* stream);
 // out[t, i] = magnitude * (cos, sin)(positions[t] * freqs[i]): fp32 [rows, pairs, 2], the table of the pairwise rotations below and in
 // head_prep.h, latent_attention.h
 int rb_rotary_table(const long long* positions, const double* freqs, float magnitude, float* out, long long rows, int pairs,
