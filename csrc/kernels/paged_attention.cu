@@ -543,11 +543,12 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
   long long span = static_cast<long long>(a.max_blocks) * a.block_size;      // most keys a row can see
   if (a.chunk > 0 && a.chunk < span) span = a.chunk;
   if (a.window > 0 && static_cast<long long>(a.window) + a.keep_first < span) span = a.window + a.keep_first;
-  // About four CTAs for each of the 148 x 3 that fit at a time.  The tables are as wide as the model's context, so slices of 256 tokens for
-  // all of it were mostly CTAs without a token, each of which still takes its turn: 64 sequences of 100 to 4000 tokens in tables for
-  // 16384, 4 KV heads of 128: 74.5 us as 16384 CTAs, 64.9 us (4.1 TB/s) with 7 slices of each sequence, merges included.
+  // About three CTAs for each of the 148 x 3 that fit at a time.  The tables are as wide as the model's context, so slices of 256 tokens for
+  // all of it were mostly CTAs without a token, each of which still takes its turn.  64 sequences of 100 to 4000 tokens in tables for 16384, 4
+  // KV heads of 128: 74.5 us as 16384 CTAs, 64.4 us (4.2 TB/s) with 6 slices of each sequence, merges included; 24 of 128 to 2560, 8 KV heads:
+  // 43.5 and 39.0 (two, four, six CTAs for each: 64.8, 64.6, 69.4 and 40.8, 44.5, 44.2).
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads, most = (span + rb::kSplitTokens - 1) / rb::kSplitTokens;
-  const long long wanted = (148 * 3 * 4 + pairs - 1) / pairs;
+  const long long wanted = (148 * 3 * 3 + pairs - 1) / pairs;
   const int nsplit = static_cast<int>(wanted < most ? wanted : most);
   // dynamic shared memory: per warp a K and a V tile of 32 padded rows, plus the 16 padded query rows
   const int smem = (rb::kPaWarps * 32 * (DK + 8 + DV + 8) + rb::kMaxGroup * (DK + 8)) * 2;
