@@ -336,7 +336,8 @@ __device__ __forceinline__ void stage_put(uint32_t addr, uint32_t a, uint32_t b,
 
 // Epilogue of one warp through tiles of 32 rows x 128 bytes in shared memory that TMA moves: bf16 in 64-column blocks (staged 2), fp32 in
 // 32-column blocks (3; 4 adds to d: every element is added to by one warp once, so the sum does not depend on any order).  With two tiles
-// per warp (SLOTS) one is filled while the other is stored.  With `side`, TMA has loaded the residual or aux_in into the tiles (`epilogue_side_load`,
+// per warp (SLOTS) one is filled while the other is stored: blocks take them in turn, on into the next output tile (`t` counts those).
+// With `side`, TMA has loaded the residual or aux_in into the tiles (`epilogue_side_load`,
 // issued before the accumulator is waited for); results replace it in place.  Reading those through the SM's own loads instead, each
 // lane 64 bytes of its row, cost more than the products at K = 768: 32768 x 3072 with gelu'(aux_in) 292 us, residual 32768 x 768 61 us.
 // `arrive` hands the accumulator back; `row0` is the warp's first row, `col` the first of its COLS columns.
@@ -463,7 +464,7 @@ __device__ __forceinline__ void tile_act(const EpiParams& ep, const uint32_t (&s
 
 template <int COLS, int SLOTS, class Arrive>
 __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensorMap* tmD, const CUtensorMap* tmAux, uint32_t stg,
-                                             uint32_t bar_side, uint32_t side_parity, uint32_t taddr, int row0, int drow, int col, int M, int N,
+                                             uint32_t bar_side, uint32_t t, uint32_t taddr, int row0, int drow, int col, int M, int N,
                                              int lane, bool empty_k, volatile int* abort_flag, unsigned int* status, Arrive arrive) {
   // rows behind the matrix are computed like the others (on what the accumulator holds for them) and clipped by the stores
   const long long row = min(row0 + lane, M - 1);
@@ -473,12 +474,13 @@ __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensor
   for (int c = 0; c < COLS; c += 32) {
     // 32 columns at a time; `half`: which part of a 64-column tile they are
     const int block = c / cols, half = (c & (cols - 1)) >> 5;
-    const uint32_t slot = stg + (two ? 0 : block % SLOTS) * 4096;
+    // The wait below leaves the newest store in flight, so no two blocks in a row may share a tile; a side tile lies where it was loaded to.
+    const uint32_t slot = stg + (two ? 0 : (block + (ep.side != 0 ? 0 : t * (COLS / cols))) % SLOTS) * 4096;
     uint32_t r[32];
     tmem_ld_32x32(taddr + c, r);
     uint32_t side[16];
     if (ep.side != 0) {
-      if (half == 0 && !mbar_wait(bar_side + 8 * block, side_parity, abort_flag, status, 7)) return;
+      if (half == 0 && !mbar_wait(bar_side + 8 * block, t & 1, abort_flag, status, 7)) return;
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(side[4 * q]), "=r"(side[4 * q + 1]), "=r"(side[4 * q + 2]),
@@ -854,7 +856,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
       };
       if (L::kTma && ep.staged >= 2) {
-        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t & 1, taddr + cgrp * (BLOCK_N / 2), row0,
+        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0,
                                   num_splits > 1 || grp.mode == 2 ? outer * M + row0 : row0, colg, M, N, lane, empty_k, abort_flag, status, arrive);
         continue;
       }
@@ -1164,7 +1166,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         continue;
       }
       if (ep.staged >= 2) {
-        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t & 1, taddr + cgrp * (BLOCK_N / 2), row0,
+        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0,
                                   num_splits > 1 ? split * M + row0 : row0, colg, M, N, lane, false, abort_flag, status, arrive);
         continue;
       }
