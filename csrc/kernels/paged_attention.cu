@@ -1,8 +1,8 @@
 // Paged KV cache: append and single-token (decode) attention through a block table (page size 16 by default).
 //
 // Decode attention is bandwidth-bound (every cached key and value is read once per step), so the kernel is built
-// around memory access and parallelism: one CTA per (sequence, KV head, 256-token slice of the context) serves all
-// query heads of that group (split-KV, so a batch of 32 sequences still fills 148 SMs); K and V rows are fetched
+// around memory access and parallelism: a CTA takes slices of 256 tokens of a sequence's context for all query heads
+// of a KV head's group (split-KV, so that few sequences still fill 148 SMs); K and V rows are fetched
 // coalesced into a padded shared tile, the group's heads are the rows of mma.sync tensor-core tiles for both
 // Q K^T and P V, and a second kernel merges the slices' (max, sum, output) triples.
 //
@@ -39,10 +39,12 @@ kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, long long ld_k, const 
 
 constexpr int kMaxGroup = 16;    // query heads per KV head served by one CTA pass (the M of the mma tile)
 constexpr int kPaWarps = 4;
-constexpr int kSplitTokens = 256;          // least tokens of a slice (split-KV): 2 passes of 32 tokens per warp
-// Tokens per slice of a sequence with `count` visible tokens when a launch has room for `nsplit` slices of each sequence.
-__device__ __forceinline__ int pa_slice(int count, int nsplit) {
-  return max(kSplitTokens, ((count + nsplit - 1) / nsplit + kPaWarps * 32 - 1) / (kPaWarps * 32) * (kPaWarps * 32));
+// Cached tokens per slice (split-KV): 2 passes of 32 tokens per warp.  A sequence is cut into slices by its own length alone, so that its
+// result has the same bits alone and beside any others.
+constexpr int kSplitTokens = 256;
+// Slices of a sequence with `count` visible tokens; at most `nsplit` have room in the scratch memory.
+__device__ __forceinline__ int pa_slices(int count, int nsplit) {
+  return max(0, min(nsplit, (count + kSplitTokens - 1) / kSplitTokens));
 }
 
 __device__ __forceinline__ void pa_ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -61,6 +63,9 @@ __device__ __forceinline__ void pa_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // 16-byte asynchronous global -> shared copy; bytes == 0 writes zeros and reads nothing
 __device__ __forceinline__ void pa_cp_async16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void pa_cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void pa_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -122,11 +127,16 @@ __device__ __forceinline__ float pa_gate(const PaRule& r, long long row, int hea
   return r.head_gate ? pa_sigmoid(r.head_gate[row * r.ld_g + head]) : 1.f;
 }
 
-template <int DK, int DV, bool RULE>
+// LIST: the slices of all sequences, numbered one sequence after the other, are dealt in equal runs to CTAs that stay (grid: CTAs for a KV head,
+// KV heads).  Sequences differ in length by any factor, so a grid over (sequence, slice) is mostly CTAs without a token, each of which still
+// takes its turn (about 1500 in a microsecond), and one with fewer, longer slices leaves the longest sequence to a few CTAs.  From one slice
+// to the next the copies of K go on: the warps' accumulators are merged in the memory of the V tiles.  Without LIST: grid (sequences, KV heads,
+// slices), a slice for each CTA, where that many fit; nothing has to be looked up first.
+template <int DK, int DV, bool RULE, bool LIST>
 __global__ void __launch_bounds__(kPaWarps * 32, 3)
 paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, const __nv_bfloat16* __restrict__ k_cache,
                           const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int max_blocks,
-                          const int* __restrict__ context_lens, int heads, int kv_heads, int dk_real, int dv_real,
+                          const int* __restrict__ context_lens, int batch, int heads, int kv_heads, int dk_real, int dv_real,
                           int block_size, long long num_blocks, float scale, int g0, int gcount, float* __restrict__ partial,
                           int nsplit, __nv_bfloat16* __restrict__ direct_out, long long ld_o, const PaRule rule
                           RB_BOUNDS_PARAM) {
@@ -137,23 +147,59 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
   constexpr int NT = DV / 8;                 // n-tiles of the output accumulator
   constexpr int kKTile = 32 * KROW, kVTile = 32 * VROW;   // one tile of one warp
   const int dk = RULE ? dk_real : DK, dv = RULE ? dv_real : DV;
-  extern __shared__ __align__(16) uint8_t big[];   // [warp][K tile, V tile] bf16, then q_sh; later the warp merge area
+  extern __shared__ __align__(16) uint8_t big[];   // [warp][K tile, V tile] bf16, then q_sh
   __nv_bfloat16* q_sh = reinterpret_cast<__nv_bfloat16*>(big) + kPaWarps * (kKTile + kVTile);
   __shared__ float m_sh[kPaWarps][kMaxGroup], l_sh[kPaWarps][kMaxGroup];
-  const int b = blockIdx.x, hk = blockIdx.y, sp = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;   // fragment coordinates: row (and row + 8), column pair
   const int group = heads / kv_heads;
-  const int ctx = context_lens[b];
-  const PaVisible vis = RULE ? pa_visible(ctx, rule) : PaVisible{0, 0, ctx};
-  const int slice = pa_slice(vis.count, nsplit);
-  const int t_begin = sp * slice;
-  if (t_begin >= vis.count) return;
-  const int t_end = min(vis.count, t_begin + slice);
-  const int h_base = hk * group + g0;        // first query head of this pass
   const uint32_t kt_u32 = smem_u32(reinterpret_cast<__nv_bfloat16*>(big) + warp * (kKTile + kVTile));
   const uint32_t vt_u32 = kt_u32 + kKTile * 2;
   const uint32_t q_u32 = smem_u32(q_sh);
+  float* merge = reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(big) + kKTile);   // [warp][16][VROW] fp32 where V tiles are
+  constexpr int kMergeStride = (kKTile + kVTile) / 2;
+  static_assert(kMaxGroup * VROW * 4 == kVTile * 2, "the warps' accumulators take the place of the V tiles");
+  auto visible = [&](int c) { return RULE ? pa_visible(c, rule) : PaVisible{0, 0, c}; };
+  auto slices_of = [&](int seq) { return pa_slices(visible(context_lens[seq]).count, nsplit); };
+
+  // ---- this CTA's run of slices, and the sequence and slice that it begins with (every warp forms the same numbers)
+  int b = 0, sp = 0, left = 1;
+  if (!LIST) {
+    b = blockIdx.x;
+    sp = blockIdx.z;
+    if (sp >= slices_of(b)) return;
+  } else {
+    int n = lane < batch ? slices_of(lane) : 0, total = n;
+    for (int i = lane + 32; i < batch; i += 32) total += slices_of(i);
+    total = __reduce_add_sync(0xffffffffu, total);
+    // at least two slices per CTA where their copies are what takes the time: 24 sequences of 128 to 2560, 8 KV heads of 128, 38.0 us, with all
+    // CTAs 45.5; for heads of 64 an even split counts more (48 of 16 to 1024, 12 KV heads: 33.2 / 29.1)
+    const int cta = blockIdx.x, most = gridDim.x, ctas = DK + DV >= 256 && total < 2 * most ? (most + 1) / 2 : most;
+    const int share = total / ctas, over = total - share * ctas;
+    left = cta < ctas ? share + (cta < over ? 1 : 0) : 0;
+    if (left == 0) return;
+    sp = cta * share + min(cta, over);
+    for (int first = 0; batch > 1; n = first + lane < batch ? slices_of(first + lane) : 0) {
+      int upto = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const unsigned int behind = __ballot_sync(0xffffffffu, upto > sp);
+      if (behind != 0u) {
+        const int at = __ffs(behind) - 1;
+        b = first + at;
+        sp -= __shfl_sync(0xffffffffu, upto - n, at);
+        break;
+      }
+      sp -= __shfl_sync(0xffffffffu, upto, 31);
+      first += 32;
+    }
+  }
+  const int hk = blockIdx.y;
+  const int h_base = hk * group + g0;        // first query head of this pass
+
   float slope0 = 0.f, slope1 = 0.f, two_over_cap = 0.f;
   float amount0 = 0.f, amount1 = 0.f, rate0 = 0.f, rate1 = 0.f;
   if (RULE) {
@@ -168,31 +214,13 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
     if (rule.softcap > 0.f) two_over_cap = 2.f / rule.softcap;
   }
 
-  // the group's query rows as bf16 [16][D] (rows >= gcount are zero)
-  for (int i = threadIdx.x; i < kMaxGroup * LPK; i += blockDim.x) {
-    const int g = i / LPK, c = (i - g * LPK) * 8;
-    uint4 u = make_uint4(0u, 0u, 0u, 0u);
-    if (g < gcount && c < dk) {
-      const __nv_bfloat16* src = q + static_cast<long long>(b) * ld_q + static_cast<long long>(h_base + g) * dk + c;
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const uint32_t*>(src + 2 * j);   // rows are 4-byte aligned at least
-      u = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    *reinterpret_cast<uint4*>(q_sh + g * KROW + c) = u;
-  }
-  __syncthreads();
-
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // rows gq and gq + 8
-  float acc[NT][4];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-
+  int ctx = 0, t_end = 0, base = 0;
+  PaVisible vis = {0, 0, 0};
   int slot = -1;                             // cache slot of token `first + lane` of the located tile (-1: past the end)
   int n_next = 0;
-  // cache slots of the 32 tokens that start at `first` (the host bounds num_blocks * block_size below 2^31)
-  auto locate = [&](int first) {
-    const int num = first + lane;
+  // cache slots of the 32 tokens from number `from` on (the host bounds num_blocks * block_size below 2^31)
+  auto locate = [&](int from) {
+    const int num = from + lane;
     slot = -1;
     if (num < t_end) {
       const int tok = RULE && num >= vis.kept ? num + vis.gap : num;
@@ -204,175 +232,244 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       }
       slot = blk * block_size + (tok - blk_idx * block_size);
     }
-    n_next = min(32, t_end - first);
+    n_next = min(32, t_end - from);
   };
-  // one tile = one asynchronous 16-byte copy per lane and piece, one commit group; rows past the context and columns past
-  // the real head size are zero-filled
+  // takes up slice sp of sequence b
+  auto enter = [&]() {
+    ctx = context_lens[b];
+    vis = visible(ctx);
+    t_end = min(vis.count, (sp + 1) * kSplitTokens);
+    base = sp * kSplitTokens + warp * 32;
+    locate(base);
+  };
+  // one tile = one asynchronous 16-byte copy per lane and piece, one commit group (empty for a warp without tokens in the slice); rows past
+  // the context and columns past the real head size are zero-filled
   auto request = [&](const __nv_bfloat16* cache, uint32_t tile_u32, auto pieces, int dim) {
     constexpr int LP = decltype(pieces)::value;
+    if (n_next > 0) {
 #pragma unroll
-    for (int i = 0; i < LP; ++i) {
-      const int idx = i * 32 + lane;
-      const int r = idx / LP, c = (idx - r * LP) * 8;
-      const int s_r = __shfl_sync(0xffffffffu, slot, r);
-      const bool ok = s_r >= 0 && c < dim;
-      pa_cp_async16(tile_u32 + (r * (LP * 8 + 8) + c) * 2,
-                    ok ? cache + (static_cast<long long>(s_r) * kv_heads + hk) * dim + c : cache, ok ? 16 : 0);
+      for (int i = 0; i < LP; ++i) {
+        const int idx = i * 32 + lane;
+        const int r = idx / LP, c = (idx - r * LP) * 8;
+        const int s_r = __shfl_sync(0xffffffffu, slot, r);
+        const bool ok = s_r >= 0 && c < dim;
+        pa_cp_async16(tile_u32 + (r * (LP * 8 + 8) + c) * 2,
+                      ok ? cache + (static_cast<long long>(s_r) * kv_heads + hk) * dim + c : cache, ok ? 16 : 0);
+      }
     }
     pa_cp_commit();
   };
+  // the group's query rows as bf16 [16][D]; rows and columns that no query fills are zero.  By copies too, where copies of K are on their way:
+  // loads would wait behind them
+  auto request_q = [&]() {
+    const __nv_bfloat16* src = q + static_cast<long long>(b) * ld_q + static_cast<long long>(h_base) * dk;
+    for (int i = threadIdx.x; i < gcount * (DK / 2); i += blockDim.x) {
+      const int g = i / (DK / 2), c = (i - g * (DK / 2)) * 2;
+      if (c < dk) pa_cp_async4(q_u32 + (g * KROW + c) * 2, src + g * dk + c);        // rows are 4-byte aligned at least
+    }
+    pa_cp_commit();
+  };
+  auto load_q = [&](bool whole) {
+    for (int i = threadIdx.x; i < kMaxGroup * LPK; i += blockDim.x) {
+      const int g = i / LPK, c = (i - g * LPK) * 8;
+      uint4 u = make_uint4(0u, 0u, 0u, 0u);
+      if (g < gcount && c < dk) {
+        if (!whole) continue;
+        const __nv_bfloat16* src = q + static_cast<long long>(b) * ld_q + static_cast<long long>(h_base + g) * dk + c;
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const uint32_t*>(src + 2 * j);
+        u = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      *reinterpret_cast<uint4*>(q_sh + g * KROW + c) = u;
+    }
+  };
   const PaInt<LPK> pk{};
   const PaInt<LPV> pv{};
-  int base = t_begin + warp * 32;
-  if (base < t_end) {
-    locate(base);
-    request(k_cache, kt_u32, pk, dk);
-    request(v_cache, vt_u32, pv, dv);
+
+  if (!LIST) {
+    load_q(true);
+    __syncthreads();
   }
-  for (; base < t_end; base += kPaWarps * 32) {
-    const int n_tok = n_next;
-    const bool more = base + kPaWarps * 32 < t_end;
-    pa_cp_wait<1>();                                                 // this pass's K tile has landed (V may be in flight)
-    __syncwarp();
-    // ---- S[16 heads, 32 tokens] = Q K^T
-    float s[4][4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-#pragma unroll
-    for (int k0 = 0; k0 < DK; k0 += 16) {
-      uint32_t a[4];
-      // A fragment: matrices (rows 0-7, k0), (rows 8-15, k0), (rows 0-7, k0 + 8), (rows 8-15, k0 + 8)
-      pa_ldsm_x4(q_u32 + ((lane & 15) * KROW + k0 + (lane >> 4) * 8) * 2, a);
-#pragma unroll
-      for (int np = 0; np < 2; ++np) {
-        uint32_t bfr[4];
-        // B fragments of two n-tiles: (tokens 16np..+7, k0), (same tokens, k0 + 8), (tokens 16np + 8.., k0), (.., k0 + 8)
-        pa_ldsm_x4(kt_u32 + ((np * 16 + (lane & 7) + ((lane >> 4) << 3)) * KROW + k0 + ((lane >> 3) & 1) * 8) * 2, bfr);
-        pa_mma(s[2 * np], a, bfr[0], bfr[1]);
-        pa_mma(s[2 * np + 1], a, bfr[2], bfr[3]);
-      }
+  enter();
+  request(k_cache, kt_u32, pk, dk);
+  if (LIST) load_q(false);
+  for (bool other = LIST;;) {
+    if (other) request_q();
+    request(v_cache, vt_u32, pv, dv);
+    if (other) {                               // query rows of another sequence: copied by all warps for all warps
+      pa_cp_wait<1>();
+      __syncthreads();
     }
-    __syncwarp();                                                    // every lane has read its K fragments
-    if (more) {                                                      // the next pass's K tile flies under softmax and P V
-      locate(base + kPaWarps * 32);
-      request(k_cache, kt_u32, pk, dk);
-    }
-    // ---- online softmax over the 32 tokens; this thread holds 8 of them for rows gq and gq + 8
-    float mx0 = -INFINITY, mx1 = -INFINITY;
+    const int b_done = b, sp_done = sp;
+    const bool another = LIST && --left > 0;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // rows gq and gq + 8
+    float acc[NT][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+
+    for (;;) {
+      const int n_tok = n_next, now = base, ctx_now = ctx;             // at most 0 tokens: a warp without a part in the slice
+      const PaVisible vis_now = vis;
+      const bool more = now + kPaWarps * 32 < t_end;
+      pa_cp_wait<1>();                                                 // this pass's K tile has landed (V may be in flight)
+      __syncwarp();
+      // ---- S[16 heads, 32 tokens] = Q K^T
+      float s[4][4];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const bool ok = n * 8 + 2 * tq + j < n_tok;
-        float v0 = s[n][j] * scale, v1 = s[n][2 + j] * scale;
-        if (RULE) {
-          if (rule.softcap > 0.f) {
-            v0 = pa_softcap(v0, rule.softcap, two_over_cap);
-            v1 = pa_softcap(v1, rule.softcap, two_over_cap);
-          }
-          const int num = base + n * 8 + 2 * tq + j;
-          const float dist = static_cast<float>(ctx - 1 - (num < vis.kept ? num : num + vis.gap));
-          v0 = fmaf(-slope0, dist, v0);
-          v1 = fmaf(-slope1, dist, v1);
-          if (rule.log_rate) {                       // distances behind the last token are masked below
-            v0 = fmaf(-amount0, __logf(fmaf(rate0, fmaxf(dist, 0.f), 1.f)), v0);
-            v1 = fmaf(-amount1, __logf(fmaf(rate1, fmaxf(dist, 0.f), 1.f)), v1);
+      for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+      if (n_tok > 0) {
+#pragma unroll
+        for (int k0 = 0; k0 < DK; k0 += 16) {
+          uint32_t a[4];
+          // A fragment: matrices (rows 0-7, k0), (rows 8-15, k0), (rows 0-7, k0 + 8), (rows 8-15, k0 + 8)
+          pa_ldsm_x4(q_u32 + ((lane & 15) * KROW + k0 + (lane >> 4) * 8) * 2, a);
+#pragma unroll
+          for (int np = 0; np < 2; ++np) {
+            uint32_t bfr[4];
+            // B fragments of two n-tiles: (tokens 16np..+7, k0), (same tokens, k0 + 8), (tokens 16np + 8.., k0), (.., k0 + 8)
+            pa_ldsm_x4(kt_u32 + ((np * 16 + (lane & 7) + ((lane >> 4) << 3)) * KROW + k0 + ((lane >> 3) & 1) * 8) * 2, bfr);
+            pa_mma(s[2 * np], a, bfr[0], bfr[1]);
+            pa_mma(s[2 * np + 1], a, bfr[2], bfr[3]);
           }
         }
-        s[n][j] = ok ? v0 : -INFINITY;
-        s[n][2 + j] = ok ? v1 : -INFINITY;
-        mx0 = fmaxf(mx0, s[n][j]);
-        mx1 = fmaxf(mx1, s[n][2 + j]);
       }
-    }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);          // finite: token 0 of the pass is always valid
-    const float al0 = (m0 == -INFINITY) ? 0.f : __expf(m0 - mn0);
-    const float al1 = (m1 == -INFINITY) ? 0.f : __expf(m1 - mn1);
-    float sum0 = 0.f, sum1 = 0.f;
-    uint32_t pfr[2][4];                                              // P as the A operand of the two 16-token k-steps
+      __syncwarp();                                                    // every lane has read its K fragments
+      // the K tile of the next pass, in this slice or the next, flies under softmax, P V and merge
+      if (more) {
+        locate(base = now + kPaWarps * 32);
+      } else if (another) {
+        if (++sp == slices_of(b)) {
+          sp = 0;
+          do ++b; while (slices_of(b) == 0);
+        }
+        enter();
+      } else {
+        n_next = 0;
+      }
+      request(k_cache, kt_u32, pk, dk);
+      if (n_tok <= 0) break;
+      // ---- online softmax over the 32 tokens; this thread holds 8 of them for rows gq and gq + 8
+      float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const float p0 = __expf(s[n][0] - mn0), p1 = __expf(s[n][1] - mn0);
-      const float p2 = __expf(s[n][2] - mn1), p3 = __expf(s[n][3] - mn1);
-      sum0 += p0 + p1;
-      sum1 += p2 + p3;
-      pfr[n >> 1][(n & 1) * 2 + 0] = pa_pack_bf16(p0, p1);          // rows gq
-      pfr[n >> 1][(n & 1) * 2 + 1] = pa_pack_bf16(p2, p3);          // rows gq + 8
+      for (int n = 0; n < 4; ++n) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const bool ok = n * 8 + 2 * tq + j < n_tok;
+          float v0 = s[n][j] * scale, v1 = s[n][2 + j] * scale;
+          if (RULE) {
+            if (rule.softcap > 0.f) {
+              v0 = pa_softcap(v0, rule.softcap, two_over_cap);
+              v1 = pa_softcap(v1, rule.softcap, two_over_cap);
+            }
+            const int num = now + n * 8 + 2 * tq + j;
+            const float dist = static_cast<float>(ctx_now - 1 - (num < vis_now.kept ? num : num + vis_now.gap));
+            v0 = fmaf(-slope0, dist, v0);
+            v1 = fmaf(-slope1, dist, v1);
+            if (rule.log_rate) {                       // distances behind the last token are masked below
+              v0 = fmaf(-amount0, __logf(fmaf(rate0, fmaxf(dist, 0.f), 1.f)), v0);
+              v1 = fmaf(-amount1, __logf(fmaf(rate1, fmaxf(dist, 0.f), 1.f)), v1);
+            }
+          }
+          s[n][j] = ok ? v0 : -INFINITY;
+          s[n][2 + j] = ok ? v1 : -INFINITY;
+          mx0 = fmaxf(mx0, s[n][j]);
+          mx1 = fmaxf(mx1, s[n][2 + j]);
+        }
+      }
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+      const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);          // finite: token 0 of the pass is always valid
+      const float al0 = (m0 == -INFINITY) ? 0.f : __expf(m0 - mn0);
+      const float al1 = (m1 == -INFINITY) ? 0.f : __expf(m1 - mn1);
+      float sum0 = 0.f, sum1 = 0.f;
+      uint32_t pfr[2][4];                                              // P as the A operand of the two 16-token k-steps
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const float p0 = __expf(s[n][0] - mn0), p1 = __expf(s[n][1] - mn0);
+        const float p2 = __expf(s[n][2] - mn1), p3 = __expf(s[n][3] - mn1);
+        sum0 += p0 + p1;
+        sum1 += p2 + p3;
+        pfr[n >> 1][(n & 1) * 2 + 0] = pa_pack_bf16(p0, p1);          // rows gq
+        pfr[n >> 1][(n & 1) * 2 + 1] = pa_pack_bf16(p2, p3);          // rows gq + 8
+      }
+      sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
+      sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
+      sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
+      sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
+      l0 = l0 * al0 + sum0;
+      l1 = l1 * al1 + sum1;
+      m0 = mn0;
+      m1 = mn1;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        acc[n][0] *= al0; acc[n][1] *= al0; acc[n][2] *= al1; acc[n][3] *= al1;
+      }
+      // ---- O[16, DV] += P[16, 32] V[32, DV]
+      pa_cp_wait<1>();                                                 // this pass's V tile has landed
+      __syncwarp();
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+#pragma unroll
+        for (int n2 = 0; n2 < NT / 2; ++n2) {
+          uint32_t bfr[4];
+          // transposed 8x8 blocks: (tokens 16ks..+7, dims 16n2), (tokens +8, same dims), (tokens.., dims + 8), (+8, + 8)
+          pa_ldsm_x4_t(vt_u32 + ((ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VROW + n2 * 16 + (lane >> 4) * 8) * 2, bfr);
+          pa_mma(acc[2 * n2], pfr[ks], bfr[0], bfr[1]);
+          pa_mma(acc[2 * n2 + 1], pfr[ks], bfr[2], bfr[3]);
+        }
+      }
+      __syncwarp();                                                    // every lane has read its V fragments
+      if (!more) break;
+      request(v_cache, vt_u32, pv, dv);
     }
-    sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
-    sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
-    sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
-    sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
-    l0 = l0 * al0 + sum0;
-    l1 = l1 * al1 + sum1;
-    m0 = mn0;
-    m1 = mn1;
+
+    // ---- merge the warps in the memory of their V tiles, write this slice's (max, sum, accumulator) per head
+    if (tq == 0) {
+      m_sh[warp][gq] = m0; l_sh[warp][gq] = l0;
+      m_sh[warp][gq + 8] = m1; l_sh[warp][gq + 8] = l1;
+    }
+    float* mine = merge + warp * kMergeStride + gq * VROW + 2 * tq;
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-      acc[n][0] *= al0; acc[n][1] *= al0; acc[n][2] *= al1; acc[n][3] *= al1;
+      if (gq < gcount) *reinterpret_cast<float2*>(mine + n * 8) = make_float2(acc[n][0], acc[n][1]);
+      if (gq + 8 < gcount) *reinterpret_cast<float2*>(mine + 8 * VROW + n * 8) = make_float2(acc[n][2], acc[n][3]);
     }
-    // ---- O[16, DV] += P[16, 32] V[32, DV]
-    if (more) pa_cp_wait<1>(); else pa_cp_wait<0>();                 // this pass's V tile has landed
-    __syncwarp();
+    __syncthreads();
+    for (int i = threadIdx.x; i < gcount * dv; i += blockDim.x) {
+      const int g = i / dv, d = i - g * dv;
+      float mx = -INFINITY;
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
+      for (int w = 0; w < kPaWarps; ++w) mx = fmaxf(mx, m_sh[w][g]);
+      float num = 0.f, den = 0.f;
 #pragma unroll
-      for (int n2 = 0; n2 < NT / 2; ++n2) {
-        uint32_t bfr[4];
-        // transposed 8x8 blocks: (tokens 16ks..+7, dims 16n2), (tokens +8, same dims), (tokens.., dims + 8), (+8, + 8)
-        pa_ldsm_x4_t(vt_u32 + ((ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VROW + n2 * 16 + (lane >> 4) * 8) * 2, bfr);
-        pa_mma(acc[2 * n2], pfr[ks], bfr[0], bfr[1]);
-        pa_mma(acc[2 * n2 + 1], pfr[ks], bfr[2], bfr[3]);
+      for (int w = 0; w < kPaWarps; ++w) {
+        const float sc = (m_sh[w][g] == -INFINITY) ? 0.f : __expf(m_sh[w][g] - mx);
+        num += merge[w * kMergeStride + g * VROW + d] * sc;
+        den += l_sh[w][g] * sc;
       }
+      if (direct_out) {                        // a single slice: this is the result
+        const long long col = static_cast<long long>(h_base + g) * dv + d;
+        if (RULE && rule.sink) {               // a score 0 without a value
+          const float top = fmaxf(mx, 0.f), sc = __expf(mx - top);
+          num *= sc;
+          den = fmaf(den, sc, __expf(-top));
+        }
+        float o = num / den;
+        if (RULE) o *= pa_gate(rule, b_done, h_base + g, col) * rule.out_scale;
+        direct_out[b_done * ld_o + col] = __float2bfloat16(o);
+        continue;
+      }
+      float* pp = partial + ((static_cast<long long>(b_done) * heads + h_base + g) * nsplit + sp_done) * (dv + 2);
+      pp[2 + d] = num;
+      if (d == 0) { pp[0] = mx; pp[1] = den; }
     }
-    __syncwarp();                                                    // every lane has read its V fragments
-    if (more) request(v_cache, vt_u32, pv, dv);
-  }
 
-  // ---- merge the warps, write this slice's (max, sum, accumulator) per head
-  __syncthreads();                            // every warp is done with its tile: the buffer becomes the merge area
-  float (*acc_sh)[kMaxGroup][DV] = reinterpret_cast<float (*)[kMaxGroup][DV]>(big);
-  if (tq == 0) {
-    m_sh[warp][gq] = m0; l_sh[warp][gq] = l0;
-    m_sh[warp][gq + 8] = m1; l_sh[warp][gq + 8] = l1;
-  }
-#pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    *reinterpret_cast<float2*>(&acc_sh[warp][gq][n * 8 + 2 * tq]) = make_float2(acc[n][0], acc[n][1]);
-    *reinterpret_cast<float2*>(&acc_sh[warp][gq + 8][n * 8 + 2 * tq]) = make_float2(acc[n][2], acc[n][3]);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < gcount * dv; i += blockDim.x) {
-    const int g = i / dv, d = i - g * dv;
-    float mx = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kPaWarps; ++w) mx = fmaxf(mx, m_sh[w][g]);
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < kPaWarps; ++w) {
-      const float sc = (m_sh[w][g] == -INFINITY) ? 0.f : __expf(m_sh[w][g] - mx);
-      num += acc_sh[w][g][d] * sc;
-      den += l_sh[w][g] * sc;
-    }
-    if (direct_out) {                        // a single slice: this is the result
-      const long long col = static_cast<long long>(h_base + g) * dv + d;
-      if (RULE && rule.sink) {               // a score 0 without a value
-        const float top = fmaxf(mx, 0.f), sc = __expf(mx - top);
-        num *= sc;
-        den = fmaf(den, sc, __expf(-top));
-      }
-      float o = num / den;
-      if (RULE) o *= pa_gate(rule, b, h_base + g, col) * rule.out_scale;
-      direct_out[b * ld_o + col] = __float2bfloat16(o);
-      continue;
-    }
-    float* pp = partial + ((static_cast<long long>(b) * heads + h_base + g) * nsplit + sp) * (dv + 2);
-    pp[2 + d] = num;
-    if (d == 0) { pp[0] = mx; pp[1] = den; }
+    if (!another) return;
+    __syncthreads();                            // the merge area has been read: it becomes V tiles again
+    other = b != b_done;
   }
 }
 
@@ -385,8 +482,7 @@ paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restri
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   if (d >= dv) return;
   const int ctx = context_lens[b];
-  const int count = pa_visible(ctx, rule).count, slice = pa_slice(count, nsplit);
-  const int n = (count + slice - 1) / slice;
+  const int n = pa_slices(pa_visible(ctx, rule).count, nsplit);
   const float* base = partial + (static_cast<long long>(b) * heads + h) * nsplit * (dv + 2);
   float mx = -INFINITY;
   for (int s = 0; s < n; ++s) mx = fmaxf(mx, base[s * (dv + 2)]);
@@ -543,32 +639,34 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
   long long span = static_cast<long long>(a.max_blocks) * a.block_size;      // most keys a row can see
   if (a.chunk > 0 && a.chunk < span) span = a.chunk;
   if (a.window > 0 && static_cast<long long>(a.window) + a.keep_first < span) span = a.window + a.keep_first;
-  // About three CTAs for each of the 148 x 3 that fit at a time.  The tables are as wide as the model's context, so slices of 256 tokens for
-  // all of it were mostly CTAs without a token, each of which still takes its turn.  64 sequences of 100 to 4000 tokens in tables for 16384, 4
-  // KV heads of 128: 74.5 us as 16384 CTAs, 64.4 us (4.2 TB/s) with 6 slices of each sequence, merges included; 24 of 128 to 2560, 8 KV heads:
-  // 43.5 and 39.0 (two, four, six CTAs for each: 64.8, 64.6, 69.4 and 40.8, 44.5, 44.2).
-  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads, most = (span + rb::kSplitTokens - 1) / rb::kSplitTokens;
-  const long long wanted = (148 * 3 * 3 + pairs - 1) / pairs;
-  const int nsplit = static_cast<int>(wanted < most ? wanted : most);
+  const int nsplit = static_cast<int>((span + rb::kSplitTokens - 1) / rb::kSplitTokens);
+  // A CTA for every slice that the tables have room for, where that is no more than twice what fits at a time (three per SM); else twice as many
+  // as fit, over the slices that there are.  One B200, merge included, us: grid of slices / fewer, longer slices per sequence (six CTAs per SM
+  // over batch x KV heads, results then depend on the batch) / list.  64 sequences of 100 to 4000 tokens in tables for 16384, 4 KV heads of
+  // 128: 74.7 / 64.6 / 65.5; 24 of 128 to 2560, 8 KV heads: 47.7 / 45.2 / 38.0; 63 of 300 and one of 16384: 48.5 / 78.4 / 35.7; 332 and one: 138 /
+  // 343 / 85; 400 of 500, 8 KV heads: 298 / 155 / 167.  One sequence of 2047, 4 KV heads: 12.4 / 11.6 / 12.4 as a list, 11.3 as a grid.  With
+  // as many CTAs as fit at a time the first takes 68 to 70 us, with three times as many 67.
+  const long long room = static_cast<long long>(a.batch) * a.kv_heads * nsplit, some = 6ll * rbhost::device_sm_count();
+  const bool list = room > some;
+  const dim3 grid = list ? dim3(static_cast<unsigned int>(some < a.kv_heads ? 1 : some / a.kv_heads), a.kv_heads) : dim3(a.batch, a.kv_heads, nsplit);
   // dynamic shared memory: per warp a K and a V tile of 32 padded rows, plus the 16 padded query rows
   const int smem = (rb::kPaWarps * 32 * (DK + 8 + DV + 8) + rb::kMaxGroup * (DK + 8)) * 2;
-  auto kern = rb::paged_decode_split_kernel<DK, DV, RULE>;
-  static bool attr_set[64] = {};
+  auto kern = list ? rb::paged_decode_split_kernel<DK, DV, RULE, true> : rb::paged_decode_split_kernel<DK, DV, RULE, false>;
+  static bool attr_set[2][64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
-  if (!attr_set[dev]) {
+  if (!attr_set[list][dev]) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
-    attr_set[dev] = true;
+    attr_set[list][dev] = true;
   }
   auto O = reinterpret_cast<__nv_bfloat16*>(a.out);
   const rb::PaRule rule = {a.softcap, a.slopes, a.chunk, reinterpret_cast<const __nv_bfloat16*>(a.gate), a.head_gate, a.ld_g,
                            a.window, a.keep_first, a.sink, a.log_amount, a.log_rate, a.out_scale};
-  const dim3 grid(a.batch, a.kv_heads, nsplit);
   for (int g0 = 0; g0 < group; g0 += rb::kMaxGroup)       // groups wider than 16 heads take several passes
-    rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kPaWarps * 32), smem, stream, 1, 
+    rbhost::launch_pdl(kern, grid, dim3(rb::kPaWarps * 32), smem, stream, 1,
         reinterpret_cast<const __nv_bfloat16*>(a.q), a.ld_q, reinterpret_cast<const __nv_bfloat16*>(a.k_cache),
-        reinterpret_cast<const __nv_bfloat16*>(a.v_cache), a.block_tables, a.max_blocks, a.context_lens, a.heads, a.kv_heads,
+        reinterpret_cast<const __nv_bfloat16*>(a.v_cache), a.block_tables, a.max_blocks, a.context_lens, a.batch, a.heads, a.kv_heads,
         a.dk, a.dv, a.block_size, a.num_blocks, a.scale, g0, group - g0 < rb::kMaxGroup ? group - g0 : rb::kMaxGroup,
         a.scratch, nsplit, nsplit == 1 ? O : nullptr, a.ld_o, rule RB_BOUNDS_ARG);
   if (nsplit > 1)

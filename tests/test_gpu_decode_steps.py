@@ -37,7 +37,7 @@ def test_rope_append_is_rope_and_append(tokens, heads, kv, dim, cuda_status):
 @pytest.mark.parametrize("batch,heads,kv,dim,longest,width", [(1, 8, 2, 128, 2500, 400), (64, 8, 4, 128, 1300, 1024), (120, 32, 16, 64, 700, 64),
                                                              (3, 4, 4, 64, 257, 1024)])
 def test_slices_of_the_context(batch, heads, kv, dim, longest, width, cuda_status):
-    """Slices of 256 tokens, of more (many sequences), and one slice for everything; lengths from 1 to the longest."""
+    """Several slices per CTA and fewer slices than CTAs, up to four warps' worth of sequences; lengths from 1 to the longest."""
     g = torch.Generator(device="cuda").manual_seed(batch)
     need = (longest + 15) // 16
     blocks = batch * need
@@ -56,3 +56,30 @@ def test_slices_of_the_context(batch, heads, kv, dim, longest, width, cuda_statu
         want = torch.einsum("hn,nhd->hd", p, v)
         # weights rounded to bf16 (2^-9 each, against the unrounded sum) and a bf16 result
         assert ((got[b] - want).abs() <= 2.0 ** -8 * torch.einsum("hn,nhd->hd", p, v.abs()) + 1e-3).all(), b
+
+
+@pytest.mark.parametrize("rule", [None, dict(chunk=300), dict(window=500, keep_first=7, sink=True, softcap=20.0)])
+@pytest.mark.parametrize("heads,kv,dim", [(8, 2, 128), (40, 2, 64)])
+def test_a_sequence_has_the_same_bits_alone_and_beside_others(heads, kv, dim, rule, cuda_status):
+    """Slices are cut by a sequence's own length: neither the batch, nor the others' lengths (among them none and a very long one), nor the
+    width of the tables changes a bit.  40 heads on 2 take two passes of 16 and one of 8."""
+    from rustral_b200.ops.attention import ScoreRule
+    rule = ScoreRule(**rule) if rule else None
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    lens = [1, 255, 256, 257, 9000, 0, 2000, 640] + [33 * i % 700 + 1 for i in range(62)]
+    need = [(n + 15) // 16 for n in lens]
+    kc, vc = (torch.randn(sum(need), 16, kv, dim, device="cuda", generator=g).bfloat16() for _ in range(2))
+    pages = torch.randperm(sum(need), device="cuda", generator=g).int()
+    table = torch.zeros(len(lens), 1024, dtype=torch.int32, device="cuda")
+    for i, n in enumerate(need):
+        table[i, :n] = pages[sum(need[:i]):sum(need[:i + 1])]
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = torch.randn(len(lens), heads * dim, device="cuda", generator=g).bfloat16()
+    run = lambda rows, width: paged.paged_attention_decode(q[rows], kc, vc, table[rows, :width].contiguous(), ctx[rows], rule=rule)  # noqa: E731
+    together = run(list(range(len(lens))), 1024)
+    for i in (0, 1, 2, 3, 4, 6, 7, 40, 69):
+        assert torch.equal(run([i], 1024)[0], together[i]), i
+        if need[i] > 16:
+            assert torch.equal(run([i], need[i])[0], together[i]), i
+    some = [3, 4, 69, 6]
+    assert torch.equal(run(some, 700), together[some])
