@@ -480,19 +480,48 @@ paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restri
   pdl_wait();
   pdl_launch();
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
-  if (d >= dv) return;
   const int ctx = context_lens[b];
   const int n = pa_slices(pa_visible(ctx, rule).count, nsplit);
   const float* base = partial + (static_cast<long long>(b) * heads + h) * nsplit * (dv + 2);
-  float mx = -INFINITY;
-  for (int s = 0; s < n; ++s) mx = fmaxf(mx, base[s * (dv + 2)]);
-  if (rule.sink) mx = fmaxf(mx, 0.f);
-  float num = 0.f, den = rule.sink ? __expf(-mx) : 0.f;      // a sink is a score 0 without a value
-  for (int s = 0; s < n; ++s) {
-    const float ms = base[s * (dv + 2)];
-    const float sc = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-    num += base[s * (dv + 2) + 2 + d] * sc;
-    den += base[s * (dv + 2) + 1] * sc;
+  float mx = rule.sink ? 0.f : -INFINITY, num = 0.f, den;    // a sink is a score 0 without a value
+  if (n <= 8) {
+    if (d >= dv) return;
+    for (int s = 0; s < n; ++s) mx = fmaxf(mx, base[s * (dv + 2)]);
+    den = rule.sink ? __expf(-mx) : 0.f;
+    for (int s = 0; s < n; ++s) {
+      const float ms = base[s * (dv + 2)];
+      const float sc = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
+      num += base[s * (dv + 2) + 2 + d] * sc;
+      den += base[s * (dv + 2) + 1] * sc;
+    }
+  } else {
+    // Long contexts: a slice's factor is formed once, by one thread, and the sums run over independent loads (in the same order).  Attention of
+    // one sequence of 16000 tokens 24.7 us, so 19.1; 64 of 100 to 4000 66.0 and 64.7; with up to 8 slices the two barriers cost 0.2 us.
+    __shared__ float scale_sh[128], sum_sh[128], top_sh[4];
+    for (int s = d; s < n; s += 128) mx = fmaxf(mx, base[s * (dv + 2)]);
+    mx = warp_max(mx);
+    if ((d & 31) == 0) top_sh[d >> 5] = mx;
+    __syncthreads();
+    mx = fmaxf(fmaxf(top_sh[0], top_sh[1]), fmaxf(top_sh[2], top_sh[3]));
+    den = rule.sink ? __expf(-mx) : 0.f;
+    for (int from = 0; from < n; from += 128) {
+      const int m = min(128, n - from);
+      if (from) __syncthreads();
+      if (d < m) {
+        const float ms = base[(from + d) * (dv + 2)];
+        scale_sh[d] = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
+        sum_sh[d] = base[(from + d) * (dv + 2) + 1];
+      }
+      __syncthreads();
+      if (d < dv) {
+#pragma unroll 8
+        for (int s = 0; s < m; ++s) {
+          num += base[(from + s) * (dv + 2) + 2 + d] * scale_sh[s];
+          den += sum_sh[s] * scale_sh[s];
+        }
+      }
+    }
+    if (d >= dv) return;
   }
   const long long col = static_cast<long long>(h) * dv + d;
   float o = den > 0.f ? num / den : 0.f;
@@ -643,7 +672,7 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
   // A CTA for every slice that the tables have room for, where that is no more than twice what fits at a time (three per SM); else twice as many
   // as fit, over the slices that there are.  One B200, merge included, us: grid of slices / fewer, longer slices per sequence (six CTAs per SM
   // over batch x KV heads, results then depend on the batch) / list.  64 sequences of 100 to 4000 tokens in tables for 16384, 4 KV heads of
-  // 128: 74.7 / 64.6 / 65.5; 24 of 128 to 2560, 8 KV heads: 47.7 / 45.2 / 38.0; 63 of 300 and one of 16384: 48.5 / 78.4 / 35.7; 332 and one: 138 /
+  // 128: 74.7 / 64.6 / 64.7; 24 of 128 to 2560, 8 KV heads: 47.7 / 45.2 / 38.0; 63 of 300 and one of 16384: 48.5 / 78.4 / 35.7; 332 and one: 138 /
   // 343 / 85; 400 of 500, 8 KV heads: 298 / 155 / 167.  One sequence of 2047, 4 KV heads: 12.4 / 11.6 / 12.4 as a list, 11.3 as a grid.  With
   // as many CTAs as fit at a time the first takes 68 to 70 us, with three times as many 67.
   const long long room = static_cast<long long>(a.batch) * a.kv_heads * nsplit, some = 6ll * rbhost::device_sm_count();

@@ -66,7 +66,7 @@ def test_a_sequence_has_the_same_bits_alone_and_beside_others(heads, kv, dim, ru
     from rustral_b200.ops.attention import ScoreRule
     rule = ScoreRule(**rule) if rule else None
     g = torch.Generator(device="cuda").manual_seed(dim)
-    lens = [1, 255, 256, 257, 9000, 0, 2000, 640] + [33 * i % 700 + 1 for i in range(62)]
+    lens = [1, 255, 256, 257, 9000, 0, 2049, 2048] + [33 * i % 700 + 1 for i in range(62)]
     need = [(n + 15) // 16 for n in lens]
     kc, vc = (torch.randn(sum(need), 16, kv, dim, device="cuda", generator=g).bfloat16() for _ in range(2))
     pages = torch.randperm(sum(need), device="cuda", generator=g).int()
@@ -77,6 +77,14 @@ def test_a_sequence_has_the_same_bits_alone_and_beside_others(heads, kv, dim, ru
     q = torch.randn(len(lens), heads * dim, device="cuda", generator=g).bfloat16()
     run = lambda rows, width: paged.paged_attention_decode(q[rows], kc, vc, table[rows, :width].contiguous(), ctx[rows], rule=rule)  # noqa: E731
     together = run(list(range(len(lens))), 1024)
+    for i in (4, 6, 7):                                       # 36, 9 and 8 slices: both forms of the merge (without a rule: all are seen)
+        rows = table[i, :need[i]].long()
+        k, v = (c[rows].reshape(-1, kv, dim)[:lens[i]].repeat_interleave(heads // kv, 1).double() for c in (kc, vc))
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[i].double().view(heads, dim), k) * dim ** -0.5, -1)
+        # weights rounded to bf16 (2^-9 each, against the unrounded sum) and a bf16 result
+        bound = 2.0 ** -8 * torch.einsum("hn,nhd->hd", p, v.abs()) + 1e-3
+        off = (together[i].double().view(heads, dim) - torch.einsum("hn,nhd->hd", p, v)).abs()
+        assert rule is not None or (off <= bound).all(), i
     for i in (0, 1, 2, 3, 4, 6, 7, 40, 69):
         assert torch.equal(run([i], 1024)[0], together[i]), i
         if need[i] > 16:
