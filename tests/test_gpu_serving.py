@@ -64,3 +64,35 @@ def test_tensor_parallel_serving_matches_single_gpu(transport):
     assert out["prefill_rel_err"] < 3e-2, out
     # greedy decoding of random-init logits can flip on near ties; the first tokens must agree
     assert out["tokens_ref"][:4] == out["tokens_tp"][:4], out
+
+
+def test_steps_keep_their_host_memory(cuda_status):
+    """Steps that are issued one behind another share two page-locked blocks, whatever their batch size, and what they copy is theirs: a
+    block is not written again before its copy has been made."""
+    cfg = preset("llama-test")
+    r = ModelRunner(cfg, device="cuda", num_blocks=128, seed=3)
+    for i in range(5):
+        assert r.cache.allocate(i, 40)
+    prompts = torch.arange(5 * 8).view(5, 8).tolist()
+
+    def steps():
+        got = {}
+        for B in (1, 3, 5):
+            for n in (1, 8, 20):
+                got[B, n] = r.decode(list(range(B)), [7 * n + i for i in range(B)], [n] * B).clone()
+        got["prompts"] = torch.stack(r.step_mixed([(i, t, 20, True) for i, t in enumerate(prompts)], [], [], [])[0])
+        return got
+
+    steps()                                                    # graphs are captured, every slot that is seen below is written
+    want = steps()
+    torch.cuda.synchronize()
+    before = torch.cuda.host_memory_stats()["num_host_alloc"]
+    rounds = []
+    for _ in range(30):
+        torch.cuda._sleep(200000)                              # the copies below wait in the stream
+        rounds.append(steps())
+    assert len(r._memory.free) <= 2
+    assert torch.cuda.host_memory_stats()["num_host_alloc"] == before
+    for got in rounds:
+        for key, logits in want.items():
+            assert torch.equal(got[key], logits), key
