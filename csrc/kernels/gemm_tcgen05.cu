@@ -139,12 +139,10 @@ struct SmemLayout {
 // Epilogue arithmetic on 32 consecutive accumulator columns of one output row (everything but the final store).
 // STORE_AUX: write the pre-activation to aux_out from here (one 64-byte piece per thread).  PRE_ONLY: stop after
 // the bias, leaving the pre-activation in v (the staged path writes it out itself, coalesced).
-// POST_ONLY: v already holds the pre-activation; only the activation and the residual are applied.
-template <bool STORE_AUX = true, bool PRE_ONLY = false, bool POST_ONLY = false>
+template <bool STORE_AUX = true, bool PRE_ONLY = false>
 __device__ __forceinline__ void epilogue_math(const EpiParams& ep, uint32_t (&r)[32], long long row, int col0, int N,
                                               float (&v)[32]) {
   const bool full = (col0 + 32 <= N);
-  if (!POST_ONLY) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * ep.alpha;
 
@@ -185,8 +183,6 @@ __device__ __forceinline__ void epilogue_math(const EpiParams& ep, uint32_t (&r)
     }
   }
 
-  }   // !POST_ONLY
-
   if (PRE_ONLY) return;
 
   if (ep.act == RB_ACT_GELU || ep.act == RB_ACT_RELU || ep.act == RB_ACT_SILU || ep.act == RB_ACT_RELU2) {
@@ -206,9 +202,9 @@ __device__ __forceinline__ void epilogue_math(const EpiParams& ep, uint32_t (&r)
         for (int j = 0; j < 32; ++j)
           if (col0 + j < N) ap[j] = __float2bfloat16(v[j]);
       }
-      // The activation is applied to the unrounded fp32 value; the backward pass differentiates at the bf16-rounded
-      // one it reads back (a relative difference of 2^-9 in the argument).  Rounding here as well costs two conversions
-      // per element in an epilogue whose conversion and special-function work already exceeds the main loop at K = 768.
+      // Here the activation is applied to the unrounded fp32 value, while the backward pass differentiates at the bf16-rounded one that it
+      // reads back (a relative difference of 2^-9 in the argument).  Results that leave through TMA (`epilogue_tma`) are formed from the
+      // rounded value, which their tile holds.
     }
     if (ep.act == RB_ACT_GELU) {
 #pragma unroll
@@ -462,7 +458,35 @@ __device__ __forceinline__ void tile_act(const EpiParams& ep, const uint32_t (&s
   }
 }
 
-template <int COLS, int SLOTS, class Arrive>
+// 32 columns of a side input as packed pairs, by the SM's own loads; N is a multiple of 8.
+__device__ __forceinline__ void side_get(const __nv_bfloat16* src, int col0, int N, uint32_t (&side)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 u = make_uint4(0u, 0u, 0u, 0u);
+    if (col0 + 8 * q < N) u = *reinterpret_cast<const uint4*>(src + col0 + 8 * q);
+    side[4 * q] = u.x; side[4 * q + 1] = u.y; side[4 * q + 2] = u.z; side[4 * q + 3] = u.w;
+  }
+}
+__device__ __forceinline__ void tile_get(uint32_t slot, int lane, int half, uint32_t (&v)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[4 * q]), "=r"(v[4 * q + 1]), "=r"(v[4 * q + 2]), "=r"(v[4 * q + 3])
+                 : "r"(stage_addr(slot, lane, half * 4 + q)));
+}
+__device__ __forceinline__ void tile_put(uint32_t slot, int lane, int half, const Pair (&v)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    stage_put(stage_addr(slot, lane, half * 4 + q), packed(v[4 * q]), packed(v[4 * q + 1]), packed(v[4 * q + 2]), packed(v[4 * q + 3]));
+}
+__device__ __forceinline__ void tile_add(const uint32_t (&r)[16], Pair (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = add2(v[j], pair_of(r[j]));
+}
+
+// EXTRA: the forms that the tiles do not suffice for: side inputs beside a second result, two side inputs, and any of them with one tile per
+// warp.  What finds no tile is read by the SM's own loads.  Kernels of their own: as branches of the common ones, not taken, these cost 10 % of a
+// short contraction and 2.5 of 20 us of a small one.
+template <int COLS, int SLOTS, bool EXTRA, class Arrive>
 __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensorMap* tmD, const CUtensorMap* tmAux, uint32_t stg,
                                              uint32_t bar_side, uint32_t t, uint32_t taddr, int row0, int drow, int col, int M, int N,
                                              int lane, bool empty_k, volatile int* abort_flag, unsigned int* status, Arrive arrive) {
@@ -478,13 +502,14 @@ __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensor
     const uint32_t slot = stg + (two ? 0 : (block + (ep.side != 0 ? 0 : t * (COLS / cols))) % SLOTS) * 4096;
     uint32_t r[32];
     tmem_ld_32x32(taddr + c, r);
-    uint32_t side[16];
+    uint32_t side[16], residual[16];
+    if (EXTRA) {                               // requested before the accumulator is waited for
+      if (ep.residual != nullptr && ep.side != 1) side_get(ep.residual + row * ep.ldr, col + c, N, residual);
+      if (ep.aux_in != nullptr && ep.side != 2) side_get(ep.aux_in + row * ep.ld_aux_in, col + c, N, side);
+    }
     if (ep.side != 0) {
       if (half == 0 && !mbar_wait(bar_side + 8 * block, t & 1, abort_flag, status, 7)) return;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(side[4 * q]), "=r"(side[4 * q + 1]), "=r"(side[4 * q + 2]),
-                     "=r"(side[4 * q + 3]) : "r"(stage_addr(slot, lane, half * 4 + q)));
+      tile_get(slot, lane, half, side);
     } else if (half == 0) {
       // with two results the first tile may be filled again while the second one, stored later, still leaves
       if (lane == 0) tma_store_wait_read<SLOTS - 1>();
@@ -507,28 +532,25 @@ __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensor
     } else {
       if (!two) {
         tile_act(ep, side, v);
-        if (ep.side == 1) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = add2(v[j], pair_of(side[j]));
-        }
+        if (ep.side == 1) tile_add(side, v);
+        else if (EXTRA && ep.residual != nullptr) tile_add(residual, v);
       }
       uint32_t o[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) o[j] = packed(v[j]);
 #pragma unroll
       for (int q = 0; q < 4; ++q) stage_put(stage_addr(slot, lane, half * 4 + q), o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-      if (two) {
+      if (two && SLOTS > 1) {
         // the result is formed from the rounded pre-activation, in the second tile
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = pair_of(o[j]);
         tile_act(ep, side, v);
+        if (EXTRA && ep.residual != nullptr) tile_add(residual, v);
         if (half == 0) {
           if (lane == 0) tma_store_wait_read<0>();
           __syncwarp();
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          stage_put(stage_addr(slot + 4096, lane, half * 4 + q), packed(v[4 * q]), packed(v[4 * q + 1]), packed(v[4 * q + 2]), packed(v[4 * q + 3]));
+        tile_put(slot + 4096, lane, half, v);
       }
       if (half == 0) continue;
     }
@@ -540,8 +562,33 @@ __device__ __forceinline__ void epilogue_tma(const EpiParams& ep, const CUtensor
       else if (ep.staged == 4) tma_reduce_add_2d(tmD, slot, x, drow);
       else tma_store_2d(two ? tmAux : tmD, slot, x, drow);
       tma_store_commit();
-      if (two) {
+      if (two && SLOTS > 1) {
         if (row0 < M) tma_store_2d(tmD, slot + 4096, x, drow);
+        tma_store_commit();
+      }
+    }
+    if (EXTRA && SLOTS == 1 && two) {
+      // one tile: the result takes the place of the rounded pre-activation when that has been read out, each lane from its own row
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        uint32_t o[16];
+        tile_get(slot, lane, h, o);
+        Pair v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = pair_of(o[j]);
+        tile_act(ep, o, v);
+        if (ep.residual != nullptr) {
+          side_get(ep.residual + row * ep.ldr, col + c - 32 + 32 * h, N, o);
+          tile_add(o, v);
+        }
+        tile_put(slot, lane, h, v);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (row0 < M) tma_store_2d(tmD, slot, col + c - 32, drow);
         tma_store_commit();
       }
     }
@@ -587,7 +634,7 @@ __device__ __forceinline__ void epilogue_swiglu(const CUtensorMap* tmD, uint32_t
 
 // FP8 = 1: both operands hold e4m3 bytes (K-major only).  A 128-byte swizzle row then carries 128 elements, so K, lda
 // and ldb arrive halved (in units of two bytes) and only the TMA coordinates, which count elements, are doubled back.
-template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
+template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0, bool EXTRA = false>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
@@ -856,8 +903,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
       };
       if (L::kTma && ep.staged >= 2) {
-        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0,
-                                  num_splits > 1 || grp.mode == 2 ? outer * M + row0 : row0, colg, M, N, lane, empty_k, abort_flag, status, arrive);
+        const int drow = num_splits > 1 || grp.mode == 2 ? outer * M + row0 : row0;
+        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
+                                                    lane, empty_k, abort_flag, status, arrive);
         continue;
       }
       EpiParams epu = ep;
@@ -990,7 +1038,7 @@ struct SmemLayoutPair {
   static constexpr int kTotalStaged = kStagingOffset + kNumEpilogueWarps * kStagingBytesPerWarp;
 };
 
-template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0>
+template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0, bool EXTRA = false>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
@@ -1166,8 +1214,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         continue;
       }
       if (ep.staged >= 2) {
-        epilogue_tma<BLOCK_N / 2, L::kSlots>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0,
-                                  num_splits > 1 ? split * M + row0 : row0, colg, M, N, lane, false, abort_flag, status, arrive);
+        const int drow = num_splits > 1 ? split * M + row0 : row0;
+        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
+                                                    lane, false, abort_flag, status, arrive);
         continue;
       }
       EpiParams epu = ep;
@@ -1276,10 +1325,13 @@ bool tma_store_default() {
   return v == 1;
 }
 
-// Fills the epilogue's parameters and the tensor maps of what TMA moves for it.  Returns the shared memory to ask for.
+// Fills the epilogue's parameters and the tensor maps of what TMA moves for it.  Returns the shared memory to ask for.  `extra` on entry: the
+// kernel exists with the EXTRA forms; on return: it has to be that one.
 template <class L>
 int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUtensorMap*& td, const CUtensorMap*& tx,
-                  const CUtensorMap*& ts) {
+                  const CUtensorMap*& ts, bool& extra) {
+  const bool may_extra = extra;
+  extra = false;
   ep.d = g.d; ep.ldd = g.ldd;
   ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
   ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual); ep.ldr = g.ldr;
@@ -1305,18 +1357,20 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
     if (g.peer_mode != 2 && !staged_store_default()) return L::kTotal + 1024;
     ep.staged = 1;
     const bool reads = g.aux_in || g.residual;
-    if (tma && (L::kSide ? !(g.aux_in && g.residual) && !(reads && g.aux_out) : !reads && !g.aux_out)) {
+    const bool more = L::kSide ? (g.aux_in && g.residual) || (reads && g.aux_out) : reads || g.aux_out;     // than the tiles suffice for
+    if (tma && (may_extra || !more)) {
       const uint64_t n = g.N, m = g.M * stack;
       const CUtensorMap* d = rbhost::get_tmap_2d(g.d, 2, n, m, (uint64_t)g.ldd, 64, 32, 1, &err);
       const CUtensorMap* x = g.aux_out ? rbhost::get_tmap_2d(g.aux_out, 2, n, m, (uint64_t)g.ld_aux_out, 64, 32, 1, &err) : d;
       const CUtensorMap* side = nullptr;
-      if (reads) {
+      if (L::kSide && !g.aux_out) {            // a second result needs the tiles itself
         if (g.aux_in) side = rbhost::get_tmap_2d(g.aux_in, 2, n, m, (uint64_t)g.ld_aux_in, 64, 32, 1, &err);
         else if (g.residual) side = rbhost::get_tmap_2d(g.residual, 2, n, m, (uint64_t)g.ldr, 64, 32, 1, &err);
       }
-      if (d && x && (side || !reads)) {
+      if (d && x && (side || more || !reads)) {
         ep.staged = 2; td = d; tx = x;
         if (side) { ts = side; ep.side = g.aux_in ? 2 : 1; }
+        extra = more;
       }
     }
   } else if (tma && (stack == 1 || stacked) && ep.ldd % 4 == 0 && g.N % 4 == 0 && g.act == RB_ACT_NONE &&
@@ -1342,11 +1396,15 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
   }
   const CUtensorMap *td = ta, *tx = ta, *ts = ta;         // placeholders unless TMA moves the results
   auto kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8>;
+  constexpr bool kExtra = !A_MN && !FP8 && L::kTma;       // forward products and input gradients
+  bool extra = kExtra;
   rb::EpiParams ep;
-  const int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts);
+  const int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts, extra);
+  if constexpr (kExtra)
+    if (extra) kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8, true>;
   if (g.peer_mode == 2 && !ep.staged) return -11;
-  static int configured_dev[64] = {0};   // per instantiation and device: largest size set so far
-  int& configured = configured_dev[rbhost::device_slot()];
+  static int configured_dev[2][64] = {{0}};   // per instantiation and device: largest size set so far
+  int& configured = configured_dev[extra][rbhost::device_slot()];
   if (configured < smem) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -1420,11 +1478,15 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
   }
   const CUtensorMap *td = ta, *tx = ta, *ts = ta;
   rb::EpiParams ep;
-  int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts);
+  constexpr bool kExtra = !A_MN && !FP8;                  // forward products and input gradients
+  bool extra = kExtra;
+  int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts, extra);
+  if constexpr (kExtra)
+    if (extra) kern = rb::gemm_bf16_pair_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8, true>;
   if (g.act == RB_ACT_SWIGLU && ep.staged != 2) return -9;
   if (ep.staged == 1) ep.staged = 0, smem = L::kTotal + 1024;       // this kernel stores through TMA or straight from registers
-  static int configured_dev[64] = {0};
-  int& configured = configured_dev[rbhost::device_slot()];
+  static int configured_dev[2][64] = {{0}};
+  int& configured = configured_dev[extra][rbhost::device_slot()];
   if (configured < smem) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
