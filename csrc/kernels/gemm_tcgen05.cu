@@ -1555,13 +1555,18 @@ int gemm_swiglu(const RbGemmArgs& g, cudaStream_t stream) {
     return -9;
   if (rbhost::gemm_rows_takes(g)) return rbhost::gemm_rows(g, stream);
   if (g.M <= 128 || !pair_kernel_enabled() || !tma_store_default() || !staged_store_default()) return -9;
+  // The tiles of this form are 256 x 128 only.  Where they leave most pairs of SMs idle, a product of narrower tiles and a second launch are the
+  // faster way, at the shorter contractions less so (us, this form / two launches): 256 x 512 x 4096 24.7 / 12.9, 512 x 512 x 8192 43.5 / 19.1, 256
+  // x 2304 x 4096 (18 tiles) 26.2 / 21.3, 256 x 3072 x 4096 (24) 26.8 / 26.2, 300 x 1792 x 4096 (28) 26.1 / 36.6; 256 x 1024 x 1024 (8) 11.0 / 9.5, 1024
+  // x 512 x 768 (16) 9.9 / 10.9, 768 x 768 x 768 (18) 10.3 / 10.9.
+  const long long tiles = (long long)((g.M + 255) / 256) * ((g.N + 127) / 128);
+  const int most = rbhost::device_sm_count() / 2;
+  if (tiles * (g.K >= 2048 ? 4 : 5) <= most) return -9;
   int err = 0;
   const CUtensorMap* ta = rbhost::get_tmap_2d(g.a, 2, (uint64_t)g.K, (uint64_t)g.M, (uint64_t)g.lda, 64, 128, 1, &err);
   if (!ta) return err ? err : -5;
   const CUtensorMap* tb = rbhost::get_tmap_2d(g.b, 2, (uint64_t)g.K, 2 * (uint64_t)g.N, (uint64_t)g.ldb, 64, 128, 1, &err);
   if (!tb) return err ? err : -5;
-  const long long tiles = (long long)((g.M + 255) / 256) * ((g.N + 127) / 128);
-  const int most = rbhost::device_sm_count() / 2;
   return launch_pair<0, 0>(g, ta, tb, static_cast<int>(tiles < most ? tiles : most), 1, stream);
 }
 

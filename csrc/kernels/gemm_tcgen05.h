@@ -16,7 +16,7 @@ enum RbAct {
   RB_ACT_MUL = 7,     // multiply the result by aux_in
   RB_ACT_RELU2 = 8,   // the square of relu (inference: no pre-activation is kept)
   RB_ACT_SWIGLU = 9   // B holds 2 N rows, gates over ups: d = silu(A gate^T) * (A up^T).  K-major bf16 operands and result, no other
-                      // epilogue, at most 96 or more than 128 rows; what is not taken is refused with -9
+                      // epilogue, at most 96 or more than 128 rows and not too few tiles; what is not taken is refused with -9
 };
 
 typedef struct RbGemmArgs {

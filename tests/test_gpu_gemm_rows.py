@@ -61,10 +61,10 @@ def test_residual_in_place_and_graph_replay(cuda_status):
 
 
 @pytest.mark.parametrize("M", [1, 17, 96, 97, 129, 300, 513])
-@pytest.mark.parametrize("F,K", [(8, 64), (64, 72), (72, 768), (200, 2048), (1000, 264)])
+@pytest.mark.parametrize("F,K", [(8, 64), (64, 72), (72, 768), (200, 2048), (1000, 264), (2504, 72), (3200, 2048)])
 def test_swiglu_product(M, F, K, cuda_status):
     """Gates and ups of one result column come from two places of the weight: edges of 64- and 128-column tiles, rows of both kernels and of
-    neither, and a weight whose rows behind the gates are the ups (a tile that ends in the middle reads into them)."""
+    neither, with more than 128 rows few tiles (two launches) and many, and a weight whose rows behind the gates are the ups (a tile that ends in the middle reads into them)."""
     from rustral_b200.ops.rotary import swiglu_product
     x, w, _, _ = _operands(M, 2 * F, K)
     w = (w.float() * K ** -0.5).bfloat16()
