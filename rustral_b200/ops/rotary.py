@@ -205,6 +205,8 @@ def swiglu_product(a: torch.Tensor, w: torch.Tensor, b_constant: bool = False) -
     from . import matmul
     M, K = a.shape
     F = w.shape[0] // 2
+    if w.shape[0] % 2 or a.device != w.device:
+        raise ValueError("swiglu_product: as many gates as ups, on the device of the rows, are required")
     if a.is_cuda and a.dtype == w.dtype == torch.bfloat16 and M and F % 8 == 0 and K == w.shape[1] and a.stride(1) == 1 and w.stride(1) == 1 and \
             not (a.stride(0) | w.stride(0) | K) & 7 and not (a.data_ptr() | w.data_ptr()) & 15:
         out = torch.empty((M, F), dtype=a.dtype, device=a.device)

@@ -75,3 +75,11 @@ def test_swiglu_product(M, F, K, cuda_status):
     bound = 2.0 ** -7 * want.abs() + 2.0 ** -7 * 1.1 * (g * u).abs() + 1e-5
     assert ((got.double() - want).abs() <= bound).all()
     assert torch.equal(got, swiglu_product(x, w, b_constant=True))
+
+
+def test_swiglu_product_refuses_weights_that_are_no_gates_and_ups(cuda_status):
+    from rustral_b200.ops.rotary import swiglu_product
+    x, w, _, _ = _operands(5, 34, 64)
+    for a, b in ((x, w[:33]), (x.cpu(), w[:33].cpu()), (x, w.cpu()), (x, w[:, :56])):
+        with pytest.raises(ValueError):
+            swiglu_product(a, b)
