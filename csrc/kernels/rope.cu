@@ -21,7 +21,7 @@ __device__ __forceinline__ void rope_unit(const float (&c)[8], const float (&s)[
   }
 }
 
-// Where rotated keys and the values behind them go besides their own place (rb_rope_append); slots nullptr: nowhere.
+// Where rotated keys and the values behind them go besides their own place (rb_rope_append).
 struct RopeCache {
   __nv_bfloat16* k;
   __nv_bfloat16* v;
@@ -33,7 +33,7 @@ struct RopeCache {
 // One thread handles 8 neighbouring pairs of HPT heads of a token: the angles' cosines and sines (with their range reduction most of the
 // work) are formed once for all of them.  Per token: (heads / HPT, rounded up) x (half / 8) rotating units, then, with a cache, units that copy
 // 16 bytes of the values.
-template <int HPT, typename Index>
+template <int HPT, bool CACHE, typename Index>
 __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __restrict__ positions, long long tokens,
             int heads, int head_dim, int seq_len, long long pos_offset, float log2_theta, int inverse, const RopeCache cache RB_BOUNDS_PARAM) {
@@ -42,14 +42,14 @@ rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __rest
   const int half = head_dim / 2;
   const int groups = half / 8;
   const int turns = (heads + HPT - 1) / HPT * groups;
-  const int units = turns + (cache.slots ? cache.kv_heads * head_dim / 8 : 0);
+  const int units = turns + (CACHE ? cache.kv_heads * head_dim / 8 : 0);
   const Index total = static_cast<Index>(tokens) * units, stride = static_cast<Index>(gridDim.x) * blockDim.x;
   for (Index i = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     const Index row_of = i / units;
     const long long t = static_cast<long long>(row_of);
     const int u = static_cast<int>(i - row_of * units);
     long long slot = -1;                                   // a negative slot means "skip this token"
-    if (cache.slots) {
+    if (CACHE) {
       slot = cache.slots[t];
       if (slot >= cache.num_slots) {
         if (u == 0) RB_BOUNDS_HIT(103);
@@ -57,7 +57,7 @@ rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __rest
       }
     }
     const long long row = slot * cache.kv_heads * head_dim;
-    if (u >= turns) {
+    if (CACHE && u >= turns) {
       const int c = (u - turns) * 8;
       if (slot >= 0) *reinterpret_cast<uint4*>(cache.v + row + c) = *reinterpret_cast<const uint4*>(x + t * ld + static_cast<long long>(heads) * head_dim + c);
       continue;
@@ -81,7 +81,7 @@ rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __rest
       rope_unit(c, s, lo, hi);
       *reinterpret_cast<uint4*>(p) = lo;
       *reinterpret_cast<uint4*>(p + half) = hi;
-      if (slot >= 0 && h >= cache.heads) {
+      if (CACHE && slot >= 0 && h >= cache.heads) {
         __nv_bfloat16* k = cache.k + row + static_cast<long long>(h - cache.heads) * head_dim + gidx * 8;
         *reinterpret_cast<uint4*>(k) = lo;
         *reinterpret_cast<uint4*>(k + half) = hi;
@@ -209,13 +209,15 @@ void rope_launch(__nv_bfloat16* x, long long ld, const long long* positions, lon
                  long long pos_offset, float theta, int inverse, const rb::RopeCache& cache, cudaStream_t stream) {
   const int len = seq_len < 1 ? 1 : seq_len;
   const long long copies = cache.slots ? cache.kv_heads * head_dim / 8 : 0, groups = head_dim / 16;
-  // Four heads per thread where that still leaves a thread for every lane of the GPU: 40 heads of 128, rotation and append of 8192 tokens
-  // 65.0 us with one head per thread, 47.0 with four (64 tokens, one head per thread, one launch: 3.3 instead of 4.6).  32-bit divisions where the
-  // counts allow.
-  const bool wide = tokens * ((heads + 3) / 4 * groups + copies) >= 148 * 2048;
+  // Four heads per thread where that still leaves a thread for every lane of the GPU, and only where nothing is copied beside the rotation: 40
+  // heads of 128, 8192 tokens 65.0 us with one head per thread, 47.0 with four (rotation and append in one launch 53.3; 64 tokens, one head per
+  // thread, one launch: 3.3 instead of 4.6).  32-bit divisions where the counts allow.
+  const bool wide = !cache.slots && tokens * ((heads + 3) / 4 * groups) >= 148 * 2048;
   const long long total = tokens * ((wide ? (heads + 3) / 4 : heads) * groups + copies);
-  auto kern = total >= (1ll << 31) ? rb::rope_kernel<4, unsigned long long>
-                                   : wide ? rb::rope_kernel<4, unsigned int> : rb::rope_kernel<1, unsigned int>;
+  const bool large = total >= (1ll << 31);
+  auto kern = cache.slots ? (large ? rb::rope_kernel<1, true, unsigned long long> : rb::rope_kernel<1, true, unsigned int>)
+              : wide      ? (large ? rb::rope_kernel<4, false, unsigned long long> : rb::rope_kernel<4, false, unsigned int>)
+                          : rb::rope_kernel<1, false, unsigned int>;
   rbhost::launch_pdl(kern, dim3(rb::grid1d(total)), dim3(256), 0, stream, 1, x, ld, positions, tokens, heads, head_dim, len, pos_offset,
                      log2f(theta), inverse, cache RB_BOUNDS_ARG);
 }

@@ -51,6 +51,14 @@ def rope_append_(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, po
     """Rotates the query and key heads of qkv [tokens, (heads + 2 kv_heads) * head_dim] in place and stores keys and values in their cache
     slots (int64, negative: not stored): `rope_` and `paged.kv_append`, in one launch where that is faster."""
     nb, bs, hk, d = k_cache.shape
+    if qkv.is_cuda:
+        caches = (k_cache, v_cache)
+        if qkv.dtype != torch.bfloat16 or qkv.stride(1) != 1 or (hk, d) != (kv_heads, head_dim) or v_cache.shape != k_cache.shape or \
+                any(c.dtype != torch.bfloat16 or not c.is_contiguous() or c.device != qkv.device for c in caches):
+            raise TypeError("rope_append: bf16 rows with a contiguous last dimension and contiguous bf16 caches of the same heads are required")
+        if slots.dtype != torch.int64 or not slots.is_contiguous() or slots.shape != qkv.shape[:1] or positions.shape != qkv.shape[:1] or \
+                slots.device != qkv.device or positions.device != qkv.device:
+            raise TypeError("rope_append: a position and an int64 slot for every row, on its device, are required")
     # Prompts of many tokens (a thread for every lane of the GPU, see rope.cu): there the copies of the values only hold up threads that
     # rotate, and two launches are the faster way (8192 tokens, 40 heads of 128: 47.0 us against 53.3; 64 tokens: 4.6 against 3.3)
     many = qkv.shape[0] * ((heads + kv_heads + 3) // 4 * (head_dim // 16) + kv_heads * head_dim // 8) >= 148 * 2048
@@ -59,8 +67,6 @@ def rope_append_(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, po
         rope_(qkv, heads + kv_heads, head_dim, positions=positions, theta=theta)
         paged.kv_append(qkv[:, heads * head_dim:(heads + kv_heads) * head_dim], qkv[:, (heads + kv_heads) * head_dim:], k_cache, v_cache, slots)
         return qkv
-    if qkv.dtype != torch.bfloat16 or qkv.stride(1) != 1 or (hk, d) != (kv_heads, head_dim) or v_cache.shape != k_cache.shape:
-        raise TypeError("rope_append: bf16 rows with a contiguous last dimension and a cache of the same heads are required")
     N.check(N.kernels().rb_rope_append(qkv.data_ptr(), qkv.stride(0), positions.to(torch.int64).contiguous().data_ptr(), qkv.shape[0], heads, kv_heads,
                                        head_dim, theta, k_cache.data_ptr(), v_cache.data_ptr(), slots.data_ptr(), nb * bs, N.stream_ptr()),
             "rb_rope_append")

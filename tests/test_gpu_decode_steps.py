@@ -2,15 +2,25 @@
 import pytest
 import torch
 
+from rustral_b200 import _native as N
 from rustral_b200.ops import paged
 from rustral_b200.ops import rotary
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("tokens,heads,kv,dim", [(1, 4, 1, 64), (7, 6, 2, 80), (33, 16, 4, 128), (9000, 30, 5, 64)])
+def _rotated(x, pos, heads, dim, inverse):
+    """x [rows, heads * dim] in 64 bits, turned by its positions; the bound: a bf16 result, fp32 angles up to 20000 (2^-24 of them)."""
+    freq = 10000.0 ** (-torch.arange(dim // 2, device="cuda").double() * 2 / dim)
+    a = pos.double()[:, None, None] * freq * (-1 if inverse else 1)
+    u, v = x.double().view(x.shape[0], heads, dim).split(dim // 2, -1)
+    want = torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], -1)
+    return want, 2.0 ** -8 * want.abs() + 20000 * 2.0 ** -22 * (u.abs() + v.abs()).repeat(1, 1, 2)
+
+
+@pytest.mark.parametrize("tokens,heads,kv,dim", [(1, 4, 1, 64), (7, 6, 2, 80), (33, 16, 4, 128), (3000, 30, 5, 64)])
 def test_rope_append_is_rope_and_append(tokens, heads, kv, dim, cuda_status):
-    """One head per thread and four (the last case, with a count of heads that four does not divide); skipped tokens; wide rows."""
+    """The one launch against the two, bit for bit; skipped tokens; wide rows."""
     g = torch.Generator(device="cuda").manual_seed(tokens)
     cols = (heads + 2 * kv) * dim
     qkv = torch.randn(tokens, cols + 8, device="cuda", generator=g).bfloat16()[:, :cols]
@@ -20,18 +30,42 @@ def test_rope_append_is_rope_and_append(tokens, heads, kv, dim, cuda_status):
     slots[::5] = -1
     kc, vc = (torch.zeros((tokens + 47) // 16, 16, kv, dim, device="cuda", dtype=torch.bfloat16) for _ in range(2))
     kc2, vc2 = kc.clone(), vc.clone()
+    before = N.launch_count
     rotary.rope_append_(qkv, heads, kv, dim, pos, 10000.0, kc, vc, slots)
+    assert N.launch_count == before + 1                       # none of these is long enough for two launches
     rotary.rope_(other, heads + kv, dim, positions=pos, theta=10000.0)
     paged.kv_append(other[:, heads * dim:(heads + kv) * dim], other[:, (heads + kv) * dim:], kc2, vc2, slots)
     assert torch.equal(qkv, other) and torch.equal(kc, kc2) and torch.equal(vc, vc2)
-    # against 64 bits: bf16 result, fp32 angles up to 20000 (2^-24 of them)
-    x = torch.randn(tokens, heads * dim, device="cuda", generator=g).bfloat16()
-    freq = 10000.0 ** (-torch.arange(dim // 2, device="cuda").double() * 2 / dim)
-    a = pos.double()[:, None] * freq
-    u, v = x.double().view(tokens, heads, dim).split(dim // 2, -1)
-    want = torch.cat([u * a.cos()[:, None] - v * a.sin()[:, None], v * a.cos()[:, None] + u * a.sin()[:, None]], -1)
-    got = rotary.rope_(x.clone(), heads, dim, positions=pos, theta=10000.0).view(tokens, heads, dim).double()
-    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 20000 * 2.0 ** -22 * (u.abs() + v.abs()).repeat(1, 1, 2)).all()
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+@pytest.mark.parametrize("tokens,heads,dim", [(7, 6, 80), (12000, 30, 64), (6000, 29, 128)])
+def test_rotation_against_64_bit(tokens, heads, dim, inverse, cuda_status):
+    """One head per thread, and four where that leaves a thread for every lane of the GPU (the two long ones), with counts of heads that four
+    does not divide."""
+    assert (tokens * ((heads + 3) // 4) * (dim // 16) >= 148 * 2048) == (tokens > 1000)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    pos = torch.randint(0, 20000, (tokens,), device="cuda", generator=g)
+    x = torch.randn(tokens, heads * dim + 8, device="cuda", generator=g).bfloat16()
+    want, bound = _rotated(x[:, :heads * dim].contiguous(), pos, heads, dim, inverse)
+    got = x.clone()
+    rotary.rope_(got, heads, dim, positions=pos, theta=10000.0, inverse=inverse)
+    assert torch.equal(got[:, heads * dim:], x[:, heads * dim:])
+    assert ((got[:, :heads * dim].double().view(tokens, heads, dim) - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("tokens", [3, 9000])
+def test_rope_append_refuses_what_it_cannot_address(tokens, cuda_status):
+    """The one launch and the two refuse the same: caches of other heads or types, slots of another type or number."""
+    heads, kv, dim = 30, 5, 64
+    qkv = torch.zeros(tokens, (heads + 2 * kv) * dim, device="cuda").bfloat16()
+    pos, slots = torch.arange(tokens, device="cuda"), torch.full((tokens,), -1, device="cuda")
+    cache = torch.zeros(2, 16, kv, dim, device="cuda").bfloat16()
+    rotary.rope_append_(qkv, heads, kv, dim, pos.int(), 10000.0, cache, cache.clone(), slots)
+    for bad in (dict(k=cache.view(2, 16, 1, kv * dim), v=cache.view(2, 16, 1, kv * dim)), dict(v=cache.float()), dict(k=cache.cpu()),
+                dict(slots=slots.int()), dict(slots=slots[1:]), dict(slots=torch.stack([slots, slots], 1)[:, 0]), dict(pos=pos[1:])):
+        with pytest.raises(TypeError):
+            rotary.rope_append_(qkv, heads, kv, dim, bad.get("pos", pos), 10000.0, bad.get("k", cache), bad.get("v", cache), bad.get("slots", slots))
 
 
 @pytest.mark.parametrize("batch,heads,kv,dim,longest,width", [(1, 8, 2, 128, 2500, 400), (64, 8, 4, 128, 1300, 1024), (120, 32, 16, 64, 700, 64),
