@@ -1601,6 +1601,16 @@ int gemm_fp8(const RbGemmArgs& g, int sms, int bn, int splits, cudaStream_t stre
 
 }  // namespace
 
+RB_API long long rb_gemm_workspace(const RbGemmArgs* args, long long most) {
+  RbGemmArgs g = *args;
+  g.workspace = &g;                           // any address: nothing is launched
+  g.workspace_bytes = most;
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.act == RB_ACT_SWIGLU || rbhost::gemm_rows_takes(g)) return 0;
+  int bn = 128, splits = 1;
+  pick_plan(g, rbhost::device_sm_count(), bn, splits);
+  return splits > 1 ? static_cast<long long>(splits) * g.M * g.N * 4 : 0;
+}
+
 RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
   const RbGemmArgs& g = *args;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);

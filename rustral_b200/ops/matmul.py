@@ -163,6 +163,21 @@ def _workspace(device) -> torch.Tensor:
     return ws
 
 
+N.optional_sig("rb_gemm_workspace", [N.C.POINTER(N.RbGemmArgs), N.c_ll], N.c_ll)
+
+
+def _give_workspace(g, device):
+    """Names the split-K scratch in `g`; what is returned has to live until the launch.  A captured graph gets its own, as much as the plan
+    takes: graphs that name one buffer could not be replayed side by side."""
+    if torch.cuda.is_current_stream_capturing():
+        n = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES)
+        ws = torch.empty(n, dtype=torch.uint8, device=device) if n > 0 else None
+    else:
+        ws = _workspace(device)
+    g.workspace, g.workspace_bytes = N.ptr(ws), ws.numel() if ws is not None else 0
+    return ws
+
+
 _plain_tls = threading.local()
 
 
@@ -296,8 +311,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             cache[key] = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
         if splits != 1 and K >= 2048 and act == "none":
-            ws = _workspace(a.device)
-            g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
+            ws = _give_workspace(g, a.device)  # noqa: F841
         N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
         return out
     for t, nm in ((bias, "bias"), (residual, "residual"), (aux_in, "aux_in"), (aux_out, "aux_out")):
@@ -335,8 +349,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.peer_ptrs[r] = pp
         g.splits = 1
     elif splits != 1 and K >= 2048 and act == "none":
-        ws = _workspace(a.device)
-        g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
+        ws = _give_workspace(g, a.device)  # noqa: F841
     N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
     return out
 

@@ -155,3 +155,33 @@ def test_a_captured_graph_owns_its_scratch(cuda_status):
     torch.cuda.empty_cache()
     graph.replay()
     assert torch.equal(got, want) and torch.equal(got_wide, want_wide) and torch.isfinite(total)
+
+
+@pytest.mark.parametrize("splits", [0, 3])
+def test_a_captured_graph_owns_its_split_products_scratch(splits, cuda_status):
+    """Two graphs whose products split their contraction, replayed side by side on two streams: each has slabs of its own, and the buffer of
+    the streams' direct calls is not among them."""
+    from rustral_b200.ops import matmul
+    from rustral_b200.ops.matmul import gemm
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    a, b = ([torch.randn(16384, n, device="cuda", generator=g).bfloat16() for _ in range(2)] for n in (256, 384))
+    want = [gemm(x, y, a_mn=True, b_mn=True, out_dtype=torch.float32, splits=splits) for x, y in zip(a, b)]
+    before = {k: v.data_ptr() for k, v in matmul._workspaces.items()}
+    graphs, got = [], []
+    for x, y in zip(a, b):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            got.append(gemm(x, y, a_mn=True, b_mn=True, out_dtype=torch.float32, splits=splits))
+    assert {k: v.data_ptr() for k, v in matmul._workspaces.items()} == before
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(5):
+        for t in got:
+            t.zero_()
+        torch.cuda.synchronize()
+        for s, graph in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                for _ in range(10):
+                    graph.replay()
+        torch.cuda.synchronize()
+        for t, w in zip(got, want):
+            assert torch.equal(t, w)
