@@ -165,9 +165,12 @@ def route_backward(probs, idx, w, dw, counts, renorm: bool, aux_grad_scale):
         dp = dp + aux_grad_scale * E * (counts.float() / (T * k))[None, :] / T
         return probs * (dp - (dp * probs).sum(-1, keepdim=True))
     out = torch.empty_like(probs)
-    scale = torch.as_tensor(aux_grad_scale, dtype=torch.float32, device=probs.device)
+    if isinstance(aux_grad_scale, torch.Tensor):
+        scale = aux_grad_scale.to(device=probs.device, dtype=torch.float32)
+    else:                                       # filled there: a copy from the host would wait, and cannot be captured
+        scale = torch.full((), float(aux_grad_scale), device=probs.device) if aux_grad_scale else None
     N.check(N.kernels().rb_moe_route_bwd(probs.data_ptr(), idx.data_ptr(), w.data_ptr(), dw.contiguous().data_ptr(),
-                                         counts.data_ptr(), T, E, k, int(renorm), scale.data_ptr(), out.data_ptr(),
+                                         counts.data_ptr(), T, E, k, int(renorm), N.ptr(scale), out.data_ptr(),
                                          N.stream_ptr()), "rb_moe_route_bwd")
     return out
 

@@ -185,3 +185,22 @@ def test_a_captured_graph_owns_its_split_products_scratch(splits, cuda_status):
         torch.cuda.synchronize()
         for t, w in zip(got, want):
             assert torch.equal(t, w)
+
+
+def test_routing_gradient_takes_a_number_under_capture(cuda_status):
+    """The scale of the balancing loss as a number, as a tensor and as nothing, directly and captured."""
+    from rustral_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(1)
+    logits, dw = torch.randn(40, 8, device="cuda", generator=g), torch.randn(40, 2, device="cuda", generator=g)
+    idx, w, probs = moe.route(logits, 2, True)
+    counts = torch.bincount(idx.reshape(-1).long(), minlength=8).int()
+    call = lambda s: moe.route_backward(probs, idx, w, dw, counts, True, s)  # noqa: E731
+    want = [call(torch.tensor(s, device="cuda")) for s in (0.25, 0.0)]
+    cpu = moe.route_backward(probs.cpu(), idx.cpu(), w.cpu(), dw.cpu(), counts.cpu(), True, 0.25)
+    assert torch.allclose(want[0].cpu(), cpu, rtol=1e-4, atol=1e-6)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [call(0.25), call(0.0)]
+    graph.replay()
+    for a, b, c in zip(want, got, (0.25, 0.0)):
+        assert torch.equal(a, b) and torch.equal(a, call(c))
