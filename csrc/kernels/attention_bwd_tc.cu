@@ -537,10 +537,10 @@ RB_API int rb_attention_delta_tc(const RbAttnArgs* a, void* stream_v) {
   const __nv_bfloat16* o = reinterpret_cast<const __nv_bfloat16*>(a->o);
   const __nv_bfloat16* d_o = reinterpret_cast<const __nv_bfloat16*>(a->d_o);
   if (D == 64)
-    rbhost::launch_pdl(rb::attn_delta_tc_kernel<64>, dim3(dgrid), dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
+    rbhost::launch_pdl(rb::attn_delta_tc_kernel<64>, dgrid, dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
                                                              a->o_strides[2], a->heads, a->seq_q);
   else
-    rbhost::launch_pdl(rb::attn_delta_tc_kernel<128>, dim3(dgrid), dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
+    rbhost::launch_pdl(rb::attn_delta_tc_kernel<128>, dgrid, dim3(256), 0, stream, 1, o, d_o, a->delta, a->o_strides[0], a->o_strides[1],
                                                               a->o_strides[2], a->heads, a->seq_q);
   return static_cast<int>(cudaGetLastError());
 }

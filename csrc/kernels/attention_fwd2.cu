@@ -673,7 +673,7 @@ int f2_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* t
     if (e != cudaSuccess) return static_cast<int>(e);
     cfg = true;
   }
-  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kF2Threads), smem, stream, 1, *tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk, p, rbhost::status_ptr());
+  rbhost::launch_pdl(kern, grid, dim3(rb::kF2Threads), smem, stream, 1, *tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk, p, rbhost::status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 }  // namespace

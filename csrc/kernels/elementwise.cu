@@ -133,7 +133,7 @@ int launch_pointwise(int op, const void* a, const void* b, float s, void* out, l
     if (done < n) {
       auto A = reinterpret_cast<const __nv_bfloat16*>(a);
       auto B = reinterpret_cast<const __nv_bfloat16*>(b);
-      rbhost::launch_pdl(pointwise_kernel<__nv_bfloat16, MODE>, dim3(ew_grid(n - done)), dim3(256), 0, st, 1, 
+      rbhost::launch_pdl(pointwise_kernel<__nv_bfloat16, MODE>, dim3(ew_grid(n - done)), dim3(256), 0, st, 1,
           op, A ? A + done : A, B ? B + done : B, s, reinterpret_cast<__nv_bfloat16*>(out) + done, n - done);
     }
   } else {
@@ -466,10 +466,10 @@ RB_API int rb_sum_dim0_staged(const void* a, long long lda, float* out, float* p
   // 64 rows or more per slab: each of the 8 row lanes of a block then has its 8 loads in flight
   if ((rows + 63) / 64 < slabs) slabs = static_cast<int>((rows + 63) / 64);
   dim3 grid((cols + 255) / 256, slabs);
-  if (dtype == 0) rbhost::launch_pdl(rb::sum_dim0_stage1<float>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const float*)a, lda, partial, rows, cols);
+  if (dtype == 0) rbhost::launch_pdl(rb::sum_dim0_stage1<float>, grid, dim3(256), 0, RB_STREAM, 1, (const float*)a, lda, partial, rows, cols);
   else if ((cols % 8 == 0) && (lda % 8 == 0) && (reinterpret_cast<uintptr_t>(a) % 16 == 0))
     rbhost::launch_pdl(rb::sum_dim0_stage1_vec, dim3((cols + 255) / 256, slabs), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
-  else rbhost::launch_pdl(rb::sum_dim0_stage1<__nv_bfloat16>, dim3(grid), dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
+  else rbhost::launch_pdl(rb::sum_dim0_stage1<__nv_bfloat16>, grid, dim3(256), 0, RB_STREAM, 1, (const __nv_bfloat16*)a, lda, partial, rows, cols);
   rbhost::launch_pdl(rb::sum_dim0_stage2, dim3((cols + 31) / 32), dim3(1024), 0, RB_STREAM, 1, partial, slabs, out, cols, accumulate);
   return static_cast<int>(cudaGetLastError());
 }

@@ -206,7 +206,7 @@ RB_API int rb_embedding_fwd(const long long* ids, const void* wte, const void* w
   const long long total = tokens * (dim / 8);
   long long blocks = (total + 127) / 128;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
-  rbhost::launch_pdl(rb::embedding_fwd_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, stream, 1, 
+  rbhost::launch_pdl(rb::embedding_fwd_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, stream, 1,
       ids, reinterpret_cast<const __nv_bfloat16*>(wte), reinterpret_cast<const __nv_bfloat16*>(wpe),
       reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, seq_len < 1 ? 1 : seq_len, vocab RB_BOUNDS_ARG);
   return static_cast<int>(cudaGetLastError());

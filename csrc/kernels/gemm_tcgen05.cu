@@ -1021,7 +1021,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // TMEM.  Per k-block a CTA moves 16 KB + 16 KB instead of 16 KB + 32 KB through the L2 -> SM fabric, which is what
 // bounds the one-CTA kernel on short-K problems.  No TMA multicast: every load targets the loading CTA's own memory
 // and reports its bytes to the leader's barrier; tcgen05.commit signals both CTAs' barriers.
-// Plain (non-grouped, non-peer) problems only; the epilogue is the staged / direct epilogue of the one-CTA kernel.
+// Plain (non-grouped, non-peer) problems only; results leave through TMA (`epilogue_tma`, `epilogue_swiglu`) or, where they cannot, straight
+// from registers.
 // ------------------------------------------------------------------------------------------------------------------
 template <int BLOCK_N, int STAGES>
 struct SmemLayoutPair {

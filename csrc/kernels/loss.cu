@@ -235,7 +235,7 @@ RB_API int rb_cross_entropy(const void* logits, long long ld, const long long* t
                             long long ignore_index, void* stream_v) {
   if (rows <= 0 || n_valid <= 0 || n_pad < n_valid || !logits || !targets || !loss) return -1;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  rbhost::launch_pdl(rb::cross_entropy_kernel, dim3(rows), dim3(rb::kCeThreads), 0, stream, 1, 
+  rbhost::launch_pdl(rb::cross_entropy_kernel, dim3(rows), dim3(rb::kCeThreads), 0, stream, 1,
       reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, loss, lse, reinterpret_cast<__nv_bfloat16*>(dlogits),
       ldd, n_valid, n_pad, grad_scale, ignore_index RB_BOUNDS_ARG);
   return static_cast<int>(cudaGetLastError());

@@ -264,9 +264,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
   }
 }
 
-// out[col] (+)= sum_p partial[p][col].  Eight row groups per CTA each sum every eighth partial, then the
-// groups are folded in index order: parallel enough to hide latency, and the order is fixed.
-// 32 columns per block, 32 lanes share a column's partials and add theirs in order: with 8 lanes a fold took 5 us for rows of any length.
+// out[col] (+)= sum_p partial[p][col].  32 columns per block; 32 lanes share a column's partials, each adds every 32nd in order, and the lanes'
+// sums are folded in index order: the order is fixed.  With 8 lanes a fold took 5 us for rows of any length.
 __global__ void __launch_bounds__(1024)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int num_partials, int n, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, int accumulate) {
@@ -346,9 +345,9 @@ RB_API int rb_norm_fwd(const void* x, long long ldx, const void* gamma, const vo
   auto B = reinterpret_cast<const __nv_bfloat16*>(beta);
   auto Y = reinterpret_cast<__nv_bfloat16*>(y);
 #define RB_LAUNCH(C, W)                                                                                           \
-  if (rms) rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, true>, dim3(grid), dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, nullptr, Y, ldy,  \
+  if (rms) rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, true>, grid, dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, nullptr, Y, ldy,  \
                                                                                      nullptr, rstd, rows, n, eps);\
-  else rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, false>, dim3(grid), dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, B, Y, ldy, mean,     \
+  else rbhost::launch_pdl(rb::norm_fwd_kernel<C, W, false>, grid, dim3(rb::kNormWarps * 32), 0, stream, 1, X, ldx, G, B, Y, ldy, mean,     \
                                                                                   rstd, rows, n, eps);
   RB_NORM_DISPATCH(n, RB_LAUNCH)
 #undef RB_LAUNCH
@@ -379,12 +378,12 @@ RB_API int rb_norm_bwd(const void* dy, long long lddy, const void* x, long long 
     if (rms) {                                                                                                     \
       auto k = rb::norm_bwd_kernel<C, W, true>;                                                                    \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-      rbhost::launch_pdl(k, dim3(grid), dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
+      rbhost::launch_pdl(k, grid, dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
                                                      partial, rows, n);                                            \
     } else {                                                                                                       \
       auto k = rb::norm_bwd_kernel<C, W, false>;                                                                   \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-      rbhost::launch_pdl(k, dim3(grid), dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
+      rbhost::launch_pdl(k, grid, dim3(rb::kNormWarps * 32), smem, stream, 1, DY, lddy, X, ldx, G, mean, rstd, DR, lddres, DX, lddx,        \
                                                      partial, rows, n);                                            \
     }                                                                                                              \
   }

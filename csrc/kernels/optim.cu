@@ -151,7 +151,9 @@ __global__ void __launch_bounds__(256) sumsq_stage2(const float* __restrict__ sc
 }
 __global__ void sqrt_scalar_kernel(const float* in, float* out) {
   pdl_wait();
-  pdl_launch(); out[0] = sqrtf(in[0]); }
+  pdl_launch();
+  out[0] = sqrtf(in[0]);
+}
 
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ d, long long n) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * 4;
@@ -194,10 +196,10 @@ RB_API int rb_adam_step(float* p, float* m, float* v, const void* g, int g_bf16,
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   const int grid = rb::grid_for(n, 4);
   if (g_bf16)
-    rbhost::launch_pdl(rb::adam_kernel<true>, dim3(grid), dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
+    rbhost::launch_pdl(rb::adam_kernel<true>, grid, dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
                                                     grad_norm, found_inf);
   else
-    rbhost::launch_pdl(rb::adam_kernel<false>, dim3(grid), dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
+    rbhost::launch_pdl(rb::adam_kernel<false>, grid, dim3(256), 0, stream, 1, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16), n, *args,
                                                      grad_norm, found_inf);
   return static_cast<int>(cudaGetLastError());
 }

@@ -649,7 +649,7 @@ RB_API int rb_kv_append(const void* k_new, long long ld_k, const void* v_new, lo
   const long long total = tokens * (row / 8);
   long long blocks = (total + 127) / 128;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  rbhost::launch_pdl(rb::kv_append_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
+  rbhost::launch_pdl(rb::kv_append_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream_v), 1,
       reinterpret_cast<const __nv_bfloat16*>(k_new), ld_k, reinterpret_cast<const __nv_bfloat16*>(v_new), ld_v,
       reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), slot_mapping, tokens, row,
       num_slots RB_BOUNDS_ARG);

@@ -267,7 +267,7 @@ RB_API int rb_rotate_pairs(void* x, long long ld, const float* table, long long 
 RB_API int rb_swiglu_fwd(const void* gu, long long ld_gu, void* h, long long ld_h, long long tokens, int F, void* stream_v) {
   if (tokens <= 0 || F <= 0 || (F % 8) || (ld_gu % 8) || (ld_h % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(h)) & 15) return -2;
-  rbhost::launch_pdl(rb::swiglu_fwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
+  rbhost::launch_pdl(rb::swiglu_fwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1,
       reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(h), ld_h, tokens, F);
   return static_cast<int>(cudaGetLastError());
 }
@@ -276,7 +276,7 @@ RB_API int rb_swiglu_bwd(const void* dh, long long ld_dh, const void* gu, long l
                          long long tokens, int F, void* stream_v) {
   if (tokens <= 0 || F <= 0 || (F % 8) || (ld_gu % 8) || (ld_dh % 8) || (ld_dgu % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(dh) | reinterpret_cast<uintptr_t>(dgu)) & 15) return -2;
-  rbhost::launch_pdl(rb::swiglu_bwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1, 
+  rbhost::launch_pdl(rb::swiglu_bwd_kernel, dim3(rb::grid1d(tokens * (F / 8))), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_v), 1,
       reinterpret_cast<const __nv_bfloat16*>(dh), ld_dh, reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu,
       reinterpret_cast<__nv_bfloat16*>(dgu), ld_dgu, tokens, F);
   return static_cast<int>(cudaGetLastError());
