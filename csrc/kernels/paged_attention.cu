@@ -79,8 +79,8 @@ template <int N>
 struct PaInt { static constexpr int value = N; };
 __device__ __forceinline__ float pa_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
-// Split-KV decode attention.  One CTA = (sequence, KV head, 256-token slice of the context); the slices of a sequence
-// run on different SMs and a second kernel merges their (max, sum, accumulator) triples.  Inside a CTA a warp takes
+// Split-KV decode attention.  A CTA takes 256-token slices of the contexts for a KV head, one or a run of them; a second
+// kernel merges the (max, sum, accumulator) triples of a sequence's slices.  Inside a CTA a warp takes
 // 32 tokens at a time.  Their K rows and V rows are fetched with fully coalesced 16-byte asynchronous copies (cp.async,
 // 16 lanes per 256-byte row) into two padded shared tiles per warp; the K tile of the next pass is requested as soon
 // as the scores of this pass are computed and the V tile as soon as P V is done, so every warp always has a tile in
