@@ -166,15 +166,13 @@ def _workspace(device) -> torch.Tensor:
 N.optional_sig("rb_gemm_workspace", [N.C.POINTER(N.RbGemmArgs), N.c_ll], N.c_ll)
 
 
-def _give_workspace(g, device):
-    """Names the split-K scratch in `g`; what is returned has to live until the launch.  A captured graph gets its own, as much as the plan
-    takes: graphs that name one buffer could not be replayed side by side."""
-    if torch.cuda.is_current_stream_capturing():
-        n = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES)
-        ws = torch.empty(n, dtype=torch.uint8, device=device) if n > 0 else None
-    else:
-        ws = _workspace(device)
-    g.workspace, g.workspace_bytes = N.ptr(ws), ws.numel() if ws is not None else 0
+def _give_workspace(g, device, need: int):
+    """Names the split-K scratch in `g`; what is returned has to live until the launch.  `need`: what the plan takes (`rb_gemm_workspace`); with
+    none the plan is the same without scratch.  A captured graph gets its own: graphs that name one buffer could not be replayed side by side."""
+    if not need:
+        return None
+    ws = torch.empty(need, dtype=torch.uint8, device=device) if torch.cuda.is_current_stream_capturing() else _workspace(device)
+    g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
     return ws
 
 
@@ -308,10 +306,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.alpha = alpha
             g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
             g.b_constant = int(b_constant)
-            cache[key] = g
+            need = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES) if splits != 1 and K >= 2048 and act == "none" else 0
+            cache[key] = g, need
+        else:
+            g, need = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
-        if splits != 1 and K >= 2048 and act == "none":
-            ws = _give_workspace(g, a.device)  # noqa: F841
+        ws = _give_workspace(g, a.device, need)  # noqa: F841
         N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
         return out
     for t, nm in ((bias, "bias"), (residual, "residual"), (aux_in, "aux_in"), (aux_out, "aux_out")):
@@ -349,7 +349,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.peer_ptrs[r] = pp
         g.splits = 1
     elif splits != 1 and K >= 2048 and act == "none":
-        ws = _give_workspace(g, a.device)  # noqa: F841
+        cache = _plain_args()
+        key = (M, Nn, K, a_mn, b_mn, accumulate, block_n, group_m, max_ctas, splits, aux_in is None, aux_out is None)
+        need = cache.get(key)
+        if need is None:
+            need = cache[key] = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES)
+        ws = _give_workspace(g, a.device, need)  # noqa: F841
     N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
     return out
 

@@ -50,24 +50,28 @@ N.optional_sig("rb_rope_append", [N.c_void_p, N.c_ll, N.c_void_p, N.c_ll, N.c_in
 def rope_append_(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, positions, theta: float, k_cache, v_cache, slots) -> torch.Tensor:
     """Rotates the query and key heads of qkv [tokens, (heads + 2 kv_heads) * head_dim] in place and stores keys and values in their cache
     slots (int64, negative: not stored): `rope_` and `paged.kv_append`, in one launch where that is faster."""
-    nb, bs, hk, d = k_cache.shape
+    shape, tokens = k_cache.shape, qkv.shape[0]
+    nb, bs, hk, d = shape
     if qkv.is_cuda:
-        caches = (k_cache, v_cache)
-        if qkv.dtype != torch.bfloat16 or qkv.stride(1) != 1 or (hk, d) != (kv_heads, head_dim) or v_cache.shape != k_cache.shape or \
-                any(c.dtype != torch.bfloat16 or not c.is_contiguous() or c.device != qkv.device for c in caches):
+        dev, bf16 = qkv.device, torch.bfloat16
+        if not (qkv.dtype is bf16 and qkv.stride(1) == 1 and hk == kv_heads and d == head_dim and v_cache.shape == shape and
+                k_cache.dtype is bf16 and v_cache.dtype is bf16 and k_cache.is_contiguous() and v_cache.is_contiguous() and
+                k_cache.device == dev == v_cache.device):
             raise TypeError("rope_append: bf16 rows with a contiguous last dimension and contiguous bf16 caches of the same heads are required")
-        if slots.dtype != torch.int64 or not slots.is_contiguous() or slots.shape != qkv.shape[:1] or positions.shape != qkv.shape[:1] or \
-                slots.device != qkv.device or positions.device != qkv.device:
+        if not (slots.dtype is torch.int64 and slots.is_contiguous() and slots.dim() == 1 == positions.dim() and
+                slots.shape[0] == tokens == positions.shape[0] and slots.device == dev == positions.device):
             raise TypeError("rope_append: a position and an int64 slot for every row, on its device, are required")
     # Prompts of many tokens (a thread for every lane of the GPU, see rope.cu): there the copies of the values only hold up threads that
     # rotate, and two launches are the faster way (8192 tokens, 40 heads of 128: 47.0 us against 53.3; 64 tokens: 4.6 against 3.3)
-    many = qkv.shape[0] * ((heads + kv_heads + 3) // 4 * (head_dim // 16) + kv_heads * head_dim // 8) >= 148 * 2048
+    many = tokens * ((heads + kv_heads + 3) // 4 * (head_dim // 16) + kv_heads * head_dim // 8) >= 148 * 2048
     if not qkv.is_cuda or many:
         from . import paged
         rope_(qkv, heads + kv_heads, head_dim, positions=positions, theta=theta)
         paged.kv_append(qkv[:, heads * head_dim:(heads + kv_heads) * head_dim], qkv[:, (heads + kv_heads) * head_dim:], k_cache, v_cache, slots)
         return qkv
-    N.check(N.kernels().rb_rope_append(qkv.data_ptr(), qkv.stride(0), positions.to(torch.int64).contiguous().data_ptr(), qkv.shape[0], heads, kv_heads,
+    if positions.dtype is not torch.int64 or not positions.is_contiguous():
+        positions = positions.to(torch.int64).contiguous()
+    N.check(N.kernels().rb_rope_append(qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), tokens, heads, kv_heads,
                                        head_dim, theta, k_cache.data_ptr(), v_cache.data_ptr(), slots.data_ptr(), nb * bs, N.stream_ptr()),
             "rb_rope_append")
     return qkv
@@ -211,7 +215,7 @@ def swiglu_product(a: torch.Tensor, w: torch.Tensor, b_constant: bool = False) -
     from . import matmul
     M, K = a.shape
     F = w.shape[0] // 2
-    if w.shape[0] % 2 or a.device != w.device:
+    if w.shape[0] % 2 or a.get_device() != w.get_device():
         raise ValueError("swiglu_product: as many gates as ups, on the device of the rows, are required")
     if a.is_cuda and a.dtype == w.dtype == torch.bfloat16 and M and F % 8 == 0 and K == w.shape[1] and a.stride(1) == 1 and w.stride(1) == 1 and \
             not (a.stride(0) | w.stride(0) | K) & 7 and not (a.data_ptr() | w.data_ptr()) & 15:

@@ -98,11 +98,11 @@ class _StepMemory:
         self.pinned = device.type == "cuda"
         self.free = deque()                                       # (block, event behind its last copy), oldest first
 
-    def take(self, nbytes: int) -> torch.Tensor:
-        """`nbytes` of a block that no copy reads any more; `give` hands it back."""
+    def take(self, nbytes: int) -> tuple:
+        """A block of at least `nbytes` that no copy reads any more, and the event that `give` records behind the copies out of it."""
         if not self.pinned:
-            return torch.empty(nbytes, dtype=torch.uint8)
-        block = None
+            return torch.empty(nbytes, dtype=torch.uint8), None
+        block = copied = None
         if len(self.free) > 1:
             try:
                 block, copied = self.free.popleft()
@@ -111,12 +111,11 @@ class _StepMemory:
                 pass
         if block is None or block.numel() < nbytes:
             block = torch.empty(1 << max(16, (nbytes - 1).bit_length()), dtype=torch.uint8, pin_memory=True)
-        return block
+        return block, copied or torch.cuda.Event()
 
-    def give(self, block: torch.Tensor) -> None:
+    def give(self, block: torch.Tensor, copied) -> None:
         """All copies out of `block` have been issued on the current stream."""
         if self.pinned and len(self.free) < 8:
-            copied = torch.cuda.Event()
             copied.record()
             self.free.append((block, copied))
 
@@ -264,7 +263,7 @@ class ModelRunner:
         rd = sum(len(c[1]) for c in chunks)
         T = rd + len(dec_ids)
         width = max((len(self.cache.block_table(s_)) for s_ in dec_ids), default=0)
-        memory = self._memory.take(24 * T + 4 * len(dec_ids) * width)
+        memory, copied = self._memory.take(24 * T + 4 * len(dec_ids) * width)
         host = memory[:24 * T].view(torch.int64).view(3, T)          # token ids, positions, cache slots
         ids_h, at_pos, at_slots = host[0].numpy(), host[1].data_ptr(), host[2].data_ptr()
         spans, tables, r0 = [], [], 0
@@ -285,7 +284,7 @@ class ModelRunner:
             self.cache.fill_tables(dec_ids, bt)
             bt = bt.to(dev, non_blocking=True)
             ctx = torch.tensor(dec_len, dtype=torch.int32, device=dev)
-        self._memory.give(memory)
+        self._memory.give(memory, copied)
         segments = None
         if self.recurrent:
             table = [(r0, r1 - r0, self.cache.state_slot(c[0]), start) for (r0, r1, start), c in zip(spans, chunks)]
@@ -372,14 +371,14 @@ class ModelRunner:
             if self.recurrent:
                 g["seg"] = Segments(torch.zeros((B, 4), dtype=torch.int32, device=dev), None)
             self._graphs[(B, width)] = g
-        memory = self._memory.take(g["buf"].numel())
+        memory, copied = self._memory.take(g["buf"].numel())
         host = memory[:g["buf"].numel()]
         view = self._step_views(host, B, width)
         view["ids"].numpy()[:] = last_tokens
         view["ctx"].numpy()[:] = context_lens
         self.cache.fill_tables(seq_ids, view["bt"])
         g["buf"].copy_(host, non_blocking=True)
-        self._memory.give(memory)
+        self._memory.give(memory, copied)
         if g["seg"] is not None:
             g["seg"].table.copy_(torch.tensor(self._decode_segments(seq_ids, context_lens), dtype=torch.int32), non_blocking=True)
         if g["graph"] is None:
