@@ -166,15 +166,15 @@ class EngineLoop:
             ev.set()
 
     def _deliver(self) -> None:
-        """Hands finished requests to their handlers and drops their records."""
+        """Drops the records of finished requests and hands the results to their handlers."""
         eng = self.engine
         eng.scheduler._retire()
         for r in list(eng.scheduler.completed):
-            w = self._waiting.pop(r.id, None)
+            w, tokens = self._waiting.pop(r.id, None), list(r.generated)
+            eng.release(r.id)                        # before the handler wakes and looks
             if w is not None:
-                w[0].append((True, list(r.generated)))
+                w[0].append((True, tokens))
                 w[1].set()
-            eng.release(r.id)
 
     def _run(self) -> None:
         import queue
