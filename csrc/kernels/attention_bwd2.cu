@@ -189,7 +189,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t sRes = sbase + L::kRes, sStream = sbase + L::kStream;
 
   if (warp == kB2ComputeWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------------------------------------------------------- TMA producer
       uint32_t g = 0, wi = 0;
       bool ok = true;
@@ -232,7 +232,9 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else if (warp == kB2ComputeWarps + 1) {
-    if (lane == 0) {
+    // elect.sync, not lane 0: the compiler then knows that one lane runs this and keeps descriptors in uniform registers.  Both passes, one
+    // B200, us behind `lane == 0` / elect.sync: 4 x 4096, 32 (8 KV) heads of 128 2519 / 2230, 32 x 1024, 12 heads of 64 490 / 474
+    if (elect_one()) {
       // ---------------------------------------------------------------- MMA issuer
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, D, 0, 1);    // A from TMEM (K-major), B MN-major
