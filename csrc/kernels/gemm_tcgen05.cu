@@ -23,6 +23,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "pairs.cuh"
 #include "pdl.cuh"
 #include "rb_common.cuh"
 
@@ -351,43 +352,7 @@ __device__ __forceinline__ void epilogue_side_load(const EpiParams& ep, const CU
   __syncwarp();
 }
 
-// Pairs of neighbouring columns, for the packed fp32 instructions.
-struct Pair {
-  unsigned long long v;
-};
-__device__ __forceinline__ Pair pair_of(float lo, float hi) {
-  Pair p;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(lo), "f"(hi));
-  return p;
-}
-__device__ __forceinline__ float2 floats(Pair p) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p.v));
-  return f;
-}
-__device__ __forceinline__ Pair pair_of(uint32_t bf16x2) {
-  const float2 f = unpack_bf16x2(bf16x2);
-  return pair_of(f.x, f.y);
-}
-__device__ __forceinline__ uint32_t packed(Pair p) {
-  const float2 f = floats(p);
-  return pack_bf16x2(f.x, f.y);
-}
-__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
-  Pair d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return d;
-}
-__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
-  Pair d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
-__device__ __forceinline__ Pair add2(Pair a, Pair b) {
-  Pair d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
+// Pairs of neighbouring columns (pairs.cuh).
 __device__ __forceinline__ Pair gelu2(Pair x) {
   constexpr float k0 = 0.7978845608028654f, k1 = 0.044715f;
   const float2 u = floats(mul2(x, fma2(pair_of(k0 * k1, k0 * k1), mul2(x, x), pair_of(k0, k0))));

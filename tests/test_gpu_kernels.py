@@ -385,6 +385,25 @@ def test_flash_attention_backward_tcgen05(B, Sq, Sk, H, Hk, D, causal, impl, cud
     _close(dv, dv3, tol=3e-2, what="tc vs mma dv")
 
 
+@pytest.mark.parametrize("B,Sq,Sk,H,Hk,D,causal", [
+    (16, 290, 290, 12, 12, 64, True), (16, 300, 431, 12, 4, 64, False), (9, 257, 384, 16, 8, 128, True), (20, 130, 130, 16, 16, 128, False),
+])
+def test_flash_attention_backward_walks_several_items(B, Sq, Sk, H, Hk, D, causal, cuda_status):
+    """More owned tiles than SMs: rings, barriers and the resident operands' memory (results leave through it) go around several times, and
+    rows end inside a 32-row copy.  Packed gradients against the one-tile kernel: products of the same bf16 operands, in the same order."""
+    q, k, v, do = (_bf(s, i).cuda() for i, s in enumerate([(B, Sq, H, D), (B, Sk, Hk, D), (B, Sk, Hk, D), (B, Sq, H, D)], 1))
+    scale = 1 / math.sqrt(D)
+    o, lse = attn_ops.attention_forward(q, k, v, causal, scale, impl="tc")
+    ref = attn_ops.attention_backward(do, q, k, v, o, lse, causal, scale, impl="tc")
+    pack = torch.full((B, max(Sq, Sk), (H + 2 * Hk) * D), 7.0, dtype=torch.bfloat16, device="cuda")
+    dq = pack[:, :Sq, :H * D].view(B, Sq, H, D)
+    dk, dv = (pack[:, :Sk, (H + i * Hk) * D:(H + (i + 1) * Hk) * D].view(B, Sk, Hk, D) for i in range(2))
+    attn_ops.attention_backward(do, q, k, v, o, lse, causal, scale, dq=dq, dk=dk, dv=dv, impl="tc2")
+    for name, x, y in zip(("dq", "dk", "dv"), (dq, dk, dv), ref):
+        _close(x, y.cpu(), tol=2 ** -8, what=name)                     # one rounding of the results to bf16
+    assert (pack[:, Sq:, :H * D] == 7).all() and (pack[:, Sk:, H * D:] == 7).all(), "rows behind the sequence were written"
+
+
 @pytest.mark.parametrize("B,S,H,Hk,D,causal,lens", [
     (3, 256, 2, 2, 64, False, [256, 100, 1]), (2, 384, 4, 2, 128, True, [384, 130]), (2, 200, 2, 2, 64, False, [200, 0]),
 ])
