@@ -22,6 +22,7 @@
 //
 // Same semantics as the other forward kernels (causal alignment to the end of the keys, GQA, log-sum-exp output).
 // Replaces the reference's materialised-score attention (crates/nn/src/attention.rs:640-836).
+#define RB_INLINE_WAITS                 // registers are reallocated between warp groups
 #include "attention.h"
 
 #include "pdl.cuh"

@@ -9,6 +9,7 @@
 // launch, first load, exchange and last store are about 4.
 //
 // Roles: warp 0 TMA, warp 1 MMA issue and TMEM, warps 2 to 5 accumulator -> shared memory; then all warps the epilogue.
+#define RB_INLINE_WAITS
 #include "gemm_rows.h"
 
 #include "pdl.cuh"

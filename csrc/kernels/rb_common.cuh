@@ -119,12 +119,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 // Bounded wait.  `abort_flag` is a CTA-shared int: once any waiter gives up, everybody else
-// leaves at their next poll.  Returns false when the wait was abandoned.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned int* status, unsigned int where) {
-#pragma unroll 1
-  for (int i = 0; i < 128; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
+// leaves at their next poll.  Returns false when the wait was abandoned.  What follows the first polls is a function of its own: inlined at
+// each of a kernel's 20 or so waits it was a quarter of its code, and code that is not in the instruction cache costs a lone thread about 200
+// cycles per hundred instructions, in every kernel's first pass and in its issuing thread's every step.  Training steps of GPT-2 shapes, one
+// B200, us: 2 layers of 256 444 -> 437, 6 of 384 1443 -> 1422.  A kernel that reallocates registers cannot call functions, and `gemm_rows.cu`, with few
+// waits, was 1 % slower that way: such files define RB_INLINE_WAITS.
+#ifdef RB_INLINE_WAITS
+__device__ __forceinline__
+#else
+static __device__ __noinline__
+#endif
+bool mbar_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned int* status, unsigned int where) {
   const unsigned long long t0 = globaltimer_ns();
 #pragma unroll 1
   while (true) {
@@ -138,6 +143,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       return false;
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned int* status, unsigned int where) {
+#pragma unroll 1
+  for (int i = 0; i < 128; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_long(bar, parity, abort_flag, status, where);
 }
 
 // ---------------------------------------------------------------------------------------------
