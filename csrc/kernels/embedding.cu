@@ -16,7 +16,7 @@ namespace rb {
 __global__ void __launch_bounds__(128)
 embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ wte,
                      const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out, long long tokens, int dim,
-                     int seq_len, long long vocab RB_BOUNDS_PARAM) {
+                     int seq_len, const int* __restrict__ lengths, long long vocab RB_BOUNDS_PARAM) {
   pdl_wait();
   pdl_launch();
   const int chunks = dim / 8;
@@ -32,7 +32,12 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __r
     }
     uint4 a = __ldg(reinterpret_cast<const uint4*>(wte + id * dim + c));
     if (wpe) {
-      const uint4 b = __ldg(reinterpret_cast<const uint4*>(wpe + (t % seq_len) * dim + c));
+      long long pos = lengths ? lengths[t] - 1 : t % seq_len;
+      if (pos < 0 || pos >= seq_len) {     // positions behind the table read its last row instead of faulting
+        if (c == 0) RB_BOUNDS_HIT(102);
+        pos = seq_len - 1;
+      }
+      const uint4 b = __ldg(reinterpret_cast<const uint4*>(wpe + pos * dim + c));
       float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
       float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y), b2 = unpack_bf16x2(b.z), b3 = unpack_bf16x2(b.w);
       a.x = pack_bf16x2(a0.x + b0.x, a0.y + b0.y); a.y = pack_bf16x2(a1.x + b1.x, a1.y + b1.y);
@@ -199,7 +204,7 @@ RB_API int rb_embedding_residual(const long long* ids, const void* table, int ta
 }
 
 RB_API int rb_embedding_fwd(const long long* ids, const void* wte, const void* wpe, void* out, long long tokens,
-                            int dim, int seq_len, long long vocab, void* stream_v) {
+                            int dim, int seq_len, const int* lengths, long long vocab, void* stream_v) {
   if (tokens <= 0 || dim <= 0 || (dim & 7) || vocab <= 0 || (wpe && seq_len <= 0)) return -1;
   if ((reinterpret_cast<uintptr_t>(wte) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(wpe)) & 15) return -2;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
@@ -208,7 +213,7 @@ RB_API int rb_embedding_fwd(const long long* ids, const void* wte, const void* w
   if (blocks > 148LL * 32) blocks = 148LL * 32;
   rbhost::launch_pdl(rb::embedding_fwd_kernel, dim3(static_cast<int>(blocks)), dim3(128), 0, stream, 1,
       ids, reinterpret_cast<const __nv_bfloat16*>(wte), reinterpret_cast<const __nv_bfloat16*>(wpe),
-      reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, seq_len < 1 ? 1 : seq_len, vocab RB_BOUNDS_ARG);
+      reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, seq_len < 1 ? 1 : seq_len, lengths, vocab RB_BOUNDS_ARG);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -3,9 +3,10 @@
 #ifdef __cplusplus
 extern "C" {
 #endif
-// out[t, :] = wte[ids[t], :] (+ wpe[t % seq_len, :] when wpe != NULL); bf16 tables and output.
+// out[t, :] = wte[ids[t], :] (+ wpe[t % seq_len, :], or wpe[lengths[t] - 1, :] of seq_len rows with lengths, when wpe != NULL); bf16 tables and
+// output.
 int rb_embedding_fwd(const long long* ids, const void* wte, const void* wpe, void* out, long long tokens, int dim,
-                     int seq_len, long long vocab, void* stream);
+                     int seq_len, const int* lengths, long long vocab, void* stream);
 // Start of a 32-bit residual stream: x[t, :] = scale * table[ids[t], :], and h[t, :] = the same row in the table's type
 // (pitch ld_h) when h != NULL (operand of the first matrix products).  table bf16 or fp32.
 int rb_embedding_residual(const long long* ids, const void* table, int table_f32, float* x, void* h, long long ld_h,

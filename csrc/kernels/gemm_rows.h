@@ -7,5 +7,7 @@
 namespace rbhost {
 // Whether `gemm_rows` computes this call (arguments already checked by rb_gemm_bf16).
 bool gemm_rows_takes(const RbGemmArgs& g);
+// Whether it can take the rows through the norm that the call names.
+bool gemm_rows_norm_takes(const RbGemmArgs& g);
 int gemm_rows(const RbGemmArgs& g, cudaStream_t stream);
 }  // namespace rbhost

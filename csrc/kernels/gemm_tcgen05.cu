@@ -1595,6 +1595,11 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
   if (g.b_scale && (reinterpret_cast<uintptr_t>(g.b_scale) & 15)) return -3;
   if ((g.act >= RB_ACT_DGELU && g.act <= RB_ACT_MUL) && !g.aux_in) return -4;
   if (g.act == RB_ACT_RELU2 && g.aux_out) return -4;
+  if (g.norm_gamma) {
+    if (!rbhost::gemm_rows_norm_takes(g) || !rbhost::gemm_rows_takes(g) || (g.act == RB_ACT_SWIGLU && (g.bias || g.residual || g.out_f32))) return -9;
+    if (((reinterpret_cast<uintptr_t>(g.norm_gamma) | reinterpret_cast<uintptr_t>(g.norm_beta)) & 15)) return -3;
+    return rbhost::gemm_rows(g, stream);
+  }
 
   if (g.group_mode < 0 || g.group_mode > 2) return -8;
   if (g.group_mode == 1 && (!g.tile_expert || !g.num_m_tiles || g.b_expert_rows <= 0)) return -8;

@@ -70,6 +70,12 @@ typedef struct RbGemmArgs {
   const void* b_scale;         // fp32 [N] or NULL: one scale per row of B (per output channel)
   int b_constant;              // 1: the kernel in front of this call in its stream does not write B (a served model's weights), so
                                // that B may be read while that kernel still runs
+  // A passes through a norm first (bf16 weights [K]; norm_rms: without mean and beta): at most 8 rows and 16384 numbers, operands and epilogues of
+  // the few-row product; what is not taken is refused with -9
+  const void* norm_gamma;      // NULL: no norm
+  const void* norm_beta;       // or NULL
+  float norm_eps;
+  int norm_rms;
 } RbGemmArgs;
 
 // Returns 0 on success, a negative code for rejected arguments, a positive cudaError otherwise.

@@ -19,6 +19,28 @@ int rb_paged_attention_decode(const void* q, long long ld_q, void* out, long lon
                               const void* v_cache, const int* block_tables, int max_blocks, const int* context_lens,
                               int batch, int heads, int kv_heads, int head_dim, int block_size, long long num_blocks,
                               float scale, float* scratch, void* stream);
+// Decode attention of one layer of a decoding step, from the packed projection: rotation of queries and keys (theta 0: none), append and attention
+// in one launch.  qkv [batch, (heads + 2 kv_heads) * head_dim], pitch ld_qkv, is not changed; context_lens count the new token, whose cache slot
+// follows from the tables.  Neither tables, lengths nor the cached tokens may be written by the kernel in front in the stream.  At most 16 query
+// heads per KV head; head_dim 64 or 128.  -9 where the tables have room for more slices than fit the GPU twice (the other entries are faster
+// there; rb_paged_attention_step_takes).  arrived: [batch * kv_heads], zero before the first call; a call leaves it zero.  scratch as above.
+typedef struct RbPagedStepArgs {
+  const void* qkv;
+  long long ld_qkv;
+  void* out;
+  long long ld_o;
+  void* k_cache;
+  void* v_cache;
+  const int* block_tables;
+  const int* context_lens;
+  float* scratch;
+  unsigned int* arrived;
+  long long num_blocks;
+  int max_blocks, block_size, batch, heads, kv_heads, head_dim;
+  float scale, theta;
+} RbPagedStepArgs;
+int rb_paged_attention_step_takes(int batch, int kv_heads, int max_blocks, int block_size);
+int rb_paged_attention_step(const RbPagedStepArgs* args, void* stream);
 // The same decode attention with separate key / value head sizes (multiples of 8, at most 128), a score rule and an output
 // gate; softcap, slopes, log bias, chunk, window, sink, gates and out_scale as in RbPagedRowsArgs below.  bf16 operands.  scratch: fp32
 // [rb_paged_attention_scratch_floats(batch, heads, dv, max_blocks, block_size)].

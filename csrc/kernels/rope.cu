@@ -6,20 +6,9 @@
 
 #include "pdl.cuh"
 #include "rb_common.cuh"
+#include "rotary.cuh"
 
 namespace rb {
-
-// Rotates 8 neighbouring pairs (i, i + half) of one head: p points at the first.
-__device__ __forceinline__ void rope_unit(const float (&c)[8], const float (&s)[8], uint4& lo, uint4& hi) {
-  uint32_t* pl = reinterpret_cast<uint32_t*>(&lo);
-  uint32_t* ph = reinterpret_cast<uint32_t*>(&hi);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 a = unpack_bf16x2(pl[j]), b = unpack_bf16x2(ph[j]);
-    pl[j] = pack_bf16x2(a.x * c[2 * j] - b.x * s[2 * j], a.y * c[2 * j + 1] - b.y * s[2 * j + 1]);
-    ph[j] = pack_bf16x2(b.x * c[2 * j] + a.x * s[2 * j], b.y * c[2 * j + 1] + a.y * s[2 * j + 1]);
-  }
-}
 
 // Where rotated keys and the values behind them go besides their own place (rb_rope_append).
 struct RopeCache {
@@ -78,7 +67,7 @@ rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const long long* __rest
       if (h >= heads) break;
       __nv_bfloat16* p = x + t * ld + static_cast<long long>(h) * head_dim + gidx * 8;
       uint4 lo = *reinterpret_cast<uint4*>(p), hi = *reinterpret_cast<uint4*>(p + half);
-      rope_unit(c, s, lo, hi);
+      rope_unit(lo, hi, [&](int j) { return make_float2(c[j], s[j]); });
       *reinterpret_cast<uint4*>(p) = lo;
       *reinterpret_cast<uint4*>(p + half) = hi;
       if (CACHE && slot >= 0 && h >= cache.heads) {

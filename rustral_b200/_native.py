@@ -38,6 +38,7 @@ class RbGemmArgs(C.Structure):
         ("peer_epoch", C.c_uint), ("ready_flags", c_void_p), ("peer_ptrs", c_void_p * 8),
         ("tile_arrived", c_void_p), ("tile_expected", c_void_p),
         ("ab_fp8", c_int), ("a_scale", c_void_p), ("b_scale", c_void_p), ("b_constant", c_int),
+        ("norm_gamma", c_void_p), ("norm_beta", c_void_p), ("norm_eps", c_float), ("norm_rms", c_int),
     ]
 
 
@@ -50,6 +51,15 @@ class RbAttnArgs(C.Structure):
         ("dq_strides", c_ll * 3), ("dk_strides", c_ll * 3), ("dv_strides", c_ll * 3),
         ("batch", c_int), ("heads", c_int), ("kv_heads", c_int), ("seq_q", c_int), ("seq_k", c_int),
         ("head_dim", c_int), ("causal", c_int), ("scale", c_float), ("kv_lens", c_void_p),
+    ]
+
+
+class RbPagedStepArgs(C.Structure):
+    _fields_ = [
+        ("qkv", c_void_p), ("ld_qkv", c_ll), ("out", c_void_p), ("ld_o", c_ll), ("k_cache", c_void_p), ("v_cache", c_void_p),
+        ("block_tables", c_void_p), ("context_lens", c_void_p), ("scratch", c_void_p), ("arrived", c_void_p), ("num_blocks", c_ll),
+        ("max_blocks", c_int), ("block_size", c_int), ("batch", c_int), ("heads", c_int), ("kv_heads", c_int), ("head_dim", c_int),
+        ("scale", c_float), ("theta", c_float),
     ]
 
 
@@ -316,7 +326,7 @@ def _declare_kernels(lib: C.CDLL) -> None:
     sig("rb_sqrt_scalar", [P, P, P])
     sig("rb_cast_f32_to_bf16", [P, P, c_ll, P])
     sig("rb_cast_bf16_to_f32", [P, P, c_ll, P])
-    sig("rb_embedding_fwd", [P, P, P, P, c_ll, c_int, c_int, c_ll, P])
+    sig("rb_embedding_fwd", [P, P, P, P, c_ll, c_int, c_int, P, c_ll, P])
     sig("rb_embedding_bwd_scratch_ints", [c_ll, c_ll], c_ll)
     sig("rb_embedding_bwd", [P, P, P, P, P, c_ll, c_int, c_int, c_ll, P])
     sig("rb_attention_fwd", [C.POINTER(RbAttnArgs), P])

@@ -12,15 +12,16 @@ def _int_scratch(device, n: int) -> torch.Tensor:
     return N.scratch(_scratch, device, n, torch.int32, 0)
 
 
-def embedding_forward(ids: torch.Tensor, wte: torch.Tensor, wpe=None, seq_len: int = 0, out=None) -> torch.Tensor:
-    """ids: int64 [tokens]; wte: [vocab, dim]; wpe: [max_pos, dim] added by position ``t % seq_len``."""
+def embedding_forward(ids: torch.Tensor, wte: torch.Tensor, wpe=None, seq_len: int = 0, out=None, lengths=None) -> torch.Tensor:
+    """ids: int64 [tokens]; wte: [vocab, dim]; wpe: [max_pos, dim] added by position ``t % seq_len``, or by position ``lengths[t] - 1``
+    (int32 [tokens]: the sequences' lengths with their new tokens)."""
     tokens = ids.numel()
     dim = wte.shape[1]
     flat = ids.reshape(-1)
     if not wte.is_cuda:
         y = wte[flat]
         if wpe is not None:
-            pos = torch.arange(tokens) % seq_len
+            pos = torch.arange(tokens) % seq_len if lengths is None else lengths.long() - 1
             y = (y.float() + wpe[pos].float()).to(wte.dtype)
         if out is not None:
             out.copy_(y)
@@ -32,8 +33,12 @@ def embedding_forward(ids: torch.Tensor, wte: torch.Tensor, wpe=None, seq_len: i
     y = out if out is not None else torch.empty((tokens, dim), dtype=wte.dtype, device=wte.device)
     if tokens == 0:
         return y
+    if lengths is not None:
+        if lengths.dtype != torch.int32 or not lengths.is_contiguous() or lengths.numel() != tokens or lengths.device != wte.device:
+            raise TypeError("embedding: a length (int32, on the table's device) for every token is required")
+        seq_len = wpe.shape[0] if wpe is not None else 1
     N.check(N.kernels().rb_embedding_fwd(flat.data_ptr(), wte.data_ptr(), N.ptr(wpe), y.data_ptr(), tokens, dim,
-                                         seq_len, wte.shape[0], N.stream_ptr()), "rb_embedding_fwd")
+                                         seq_len, N.ptr(lengths), wte.shape[0], N.stream_ptr()), "rb_embedding_fwd")
     return y
 
 

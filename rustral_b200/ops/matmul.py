@@ -359,6 +359,36 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
+def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta, eps: float, rms: bool, w: torch.Tensor, *, bias=None, act: str = "none",
+              b_constant: bool = False) -> torch.Tensor:
+    """act(norm(x) @ w^T + bias) for inference (`act` "swiglu": w = [gate; up], see rotary.swiglu_product).  For a few rows one launch, in which
+    every block forms the norm itself; else the norm's kernel and the product's, with the same result up to the order of the norm's sums."""
+    from . import norm as norm_ops
+    from .rotary import swiglu_product
+    M, K = x.shape
+    glu = act == "swiglu"
+    F = w.shape[0] // 2 if glu else w.shape[0]
+    if x.is_cuda and 0 < M <= 8 and K <= 4096 and M * K <= 16384 and x.dtype is gamma.dtype is w.dtype is torch.bfloat16 and \
+            w.shape[1] == K == gamma.numel() and not (F | K | x.stride(0) | w.stride(0)) & 7 and x.stride(1) == 1 == w.stride(1) and \
+            gamma.is_contiguous() and not (x.data_ptr() | gamma.data_ptr() | w.data_ptr()) & 15 and not (rms and beta is not None) and \
+            x.device == w.device == gamma.device and not (glu and (bias is not None or w.shape[0] & 1)) and \
+            all(t is None or (t.dtype is torch.bfloat16 and t.is_contiguous() and t.numel() == n and not t.data_ptr() & 15 and t.device == x.device)
+                for t, n in ((beta, K), (bias, F))):
+        out = torch.empty((M, F), dtype=x.dtype, device=x.device)
+        g = N.RbGemmArgs()
+        g.a, g.b, g.d, g.bias = x.data_ptr(), w.data_ptr(), out.data_ptr(), N.ptr(bias)
+        g.lda, g.ldb, g.ldd = x.stride(0), w.stride(0), F
+        g.M, g.N, g.K = M, F, K
+        g.act, g.alpha, g.b_constant = 9 if glu else N.ACT[act], 1.0, int(b_constant)              # 9: RB_ACT_SWIGLU
+        g.norm_gamma, g.norm_beta, g.norm_eps, g.norm_rms = gamma.data_ptr(), N.ptr(beta), eps, int(rms)
+        rc = N.kernels().rb_gemm_bf16(g, N.stream_ptr())
+        if rc != -9:
+            N.check(rc, "rb_gemm_bf16[norm]")
+            return out
+    h, _, _ = norm_ops.norm_forward(x, gamma, beta, eps, rms)
+    return swiglu_product(h, w, b_constant=b_constant) if glu else gemm(h, w, bias=bias, act=act, b_constant=b_constant)
+
+
 class WeightGradStore:
     """Deferred weight-gradient work of `linear` layers.
 

@@ -104,6 +104,45 @@ def paged_attention_decode(q, k_cache, v_cache, block_tables, context_lens, scal
     return out
 
 
+N.optional_sig("rb_paged_attention_step", [N.C.POINTER(N.RbPagedStepArgs), N.c_void_p])
+
+
+N.optional_sig("rb_paged_attention_step_takes", [N.c_int, N.c_int, N.c_int, N.c_int])
+
+
+def step_supported(qkv, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables) -> bool:
+    """Whether `attention_step` takes these operands: a step of a few sequences, for which its one launch is the faster way."""
+    return qkv.is_cuda and qkv.dtype is torch.bfloat16 and head_dim in (64, 128) and heads <= 16 * kv_heads and qkv.stride(1) == 1 and \
+        not qkv.stride(0) & 7 and not qkv.data_ptr() & 15 and k_cache.is_contiguous() and v_cache.is_contiguous() and \
+        k_cache.dtype is torch.bfloat16 and k_cache.shape == v_cache.shape and k_cache.shape[2:] == (kv_heads, head_dim) and \
+        bool(N.kernels().rb_paged_attention_step_takes(block_tables.shape[0], kv_heads, block_tables.shape[1], k_cache.shape[1]))
+
+
+def attention_step(qkv, heads: int, kv_heads: int, head_dim: int, theta: float, k_cache, v_cache, block_tables, context_lens, arrived, scale: float):
+    """Decode attention of one layer from its packed projection qkv [batch, (heads + 2 kv_heads) * head_dim]: rotates queries and keys (theta 0:
+    not), stores keys and values of the new tokens at positions context_lens - 1 and attends, in one launch; qkv is not changed.  The tables,
+    the lengths and the cached tokens must be older than the kernel in front of this call in its stream.  `arrived`: int32, at least batch *
+    kv_heads zeros that no other stream uses; a call leaves them zero.  Lengths count the new tokens, so they are 1 or more."""
+    nb, bs = k_cache.shape[:2]
+    B, width = block_tables.shape
+    if not (block_tables.dtype is context_lens.dtype is arrived.dtype is torch.int32 and block_tables.is_contiguous() and
+            context_lens.is_contiguous() and arrived.is_contiguous() and qkv.shape[0] == B == context_lens.numel() and
+            qkv.shape[1] == (heads + 2 * kv_heads) * head_dim and arrived.numel() >= B * kv_heads and
+            block_tables.device == context_lens.device == arrived.device == qkv.device == k_cache.device):
+        raise TypeError("attention_step: a packed projection row, a table row and an int32 length per sequence, on one device, are required")
+    lib = N.kernels()
+    out = torch.empty((B, heads * head_dim), dtype=qkv.dtype, device=qkv.device)
+    scratch = torch.empty(lib.rb_paged_attention_scratch_floats(B, heads, head_dim, width, bs), dtype=torch.float32, device=qkv.device)
+    a = N.RbPagedStepArgs()
+    a.qkv, a.ld_qkv, a.out, a.ld_o = qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0)
+    a.k_cache, a.v_cache, a.num_blocks, a.block_size = k_cache.data_ptr(), v_cache.data_ptr(), nb, bs
+    a.block_tables, a.max_blocks, a.context_lens = block_tables.data_ptr(), width, context_lens.data_ptr()
+    a.scratch, a.arrived, a.batch, a.heads, a.kv_heads, a.head_dim = scratch.data_ptr(), arrived.data_ptr(), B, heads, kv_heads, head_dim
+    a.scale, a.theta = scale, theta
+    N.check(lib.rb_paged_attention_step(a, N.stream_ptr()), "rb_paged_attention_step")
+    return out
+
+
 N.optional_sig("rb_paged_attention_rows", [N.C.POINTER(N.RbPagedRowsArgs), N.c_void_p])
 
 

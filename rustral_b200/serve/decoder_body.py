@@ -23,7 +23,7 @@ from ..ops import recurrent as rc_ops
 from ..ops import rotary as rope_ops
 from ..ops.attention import ScoreRule, distance_slopes
 from ..ops.heads import head_prep_, row_prep_
-from ..ops.matmul import gemm
+from ..ops.matmul import gemm, norm_gemm
 from .kv_cache import CacheLayer
 from .weights import latent_columns, mixer_columns, packed_columns
 
@@ -50,6 +50,10 @@ class GPTBody:
         y, _, _ = norm_ops.norm_forward(x, P.w(name + ".weight"), None if rms else P.w(name + ".bias"), self.cfg.norm_eps, rms)
         return y
 
+    def _norm_product(self, x, name, w, **kw):
+        P, rms = self.r.params, self.rms
+        return norm_gemm(x, P.w(name + ".weight"), None if rms else P.w(name + ".bias"), self.cfg.norm_eps, rms, w, b_constant=True, **kw)
+
     def _row_parallel(self, a, w, bias, residual):
         """a @ w^T (+ bias) + residual; with tensor parallelism the partial products are summed over the ranks."""
         tp = self.r.tp
@@ -61,6 +65,8 @@ class GPTBody:
 
     def embed(self, sb):
         P, cfg = self.r.params, self.cfg
+        if cfg.arch == "gpt2" and sb.arrived is not None:
+            return ops.embedding_forward(sb.ids, P.w("tok_embed.embed"), P.w("pos_embed.embed"), lengths=sb.ctx)
         x = ops.embedding_forward(sb.ids, P.w("tok_embed.embed"))
         if cfg.arch == "gpt2":
             x = ops.binary("add", x, ops.gather_rows(P.w("pos_embed.embed"), sb.pos))
@@ -70,31 +76,35 @@ class GPTBody:
         P, r, rms = self.r.params, self.r, self.rms
         H, Hk, D = r.n_head, r.n_kv_head, self.cfg.head_dim
         p = f"layers.{l}."
-        h = self._norm(x, p + "ln1")
-        qkv = _product(h, P.w(p + "attn.wqkv.weight"), bias=None if rms else P.w(p + "attn.wqkv.bias"))
-        k2, v2 = qkv[:, H * D:(H + Hk) * D], qkv[:, (H + Hk) * D:]
-        if rms:
-            rope_ops.rope_append_(qkv, H, Hk, D, sb.pos, self.cfg.rope_theta, r.cache.k[l], r.cache.v[l], sb.slots)
+        kc, vc = r.cache.k[l], r.cache.v[l]
+        qkv = self._norm_product(x, p + "ln1", P.w(p + "attn.wqkv.weight"), bias=None if rms else P.w(p + "attn.wqkv.bias"))
+        if sb.arrived is not None and paged_ops.step_supported(qkv, H, Hk, D, kc, vc, sb.bt):
+            # the kernel in front is the projection: tables, lengths and cached tokens are older
+            a = paged_ops.attention_step(qkv, H, Hk, D, self.cfg.rope_theta if rms else 0.0, kc, vc, sb.bt, sb.ctx, sb.arrived, self.scale)
         else:
-            paged_ops.kv_append(k2, v2, r.cache.k[l], r.cache.v[l], sb.slots)
-        a = r.attend(l, qkv[:, :H * D], k2, v2, sb, self.scale)
+            k2, v2 = qkv[:, H * D:(H + Hk) * D], qkv[:, (H + Hk) * D:]
+            if rms:
+                rope_ops.rope_append_(qkv, H, Hk, D, sb.pos, self.cfg.rope_theta, kc, vc, sb.slots)
+            else:
+                paged_ops.kv_append(k2, v2, kc, vc, sb.slots)
+            a = r.attend(l, qkv[:, :H * D], k2, v2, sb, self.scale)
         x = self._row_parallel(a, P.w(p + "attn.wo.weight"), None if rms else P.w(p + "attn.wo.bias"), x)
-        h = self._norm(x, p + "ln2")
         if rms:
-            return self._row_parallel(rope_ops.swiglu_product(h, P.w(p + "ffn.gate_up.weight"), b_constant=True), P.w(p + "ffn.down.weight"), None, x)
-        h = _product(h, P.w(p + "ffn.fc1.weight"), bias=P.w(p + "ffn.fc1.bias"), act="gelu")
+            h = self._norm_product(x, p + "ln2", P.w(p + "ffn.gate_up.weight"), act="swiglu")
+            return self._row_parallel(h, P.w(p + "ffn.down.weight"), None, x)
+        h = self._norm_product(x, p + "ln2", P.w(p + "ffn.fc1.weight"), bias=P.w(p + "ffn.fc1.bias"), act="gelu")
         return _product(h, P.w(p + "ffn.fc2.weight"), bias=P.w(p + "ffn.fc2.bias"), residual=x)
 
     def head(self, x, rows):
         P, cfg, tp = self.r.params, self.cfg, self.r.tp
         if rows is not None:
             x = x.index_select(0, rows)
+        if tp is None:
+            return self._norm_product(x.contiguous(), "final_norm", P.w("tok_embed.embed" if cfg.tie_embeddings else "head.weight"))
         xf = self._norm(x.contiguous(), "final_norm")
-        if tp is not None:
-            w = P.w("head.weight")
-            _product(xf, w, out=tp.staging(xf.shape[0], w.shape[0]))
-            return tp.all_gather_cols(xf.shape[0], w.shape[0])
-        return _product(xf, P.w("tok_embed.embed" if cfg.tie_embeddings else "head.weight"))
+        w = P.w("head.weight")
+        _product(xf, w, out=tp.staging(xf.shape[0], w.shape[0]))
+        return tp.all_gather_cols(xf.shape[0], w.shape[0])
 
 
 class Stream:

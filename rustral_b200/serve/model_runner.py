@@ -30,10 +30,12 @@ from .kv_cache import PagedCache
 
 class StepBatch:
     """The rows of one model pass: prompt portions first (`spans`), then one row per decoded sequence (from row `rd`).
-    `segments`: the same sequences for layers with recurrent state (None: the model has none)."""
+    `segments`: the same sequences for layers with recurrent state (None: the model has none).  `arrived`: given for a step of decoded
+    sequences only whose tables and lengths were complete before it began (see ops.paged.attention_step); positions and slots (None) then
+    follow from them where a layer asks."""
 
-    def __init__(self, ids, pos, slots, spans, rd, tables, bt, ctx, block_size, segments=None):
-        self.ids, self.pos, self.slots = ids, pos, slots          # int64 device tensors, one entry per row
+    def __init__(self, ids, pos, slots, spans, rd, tables, bt, ctx, block_size, segments=None, arrived=None):
+        self.ids, self._pos, self._slots, self.arrived = ids, pos, slots, arrived      # int64 device tensors, one entry per row
         self.spans = spans                                        # (first row, end row, first position) per portion
         self.rd, self.rows = rd, ids.shape[0]
         self.tables = tables                                      # block table (list) of every portion's sequence
@@ -41,6 +43,19 @@ class StepBatch:
         self.block_size = block_size
         self.segments = segments
         self._keys, self._row_tables, self._rotations, self._all_keys = {}, None, {}, None
+
+    @property
+    def pos(self) -> torch.Tensor:
+        if self._pos is None:
+            self._pos = (self.ctx - 1).to(torch.int64)
+        return self._pos
+
+    @property
+    def slots(self) -> torch.Tensor:
+        if self._slots is None:
+            bs = self.block_size
+            self._slots = self.bt.gather(1, (self.pos // bs).view(-1, 1)).view(-1).to(torch.int64) * bs + self.pos % bs
+        return self._slots
 
     def rotation(self, rot, freqs: torch.Tensor) -> torch.Tensor:
         """Cosines and sines of the rows' positions for the rotary positions `rot` (models.layered.RotarySpec), one table for all
@@ -319,12 +334,15 @@ class ModelRunner:
     def _decode_segments(self, seq_ids, context_lens) -> list:
         return [(i, 1, self.cache.state_slot(s), n - 1) for i, (s, n) in enumerate(zip(seq_ids, context_lens))]
 
-    def _decode_body(self, ids, ctx, bt, segments=None):
+    def _step_counters(self, batch: int):
+        """Zeros that the steps of one stream share (see ops.paged.attention_step); None: the model's layers do not use them."""
+        if self.device.type != "cuda" or not isinstance(self.body, decoder_body.GPTBody):
+            return None
+        return torch.zeros(batch * self.n_kv_head, dtype=torch.int32, device=self.device)
+
+    def _decode_body(self, ids, ctx, bt, segments=None, arrived=None):
         """The device-side part of a decode step on static tensors (captured into a CUDA graph per batch size)."""
-        B, bs = ids.shape[0], self.block_size
-        pos = (ctx - 1).to(torch.int64)
-        slots = bt.gather(1, (pos // bs).view(B, 1)).view(B).to(torch.int64) * bs + pos % bs
-        return self._run(StepBatch(ids, pos, slots, [], 0, [], bt, ctx, bs, segments), None)
+        return self._run(StepBatch(ids, None, None, [], 0, [], bt, ctx, self.block_size, segments, arrived), None)
 
     @torch.no_grad()
     def decode(self, seq_ids: list, last_tokens: list, context_lens: list) -> torch.Tensor:
@@ -340,7 +358,7 @@ class ModelRunner:
         self.cache.fill_tables(seq_ids, bt)
         bt = bt.to(dev)
         seg = Segments.of(self._decode_segments(seq_ids, context_lens), dev) if self.recurrent else None
-        return self._decode_body(ids, ctx, bt, seg)
+        return self._decode_body(ids, ctx, bt, seg, self._step_counters(len(seq_ids)))
 
     def _table_width(self, context_lens) -> int:
         """Block-table columns of a graphed decode step: the model's whole context when that is at most 1024 blocks, else
@@ -367,7 +385,7 @@ class ModelRunner:
         if g is None:
             # ids (int64), context lengths and block tables (int32) behind one another: one copy refreshes all three
             buf = torch.zeros(12 * B + 4 * B * width, dtype=torch.uint8, device=dev)
-            g = {"buf": buf, "seg": None, "graph": None, "out": None, **self._step_views(buf, B, width)}
+            g = {"buf": buf, "seg": None, "graph": None, "out": None, "arrived": self._step_counters(B), **self._step_views(buf, B, width)}
             if self.recurrent:
                 g["seg"] = Segments(torch.zeros((B, 4), dtype=torch.int32, device=dev), None)
             self._graphs[(B, width)] = g
@@ -383,7 +401,7 @@ class ModelRunner:
             g["seg"].table.copy_(torch.tensor(self._decode_segments(seq_ids, context_lens), dtype=torch.int32), non_blocking=True)
         if g["graph"] is None:
             # first use of this batch size: one eager run (lazy kernel configuration, tensor-map cache), then capture
-            out = self._decode_body(g["ids"], g["ctx"], g["bt"], g["seg"])
+            out = self._decode_body(g["ids"], g["ctx"], g["bt"], g["seg"], g["arrived"])
             torch.cuda.current_stream().synchronize()
             graph = torch.cuda.CUDAGraph()
             # A collection in the middle of a capture could destroy an earlier runner's graphs, which ends the capture with an error
@@ -391,7 +409,7 @@ class ModelRunner:
             gc.disable()
             try:
                 with torch.cuda.graph(graph):
-                    g["out"] = self._decode_body(g["ids"], g["ctx"], g["bt"], g["seg"])
+                    g["out"] = self._decode_body(g["ids"], g["ctx"], g["bt"], g["seg"], g["arrived"])
             finally:
                 if collecting:
                     gc.enable()

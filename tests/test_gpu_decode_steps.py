@@ -125,3 +125,70 @@ def test_a_sequence_has_the_same_bits_alone_and_beside_others(heads, kv, dim, ru
             assert torch.equal(run([i], need[i])[0], together[i]), i
     some = [3, 4, 69, 6]
     assert torch.equal(run(some, 700), together[some])
+
+
+@pytest.mark.parametrize("batch,heads,kv,dim,longest,width,theta", [
+    (1, 8, 2, 128, 2500, 400, 10000.0), (36, 8, 4, 128, 1300, 96, 500000.0), (10, 32, 16, 64, 700, 64, 10000.0), (3, 4, 4, 64, 257, 1024, 0.0),
+    (5, 16, 1, 128, 20000, 1250, 10000.0), (2, 12, 12, 64, 1, 1, 0.0)])
+def test_attention_step_is_rotation_append_and_attention(batch, heads, kv, dim, longest, width, theta, cuda_status):
+    """The one launch of a decoding step against the three, for lengths at the edges of tiles and slices, in wide rows, twice in a
+    row on the same counters; a table entry out of range keeps its token out of the cache."""
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    need = (longest + 15) // 16
+    blocks = batch * need + 1
+    kc, vc = (torch.randn(blocks, 16, kv, dim, device="cuda", generator=g).bfloat16() for _ in range(2))
+    table = torch.zeros(batch, width, dtype=torch.int32, device="cuda")
+    table[:, :need] = 1 + torch.randperm(blocks - 1, device="cuda", generator=g).view(batch, need).int()
+    edges = [n for n in (1, 32, 33, 128, 129, 256, 257, 512, 513, longest) if n <= longest]
+    lens = torch.tensor([longest] + [edges[i % len(edges)] for i in range(batch - 1)], dtype=torch.int32, device="cuda")
+    cols = (heads + 2 * kv) * dim
+    arrived = torch.zeros(batch * kv, dtype=torch.int32, device="cuda")
+    pos = (lens - 1).long()
+    slots = table.gather(1, (pos // 16)[:, None]).view(-1).long() * 16 + pos % 16
+    for turn in range(2):
+        qkv = torch.randn(batch, cols + 8, device="cuda", generator=g).bfloat16()[:, :cols]
+        other, k2, v2 = qkv.clone(), kc.clone(), vc.clone()
+        if theta:
+            rotary.rope_append_(other, heads, kv, dim, pos, theta, k2, v2, slots)
+        else:
+            paged.kv_append(other[:, heads * dim:(heads + kv) * dim], other[:, (heads + kv) * dim:], k2, v2, slots)
+        want = paged.paged_attention_decode(other[:, :heads * dim], k2, v2, table, lens, 0.1)
+        assert paged.step_supported(qkv, heads, kv, dim, kc, vc, table)
+        before = qkv.clone()
+        got = paged.attention_step(qkv, heads, kv, dim, theta, kc, vc, table, lens, arrived, 0.1)
+        torch.cuda.synchronize()
+        assert torch.equal(qkv, before) and torch.equal(kc, k2) and torch.equal(vc, v2) and not arrived.any()
+        # the same arithmetic in the same order, but for contractions the compiler chooses: one rounding to bf16
+        assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-6).all()
+    # an entry out of range: nothing is stored for that sequence
+    table[0, pos[0] // 16] = blocks
+    k2, v2 = kc.clone(), vc.clone()
+    paged.attention_step(torch.full((batch, cols), 3.0, device="cuda").bfloat16(), heads, kv, dim, theta, kc, vc, table, lens, arrived, 0.1)
+    own = torch.ones(blocks * 16, dtype=torch.bool, device="cuda")
+    own[slots[1:]] = False
+    assert torch.equal(kc.view(-1, kv, dim)[own], k2.view(-1, kv, dim)[own]) and torch.equal(vc.view(-1, kv, dim)[own], v2.view(-1, kv, dim)[own])
+    N.read_status(clear=True)
+
+
+@pytest.mark.parametrize("rows,n,k", [(1, 768, 768), (1, 50304, 768), (4, 640, 4096), (8, 528, 2048), (3, 272, 200), (1, 3072, 1032), (2, 28672, 4096),
+                                      (9, 256, 256), (5, 256, 4096)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_inside_a_product_with_few_rows(rows, n, k, rms, cuda_status):
+    """The norm formed by the product's own blocks against norm and product, at one and several parts of the contraction, with stages that are filled
+    again, blocks that end inside 64 columns, and one size too many (rows, numbers): two launches.  Both round the normed rows to bf16; their
+    statistics differ in the order of fp32 sums, so a number may round the other way: 2^-8 of sqrt(k) terms beside the result's own rounding."""
+    from rustral_b200.ops import matmul, norm as norm_ops
+    g = torch.Generator(device="cuda").manual_seed(rows * n)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    x, w, gamma = rand(rows, k + 8)[:, :k] * 3 + 1, rand(n, k) * 0.05, rand(k)
+    beta, bias = (None, None) if rms else (rand(k), rand(n))
+    for act, weight in (("none", w), ("gelu", w), ("swiglu", w)):
+        b = None if act == "swiglu" else bias
+        before = N.launch_count
+        got = matmul.norm_gemm(x, gamma, beta, 1e-5, rms, weight, bias=b, act=act, b_constant=True)
+        one = rows <= 8 and rows * k <= 16384
+        assert (N.launch_count - before == 1) == one
+        h = norm_ops.norm_forward(x, gamma, beta, 1e-5, rms)[0]
+        want = rotary.swiglu_product(h, weight) if act == "swiglu" else matmul.gemm(h, weight, bias=b, act=act)
+        e = (got.float() - want.float()).abs()
+        assert (e <= 2.0 ** -7 * want.float().abs() + 2.0 ** -8 * want.float().pow(2).mean().sqrt()).all(), e.max()
