@@ -14,7 +14,6 @@
 
 #include "pdl.cuh"
 #include "rb_common.cuh"
-#include "rotary.cuh"
 
 namespace rb {
 
@@ -128,121 +127,21 @@ __device__ __forceinline__ float pa_gate(const PaRule& r, long long row, int hea
   return r.head_gate ? pa_sigmoid(r.head_gate[row * r.ld_g + head]) : 1.f;
 }
 
-// What a decoding step brings to the attention of a layer (STEP form): the packed projection's queries, keys and values of the new tokens, not
-// rotated and not in the cache yet.
-struct PaStep {
-  const __nv_bfloat16* k;        // [batch, kv_heads * size], pitch ld
-  const __nv_bfloat16* v;
-  long long ld;
-  __nv_bfloat16* k_cache;
-  __nv_bfloat16* v_cache;
-  float log2_theta;              // base of the rotary positions (0: queries and keys are taken as they are)
-  unsigned int* arrived;         // [batch * kv_heads], zero before and after
-};
-
-// The slices of a sequence for `gcount` heads, added up by the 128 threads of one CTA in the order of the slices, as paged_decode_merge_kernel does.
-// Up to 8 slices: eight threads per head hold maxima and sums, and everything is asked for at once.  `sh`: room for 2 * kMaxGroup * chunk floats.
-__device__ __noinline__ void pa_merge_here(const float* partial, int n, int nsplit, int gcount, int dv, __nv_bfloat16* out, float* sh, int chunk) {
-  const int pitch = dv + 2, tid = threadIdx.x, g0 = tid >> 3, s0 = tid & 7;      // 16 heads x 8
-  float* factor = sh;
-  float* sums = sh + kMaxGroup * chunk;
-  const float* mine = partial + (static_cast<long long>(min(g0, gcount - 1)) * nsplit + s0) * pitch;
-  if (n <= 8) {
-    const float ms = s0 < n ? __ldcg(mine) : -INFINITY, ls = s0 < n ? __ldcg(mine + 1) : 0.f;
-    float v[4][8];                                         // 512 results at a time
-    auto fetch = [&](int i0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = i0 + j * 128 + tid, g = i / dv;
-        const float* col = partial + static_cast<long long>(g) * nsplit * pitch + 2 + (i - g * dv);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) v[j][s] = i < gcount * dv && s < n ? __ldcg(col + s * pitch) : 0.f;
-      }
-    };
-    fetch(0);
-    float mx = ms;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    factor[g0 * 8 + s0] = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-    sums[g0 * 8 + s0] = ls;
-    __syncthreads();
-    for (int i0 = 0; i0 < gcount * dv; i0 += 512) {
-      if (i0) fetch(i0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = i0 + j * 128 + tid, g = i / dv;
-        if (i >= gcount * dv) break;
-        float num = 0.f, den = 0.f;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          num += v[j][s] * factor[g * 8 + s];
-          den += sums[g * 8 + s] * factor[g * 8 + s];
-        }
-        out[i] = __float2bfloat16(den > 0.f ? num / den : 0.f);
-      }
-    }
-    return;
-  }
-  float mx = -INFINITY;
-  if (g0 < gcount)
-    for (int s = 0; s0 + s < n; s += 8) mx = fmaxf(mx, __ldcg(mine + static_cast<long long>(s) * pitch));
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  for (int i0 = 0; i0 < gcount * dv; i0 += kPaWarps * 32) {
-    const int i = i0 + tid, g = min(i / dv, gcount - 1), d = i - g * dv;
-    float num = 0.f, den = 0.f;
-    for (int from = 0; from < n; from += chunk) {
-      const int m = min(chunk, n - from);
-      if (i0 == 0 || n > chunk) {                          // a slice's factor is formed once
-        __syncthreads();
-        if (g0 < gcount)
-          for (int s = s0; s < m; s += 8) {
-            const float* pp = mine + static_cast<long long>(from + s - s0) * pitch;
-            const float ms = __ldcg(pp);
-            factor[g0 * chunk + s] = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-            sums[g0 * chunk + s] = __ldcg(pp + 1);
-          }
-        __syncthreads();
-      }
-      if (i < gcount * dv) {
-        const float* col = partial + (static_cast<long long>(g) * nsplit + from) * pitch + 2 + d;
-#pragma unroll 8
-        for (int s = 0; s < m; ++s) {
-          num += __ldcg(col + static_cast<long long>(s) * pitch) * factor[g * chunk + s];
-          den += sums[g * chunk + s] * factor[g * chunk + s];
-        }
-      }
-    }
-    if (i < gcount * dv) out[i] = __float2bfloat16(den > 0.f ? num / den : 0.f);
-  }
-}
-
 // LIST: the slices of all sequences, numbered one sequence after the other, are dealt in equal runs to CTAs that stay (grid: CTAs for a KV head,
 // KV heads).  Sequences differ in length by any factor, so a grid over (sequence, slice) is mostly CTAs without a token, each of which still
 // takes its turn (about 1500 in a microsecond), and one with fewer, longer slices leaves the longest sequence to a few CTAs.  From one slice
 // to the next the copies of K go on: the warps' accumulators are merged in the memory of the V tiles.  Without LIST: grid (sequences, KV heads,
 // slices), a slice for each CTA, where that many fit; nothing has to be looked up first.
-//
-// STEP: rotation and append of the new token and the merge of the slices in the same launch, for decoding steps.  The tables, the lengths and
-// the cached tokens are older than the kernel in front (the projection), so the first K and V tiles and the angles are asked for while
-// that kernel still runs; behind it come only the queries and the new token's row, which goes from the projection into the tiles (and into the
-// cache) without being read back.  The CTA whose slice is a sequence's last one stores it; the last CTA of a sequence and KV head to count itself in
-// adds up the slices, in their order.  A layer of a decoding step, us, three launches / this one: 1 sequence of 2047, 4 KV heads of 128 14.0 / 12.8, of
-// 300, 12 heads of 64 9.2 / 8.5.  Not for lists: there the count and the sum at a CTA's end cost more than the launches (64 sequences of 100 to
-// 4000 69.2 / 90.6, 24 of 128 to 2560 42.6 / 46.7).
-template <int DK, int DV, bool RULE, bool LIST, bool STEP>
+template <int DK, int DV, bool RULE, bool LIST>
 __global__ void __launch_bounds__(kPaWarps * 32, 3)
 paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, const __nv_bfloat16* __restrict__ k_cache,
                           const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int max_blocks,
                           const int* __restrict__ context_lens, int batch, int heads, int kv_heads, int dk_real, int dv_real,
                           int block_size, long long num_blocks, float scale, int g0, int gcount, float* __restrict__ partial,
-                          int nsplit, __nv_bfloat16* __restrict__ direct_out, long long ld_o, const PaRule rule, const PaStep step
+                          int nsplit, __nv_bfloat16* __restrict__ direct_out, long long ld_o, const PaRule rule
                           RB_BOUNDS_PARAM) {
-  static_assert(!STEP || (!RULE && !LIST), "steps of plain attention, one slice per CTA");
-  if (!STEP) {
-    pdl_wait();
-    pdl_launch();
-  }
+  pdl_wait();
+  pdl_launch();
   constexpr int LPK = DK / 8, LPV = DV / 8;  // 16-byte pieces per K / V row = copies per lane for a 32-row tile
   constexpr int KROW = DK + 8, VROW = DV + 8;  // padded rows (elements): ldmatrix rows 272 (144) bytes apart hit distinct banks
   constexpr int NT = DV / 8;                 // n-tiles of the output accumulator
@@ -251,8 +150,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
   extern __shared__ __align__(16) uint8_t big[];   // [warp][K tile, V tile] bf16, then q_sh
   __nv_bfloat16* q_sh = reinterpret_cast<__nv_bfloat16*>(big) + kPaWarps * (kKTile + kVTile);
   __shared__ float m_sh[kPaWarps][kMaxGroup], l_sh[kPaWarps][kMaxGroup];
-  __shared__ float2 turn_sh[STEP ? DK / 2 : 1];       // STEP: cosine and sine of the new token's angles
-  __shared__ int last_sh;                            // STEP: this CTA was the last to arrive for its sequence and head
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;   // fragment coordinates: row (and row + 8), column pair
   const int group = heads / kv_heads;
@@ -321,7 +218,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
   PaVisible vis = {0, 0, 0};
   int slot = -1;                             // cache slot of token `first + lane` of the located tile (-1: past the end)
   int n_next = 0;
-  int fresh = -1;                            // STEP: row of the new token in the located tile
   // cache slots of the 32 tokens from number `from` on (the host bounds num_blocks * block_size below 2^31)
   auto locate = [&](int from) {
     const int num = from + lane;
@@ -337,10 +233,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       slot = blk * block_size + (tok - blk_idx * block_size);
     }
     n_next = min(32, t_end - from);
-    if (STEP) {                                // its row is filled with zeros and written behind the copies
-      fresh = from < ctx && ctx <= t_end && ctx - 1 - from < 32 ? ctx - 1 - from : -1;
-      if (num == ctx - 1) slot = -1;
-    }
   };
   // takes up slice sp of sequence b
   auto enter = [&]() {
@@ -394,109 +286,20 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
   };
   const PaInt<LPK> pk{};
   const PaInt<LPV> pv{};
-  // STEP: angles of sequence b's new token (formed like rope_kernel's), for all heads
-  auto form_angles = [&]() {
-    if (step.log2_theta != 0.f && threadIdx.x < DK / 2) {
-      const float inv_freq = exp2f(-step.log2_theta * (2.f * threadIdx.x) / static_cast<float>(DK));
-      float sn, cs;
-      sincosf(static_cast<float>(context_lens[b] - 1) * inv_freq, &sn, &cs);
-      turn_sh[threadIdx.x] = make_float2(cs, sn);
-    }
-  };
-  auto rotate8 = [&](int unit, uint4& lo, uint4& hi) {       // pairs 8 unit .. 8 unit + 7 of a head
-    if (step.log2_theta != 0.f) rope_unit(lo, hi, [&](int j) { return turn_sh[unit * 8 + j]; });
-  };
-  // STEP: the group's rotated query rows; rows and columns that no query fills are zero
-  auto load_q_step = [&]() {
-    constexpr int U = DK / 16;
-    for (int i = threadIdx.x; i < kMaxGroup * U; i += blockDim.x) {
-      const int g = i / U, u = i - g * U;
-      uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-      if (g < gcount) {
-        const __nv_bfloat16* src = q + static_cast<long long>(b) * ld_q + static_cast<long long>(h_base + g) * DK + u * 8;
-        lo = *reinterpret_cast<const uint4*>(src);
-        hi = *reinterpret_cast<const uint4*>(src + DK / 2);
-        rotate8(u, lo, hi);
-      }
-      *reinterpret_cast<uint4*>(q_sh + g * KROW + u * 8) = lo;
-      *reinterpret_cast<uint4*>(q_sh + g * KROW + DK / 2 + u * 8) = hi;
-    }
-  };
-  // STEP: the new token's key (rotated) and value, taken up by the warp whose tile they belong to when the CTA enters a sequence's last slice, and
-  // stored in the cache: lane u < DK / 16 holds pairs 8 u .., lane c < DV / 8 eight values
-  uint4 new_lo, new_hi, new_v;
-  auto take_new = [&]() {
-    if (ctx > t_end || ((ctx - 1) >> 5) % kPaWarps != warp) return;
-    const __nv_bfloat16* k = step.k + static_cast<long long>(b) * step.ld + static_cast<long long>(hk) * DK;
-    const __nv_bfloat16* v = step.v + static_cast<long long>(b) * step.ld + static_cast<long long>(hk) * DV;
-    if (lane < DK / 16) {
-      new_lo = *reinterpret_cast<const uint4*>(k + lane * 8);
-      new_hi = *reinterpret_cast<const uint4*>(k + DK / 2 + lane * 8);
-    }
-    if (lane < LPV) new_v = *reinterpret_cast<const uint4*>(v + lane * 8);
-    const int tok = ctx - 1, blk_idx = tok / block_size;
-    const int blk = blk_idx < max_blocks ? block_tables[static_cast<long long>(b) * max_blocks + blk_idx] : -1;
-    const bool keep = blk >= 0 && blk < num_blocks;                // no place in a corrupt table
-    const long long at = (static_cast<long long>(blk) * block_size + (tok - blk_idx * block_size)) * kv_heads + hk;
-    if (lane < DK / 16) {
-      rotate8(lane, new_lo, new_hi);
-      if (keep) {
-        *reinterpret_cast<uint4*>(step.k_cache + at * DK + lane * 8) = new_lo;
-        *reinterpret_cast<uint4*>(step.k_cache + at * DK + DK / 2 + lane * 8) = new_hi;
-      }
-    }
-    if (lane < LPV && keep) *reinterpret_cast<uint4*>(step.v_cache + at * DV + lane * 8) = new_v;
-  };
-  auto put = [&](int row, bool key) {          // into the landed tile
-    if (row < 0) return;
-    __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(big) + warp * (kKTile + kVTile);
-    if (key && lane < DK / 16) {
-      *reinterpret_cast<uint4*>(tile + row * KROW + lane * 8) = new_lo;
-      *reinterpret_cast<uint4*>(tile + row * KROW + DK / 2 + lane * 8) = new_hi;
-    }
-    if (!key && lane < LPV) *reinterpret_cast<uint4*>(tile + kKTile + row * VROW + lane * 8) = new_v;
-    __syncwarp();
-  };
-  // STEP: called by all threads when the slice is done
-  auto finish = [&](int slices) {
-    __syncthreads();                           // all partial results are written
-    if (threadIdx.x == 0) {
-      __threadfence();                         // for the whole CTA, behind its barrier; the counter goes back to zero with the last arrival
-      last_sh = atomicInc(step.arrived + static_cast<long long>(b) * kv_heads + hk, slices - 1) == static_cast<unsigned>(slices - 1);
-    }
-    __syncthreads();
-    if (!last_sh) return;
-    __threadfence();
-    pa_merge_here(partial + (static_cast<long long>(b) * heads + h_base) * nsplit * (DV + 2), slices, nsplit, gcount, DV,
-                  direct_out + b * ld_o + static_cast<long long>(h_base) * DV, merge, DV >= 128 ? 64 : 32);
-  };
 
-  if (!LIST && !STEP) {
+  if (!LIST) {
     load_q(true);
     __syncthreads();
   }
   enter();
   request(k_cache, kt_u32, pk, dk);
-  if (STEP) {
-    request(v_cache, vt_u32, pv, dv);
-    form_angles();
-    pdl_wait();                                // behind it only what the kernel in front has written is read
-    pdl_launch();
-    __syncthreads();
-    take_new();
-    load_q_step();
-    __syncthreads();
-  } else if (LIST) {
-    load_q(false);
-  }
+  if (LIST) load_q(false);
   for (bool other = LIST;;) {
-    if (!STEP) {
-      if (other) request_q();
-      request(v_cache, vt_u32, pv, dv);
-      if (other) {                             // query rows of another sequence: copied by all warps for all warps
-        pa_cp_wait<1>();
-        __syncthreads();
-      }
+    if (other) request_q();
+    request(v_cache, vt_u32, pv, dv);
+    if (other) {                               // query rows of another sequence: copied by all warps for all warps
+      pa_cp_wait<1>();
+      __syncthreads();
     }
     const int b_done = b, sp_done = sp;
     const bool another = LIST && --left > 0;
@@ -509,10 +312,8 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       const int n_tok = n_next, now = base, ctx_now = ctx;             // at most 0 tokens: a warp without a part in the slice
       const PaVisible vis_now = vis;
       const bool more = now + kPaWarps * 32 < t_end;
-      const int new_row = STEP ? fresh : -1;
       pa_cp_wait<1>();                                                 // this pass's K tile has landed (V may be in flight)
       __syncwarp();
-      if (STEP) put(new_row, true);
       // ---- S[16 heads, 32 tokens] = Q K^T
       float s[4][4];
 #pragma unroll
@@ -609,7 +410,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       // ---- O[16, DV] += P[16, 32] V[32, DV]
       pa_cp_wait<1>();                                                 // this pass's V tile has landed
       __syncwarp();
-      if (STEP) put(new_row, false);
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
 #pragma unroll
@@ -638,8 +438,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       if (gq + 8 < gcount) *reinterpret_cast<float2*>(mine + 8 * VROW + n * 8) = make_float2(acc[n][2], acc[n][3]);
     }
     __syncthreads();
-    const int slices = STEP ? slices_of(b_done) : nsplit;
-    const bool direct = STEP ? slices == 1 : direct_out != nullptr;
     for (int i = threadIdx.x; i < gcount * dv; i += blockDim.x) {
       const int g = i / dv, d = i - g * dv;
       float mx = -INFINITY;
@@ -652,7 +450,7 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
         num += merge[w * kMergeStride + g * VROW + d] * sc;
         den += l_sh[w][g] * sc;
       }
-      if (direct) {                            // a single slice: this is the result
+      if (direct_out) {                        // a single slice: this is the result
         const long long col = static_cast<long long>(h_base + g) * dv + d;
         if (RULE && rule.sink) {               // a score 0 without a value
           const float top = fmaxf(mx, 0.f), sc = __expf(mx - top);
@@ -669,7 +467,6 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       if (d == 0) { pp[0] = mx; pp[1] = den; }
     }
 
-    if (STEP && !direct) finish(slices);
     if (!another) return;
     __syncthreads();                            // the merge area has been read: it becomes V tiles again
     other = b != b_done;
@@ -865,8 +662,8 @@ RB_API long long rb_paged_attention_scratch_floats(int batch, int heads, int hea
 }
 
 namespace {
-template <int DK, int DV, bool RULE, bool STEP = false>
-int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream, const rb::PaStep& step = rb::PaStep{}) {
+template <int DK, int DV, bool RULE>
+int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream) {
   const int group = a.heads / a.kv_heads;
   long long span = static_cast<long long>(a.max_blocks) * a.block_size;      // most keys a row can see
   if (a.chunk > 0 && a.chunk < span) span = a.chunk;
@@ -880,11 +677,10 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream, const rb::PaStep&
   // as many CTAs as fit at a time the first takes 68 to 70 us, with three times as many 67.
   const long long room = static_cast<long long>(a.batch) * a.kv_heads * nsplit, some = 6ll * rbhost::device_sm_count();
   const bool list = room > some;
-  if (STEP && list) return -9;
   const dim3 grid = list ? dim3(static_cast<unsigned int>(some < a.kv_heads ? 1 : some / a.kv_heads), a.kv_heads) : dim3(a.batch, a.kv_heads, nsplit);
   // dynamic shared memory: per warp a K and a V tile of 32 padded rows, plus the 16 padded query rows
   const int smem = (rb::kPaWarps * 32 * (DK + 8 + DV + 8) + rb::kMaxGroup * (DK + 8)) * 2;
-  auto kern = list ? rb::paged_decode_split_kernel<DK, DV, RULE, true, false> : rb::paged_decode_split_kernel<DK, DV, RULE, false, STEP>;
+  auto kern = list ? rb::paged_decode_split_kernel<DK, DV, RULE, true> : rb::paged_decode_split_kernel<DK, DV, RULE, false>;
   static bool attr_set[2][64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
@@ -901,8 +697,8 @@ int pd_launch(const RbPagedDecodeArgs& a, cudaStream_t stream, const rb::PaStep&
         reinterpret_cast<const __nv_bfloat16*>(a.q), a.ld_q, reinterpret_cast<const __nv_bfloat16*>(a.k_cache),
         reinterpret_cast<const __nv_bfloat16*>(a.v_cache), a.block_tables, a.max_blocks, a.context_lens, a.batch, a.heads, a.kv_heads,
         a.dk, a.dv, a.block_size, a.num_blocks, a.scale, g0, group - g0 < rb::kMaxGroup ? group - g0 : rb::kMaxGroup,
-        a.scratch, nsplit, STEP || nsplit == 1 ? O : nullptr, a.ld_o, rule, step RB_BOUNDS_ARG);
-  if (nsplit > 1 && !STEP)
+        a.scratch, nsplit, nsplit == 1 ? O : nullptr, a.ld_o, rule RB_BOUNDS_ARG);
+  if (nsplit > 1)
     rbhost::launch_pdl(rb::paged_decode_merge_kernel, dim3(a.batch, a.heads), dim3(128), 0, stream, 1, a.scratch, a.context_lens, a.heads, a.dv, nsplit,
                                                                               O, a.ld_o, rule);
   return static_cast<int>(cudaGetLastError());
@@ -947,36 +743,4 @@ RB_API int rb_paged_attention_decode(const void* q, long long ld_q, void* out, l
   a.scale = scale; a.scratch = scratch; a.out_scale = 1.f;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   return head_dim == 128 ? pd_launch<128, 128, false>(a, stream) : pd_launch<64, 64, false>(a, stream);
-}
-
-RB_API int rb_paged_attention_step_takes(int batch, int kv_heads, int max_blocks, int block_size) {
-  const long long nsplit = (static_cast<long long>(max_blocks) * block_size + rb::kSplitTokens - 1) / rb::kSplitTokens;
-  return batch > 0 && static_cast<long long>(batch) * kv_heads * nsplit <= 6ll * rbhost::device_sm_count();
-}
-
-RB_API int rb_paged_attention_step(const RbPagedStepArgs* args, void* stream_v) {
-  const RbPagedStepArgs& t = *args;
-  if (t.batch <= 0) return 0;
-  if (t.heads <= 0 || t.kv_heads <= 0 || t.heads % t.kv_heads || t.heads / t.kv_heads > rb::kMaxGroup || (t.head_dim != 64 && t.head_dim != 128) ||
-      t.block_size <= 0 || t.max_blocks <= 0 || !t.scratch || !t.arrived || t.num_blocks * t.block_size >= (1ll << 31) || (t.ld_qkv % 8) ||
-      t.theta < 0.f)
-    return -1;
-  if ((reinterpret_cast<uintptr_t>(t.qkv) | reinterpret_cast<uintptr_t>(t.k_cache) | reinterpret_cast<uintptr_t>(t.v_cache)) & 15) return -2;
-  const int D = t.head_dim;
-  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(t.qkv);
-  RbPagedDecodeArgs a = {};
-  a.q = x; a.ld_q = t.ld_qkv; a.out = t.out; a.ld_o = t.ld_o; a.k_cache = t.k_cache; a.v_cache = t.v_cache;
-  a.block_tables = t.block_tables; a.max_blocks = t.max_blocks; a.context_lens = t.context_lens; a.batch = t.batch;
-  a.heads = t.heads; a.kv_heads = t.kv_heads; a.dk = a.dv = D; a.block_size = t.block_size; a.num_blocks = t.num_blocks;
-  a.scale = t.scale; a.scratch = t.scratch; a.out_scale = 1.f;
-  rb::PaStep step;
-  step.k = x + static_cast<long long>(t.heads) * D;
-  step.v = step.k + static_cast<long long>(t.kv_heads) * D;
-  step.ld = t.ld_qkv;
-  step.k_cache = reinterpret_cast<__nv_bfloat16*>(t.k_cache);
-  step.v_cache = reinterpret_cast<__nv_bfloat16*>(t.v_cache);
-  step.log2_theta = t.theta > 0.f ? log2f(t.theta) : 0.f;
-  step.arrived = t.arrived;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  return D == 128 ? pd_launch<128, 128, false, true>(a, stream, step) : pd_launch<64, 64, false, true>(a, stream, step);
 }
