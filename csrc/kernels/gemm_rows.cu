@@ -14,6 +14,10 @@
 // decoding step; here every CTA reads the whole rows (at most 32 KB, from L2), forms their statistics and puts its part of the normed rows, rounded
 // to bf16 as the norm's own kernel does, into the operand tiles itself, while the first stages of W are on their way.  Warps 2 to 5 do that.
 // A decoded token of GPT-2 small, 25 norms, with the attention step in one launch 479 -> 392 us on one B200; of 8 Llama style layers of 2048 518 -> 497.
+//
+// A kernel's last barrier across the cluster only keeps shared memory alive: as a release it waited 2000 to 3000 cycles for the results' stores.  Without
+// that, with the partial sums of all CTAs asked for at once and the norm's weights under the kernel in front, us per product in a chain, before /
+// now: 1 row 768 x 3072 6.45 / 5.63, 2048 x 2048 8.1 / 7.1, 2048 x 8192 13.4 / 12.3; 64 rows 2048 x 8192 15.8 / 14.1.
 #define RB_INLINE_WAITS
 #include "gemm_rows.h"
 
@@ -78,9 +82,24 @@ __device__ __forceinline__ float rows_sum128(float v, float* red) {
 // kb0 .. kb1 into the first stages and, for stages that are filled again, into `later`.
 template <int NORM>
 __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int kb0, int kb1, int stages, int stage_bytes, uint32_t base,
-                                          uint8_t* later, float* red) {
+                                          uint8_t* later, float* red, bool w_constant) {
   const int t = threadIdx.x - 64;
   const float inv_n = 1.f / static_cast<float>(K);
+  // the norm's weights are the model's like W: asked for before the kernel in front has ended
+  uint4 gamma[NORM], beta[NORM];
+  auto weights = [&]() {
+#pragma unroll
+    for (int i = 0; i < NORM; ++i) {
+      const int c = (i * 128 + t) * 8, kb = c >> 6;
+      const bool mine = c < K && kb >= kb0 && kb < kb1;
+      gamma[i] = mine ? *reinterpret_cast<const uint4*>(nm.gamma + c) : make_uint4(0u, 0u, 0u, 0u);
+      beta[i] = mine && nm.beta ? *reinterpret_cast<const uint4*>(nm.beta + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  if (w_constant) weights();
+  pdl_wait();
+  pdl_launch();
+  if (!w_constant) weights();
   uint4 next[NORM];
   auto fetch = [&](int m) {
 #pragma unroll
@@ -130,11 +149,11 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
         float v[8] = {}, g[8];
         if (c < K) {
           unpack(u[i], v);
-          unpack(__ldg(reinterpret_cast<const uint4*>(nm.gamma + c)), g);
+          unpack(gamma[i], g);
 #pragma unroll
           for (int j = 0; j < 8; ++j) v[j] = (v[j] - mean) * rstd * g[j];
           if (nm.beta) {
-            unpack(__ldg(reinterpret_cast<const uint4*>(nm.beta + c)), g);
+            unpack(beta[i], g);
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[j] += g[j];
           }
@@ -237,10 +256,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       if (ok) umma_commit(bar_acc);
     }
   } else {
-    pdl_wait();
-    pdl_launch();
-    if constexpr (NORM != 0) {
-      rows_norm<NORM>(nm, M, K, kb0, kb1, stages, stage_bytes, base, later, red);
+    if constexpr (NORM == 0) {
+      pdl_wait();
+      pdl_launch();
+    } else {
+      rows_norm<NORM>(nm, M, K, kb0, kb1, stages, stage_bytes, base, later, red, w_constant);
       if (warp == 2) {
         if (lane < min(stages, kb1 - kb0)) mbar_arrive(bar_full + 8 * lane);
         for (int it = stages; it < kb1 - kb0; ++it) {
@@ -280,16 +300,19 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   // ---- results: four neighbouring columns per item, items dealt to the CTAs of the cluster
   if (!*abort_flag) {
-    const int per_row = tile_n / 4;
-    for (int i = part * kRowsThreads + threadIdx.x; i < M * per_row; i += parts * kRowsThreads) {
-      const int m = i / per_row, n = (i - m * per_row) * 4, col = tile * tile_n + n;
+    const int shift = glu ? 4 : 5;                       // of 16 or 32 items in a row
+    for (int i = part * kRowsThreads + threadIdx.x; i < M << shift; i += parts * kRowsThreads) {
+      const int m = i >> shift, n = (i - (m << shift)) * 4, col = tile * tile_n + n;
       if (col >= N) continue;
       auto sum = [&](int at) {
         if (parts == 1) return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem) + at);
-        float4 a = ld_cluster_f4(mapa_shared(base + at * 4, 0));
-        for (int s = 1; s < parts; ++s) {
-          const float4 b = ld_cluster_f4(mapa_shared(base + at * 4, s));
-          a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        float4 v[8];                                     // all parts are asked for, then added in rank order
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = s < parts ? ld_cluster_f4(mapa_shared(base + at * 4, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 a = v[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s) {
+          if (s < parts) { a.x += v[s].x; a.y += v[s].y; a.z += v[s].z; a.w += v[s].w; }
         }
         return a;
       };
@@ -330,7 +353,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     }
   }
-  if (parts > 1) cluster_sync_all();                     // nobody leaves while another CTA still reads its partial sums
+  if (parts > 1) cluster_sync_relaxed();                 // nobody leaves while another CTA still reads its partial sums
   else __syncthreads();
   if (warp == 1) {
     if (*abort_flag) {
