@@ -56,6 +56,8 @@ struct EpiParams {
   int side;     // staged == 2: what TMA loads into the tiles before the accumulator is complete: 0 nothing, 1 residual, 2 aux_in
   const float* row_scale;   // fp32 [M] or nullptr: multiplies row i of the accumulator (8-bit operands: per-token scale)
   const float* col_scale;   // fp32 [N] or nullptr: multiplies column j (per-output-channel weight scale)
+  float* col_sum;           // fp32 [M] (or [splits][M], slabs), column sums of A; kernels of the EXTRA form with MN-major A only
+  int col_accumulate;
   int fp8_b_format;         // 8-bit operands: format of B in the instruction descriptor (0 = e4m3, 1 = e5m2); A is e4m3
 };
 
@@ -125,8 +127,9 @@ struct SmemLayout {
   static constexpr int kBBytes = BLOCK_N * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarOffset = STAGES * kStageBytes;
-  // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], side[warps][2], tmem ptr, abort flag
-  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], side[warps][2], tmem ptr, abort flag; behind them read[STAGES], summed[STAGES]
+  static constexpr int kSumBars = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  static constexpr int kTotal = kSumBars + 2 * STAGES * 8;
   // optional output staging (EpiParams::staged): per epilogue warp kSlots tiles of 32 rows x kStageCols bf16 (4 KB: or 32 x 32 fp32)
   static constexpr int kStageCols = (BLOCK_N % 128 == 0) ? 64 : 32;
   static constexpr int kSlots = BLOCK_N == 128 ? 2 : 1;
@@ -597,10 +600,63 @@ __device__ __forceinline__ void epilogue_swiglu(const CUtensorMap* tmD, uint32_t
   }
 }
 
+// Column sums of A beside the products (EpiParams::col_sum): four warps of their own read the A tiles of the first column of output tiles, 16 KB per
+// k-block of 64, when the issuer has seen them land (it arrives at bar_read; for a pair of CTAs a commit does, behind the products: an arrival at the
+// peer's barrier took the issuer so long that the product took three times as long) and before they are loaded over (bar_summed, for which the
+// producer waits).  Warp w sums 32 columns: lane r + 8 c the rows r, r + 8, .. of 8 columns, a swizzle chunk, so that eight lanes read a row of banks.
+// The eight rows of a lane are added up first and then to its running sum; lanes are added by shuffles, splits by the kernel that folds the slabs: the
+// order is fixed.  As a kernel of its own the sum read dy once more and took two launches: 32768 x 3072 46 + 3 us of a step's backward pass.
+constexpr int kSumWarps = 4;
+template <int STAGES>
+struct SumProducer {                               // what the TMA producer keeps
+  uint32_t used = 0, phase = 0;                    // stages whose present contents are summed; parity of their next bar_summed phase
+  __device__ __forceinline__ bool wait(uint32_t s, uint32_t bar_summed, volatile int* abort_flag, unsigned int* status) {
+    if (used >> s & 1) {
+      if (!mbar_wait(bar_summed + 8 * s, phase >> s & 1, abort_flag, status, 8)) return false;
+      phase ^= 1u << s;
+      used &= ~(1u << s);
+    }
+    return true;
+  }
+};
+// One k-block.
+__device__ __forceinline__ void sum_block(uint32_t a_tile, int w, int lane, float (&acc)[8]) {
+  const int chunk = 4 * w + (lane >> 3), r = lane & 7;
+  const uint32_t at = a_tile + (chunk >> 3) * (kBlockK * 128) + r * 128 + (((chunk & 7) ^ r) << 4);
+  Pair v[4];
+#pragma unroll
+  for (int i = 0; i < kBlockK / 8; ++i) {
+    uint32_t u[4];
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + i * 1024));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = i == 0 ? pair_of(u[j]) : add2(v[j], pair_of(u[j]));
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = floats(v[j]);
+    acc[2 * j] += f.x;
+    acc[2 * j + 1] += f.y;
+  }
+}
+__device__ __forceinline__ void sum_store(const EpiParams& ep, int split, int num_splits, int row0, int M, int w, int lane, float (&acc)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  }
+  const int m0 = row0 + (4 * w + (lane >> 3)) * 8;
+  if ((lane & 7) == 0) {
+    float* dst = ep.col_sum + (num_splits > 1 ? static_cast<long long>(split) * M : 0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (m0 + j < M) dst[m0 + j] = ep.col_accumulate && num_splits == 1 ? dst[m0 + j] + acc[j] : acc[j];
+  }
+}
+
 // FP8 = 1: both operands hold e4m3 bytes (K-major only).  A 128-byte swizzle row then carries 128 elements, so K, lda
 // and ldb arrive halved (in units of two bytes) and only the TMA coordinates, which count elements, are doubled back.
 template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0, bool EXTRA = false>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kNumThreads + (EXTRA && A_MN ? 32 * kSumWarps : 0), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
                  const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
@@ -619,6 +675,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + 2 * kNumEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
+  constexpr bool SUMS = EXTRA && A_MN;             // column sums of A beside the products
+  const uint32_t bar_read = smem_u32(smem + L::kSumBars), bar_summed = bar_read + 8 * STAGES;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   // TMEM allocations are powers of two >= 32 columns
@@ -635,6 +693,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(bar_tempty + 8 * a, kNumEpilogueWarps);
     }
     for (int w = 0; w < 2 * kNumEpilogueWarps; ++w) mbar_init(bar_side + 8 * w, 1);
+    if (SUMS) {
+      for (int s = 0; s < STAGES; ++s) {
+        mbar_init(bar_read + 8 * s, 1);
+        mbar_init(bar_summed + 8 * s, kSumWarps);
+      }
+    }
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
@@ -698,6 +762,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // elect.sync, not lane 0: the compiler then knows that one lane runs this and keeps what it issues in uniform registers
     if (elect_one()) {
       // ------------------------------------------------------------------ TMA producer
+      SumProducer<STAGES> sums;
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_units && ok; tile += gridDim.x) {
@@ -750,6 +815,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, status, 1)) { ok = false; break; }
+          if (SUMS) {
+            if (!sums.wait(s, bar_summed, abort_flag, status)) { ok = false; break; }
+            if (n_blk == 0) sums.used |= 1u << s;
+          }
           const uint32_t full = bar_full + 8 * s;
           mbar_arrive_expect_tx(full, L::kStageBytes);
           const uint32_t sa = smem_base + s * L::kStageBytes;
@@ -793,6 +862,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, status, 3)) { ok = false; break; }
+          if (SUMS && n_blk == 0) mbar_arrive(bar_read + 8 * s);
           tc_fence_after();
           const uint64_t da = desc_a + s * (L::kStageBytes / 16), db = desc_b + s * (L::kStageBytes / 16);
 #pragma unroll
@@ -804,6 +874,26 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (ok) umma_commit(bar_tfull + 8 * acc);   // accumulator complete
       }
+    }
+  } else if (SUMS && warp >= 2 + kNumEpilogueWarps) {
+    // -------------------------------------------------------------------- column sums of A
+    const int w = warp - 2 - kNumEpilogueWarps;
+    uint32_t it = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_units && ok; tile += gridDim.x) {
+      int m_blk, n_blk, kb0, kb1, outer;
+      decode_tile(tile, m_blk, n_blk, kb0, kb1, outer);
+      if (n_blk != 0) { it += kb1 - kb0; continue; }
+      float acc[8] = {};
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % STAGES;
+        if (!mbar_wait(bar_read + 8 * s, phase >> s & 1, abort_flag, status, 9)) { ok = false; break; }
+        phase ^= 1u << s;
+        sum_block(smem_base + s * L::kStageBytes, w, lane, acc);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_summed + 8 * s);
+      }
+      if (ok) sum_store(ep, outer, num_splits, m_blk * kBlockM, M, w, lane, acc);
     }
   } else {
     // -------------------------------------------------------------------- epilogue warps
@@ -869,7 +959,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       };
       if (L::kTma && ep.staged >= 2) {
         const int drow = num_splits > 1 || grp.mode == 2 ? outer * M + row0 : row0;
-        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
+        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA && !A_MN>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
                                                     lane, empty_k, abort_flag, status, arrive);
         continue;
       }
@@ -995,7 +1085,8 @@ struct SmemLayoutPair {
   static constexpr int kBBytes = (BLOCK_N / 2) * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarOffset = STAGES * kStageBytes;
-  static constexpr int kTotal = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  static constexpr int kSumBars = kBarOffset + (2 * STAGES + 4 + 2 * kNumEpilogueWarps) * 8 + 16;
+  static constexpr int kTotal = kSumBars + 2 * STAGES * 8;
   static constexpr int kStageCols = 64;
   static constexpr int kSlots = 2;
   static constexpr bool kTma = true, kSide = true;
@@ -1005,7 +1096,7 @@ struct SmemLayoutPair {
 };
 
 template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0, bool EXTRA = false>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kNumThreads + (EXTRA && A_MN ? 32 * kSumWarps : 0), 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
                       const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
@@ -1023,6 +1114,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + 2 * kNumEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
+  constexpr bool SUMS = EXTRA && A_MN;             // column sums of A beside the products
+  const uint32_t bar_read = smem_u32(smem + L::kSumBars), bar_summed = bar_read + 8 * STAGES;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();       // 0: leader (issues the MMAs), 1: peer
@@ -1041,6 +1134,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(bar_tempty + 8 * a, 2 * kNumEpilogueWarps);   // leader: the epilogue warps of both CTAs
     }
     for (int w = 0; w < 2 * kNumEpilogueWarps; ++w) mbar_init(bar_side + 8 * w, 1);
+    if (SUMS) {
+      for (int s = 0; s < STAGES; ++s) {
+        mbar_init(bar_read + 8 * s, 1);
+        mbar_init(bar_summed + 8 * s, kSumWarps);
+      }
+    }
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
@@ -1085,6 +1184,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (warp == 0) {
     if (elect_one()) {
       // ------------------------------------------------------------------ TMA producer (both CTAs)
+      SumProducer<STAGES> sums;
       uint32_t it = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < num_units && ok; tile += num_clusters) {
@@ -1095,6 +1195,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, status, 11)) { ok = false; break; }
+          if (SUMS) {
+            if (!sums.wait(s, bar_summed, abort_flag, status)) { ok = false; break; }
+            if (n_blk == 0) sums.used |= 1u << s;
+          }
           const uint32_t full_local = bar_full + 8 * s;
           if (cta_rank == 0) mbar_arrive_expect_tx(full_local, 2 * L::kStageBytes);
           const uint32_t full = mapa_shared(full_local, 0);
@@ -1146,10 +1250,31 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             if (FP8) umma_f8_ss_pair(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
             else umma_bf16_ss_pair(tmem_d, da + k * kStepA, db + k * kStepB, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
           }
+          if (SUMS && n_blk == 0) umma_commit_pair(bar_read + 8 * s, 3);
           umma_commit_pair(bar_empty + 8 * s, 3);     // both CTAs may refill this stage
         }
         if (ok) umma_commit_pair(bar_tfull + 8 * acc, 3);   // both CTAs' accumulator halves are complete
       }
+    }
+  } else if (SUMS && warp >= 2 + kNumEpilogueWarps) {
+    // -------------------------------------------------------------------- column sums of A
+    const int w = warp - 2 - kNumEpilogueWarps;
+    uint32_t it = 0, phase = 0;
+    bool ok = true;
+    for (int tile = cluster_id; tile < num_units && ok; tile += num_clusters) {
+      int m_blk, n_blk, kb0, kb1, split;
+      decode_tile(tile, m_blk, n_blk, kb0, kb1, split);
+      if (n_blk != 0) { it += kb1 - kb0; continue; }
+      float acc[8] = {};
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % STAGES;
+        if (!mbar_wait(bar_read + 8 * s, phase >> s & 1, abort_flag, status, 9)) { ok = false; break; }
+        phase ^= 1u << s;
+        sum_block(smem_base + s * L::kStageBytes, w, lane, acc);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_summed + 8 * s);
+      }
+      if (ok) sum_store(ep, split, num_splits, m_blk * kPairM + static_cast<int>(cta_rank) * kBlockM, M, w, lane, acc);
     }
   } else {
     // -------------------------------------------------------------------- epilogue warps (both CTAs)
@@ -1181,7 +1306,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       if (ep.staged >= 2) {
         const int drow = num_splits > 1 ? split * M + row0 : row0;
-        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
+        epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA && !A_MN>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
                                                     lane, false, abort_flag, status, arrive);
         continue;
       }
@@ -1219,9 +1344,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slab, void* d, long long ldd, int M, int N,
                      int out_f32, int accumulate, const __nv_bfloat16* __restrict__ bias,
-                     const __nv_bfloat16* __restrict__ residual, long long ldr) {
+                     const __nv_bfloat16* __restrict__ residual, long long ldr, const float* __restrict__ sum_ws, float* col_sum) {
   pdl_wait();
   pdl_launch();
+  if (sum_ws != nullptr) {                          // column sums: slabs of M numbers
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+      float acc = sum_ws[i];
+      for (int s = 1; s < splits; ++s) acc += sum_ws[static_cast<long long>(s) * M + i];
+      col_sum[i] = accumulate ? col_sum[i] + acc : acc;
+    }
+  }
   const long long n4 = static_cast<long long>(M) * N / 4;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -1308,7 +1440,9 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
   ep.col_scale = reinterpret_cast<const float*>(g.b_scale);
   ep.fp8_b_format = g.ab_fp8 == 2 ? 1 : 0;
   ep.staged = 0; ep.side = 0;
+  ep.col_sum = g.col_sum; ep.col_accumulate = g.accumulate;
   if (splits > 1) {
+    if (g.col_sum) ep.col_sum = reinterpret_cast<float*>(g.workspace) + static_cast<long long>(splits) * g.M * g.N;
     ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
     ep.bias = nullptr; ep.residual = nullptr;          // applied once, by the kernel that folds the slabs
   }
@@ -1362,10 +1496,12 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
   }
   const CUtensorMap *td = ta, *tx = ta, *ts = ta;         // placeholders unless TMA moves the results
   auto kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8>;
-  constexpr bool kExtra = !A_MN && !FP8 && L::kTma;       // forward products and input gradients
-  bool extra = kExtra;
+  constexpr bool kExtra = (!A_MN && !FP8 && L::kTma) || (A_MN && B_MN);       // forward products and input gradients; weight gradients
+  bool extra = kExtra && !A_MN;
   rb::EpiParams ep;
   const int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts, extra);
+  if (A_MN) extra = kExtra && g.col_sum != nullptr;
+  const int threads = rb::kNumThreads + (A_MN && extra ? 32 * rb::kSumWarps : 0);
   if constexpr (kExtra)
     if (extra) kern = rb::gemm_bf16_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8, true>;
   if (g.peer_mode == 2 && !ep.staged) return -11;
@@ -1394,7 +1530,7 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
     peer.a_peer[r] = reinterpret_cast<const __nv_bfloat16*>(g.peer_ptrs[r]);
     peer.d_peer[r] = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(g.peer_ptrs[r]));
   }
-  rbhost::launch_pdl(kern, dim3(grid), dim3(rb::kNumThreads), smem, stream, 1, *ta, *tb, *td, *tx, *ts, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
+  rbhost::launch_pdl(kern, dim3(grid), dim3(threads), smem, stream, 1, *ta, *tb, *td, *tx, *ts, g.M, g.N, k_units, group_m, splits, kb_per, slab, ep, grp, peer,
                                                 rbhost::status_ptr());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
@@ -1403,7 +1539,8 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
   rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
-                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);
+                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr,
+                                                      g.col_sum ? ep.col_sum : nullptr, g.col_sum);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1444,9 +1581,11 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
   }
   const CUtensorMap *td = ta, *tx = ta, *ts = ta;
   rb::EpiParams ep;
-  constexpr bool kExtra = !A_MN && !FP8;                  // forward products and input gradients
-  bool extra = kExtra;
+  constexpr bool kExtra = (!A_MN && !FP8) || (A_MN && B_MN);                  // forward products and input gradients; weight gradients
+  bool extra = kExtra && !A_MN;
   int smem = plan_epilogue<L>(g, splits, ep, td, tx, ts, extra);
+  if (A_MN) extra = kExtra && g.col_sum != nullptr;
+  const int threads = rb::kNumThreads + (A_MN && extra ? 32 * rb::kSumWarps : 0);
   if constexpr (kExtra)
     if (extra) kern = rb::gemm_bf16_pair_kernel<A_MN, B_MN, BLOCK_N, STAGES, FP8, true>;
   if (g.act == RB_ACT_SWIGLU && ep.staged != 2) return -9;
@@ -1458,7 +1597,7 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = smem;
   }
-  const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(rb::kNumThreads), smem, stream, 2, *ta, *tb_half, *td, *tx, *ts, g.M, g.N,
+  const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(threads), smem, stream, 2, *ta, *tb_half, *td, *tx, *ts, g.M, g.N,
                                            k_units, group_m, splits, kb_per, slab, ep, rbhost::status_ptr());
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
   const long long n4 = slab / 4;
@@ -1466,7 +1605,8 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
   rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
-                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);
+                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr,
+                                                      g.col_sum ? ep.col_sum : nullptr, g.col_sum);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1507,7 +1647,7 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
       if (sp > 1) {
         if (!can_split) continue;
         if (g.splits <= 0 && g.K / sp < 768) continue;
-        if (static_cast<long long>(sp) * g.M * g.N * 4 > g.workspace_bytes) continue;
+        if (static_cast<long long>(sp) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4 > g.workspace_bytes) continue;
       }
       const double cost = plan_cost(g.M, g.N, g.K, bn, sp, sms, pair_ok);
       if (best < 0.0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
@@ -1574,7 +1714,7 @@ RB_API long long rb_gemm_workspace(const RbGemmArgs* args, long long most) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.act == RB_ACT_SWIGLU || rbhost::gemm_rows_takes(g)) return 0;
   int bn = 128, splits = 1;
   pick_plan(g, rbhost::device_sm_count(), bn, splits);
-  return splits > 1 ? static_cast<long long>(splits) * g.M * g.N * 4 : 0;
+  return splits > 1 ? static_cast<long long>(splits) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4 : 0;
 }
 
 RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
@@ -1630,6 +1770,9 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
       if (!g.peer_ptrs[r] || (reinterpret_cast<uintptr_t>(g.peer_ptrs[r]) & 15)) return -11;
     if (g.peer_mode == 1 && (!g.ready_flags || g.lda != g.K)) return -11;       // a_full is dense [M, K]
   }
+  if (g.col_sum && (!g.a_mn_major || !g.b_mn_major || g.group_mode || g.peer_mode || g.ab_fp8 || g.act != RB_ACT_NONE ||
+                    (reinterpret_cast<uintptr_t>(g.col_sum) & 3)))
+    return -9;
   if (g.act == RB_ACT_SWIGLU) return gemm_swiglu(g, stream);
   const int sms = rbhost::device_sm_count();
   if (g.block_n != 0 && g.block_n != 64 && g.block_n != 128 && g.block_n != 192 && g.block_n != 256) return -6;

@@ -76,6 +76,9 @@ typedef struct RbGemmArgs {
   const void* norm_beta;       // or NULL
   float norm_eps;
   int norm_rms;
+  // sums over the contraction of A's columns, fp32 [M]: col_sum[i] = sum_k A[k, i] (added to it with `accumulate`), or NULL.  MN-major A and B, plain
+  // problems only.  In a weight gradient dW = dy^T x it is the bias gradient, formed while dy is in shared memory anyway.
+  float* col_sum;
 } RbGemmArgs;
 
 // Returns 0 on success, a negative code for rejected arguments, a positive cudaError otherwise.

@@ -219,9 +219,10 @@ def _gemm_f32(a, b, out, alpha, tile_expert=None, num_tiles=None, expert_stride=
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, aux_out=None, out=None, out_dtype=None, accumulate: bool = False,
          alpha: float = 1.0, block_n: int = 0, group_m: int = 0, max_ctas: int = 0, splits: int = 0,
-         peer: dict | None = None, row_scale=None, col_scale=None, b_constant: bool = False) -> torch.Tensor:
+         peer: dict | None = None, row_scale=None, col_scale=None, b_constant: bool = False, col_sum=None) -> torch.Tensor:
     """`b_constant`: the kernel in front of this call in its stream does not write `b` (a served model's weights), so reading `b` may
-    begin while that kernel still runs.  `row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
+    begin while that kernel still runs.  `col_sum` (fp32 [M], weight gradients: both operands transposed): receives the sums of a's columns, the bias
+    gradient, added to what it holds with `accumulate`.  `row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
     scales of quantised layers).  `peer` selects the tensor-parallel modes of the kernel (see parallel/fused_tp.py): a dict with `mode`
     (1: remote row blocks of A are pulled from the peers' shards inside the kernel; 2: output row blocks are
     stored into their owner's receive slot), `world`, `rank`, `rows_per_rank`, `epoch`, `ready_flags` (pointer,
@@ -237,6 +238,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         out_dtype = a.dtype if a.dtype in (torch.bfloat16, torch.float32) else torch.float32
     if act not in N.ACT:
         raise ValueError(f"gemm: unknown epilogue activation {act!r}")
+    if col_sum is not None:
+        if not (a_mn and b_mn) or act != "none" or peer is not None or col_sum.dtype != torch.float32 or col_sum.shape != (M,) or \
+                not col_sum.is_contiguous() or col_sum.device != a.device:
+            raise ValueError("gemm: column sums go with a plain product of two transposed operands, into a contiguous fp32 vector")
+        if not a.is_cuda or a.dtype != torch.bfloat16 or not K or not M or not Nn or \
+                _needs_padding(a, b, bias, residual, aux_in, aux_out, out, out_dtype, Nn):
+            from .elementwise import sum_dim0
+            if M:
+                sum_dim0(a, out=col_sum, accumulate=accumulate and out is not None)
+            col_sum = None
     if not a.is_cuda:
         if row_scale is not None or col_scale is not None:
             a = a.float().t() if a_mn else a.float()
@@ -291,7 +302,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         # three addresses (and the split-K workspace), which halves the Python time of a small launch.
         cache = _plain_args()
         key = (M, Nn, K, a_mn, b_mn, act, out.dtype, accumulate, alpha, block_n, group_m, max_ctas, splits,
-               a.stride(0), b.stride(0), out.stride(0), b_constant)
+               a.stride(0), b.stride(0), out.stride(0), b_constant, col_sum is None)
         g = cache.get(key)
         if g is None:
             if len(cache) > 4096:
@@ -306,11 +317,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.alpha = alpha
             g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
             g.b_constant = int(b_constant)
+            g.col_sum = N.ptr(col_sum)
             need = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES) if splits != 1 and K >= 2048 and act == "none" else 0
             cache[key] = g, need
         else:
             g, need = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
+        g.col_sum = N.ptr(col_sum)
         ws = _give_workspace(g, a.device, need)  # noqa: F841
         N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
         return out
@@ -335,6 +348,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     g.alpha = alpha
     g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
     g.b_constant = int(b_constant)
+    g.col_sum = N.ptr(col_sum)
     for t, n_, nm in ((row_scale, M, "row_scale"), (col_scale, Nn, "col_scale")):
         if t is not None and (t.dtype != torch.float32 or t.numel() != n_ or not t.is_contiguous() or t.device != a.device):
             raise TypeError(f"gemm: {nm} must be a contiguous fp32 vector of {n_} elements on the operands' device")
@@ -350,7 +364,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         g.splits = 1
     elif splits != 1 and K >= 2048 and act == "none":
         cache = _plain_args()
-        key = (M, Nn, K, a_mn, b_mn, accumulate, block_n, group_m, max_ctas, splits, aux_in is None, aux_out is None)
+        key = (M, Nn, K, a_mn, b_mn, accumulate, block_n, group_m, max_ctas, splits, aux_in is None, aux_out is None, col_sum is None)
         need = cache.get(key)
         if need is None:
             need = cache[key] = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES)
@@ -479,16 +493,22 @@ class _LinearFn(torch.autograd.Function):
             w_leaf, b_leaf, want_w = ctx.w_leaf, ctx.b_leaf, ctx.needs_input_grad[1]
 
             def later():
+                sums = torch.empty(dz.shape[1], dtype=torch.float32, device=dz.device) if want_w and want_b else None
                 if want_w:
-                    WeightGradStore._accumulate(w_leaf, gemm(dz, x2, a_mn=True, b_mn=True, out_dtype=w_leaf.dtype))
-                if want_b:
+                    WeightGradStore._accumulate(w_leaf, gemm(dz, x2, a_mn=True, b_mn=True, out_dtype=w_leaf.dtype, col_sum=sums))
+                if sums is not None:
+                    WeightGradStore._accumulate(b_leaf, sums.to(b_leaf.dtype))
+                elif want_b:
                     from .elementwise import sum_dim0
                     WeightGradStore._accumulate(b_leaf, sum_dim0(dz).to(b_leaf.dtype))
             queue.append(later)
             return dx, None, None, None, dres
         if ctx.needs_input_grad[1]:
-            dw = gemm(dz, x2, a_mn=True, b_mn=True, out_dtype=w.dtype)
-        if want_b:
+            sums = torch.empty(dz.shape[1], dtype=torch.float32, device=dz.device) if want_b else None
+            dw = gemm(dz, x2, a_mn=True, b_mn=True, out_dtype=w.dtype, col_sum=sums)
+            if want_b:
+                db = sums.to(w.dtype)
+        elif want_b:
             from .elementwise import sum_dim0
             db = sum_dim0(dz).to(w.dtype)
         return dx, dw, db, None, dres

@@ -383,19 +383,16 @@ class FusedGPTEngine:
                 gemm(dgu, L["ln2"], a_mn=True, b_mn=True, out=P.g(p + "ffn.gate_up.weight"), accumulate=acc)
                 dln2 = gemm(dgu, P.w(p + "ffn.gate_up.weight"), b_mn=True, out_dtype=self.act_dtype)
             else:
-                gemm(dx, L["h"], a_mn=True, b_mn=True, out=P.g(p + "ffn.fc2.weight"), accumulate=acc)
-                ops.sum_dim0(dx, out=P.g(p + "ffn.fc2.bias"), accumulate=acc)
+                gemm(dx, L["h"], a_mn=True, b_mn=True, out=P.g(p + "ffn.fc2.weight"), accumulate=acc, col_sum=P.g(p + "ffn.fc2.bias"))
                 dhp = gemm(dx, P.w(p + "ffn.fc2.weight"), b_mn=True, act="dgelu", aux_in=L["hpre"],
                            out_dtype=self.act_dtype)
-                gemm(dhp, L["ln2"], a_mn=True, b_mn=True, out=P.g(p + "ffn.fc1.weight"), accumulate=acc)
-                ops.sum_dim0(dhp, out=P.g(p + "ffn.fc1.bias"), accumulate=acc)
+                gemm(dhp, L["ln2"], a_mn=True, b_mn=True, out=P.g(p + "ffn.fc1.weight"), accumulate=acc, col_sum=P.g(p + "ffn.fc1.bias"))
                 dln2 = gemm(dhp, P.w(p + "ffn.fc1.weight"), b_mn=True, out_dtype=self.act_dtype)
             dx1, _, _ = norm_ops.norm_backward(dln2, L["x1"], P.w(p + "ln2.weight"), None if rms else L["mean2"],
                                                L["rstd2"], rms, dres=dx, dgamma=P.g(p + "ln2.weight"),
                                                dbeta=None if rms else P.g(p + "ln2.bias"), accumulate=acc)
-            gemm(dx1, L["attn"], a_mn=True, b_mn=True, out=P.g(p + "attn.wo.weight"), accumulate=acc)
-            if not rms:
-                ops.sum_dim0(dx1, out=P.g(p + "attn.wo.bias"), accumulate=acc)
+            gemm(dx1, L["attn"], a_mn=True, b_mn=True, out=P.g(p + "attn.wo.weight"), accumulate=acc,
+                 col_sum=None if rms else P.g(p + "attn.wo.bias"))
             dattn = gemm(dx1, P.w(p + "attn.wo.weight"), b_mn=True, out_dtype=self.act_dtype)
             qkv = L["qkv"]
             q = qkv[:, :H * D].view(B, S, H, D)
@@ -412,9 +409,8 @@ class FusedGPTEngine:
                 self._attention_backward_cpu(dattn.view(B, S, H, D), q, k, v, scale, dq, dk, dv)
             if rms:
                 rope_ops.rope_(dqkv, H + Hk, D, S, theta=cfg.rope_theta, inverse=True)
-            gemm(dqkv, L["ln1"], a_mn=True, b_mn=True, out=P.g(p + "attn.wqkv.weight"), accumulate=acc)
-            if not rms:
-                ops.sum_dim0(dqkv, out=P.g(p + "attn.wqkv.bias"), accumulate=acc)
+            gemm(dqkv, L["ln1"], a_mn=True, b_mn=True, out=P.g(p + "attn.wqkv.weight"), accumulate=acc,
+                 col_sum=None if rms else P.g(p + "attn.wqkv.bias"))
             dln1 = gemm(dqkv, P.w(p + "attn.wqkv.weight"), b_mn=True, out_dtype=self.act_dtype)
             dx, _, _ = norm_ops.norm_backward(dln1, L["x"], P.w(p + "ln1.weight"), None if rms else L["mean1"],
                                               L["rstd1"], rms, dres=dx1, dgamma=P.g(p + "ln1.weight"),

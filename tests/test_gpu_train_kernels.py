@@ -204,3 +204,29 @@ def test_routing_gradient_takes_a_number_under_capture(cuda_status):
     graph.replay()
     for a, b, c in zip(want, got, (0.25, 0.0)):
         assert torch.equal(a, b) and torch.equal(a, call(c))
+
+
+@pytest.mark.parametrize("tokens,out,inp,splits,block", [
+    (64, 64, 64, 0, 0), (1998, 1152, 384, 0, 0), (2100, 384, 1536, 3, 0), (4096, 2304, 768, 0, 0), (4096, 768, 768, 4, 256), (1024, 264, 520, 1, 128),
+    (333, 136, 200, 1, 192), (70, 8, 24, 1, 64), (32768, 256, 256, 0, 0), (8192, 3072, 768, 2, 0)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_bias_gradient_inside_the_weight_gradient(tokens, out, inp, splits, block, accumulate, cuda_status):
+    """Column sums of the first operand beside the product: one- and two-CTA tiles of every width, ragged tiles and contractions, slabs of splits, added to
+    what is there.  Bound: fp32 sums of at most `tokens` bf16 numbers (2^-24 of the sum of magnitudes per addition, about tokens / 64 + 16 of them in
+    a row); twice the same bits; the product is the one without sums."""
+    from rustral_b200.ops import matmul
+    g = torch.Generator(device="cuda").manual_seed(tokens + out)
+    dy = (torch.randn(tokens, out + 8, device="cuda", generator=g) + 0.5).bfloat16()[:, :out]
+    x = torch.randn(tokens, inp, device="cuda", generator=g).bfloat16()
+    w0, b0 = torch.randn(out, inp, device="cuda", generator=g), torch.randn(out, device="cuda", generator=g)
+    runs = []
+    for _ in range(2):
+        w, b = w0.clone(), b0.clone()
+        matmul.gemm(dy, x, a_mn=True, b_mn=True, out=w, accumulate=accumulate, splits=splits, block_n=block, col_sum=b)
+        runs.append((w, b))
+    plain = w0.clone()
+    matmul.gemm(dy, x, a_mn=True, b_mn=True, out=plain, accumulate=accumulate, splits=splits, block_n=block)
+    want = dy.double().sum(0) + (b0.double() if accumulate else 0)
+    bound = 2.0 ** -24 * (tokens / 64 + 16) * dy.double().abs().sum(0) + 2.0 ** -23 * want.abs()
+    assert torch.equal(runs[0][1], runs[1][1]) and torch.equal(runs[0][0], plain)
+    assert ((runs[0][1].double() - want).abs() <= bound).all()
