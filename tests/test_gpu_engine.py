@@ -41,3 +41,30 @@ def test_trainer_public_api_loss_decreases(cuda_status):
     tokens = torch.randint(0, cfg.vocab_size, (8, cfg.seq_len + 1), dtype=torch.int64).pin_memory()
     losses = [tr.step(tokens) for _ in range(8)]
     assert losses[-1] < losses[0] - 0.5, losses
+
+
+@pytest.mark.parametrize("name", ["gpt2-test", "llama-test"])
+def test_weight_gradients_beside_the_chain_are_those_in_line(name, cuda_status):
+    """The same kernels on the same operands on another stream: equal bits, eagerly (two calls of a shape) and replayed, with two micro-batches, from a
+    stream that is not the default one, while freed memory is handed out again and overwritten."""
+    cfg = preset(name)
+    g = torch.Generator().manual_seed(3)
+    grads = []
+    for beside in (False, True):
+        e = FusedGPTEngine(cfg, "cuda", micro_batch=2, seed=5, max_grad_norm=1.0)
+        assert e._beside(2 * cfg.seq_len) is not None
+        if not beside:
+            e._beside = lambda tokens: None
+        g.manual_seed(3)
+        out = []
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for _ in range(5):
+                ids, tg = (torch.randint(0, cfg.vocab_size, (4, cfg.seq_len), generator=g).cuda() for _ in range(2))
+                e.train_step(ids, tg, do_step=False)
+                junk = [torch.full((n,), float("nan"), device="cuda") for n in (1 << 10, 1 << 14, 1 << 18)]  # noqa: F841
+                out.append(e.params.grad.clone())
+        torch.cuda.synchronize()
+        grads.append(torch.stack(out))
+    assert torch.equal(grads[0], grads[1])
