@@ -50,6 +50,7 @@ int rb_attention_bwd(const RbAttnArgs* args, void* stream);
 // tcgen05 paths (attention_tc.cu, attention_fwd2.cu, attention_bwd_tc.cu, attention_bwd2.cu); -9: shape not taken
 int rb_attention_fwd_tc(const RbAttnArgs* args, void* stream);
 int rb_attention_fwd_tc2(const RbAttnArgs* args, int poly_every, void* stream);
+int rb_attention_fwd_many(const RbAttnArgs* list, int n, void* stream);
 int rb_attention_bwd_tc(const RbAttnArgs* args, void* stream);
 int rb_attention_delta_tc(const RbAttnArgs* args, void* stream);
 int rb_attention_bwd_tc2(const RbAttnArgs* args, void* stream);

@@ -239,13 +239,35 @@ struct F2Smem {
   static constexpr int kTotal = kBar + kNumBars * 8 + 16;
 };
 
-template <int D, int DV, int kPolyEvery, bool RULE, int DR = 0, bool LOG = false>
+// Several problems in one launch (portions of several prompts): each with tensor maps of its own, so that rows behind its end read as zeros and
+// nothing of another sequence can enter, and the query tiles of all of them along the grid.  A portion alone is a grid of (tiles, heads), mostly smaller
+// than the GPU: four portions of 129 to 1500 tokens, 32 heads of 64, a launch each 72 us, together @MANY@.
+constexpr int kF2Many = 8;
+struct F2One {
+  CUtensorMap q, k, v, qr, kr;
+};
+struct F2ManyMaps {
+  CUtensorMap q[kF2Many], k[kF2Many], v[kF2Many];
+  __nv_bfloat16* out[kF2Many];
+  int seq_q[kF2Many], seq_k[kF2Many], tiles_end[kF2Many];     // tiles_end: pairs of query tiles up to and with this problem
+};
+
+template <int D, int DV, int kPolyEvery, bool RULE, int DR = 0, bool LOG = false, bool MANY = false, class Maps = F2One>
 __global__ void __launch_bounds__(kF2Threads, 1)
-attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQr,
-                 const __grid_constant__ CUtensorMap tmKr, F2Params p, unsigned int* status) {
+attn_fwd2_kernel(const __grid_constant__ Maps maps, F2Params p, unsigned int* status) {
   pdl_wait();
   pdl_launch();
+  const CUtensorMap *mQ, *mK, *mV, *mQr = nullptr, *mKr = nullptr;
+  int tile = gridDim.x - 1 - blockIdx.x;                       // long causal rows first
+  if constexpr (MANY) {
+    int i = 0;
+    while (tile >= maps.tiles_end[i]) ++i;
+    tile -= i ? maps.tiles_end[i - 1] : 0;
+    mQ = &maps.q[i]; mK = &maps.k[i]; mV = &maps.v[i];
+    p.out = maps.out[i]; p.seq_q = maps.seq_q[i]; p.seq_k = maps.seq_k[i];
+  } else {
+    mQ = &maps.q; mK = &maps.k; mV = &maps.v; mQr = &maps.qr; mKr = &maps.kr;
+  }
   using L = F2Smem<D + DR, DV>;
   constexpr int kStages = L::kStages, kVStages = L::kVStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -266,7 +288,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_blk = gridDim.x - 1 - blockIdx.x;                // long causal rows first
+  const int m_blk = tile;
   const int h = blockIdx.y, b = blockIdx.z;
   const int hk = h / (p.heads / p.kv_heads);
   const int q0 = m_blk * 2 * kF2Tile;
@@ -327,9 +349,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     *abort_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(mQ);
+    tma_prefetch_desc(mK);
+    tma_prefetch_desc(mV);
   }
   if (warp == 9) {
     tmem_alloc(smem_u32(tmem_ptr_smem), kTmemCols);
@@ -351,9 +373,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive_expect_tx(bar_q + 8 * t, L::kTileBytes);
 #pragma unroll
         for (int hf = 0; hf < D / 64; ++hf)
-          tma_load_4d(sQ + t * L::kTileBytes + hf * L::kHalf, &tmQ, hf * 64, h, q0 + t * kF2Tile, b, bar_q + 8 * t);
+          tma_load_4d(sQ + t * L::kTileBytes + hf * L::kHalf, mQ, hf * 64, h, q0 + t * kF2Tile, b, bar_q + 8 * t);
         if (DR > 0)
-          tma_load_4d(sQ + t * L::kTileBytes + (D / 64) * L::kHalf, &tmQr, 0, h, q0 + t * kF2Tile, b, bar_q + 8 * t);
+          tma_load_4d(sQ + t * L::kTileBytes + (D / 64) * L::kHalf, mQr, 0, h, q0 + t * kF2Tile, b, bar_q + 8 * t);
       }
       for (int j = f_min; j < n_max; ++j) {
         const int s = (j - f_min) % kStages, use = (j - f_min) / kStages;
@@ -361,15 +383,15 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive_expect_tx(bar_kfull + 8 * s, L::kTileBytes);
 #pragma unroll
         for (int hf = 0; hf < D / 64; ++hf)
-          tma_load_4d(sK + s * L::kTileBytes + hf * L::kHalf, &tmK, hf * 64, hk, block_at(j) * kF2Tile, b, bar_kfull + 8 * s);
+          tma_load_4d(sK + s * L::kTileBytes + hf * L::kHalf, mK, hf * 64, hk, block_at(j) * kF2Tile, b, bar_kfull + 8 * s);
         if (DR > 0)
-          tma_load_4d(sK + s * L::kTileBytes + (D / 64) * L::kHalf, &tmKr, 0, 0, block_at(j) * kF2Tile, b, bar_kfull + 8 * s);
+          tma_load_4d(sK + s * L::kTileBytes + (D / 64) * L::kHalf, mKr, 0, 0, block_at(j) * kF2Tile, b, bar_kfull + 8 * s);
         const int v = (j - f_min) % kVStages, vuse = (j - f_min) / kVStages;
         if (!mbar_wait(bar_vempty + 8 * v, (vuse & 1) ^ 1, abort_flag, status, 49)) break;
         mbar_arrive_expect_tx(bar_vfull + 8 * v, L::kVTileBytes);
 #pragma unroll
         for (int hf = 0; hf < DV / 64; ++hf)
-          tma_load_4d(sV + v * L::kVTileBytes + hf * L::kHalf, &tmV, hf * 64, hk, block_at(j) * kF2Tile, b, bar_vfull + 8 * v);
+          tma_load_4d(sV + v * L::kVTileBytes + hf * L::kHalf, mV, hf * 64, hk, block_at(j) * kF2Tile, b, bar_vfull + 8 * v);
       }
     }
   } else if (warp == 9) {
@@ -674,10 +696,80 @@ int f2_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* t
     if (e != cudaSuccess) return static_cast<int>(e);
     cfg = true;
   }
-  rbhost::launch_pdl(kern, grid, dim3(rb::kF2Threads), smem, stream, 1, *tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk, p, rbhost::status_ptr());
+  const rb::F2One maps{*tq, *tk, *tv, tqr ? *tqr : *tq, tkr ? *tkr : *tk};
+  rbhost::launch_pdl(kern, grid, dim3(rb::kF2Threads), smem, stream, 1, maps, p, rbhost::status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 }  // namespace
+
+namespace {
+template <int D>
+int f2_launch_many(const rb::F2ManyMaps& maps, const rb::F2Params& p, int tiles, cudaStream_t stream) {
+  auto kern = rb::attn_fwd2_kernel<D, D, 0, false, 0, false, true, rb::F2ManyMaps>;
+  const int smem = rb::F2Smem<D, D>::kTotal + 1024;
+  static bool cfg_dev[64] = {false};
+  bool& cfg = cfg_dev[rbhost::device_slot()];
+  if (!cfg) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    cfg = true;
+  }
+  return static_cast<int>(rbhost::launch_pdl(kern, dim3(tiles, p.heads), dim3(rb::kF2Threads), smem, stream, 1, maps, p, rbhost::status_ptr()));
+}
+}  // namespace
+
+// Causal forward of `n` problems of one sequence each (batch 1; heads, head size and scale of the first), without log-sum-exp.  -9: a problem that
+// rb_attention_fwd_tc2 would not take; nothing is launched then.
+RB_API int rb_attention_fwd_many(const RbAttnArgs* list, int n, void* stream_v) {
+  if (n <= 0) return -1;
+  const int D = list[0].head_dim;
+  if (D != 64 && D != 128) return -9;
+  for (int i = 0; i < n; ++i) {
+    const RbAttnArgs& a = list[i];
+    if (a.batch != 1 || !a.causal || a.kv_lens || a.lse || a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.head_dim != D ||
+        a.heads != list[0].heads || a.kv_heads != list[0].kv_heads || a.scale != list[0].scale || a.seq_q <= 0 || a.seq_q > a.seq_k ||
+        a.o_strides[1] != list[0].o_strides[1] || a.o_strides[2] != list[0].o_strides[2])
+      return -9;
+    const void* ptrs[4] = {a.q, a.k, a.v, a.o};
+    const long long* strs[4] = {a.q_strides, a.k_strides, a.v_strides, a.o_strides};
+    for (int j = 0; j < 4; ++j) {
+      if (!ptrs[j] || (reinterpret_cast<uintptr_t>(ptrs[j]) & 15) || strs[j][1] <= 0 || strs[j][2] <= 0 || strs[j][1] % 8 || strs[j][2] % 8) return -9;
+    }
+  }
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  rb::F2Params p = {};
+  p.o_rs = list[0].o_strides[1]; p.o_hs = list[0].o_strides[2];
+  p.heads = list[0].heads; p.kv_heads = list[0].kv_heads; p.causal = 1; p.scale = list[0].scale;
+  for (int from = 0; from < n; from += rb::kF2Many) {
+    const int m = n - from < rb::kF2Many ? n - from : rb::kF2Many;
+    rb::F2ManyMaps maps;
+    // in the order of their rows' work: the grid begins with the last tiles
+    int order[rb::kF2Many];
+    for (int i = 0; i < m; ++i) {
+      int at = i;
+      while (at > 0 && list[from + order[at - 1]].seq_k > list[from + i].seq_k) { order[at] = order[at - 1]; --at; }
+      order[at] = i;
+    }
+    int tiles = 0, err = 0;
+    for (int i = 0; i < m; ++i) {
+      const RbAttnArgs& a = list[from + order[i]];
+      const long long qs[3] = {8, a.q_strides[1], a.q_strides[2]}, ks[3] = {8, a.k_strides[1], a.k_strides[2]},
+                      vs[3] = {8, a.v_strides[1], a.v_strides[2]};
+      const CUtensorMap* tq = f2_make_map(a.q, qs, a.seq_q, a.heads, 1, D, &err);
+      const CUtensorMap* tk = f2_make_map(a.k, ks, a.seq_k, a.kv_heads, 1, D, &err);
+      const CUtensorMap* tv = f2_make_map(a.v, vs, a.seq_k, a.kv_heads, 1, D, &err);
+      if (!tq || !tk || !tv) return err ? err : -5;
+      maps.q[i] = *tq; maps.k[i] = *tk; maps.v[i] = *tv;
+      maps.out[i] = reinterpret_cast<__nv_bfloat16*>(a.o);
+      maps.seq_q[i] = a.seq_q; maps.seq_k[i] = a.seq_k;
+      tiles += (a.seq_q + 2 * rb::kF2Tile - 1) / (2 * rb::kF2Tile);
+      maps.tiles_end[i] = tiles;
+    }
+    const int rc = D == 64 ? f2_launch_many<64>(maps, p, tiles, stream) : f2_launch_many<128>(maps, p, tiles, stream);
+    if (rc != 0) return rc;
+  }
+  return 0;
+}
 
 // Forward pass with two query tiles per CTA.  `poly_every`: 0 = every exponential on the special-function unit,
 // 4 = every fourth pair of keys on the FMA-pipe polynomial (measured slower on B200 at both head dims: 218 us against

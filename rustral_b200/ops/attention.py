@@ -217,6 +217,27 @@ def prompt_attention(q, k, v, scale: float, out, rule: ScoreRule | None = None, 
     return out
 
 
+N.optional_sig("rb_attention_fwd_many", [N.C.POINTER(N.RbAttnArgs), N.c_int, N.c_void_p])
+
+
+def prompt_attention_many(parts, scale: float) -> None:
+    """`prompt_attention` without a rule or a gate for several portions (q, k, v, out), eight of them in a launch where the kernel takes them."""
+    if len(parts) > 1 and parts[0][0].is_cuda and FORWARD_IMPL == "tc2" and not FORWARD_POLY_EVERY and \
+            all(t.dtype is torch.bfloat16 and t.stride(3) == 1 for part in parts for t in part) and \
+            all(q.shape[3] == k.shape[3] == v.shape[3] for q, k, v, _ in parts):
+        args = (N.RbAttnArgs * len(parts))()
+        for a, (q, k, v, out) in zip(args, parts):
+            _fill(a, q, k, v, out, True, scale)
+        lib = N.kernels()
+        rc = lib.rb_attention_fwd_many(args, len(parts), N.stream_ptr())
+        if rc != -9:
+            N.check(rc, "rb_attention_fwd_many")
+            N.launch_count += (len(parts) - 1) // 8
+            return
+    for q, k, v, out in parts:
+        prompt_attention(q, k, v, scale, out)
+
+
 def split_supported(dn: int, dr: int, dv: int, *views) -> bool:
     """Whether `prompt_attention_split` takes these head sizes and operands (2-D row-strided views; None: absent)."""
     views = [t for t in views if t is not None]

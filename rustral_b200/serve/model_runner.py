@@ -196,6 +196,7 @@ class ModelRunner:
             bt, seq = sb.row_tables()
             return paged_ops.paged_attention_rows(q, kc, vc, bt, seq, sb.pos, scale, rule, gate, out, head_gate)
         a = out if out is not None else torch.empty((T, H * dv), dtype=q.dtype, device=self.device)
+        parts = []
         for i, (r0, r1, start) in enumerate(sb.spans):
             L = r1 - r0
             kept, first = rule.key_ranges(start) if rule is not None else (0, 0)
@@ -205,9 +206,14 @@ class ModelRunner:
                 cs = sb.key_slots(i, first, kept)
                 kk = ops.gather_rows(kc.view(nb * bs, G * dk), cs).view(1, -1, G, dk)
                 vv = ops.gather_rows(vc.view(nb * bs, G * dv), cs).view(1, -1, G, dv)
-            attn_ops.prompt_attention(q[r0:r1].view(1, L, H, dk), kk, vv, scale, out=a[r0:r1].view(1, L, H, dv), rule=rule,
-                                      gate=None if gate is None else gate[r0:r1],
-                                      head_gate=None if head_gate is None else head_gate[r0:r1])
+            qq, oo = q[r0:r1].view(1, L, H, dk), a[r0:r1].view(1, L, H, dv)
+            if rule is None and gate is None and head_gate is None and dk == dv:
+                parts.append((qq, kk, vv, oo))
+            else:
+                attn_ops.prompt_attention(qq, kk, vv, scale, out=oo, rule=rule, gate=None if gate is None else gate[r0:r1],
+                                          head_gate=None if head_gate is None else head_gate[r0:r1])
+        if parts:
+            attn_ops.prompt_attention_many(parts, scale)
         if sb.rd < T:
             paged_ops.paged_attention_decode(q[sb.rd:], kc, vc, sb.bt, sb.ctx, scale, out=a[sb.rd:], rule=rule,
                                              gate=None if gate is None else gate[sb.rd:],

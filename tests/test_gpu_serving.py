@@ -96,3 +96,25 @@ def test_steps_keep_their_host_memory(cuda_status):
     for got in rounds:
         for key, logits in want.items():
             assert torch.equal(got[key], logits), key
+
+
+@pytest.mark.parametrize("H,G,D,lens", [(4, 2, 64, [(1, 1), (129, 129)]), (8, 8, 128, [(257, 600), (128, 128), (33, 2000), (256, 256)]),
+                                        (6, 2, 64, [(40 * i + 1, 60 * i + 1) for i in range(11)])])
+def test_portions_in_one_launch_are_those_alone(H, G, D, lens, cuda_status):
+    """Portions (queries, keys) of several sequences, whole and later ones, more than fit one launch: the same bits as a launch each, and nothing of the
+    rows between and behind them (NaN) enters."""
+    from rustral_b200 import _native as N
+    from rustral_b200.ops import attention as A
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    parts, alone = [], []
+    for L, S in lens:
+        q = torch.full((L + 3, (H + 2 * G) * D), float("nan"), device="cuda").bfloat16()
+        kv = torch.full((S + 3, 2 * G * D), float("nan"), device="cuda").bfloat16()
+        q[:L], kv[:S] = torch.randn(L, q.shape[1], device="cuda", generator=g).bfloat16(), torch.randn(S, kv.shape[1], device="cuda", generator=g).bfloat16()
+        view = (q[:L, :H * D].view(1, L, H, D), kv[:S, :G * D].view(1, S, G, D), kv[:S, G * D:].view(1, S, G, D))
+        parts.append((*view, torch.zeros(1, L, H, D, device="cuda").bfloat16()))
+        alone.append(A.prompt_attention(*view, 0.2, torch.zeros(1, L, H, D, device="cuda").bfloat16()))
+    before = N.launch_count
+    A.prompt_attention_many(parts, 0.2)
+    assert N.launch_count - before == -(-len(parts) // 8)
+    assert all(torch.equal(p[3], o) and torch.isfinite(o).all() for p, o in zip(parts, alone))
