@@ -241,7 +241,7 @@ struct F2Smem {
 
 // Several problems in one launch (portions of several prompts): each with tensor maps of its own, so that rows behind its end read as zeros and
 // nothing of another sequence can enter, and the query tiles of all of them along the grid.  A portion alone is a grid of (tiles, heads), mostly smaller
-// than the GPU: four portions of 129 to 1500 tokens, 32 heads of 64, a launch each 72 us, together @MANY@.
+// than the GPU: four portions of 129 to 1500 tokens, 32 heads of 64, a launch each 72 us, together 49.
 constexpr int kF2Many = 8;
 struct F2One {
   CUtensorMap q, k, v, qr, kr;

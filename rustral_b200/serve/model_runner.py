@@ -32,9 +32,10 @@ class StepBatch:
     """The rows of one model pass: prompt portions first (`spans`), then one row per decoded sequence (from row `rd`).
     `segments`: the same sequences for layers with recurrent state (None: the model has none).  `arrived`: given for a step of decoded
     sequences only whose tables and lengths were complete before it began (see ops.paged.attention_step); positions and slots (None) then
-    follow from them where a layer asks."""
+    follow from them where a layer asks.  `cached`: cache slots of all positions of the portions that do not begin at 0 (index -> int64 tensor
+    on the device), where they came with the step's other inputs."""
 
-    def __init__(self, ids, pos, slots, spans, rd, tables, bt, ctx, block_size, segments=None, arrived=None):
+    def __init__(self, ids, pos, slots, spans, rd, tables, bt, ctx, block_size, segments=None, arrived=None, cached=None):
         self.ids, self._pos, self._slots, self.arrived = ids, pos, slots, arrived      # int64 device tensors, one entry per row
         self.spans = spans                                        # (first row, end row, first position) per portion
         self.rd, self.rows = rd, ids.shape[0]
@@ -42,6 +43,7 @@ class StepBatch:
         self.bt, self.ctx = bt, ctx                               # decode rows: block tables, context lengths (int32)
         self.block_size = block_size
         self.segments = segments
+        self._cached = cached or {}
         self._keys, self._row_tables, self._rotations, self._all_keys = {}, None, {}, None
 
     @property
@@ -79,6 +81,9 @@ class StepBatch:
     def key_slots(self, i: int, first: int, kept: int = 0) -> torch.Tensor:
         """Cache slots of positions 0 .. `kept` and `first` .. end of portion i (earlier portions and this one)."""
         key = (i, first, kept)
+        if key not in self._keys and i in self._cached:
+            every = self._cached[i]
+            self._keys[key] = torch.cat([every[:kept], every[first:]]) if kept else every[first:]
         if key not in self._keys:
             r0, r1, start = self.spans[i]
             bs = self.block_size
@@ -282,46 +287,64 @@ class ModelRunner:
         (Batched and chunked prefill of the reference's scheduler: crates/nn/src/continuous_batching.rs:248-295.)"""
         dev, bs = self.device, self.block_size
         rd = sum(len(c[1]) for c in chunks)
-        T = rd + len(dec_ids)
-        width = max((len(self.cache.block_table(s_)) for s_ in dec_ids), default=0)
-        memory, copied = self._memory.take(24 * T + 4 * len(dec_ids) * width)
-        host = memory[:24 * T].view(torch.int64).view(3, T)          # token ids, positions, cache slots
-        ids_h, at_pos, at_slots = host[0].numpy(), host[1].data_ptr(), host[2].data_ptr()
-        spans, tables, r0 = [], [], 0
-        for seq_id, tokens, start, _ in chunks:
-            r1 = r0 + len(tokens)
-            spans.append((r0, r1, start))
-            tables.append(self.cache.block_table(seq_id))
-            ids_h[r0:r1] = tokens
-            self.cache.fill_slots(seq_id, start, r1 - r0, at_pos + 8 * r0, at_slots + 8 * r0)
-            r0 = r1
-        for r, (seq_id, tok, n) in enumerate(zip(dec_ids, dec_tok, dec_len), rd):
-            ids_h[r] = tok
-            self.cache.fill_slots(seq_id, n - 1, 1, at_pos + 8 * r, at_slots + 8 * r)
-        host = host.to(dev, non_blocking=True)
-        bt = ctx = None
-        if dec_ids:
-            bt = memory[24 * T:24 * T + 4 * len(dec_ids) * width].view(torch.int32).view(len(dec_ids), width)
-            self.cache.fill_tables(dec_ids, bt)
-            bt = bt.to(dev, non_blocking=True)
-            ctx = torch.tensor(dec_len, dtype=torch.int32, device=dev)
-        self._memory.give(memory, copied)
-        segments = None
-        if self.recurrent:
-            table = [(r0, r1 - r0, self.cache.state_slot(c[0]), start) for (r0, r1, start), c in zip(spans, chunks)]
-            table += [(rd + i, 1, self.cache.state_slot(s_), n - 1) for i, (s_, n) in enumerate(zip(dec_ids, dec_len))]
-            segments = Segments.of(table, dev)
-        sb = StepBatch(host[0], host[1], host[2], spans, rd, tables, bt, ctx, bs, segments)
+        nd = len(dec_ids)
+        T = rd + nd
+        spans, r0 = [], 0
+        for _, tokens, start, _ in chunks:
+            spans.append((r0, r0 + len(tokens), start))
+            r0 += len(tokens)
         # logits only where they are asked for: by default the last row of every chunk that completes its prompt, and the
         # decode rows
         want = []
         for (r0, r1, _), c in zip(spans, chunks):
             want.append([r1 - 1] if c[3] is True else [r0 + i for i in c[3]] if c[3] else [])
         rows = [r for w in want for r in w] + list(range(rd, T))
-        if rows and rows != list(range(T)):
-            sel = torch.tensor(rows, dtype=torch.int64, device=dev)
-        else:
-            sel = None if rows else []
+        every_row = rows == list(range(T))
+        # All inputs of the step in one page-locked block and one copy: a copy from other memory waits until the stream has come to it, and
+        # the host then forms the step's launches while the GPU has nothing to do.  token ids, positions, slots; rows of the logits; slots of
+        # the cached positions of later portions (their positions, not copied, at the end); block tables and lengths
+        width = max((len(self.cache.block_table(s_)) for s_ in dec_ids), default=0)
+        later = [(i, start + r1 - r0) for i, (r0, r1, start) in enumerate(spans) if start]
+        n_sel = 0 if every_row else len(rows)
+        longs = 3 * T + n_sel + sum(n for _, n in later)
+        sent = 8 * longs + 4 * nd * (width + 1)
+        memory, copied = self._memory.take((sent + 7) // 8 * 8 + 8 * max((n for _, n in later), default=0))
+        host = memory[:8 * longs].view(torch.int64)
+        numbers, at = host.numpy(), host.data_ptr()
+        tables = []
+        for (seq_id, tokens, start, _), (r0, r1, _) in zip(chunks, spans):
+            tables.append(self.cache.block_table(seq_id))
+            numbers[r0:r1] = tokens
+            self.cache.fill_slots(seq_id, start, r1 - r0, at + 8 * (T + r0), at + 8 * (2 * T + r0))
+        for r, (seq_id, tok, n) in enumerate(zip(dec_ids, dec_tok, dec_len), rd):
+            numbers[r] = tok
+            self.cache.fill_slots(seq_id, n - 1, 1, at + 8 * (T + r), at + 8 * (2 * T + r))
+        numbers[3 * T:3 * T + n_sel] = rows[:n_sel]
+        end, places = 3 * T + n_sel, {}
+        for i, n in later:
+            self.cache.fill_slots(chunks[i][0], 0, n, at + (sent + 7) // 8 * 8, at + 8 * end)
+            places[i] = (end, end + n)
+            end += n
+        bt = ctx = None
+        if dec_ids:
+            ints = memory[8 * longs:sent].view(torch.int32)
+            self.cache.fill_tables(dec_ids, ints[:nd * width].view(nd, width))
+            ints[nd * width:].numpy()[:] = dec_len
+        block = memory[:sent].to(dev, non_blocking=True)
+        self._memory.give(memory, copied)
+        sent_longs = block[:8 * longs].view(torch.int64)
+        ids, pos, slots = sent_longs[:3 * T].view(3, T)
+        if dec_ids:
+            ints = block[8 * longs:].view(torch.int32)
+            bt, ctx = ints[:nd * width].view(nd, width), ints[nd * width:]
+        segments = None
+        if self.recurrent:
+            table = [(r0, r1 - r0, self.cache.state_slot(c[0]), start) for (r0, r1, start), c in zip(spans, chunks)]
+            table += [(rd + i, 1, self.cache.state_slot(s_), n - 1) for i, (s_, n) in enumerate(zip(dec_ids, dec_len))]
+            segments = Segments.of(table, dev)
+        sb = StepBatch(ids, pos, slots, spans, rd, tables, bt, ctx, bs, segments,
+                       cached={i: sent_longs[lo:hi] for i, (lo, hi) in places.items()})
+        sel = sent_longs[3 * T:3 * T + n_sel] if n_sel else None if rows else []
         logits = self._run(sb, sel)
         out, at = [], 0
         for w, c in zip(want, chunks):
