@@ -1099,8 +1099,8 @@ template <int A_MN, int B_MN, int BLOCK_N, int STAGES, int FP8 = 0, bool EXTRA =
 __global__ void __launch_bounds__(kNumThreads + (EXTRA && A_MN ? 32 * kSumWarps : 0), 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux,
-                      const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride, EpiParams ep,
-                      unsigned int* status) {
+                      const __grid_constant__ CUtensorMap tmSide, int M, int N, int K, int group_m, int num_splits, int kb_per_split, long long d_split_stride,
+                      const int* expert_offsets, EpiParams ep, unsigned int* status) {
   using L = SmemLayoutPair<BLOCK_N, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1171,8 +1171,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   auto decode_tile = [&](int unit, int& m_blk, int& n_blk, int& kb0, int& kb1, int& split) {
     split = unit / num_tiles;
     const int tile = unit - split * num_tiles;
-    kb0 = split * kb_per_split;
-    kb1 = min(num_kb_total, kb0 + kb_per_split);
+    if (A_MN && B_MN && expert_offsets != nullptr) {   // grouped weight gradients: a slab for each expert, from that expert's rows
+      kb0 = __ldg(expert_offsets + split) / kBlockK;
+      kb1 = __ldg(expert_offsets + split + 1) / kBlockK;
+    } else {
+      kb0 = split * kb_per_split;
+      kb1 = min(num_kb_total, kb0 + kb_per_split);
+    }
     const int group = tile / group_size;
     const int first_m = group * group_m;
     const int gm = min(group_m, num_m - first_m);
@@ -1285,6 +1290,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     for (int tile = cluster_id; tile < num_units; tile += num_clusters, ++t) {
       int m_blk, n_blk, kb0, kb1, split;
       decode_tile(tile, m_blk, n_blk, kb0, kb1, split);
+      const bool empty_k = A_MN && B_MN && kb1 <= kb0;   // an expert without rows: the accumulator was never written
       const uint32_t acc = t & 1, acc_ph = (t >> 1) & 1;
       const uint32_t stg = smem_base + L::kStagingOffset + ew * L::kStagingBytesPerWarp;
       const uint32_t side_bars = bar_side + 16 * ew;
@@ -1307,17 +1313,21 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (ep.staged >= 2) {
         const int drow = num_splits > 1 ? split * M + row0 : row0;
         epilogue_tma<BLOCK_N / 2, L::kSlots, EXTRA && !A_MN>(ep, &tmD, &tmAux, stg, side_bars, t, taddr + cgrp * (BLOCK_N / 2), row0, drow, colg, M, N,
-                                                    lane, false, abort_flag, status, arrive);
+                                                    lane, empty_k, abort_flag, status, arrive);
         continue;
       }
       EpiParams epu = ep;
       if (num_splits > 1)
-        epu.d = reinterpret_cast<float*>(ep.d) + static_cast<long long>(split) * d_split_stride;
+        epu.d = static_cast<char*>(ep.d) + static_cast<long long>(split) * d_split_stride * (ep.out_f32 ? 4 : 2);
 #pragma unroll 1
       for (int c = cgrp * (BLOCK_N / 64); c < (cgrp + 1) * (BLOCK_N / 64); ++c) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
+        if (empty_k) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = 0;
+        }
         if (c == (cgrp + 1) * (BLOCK_N / 64) - 1) arrive();
         const int col0 = n_blk * BLOCK_N + c * 32;
         if (row < M && col0 < N) epilogue_chunk(epu, r, row, col0, N);
@@ -1563,6 +1573,17 @@ bool pair_kernel_enabled() {
   return v == 1;
 }
 
+// Problems for the two-CTA kernel (where their tiles are 256 wide).  Of the grouped ones the weight gradients whose experts' results are
+// stacked in whole 32-row tiles, so that TMA stores them: every expert has all M x N of its tiles and only the contraction is ragged,
+// which costs a pair nothing: eight experts of 16384 x 2048 and 2048 x 8192 over about 750 rows each, forward and backward of the layer
+// 2226 us with single CTAs, 2130 with pairs.
+// The grouped products over permuted rows stay: an expert's rows come in 128-row tiles, and a pair would leave half a tile idle behind
+// every second expert.
+bool pair_takes(const RbGemmArgs& g) {
+  if (g.peer_mode != 0 || g.M <= 128 || g.max_ctas != 0 || !pair_kernel_enabled()) return false;
+  return g.group_mode == 0 || (g.group_mode == 2 && g.M % 32 == 0 && g.d_expert_stride == static_cast<long long>(g.M) * g.ldd);
+}
+
 template <int A_MN, int B_MN, int FP8 = 0>
 int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb_half, int clusters, int splits,
                 cudaStream_t stream) {
@@ -1579,6 +1600,8 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
     splits = (num_kb + kb_per - 1) / kb_per;
     slab = static_cast<long long>(g.M) * g.N;
   }
+  const bool grouped = g.group_mode == 2;                 // a slab for each expert, not folded
+  if (grouped) slab = g.d_expert_stride;
   const CUtensorMap *td = ta, *tx = ta, *ts = ta;
   rb::EpiParams ep;
   constexpr bool kExtra = (!A_MN && !FP8) || (A_MN && B_MN);                  // forward products and input gradients; weight gradients
@@ -1598,7 +1621,8 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
     configured = smem;
   }
   const cudaError_t e = rbhost::launch_pdl(kern, dim3(2 * clusters), dim3(threads), smem, stream, 2, *ta, *tb_half, *td, *tx, *ts, g.M, g.N,
-                                           k_units, group_m, splits, kb_per, slab, ep, rbhost::status_ptr());
+                                           k_units, group_m, grouped ? g.num_experts : splits, kb_per, slab,
+                                           grouped ? reinterpret_cast<const int*>(g.expert_offsets) : nullptr, ep, rbhost::status_ptr());
   if (e != cudaSuccess || splits <= 1) return static_cast<int>(e);
   const long long n4 = slab / 4;
   int rgrid = static_cast<int>((n4 + 255) / 256 < 148 * 8 ? (n4 + 255) / 256 : 148 * 8);
@@ -1617,13 +1641,13 @@ int width_cost(int bn) { return bn == 256 ? 100 : bn == 192 ? 104 : bn == 128 ? 
 // Microseconds of a plan: waves of tiles at the measured rate (6.5 ns per unit of K for a 128 x 256 tile), the last tile's results, and
 // for a split contraction a second launch and the slabs' way through memory.  Leaving the slabs out of the sum had wide results split
 // that should not be (measured, split / whole): 2048 x 8192 x 4096 135 / 101 us, 4096 x 2048 x 8192 131 / 98, 2704 x 2048 x 2048 42 / 25.
-double plan_cost(int M, int N, int K, int bn, int splits, int sms, bool pair_ok) {
-  const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn) * splits;
+double plan_cost(int M, int N, int K, int bn, int splits, int experts, int sms, bool pair_ok) {
+  const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn) * splits * experts;
   const long long waves = (tiles + sms - 1) / sms;
   // 256-wide plans of plain problems run on the two-CTA kernel, measured about 10 % faster per tile
   const int wc = (bn == 256 && pair_ok) ? 88 : width_cost(bn);
   const double width = bn / 256.0;
-  double us = waves * width * (wc / 100.0) * (static_cast<double>(K) / splits) * 0.0065 + 1.5 * width;
+  double us = waves * width * (wc / 100.0) * (static_cast<double>(K) / (splits * experts)) * 0.0065 + 1.5 * width;
   if (splits > 1) us += 2.0 + (2.0 * splits + 1.0) * M * static_cast<double>(N) * 4.0 / 5.0e6;
   return us;
 }
@@ -1634,7 +1658,8 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
   const bool can_split = g.group_mode == 0 && g.peer_mode == 0 && g.workspace != nullptr && g.act == RB_ACT_NONE && !g.aux_out &&
                          !g.a_scale && !g.b_scale && !g.ab_fp8 &&
                          (g.N % 4 == 0) && (static_cast<long long>(g.M) * g.N % 4 == 0) && (!g.residual || (g.ldr % 4 == 0));
-  const bool pair_ok = g.peer_mode == 0 && g.group_mode == 0 && g.M > 128 && g.max_ctas == 0 && pair_kernel_enabled();
+  const bool pair_ok = pair_takes(g);
+  const int experts = g.group_mode == 2 ? g.num_experts : 1;      // each with tiles of its own and, on average, its part of the contraction
   double best = -1.0;
   bn_out = 128; splits_out = 1;
   for (int c = 0; c < 4; ++c) {
@@ -1649,7 +1674,7 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
         if (g.splits <= 0 && g.K / sp < 768) continue;
         if (static_cast<long long>(sp) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4 > g.workspace_bytes) continue;
       }
-      const double cost = plan_cost(g.M, g.N, g.K, bn, sp, sms, pair_ok);
+      const double cost = plan_cost(g.M, g.N, g.K, bn, sp, experts, sms, pair_ok);
       if (best < 0.0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
     }
   }
@@ -1794,12 +1819,12 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
                               : rbhost::get_tmap_2d(g.b, 2, (uint64_t)g.K, (uint64_t)g.N * b_experts, (uint64_t)g.ldb, 64, (uint32_t)bn, 1, &err);
   if (!tb) return err ? err : -5;
 
-  if (bn == 256 && g.peer_mode == 0 && g.group_mode == 0 && g.M > 128 && g.max_ctas == 0 && pair_kernel_enabled()) {
+  if (bn == 256 && pair_takes(g)) {
     // two-CTA kernel: 256 x 256 tiles per CTA pair, each CTA loads half of the B tile
     const CUtensorMap* tb_half =
         g.b_mn_major ? tb : rbhost::get_tmap_2d(g.b, 2, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb, 64, 128, 1, &err);
     if (!tb_half) return err ? err : -5;
-    const long long tiles2 = (long long)((g.M + 255) / 256) * ((g.N + 255) / 256) * splits;
+    const long long tiles2 = (long long)((g.M + 255) / 256) * ((g.N + 255) / 256) * (g.group_mode == 2 ? g.num_experts : splits);
     const int max_clusters = sms / 2;
     const int clusters = static_cast<int>(tiles2 < max_clusters ? tiles2 : max_clusters);
     if (!g.a_mn_major && !g.b_mn_major) return launch_pair<0, 0>(g, ta, tb_half, clusters, splits, stream);

@@ -120,3 +120,29 @@ def test_expert_weight_gradients_in_16_bits(rows, N, cuda_status):
             want = dy[m].double().T @ x[m].double()
             bound = 2.0 ** -8 * want.abs() + 2048 * 2.0 ** -24 * (dy[m].double().abs().T @ x[m].double().abs()) + 1e-30
             assert ((out[e].double() - want).abs() <= bound).all(), e
+
+
+@pytest.mark.parametrize("N", [800, 808])
+@pytest.mark.parametrize("form", ["bf16", "fp32", "fp32 added", "bf16 added"])
+def test_expert_weight_gradients_in_wide_tiles(N, form, cuda_status):
+    """256-wide tiles: on CTA pairs where the experts' results are stacked in whole 32-row tiles (800 rows, the last pair with a tile and a
+    half of nothing), on single CTAs where they are not; experts with few rows, one k-block's worth and none."""
+    from rustral_b200.ops import moe
+    E, K = 6, 760
+    counts = (1, 64, 65, 700, 0, 333)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).int()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    idx = idx[torch.randperm(len(idx), generator=torch.Generator().manual_seed(1))].cuda()[:, None].contiguous()
+    pl = moe.plan(idx, E)
+    x, dy = (torch.randn(idx.shape[0], n, device="cuda", generator=g).bfloat16() for n in (K, N))
+    xp, dyp = moe.gather(x, pl), moe.gather(dy, pl)
+    dtype = torch.float32 if form.startswith("fp32") else torch.bfloat16
+    base = torch.randn(E, N, K, device="cuda", generator=g).to(dtype)
+    out = moe.grouped_wgrad(dyp, xp, pl, out=base.clone(), accumulate=True) if form.endswith("added") else moe.grouped_wgrad(dyp, xp, pl, dtype=dtype)
+    for e in range(E):
+        m = idx[:, 0] == e
+        want = dy[m].double().T @ x[m].double() + (base[e].double() if form.endswith("added") else 0)
+        size = dy[m].double().abs().T @ x[m].double().abs() + base[e].double().abs()
+        # sums of at most 701 terms in 32 bits, any order; a result of 16 bits rounded once
+        bound = 1024 * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0) + 1e-30
+        assert ((out[e].double() - want).abs() <= bound).all(), (e, counts[e])
