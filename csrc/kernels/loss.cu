@@ -132,113 +132,6 @@ cross_entropy_kernel(const __nv_bfloat16* logits, long long ld, const long long*
   }
 }
 
-// The same for long aligned rows that fit half an SM's shared memory.  A CTA stays and takes rows blockIdx.x, + gridDim.x, ...; a bulk copy brings a row, which
-// is read from memory once, while the SM's other CTAs work on theirs.  Per row: maximum (packed bf16, no exponentials), sum of exponentials,
-// gradients.  One B200, us, before / now: 32768 rows of 50257 1690 / 1544 (traffic alone 1030, exponentials 800), 4096 of 32768 152 / 143, 8192 of 12000 141 / 131,
-// 1998 of 8192 28.0 / 25.5.  One CTA of 1024 threads with the next row on its way was slower (1619, 152, 172, 36): nothing fills its barriers.
-constexpr int kCeRowThreads = 512;
-constexpr int kCeRowBytes = 112 * 1024;                  // of a row, with padding; two CTAs of an SM hold one each
-__device__ __forceinline__ uint32_t ce_max2(uint32_t a, uint32_t b) {
-  __nv_bfloat162 m = __hmax2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
-  return *reinterpret_cast<uint32_t*>(&m);
-}
-template <class Op>
-__device__ __forceinline__ float ce_block(float v, float* sh, Op op) {      // the same value in every thread; `sh` is free again behind the next barrier
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  v = sh[threadIdx.x & 15];
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-__global__ void __launch_bounds__(kCeRowThreads, 2)
-cross_entropy_rows_kernel(const __nv_bfloat16* logits, long long ld, const long long* __restrict__ targets, float* __restrict__ loss,
-                          float* __restrict__ lse_out, __nv_bfloat16* dlogits, long long ldd, int rows, int n_valid, int n_pad, float grad_scale,
-                          long long ignore_index, unsigned int* status RB_BOUNDS_PARAM) {
-  extern __shared__ __align__(128) uint8_t ce_smem[];
-  __shared__ float sh_max[16], sh_sum[16];
-  __shared__ uint64_t bar;
-  __shared__ int abort_flag;
-  const int n8 = (n_valid + 7) / 8;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    mbar_init(smem_u32(&bar), 1);
-    abort_flag = 0;
-    fence_mbar_init();
-  }
-  __syncthreads();
-  pdl_wait();
-  pdl_launch();
-  uint32_t turn = 0;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x, ++turn) {
-    if (tid == 0) {                                                  // every thread has read the row before this one (barrier below)
-      mbar_arrive_expect_tx(smem_u32(&bar), n8 * 16);
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                   ::"r"(smem_u32(ce_smem)), "l"(logits + row * ld), "r"(n8 * 16), "r"(smem_u32(&bar)) : "memory");
-    }
-    const long long tgt = targets[row];
-    const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= n_valid;
-    if (ignored && tgt != ignore_index && tid == 0) RB_BOUNDS_HIT(105);
-    if (!mbar_wait(smem_u32(&bar), turn & 1, &abort_flag, status, 51)) break;
-    const uint4* x = reinterpret_cast<const uint4*>(ce_smem);
-    const __nv_bfloat16* xs = reinterpret_cast<const __nv_bfloat16*>(x);
-    const int tail = n_valid & 7, whole = n_valid / 8;               // the last piece may hold padding
-    uint32_t m2 = 0xff80ff80u;                                       // two -inf
-    float own = -INFINITY;
-    for (int i = tid; i < whole; i += kCeRowThreads) {
-      const uint4 u = x[i];
-      m2 = ce_max2(m2, ce_max2(ce_max2(u.x, u.y), ce_max2(u.z, u.w)));
-    }
-    if (tid < tail) own = __bfloat162float(xs[whole * 8 + tid]);
-    const float2 mm = unpack_bf16x2(m2);
-    const float m = ce_block(fmaxf(fmaxf(mm.x, mm.y), own), sh_max, [](float a, float b) { return fmaxf(a, b); });
-    float s = 0.f;
-    for (int i = tid; i < whole; i += kCeRowThreads) {
-      const uint4 u = x[i];
-      const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
-      s += (__expf(f0.x - m) + __expf(f0.y - m)) + (__expf(f1.x - m) + __expf(f1.y - m)) + (__expf(f2.x - m) + __expf(f2.y - m)) +
-           (__expf(f3.x - m) + __expf(f3.y - m));
-    }
-    if (tid < tail) s += __expf(own - m);
-    s = ce_block(s, sh_sum, [](float a, float b) { return a + b; });
-    if (m == -INFINITY) s = 0.f;                                     // nothing but -inf
-    const float lse = m + logf(s);
-    if (tid == 0) {
-      if (lse_out) lse_out[row] = lse;
-      loss[row] = ignored ? 0.f : lse - __bfloat162float(xs[tgt]);
-    }
-    if (dlogits != nullptr) {
-      uint4* dx = reinterpret_cast<uint4*>(dlogits + row * ldd);
-      const float gs = ignored ? 0.f : grad_scale;
-      const int t8 = ignored ? -1 : static_cast<int>(tgt >> 3), te = static_cast<int>(tgt & 7);
-      for (int i = tid; i < n_pad / 8; i += kCeRowThreads) {
-        float f[8] = {};
-        if (i < n8) {
-          const uint4 u = x[i];
-          const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
-          f[0] = f0.x; f[1] = f0.y; f[2] = f1.x; f[3] = f1.y; f[4] = f2.x; f[5] = f2.y; f[6] = f3.x; f[7] = f3.y;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            f[j] = __expf(f[j] - lse);
-            if (i == t8 && j == te) f[j] -= 1.f;
-            f[j] *= gs;
-          }
-          if (i >= whole) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (j >= tail) f[j] = 0.f;
-          }
-        }
-        dx[i] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
-      }
-    }
-    __syncthreads();                                                 // the row has been read: the next goes into its place
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ float ld_as_float(const T* p);
 template <>
@@ -342,24 +235,6 @@ RB_API int rb_cross_entropy(const void* logits, long long ld, const long long* t
                             long long ignore_index, void* stream_v) {
   if (rows <= 0 || n_valid <= 0 || n_pad < n_valid || !logits || !targets || !loss) return -1;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  // Rows that bulk copies can bring (16-byte aligned, whole pieces of 8 inside the row's pitch), fit twice and are long enough for 1024 threads.  Shorter
-  // ones are the other kernel's.
-  const int pieces = (n_valid + 7) / 8;
-  if (n_valid >= 8192 && pieces * 16 <= rb::kCeRowBytes && !(ld & 7) && n_pad >= pieces * 8 && ld >= n_pad && !(reinterpret_cast<uintptr_t>(logits) & 15) &&
-      (!dlogits || (!(ldd & 7) && !(n_pad & 7) && !(reinterpret_cast<uintptr_t>(dlogits) & 15)))) {
-    const int smem = (pieces * 16 + 127) & ~127;
-    static bool cfg_dev[64] = {false};
-    bool& cfg = cfg_dev[rbhost::device_slot()];
-    if (!cfg) {
-      const cudaError_t e = cudaFuncSetAttribute(rb::cross_entropy_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rb::kCeRowBytes);
-      if (e != cudaSuccess) return static_cast<int>(e);
-      cfg = true;
-    }
-    const int fit = 227 * 1024 / (smem + 2048), most = rbhost::device_sm_count() * (fit < 4 ? fit : 4);
-    return static_cast<int>(rbhost::launch_pdl(rb::cross_entropy_rows_kernel, dim3(rows < most ? rows : most), dim3(rb::kCeRowThreads), smem, stream, 1,
-        reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, loss, lse, reinterpret_cast<__nv_bfloat16*>(dlogits), ldd, rows, n_valid, n_pad,
-        grad_scale, ignore_index, rbhost::status_ptr() RB_BOUNDS_ARG));
-  }
   rbhost::launch_pdl(rb::cross_entropy_kernel, dim3(rows), dim3(rb::kCeThreads), 0, stream, 1,
       reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, loss, lse, reinterpret_cast<__nv_bfloat16*>(dlogits),
       ldd, n_valid, n_pad, grad_scale, ignore_index RB_BOUNDS_ARG);
