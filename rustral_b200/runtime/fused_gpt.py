@@ -396,7 +396,8 @@ class FusedGPTEngine:
                                                           dlogits=logits)
         ops.binary("add", self.loss_acc.view(1), ops.sum_all(loss_rows).view(1), out=self.loss_acc.view(1))
 
-        beside = self._beside(T)
+        # An eager pass waits for the host's launches, to which every hand-over adds about 10 us (first step of 2 layers, in line / beside, 1622 / 1908 us)
+        beside = self._beside(T) if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing() else None
 
         def weight_grad(dy, x, name, bias=None):
             """dW = dy^T x, and the bias gradient with it."""
