@@ -45,8 +45,8 @@ def test_trainer_public_api_loss_decreases(cuda_status):
 
 @pytest.mark.parametrize("name", ["gpt2-test", "llama-test"])
 def test_weight_gradients_beside_the_chain_are_those_in_line(name, cuda_status):
-    """The same kernels on the same operands on another stream: equal bits, in line for the eager calls (the first two of a shape) and replayed, with two micro-batches, from a
-    stream that is not the default one, while freed memory is handed out again and overwritten."""
+    """The same kernels on the same operands on another stream: equal bits, in line for the eager calls (the first two of a shape) and replayed, with
+    two micro-batches, from a stream that is not the default one, while freed memory is handed out again and overwritten."""
     cfg = preset(name)
     g = torch.Generator().manual_seed(3)
     grads = []
