@@ -1682,6 +1682,11 @@ double plan_cost(int M, int N, int K, int bn, int splits, int experts, int sms, 
   return us;
 }
 
+// Workspace of a split contraction: a slab of results for each part, and behind them one of column sums where the call wants those.
+long long split_bytes(const RbGemmArgs& g, int splits) {
+  return static_cast<long long>(splits) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4;
+}
+
 void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
   const int cands[4] = {256, 192, 128, 64};
   const int split_cands[7] = {1, 2, 3, 4, 6, 8, 12};
@@ -1702,7 +1707,7 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
       if (sp > 1) {
         if (!can_split) continue;
         if (g.splits <= 0 && g.K / sp < 768) continue;
-        if (static_cast<long long>(sp) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4 > g.workspace_bytes) continue;
+        if (split_bytes(g, sp) > g.workspace_bytes) continue;
       }
       const double cost = plan_cost(g.M, g.N, g.K, bn, sp, experts, sms, pair_ok);
       if (best < 0.0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
@@ -1767,9 +1772,11 @@ RB_API long long rb_gemm_workspace(const RbGemmArgs* args, long long most) {
   g.workspace = &g;                           // any address: nothing is launched
   g.workspace_bytes = most;
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.act == RB_ACT_SWIGLU || rbhost::gemm_rows_takes(g)) return 0;
+  // `most` bounds the slabs alone: the plan of a weight gradient, chosen here or named by a table, is the same with column sums as without
+  g.col_sum = nullptr;
   int bn = 128, splits = 1;
   pick_plan(g, rbhost::device_sm_count(), bn, splits);
-  return splits > 1 ? static_cast<long long>(splits) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4 : 0;
+  return splits > 1 ? split_bytes(*args, splits) : 0;
 }
 
 RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {

@@ -83,7 +83,8 @@ typedef struct RbGemmArgs {
 
 // Returns 0 on success, a negative code for rejected arguments, a positive cudaError otherwise.
 int rb_gemm_bf16(const RbGemmArgs* args, void* stream);
-// Bytes of workspace that rb_gemm_bf16 makes use of for this call when it may have up to `most`; 0: none.
+// Bytes of workspace that rb_gemm_bf16 makes use of for this call when its slabs may take up to `most` (col_sum: a slab of sums each comes on top);
+// 0: none.
 long long rb_gemm_workspace(const RbGemmArgs* args, long long most);
 
 #ifdef __cplusplus

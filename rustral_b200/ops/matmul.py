@@ -168,10 +168,12 @@ N.optional_sig("rb_gemm_workspace", [N.C.POINTER(N.RbGemmArgs), N.c_ll], N.c_ll)
 
 def _give_workspace(g, device, need: int):
     """Names the split-K scratch in `g`; what is returned has to live until the launch.  `need`: what the plan takes (`rb_gemm_workspace`); with
-    none the plan is the same without scratch.  A captured graph gets its own: graphs that name one buffer could not be replayed side by side."""
+    none the plan is the same without scratch.  A captured graph gets its own: graphs that name one buffer could not be replayed side by side.  So does
+    a call whose column sums come on top of slabs that fill the kept buffer."""
     if not need:
         return None
-    ws = torch.empty(need, dtype=torch.uint8, device=device) if torch.cuda.is_current_stream_capturing() else _workspace(device)
+    own = need > WORKSPACE_BYTES or torch.cuda.is_current_stream_capturing()
+    ws = torch.empty(need, dtype=torch.uint8, device=device) if own else _workspace(device)
     g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
     return ws
 

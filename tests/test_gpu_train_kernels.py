@@ -246,3 +246,33 @@ def test_embedding_gradient_for_vocabularies_around_a_scan_round(vocab, tokens, 
     often = torch.zeros(vocab, 64, dtype=torch.float64, device="cuda").index_add(0, ids, dy.double().abs())
     count = torch.bincount(ids, minlength=vocab)[:, None]
     assert ((got.double() - want).abs() <= 2.0 ** -24 * (count + 1) * often).all()
+
+
+@pytest.mark.parametrize("hook", [False, True])
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_split_that_fills_the_scratch_takes_column_sums_too(hook, captured, cuda_status):
+    """Eight parts of 4096 x 1024 are exactly the scratch of split contractions: asked for directly or by a plan table, they are taken with column sums
+    as without.  The product is the one without sums; the sums' bound as above."""
+    from rustral_b200.ops import matmul
+    tokens, out, inp = 8192, 4096, 1024
+    assert 8 * out * inp * 4 == matmul.WORKSPACE_BYTES
+    g = torch.Generator(device="cuda").manual_seed(5)
+    dy = torch.randn(tokens, out, device="cuda", generator=g).bfloat16()
+    x = torch.randn(tokens, inp, device="cuda", generator=g).bfloat16()
+    w, b, plain = torch.empty(out, inp, device="cuda"), torch.empty(out, device="cuda"), torch.empty(out, inp, device="cuda")
+    call = lambda dst, splits, sums: matmul.gemm(dy, x, a_mn=True, b_mn=True, out=dst, splits=splits, col_sum=sums)  # noqa: E731
+    call(plain, 8, None)
+    matmul._PLAN_HOOK = (lambda *a: {"block_n": 0, "splits": 8, "group_m": 0}) if hook else None
+    try:
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                call(w, 0 if hook else 8, b)
+            graph.replay()
+        else:
+            call(w, 0 if hook else 8, b)
+    finally:
+        matmul._PLAN_HOOK = None
+    assert torch.equal(w, plain)
+    want = dy.double().sum(0)
+    assert ((b.double() - want).abs() <= 2.0 ** -24 * (tokens / 64 + 16) * dy.double().abs().sum(0) + 2.0 ** -23 * want.abs()).all()
