@@ -235,21 +235,33 @@ def state_to_flat(cfg: GPTConfig, specs: list, state: dict, host: torch.Tensor) 
 
 
 class _Beside:
-    """Weight gradients of one backward pass on a stream of their own, beside the chain of input gradients that nothing waits for them in.  What they
-    read was allocated on the main stream, so it is held until that stream has waited for them."""
+    """Weight gradients of one backward pass on a stream of their own, beside the chain of input gradients that nothing waits for them in.  The
+    gradients they read were allocated on the main stream, so they are held until that stream has waited for them; it does so whenever more than
+    `MOST_HELD` bytes are held, whatever the depth and the widths of the model are."""
+
+    # Six layers of 2048 tokens x 384 hold 105 MB, twelve of 4096 x 768 700 MB (without a limit).
+    MOST_HELD = 256 << 20
 
     def __init__(self, stream):
-        self.main, self.stream, self.held = torch.cuda.current_stream(stream.device), stream, []
+        self.main, self.stream, self.held, self.held_bytes = torch.cuda.current_stream(stream.device), stream, [], 0
 
-    def run(self, fn, *reads) -> None:
-        self.held.append(reads)
+    def run(self, fn, dy, x) -> None:
+        """`fn` on the other stream; it reads `dy` and an activation `x`, which lives longer than the pass anyway."""
+        size = dy.numel() * dy.element_size()
+        if self.held_bytes + size > self.MOST_HELD:
+            self.join()
+        self.held.append((dy, x))
+        self.held_bytes += size
         self.stream.wait_stream(self.main)
         with torch.cuda.stream(self.stream):
             fn()
 
     def join(self) -> None:
+        if not self.held:              # a capture does not know the other stream before its first work
+            return
         self.main.wait_stream(self.stream)
         self.held.clear()
+        self.held_bytes = 0
 
 
 class FusedGPTEngine:
@@ -368,8 +380,8 @@ class FusedGPTEngine:
         """Where the weight gradients of a micro-batch run (None: in line).  Products of few tokens leave most of the GPU idle and last as long as their
         latencies; beside the chain they cost it nothing.  One B200, us per step, in line / beside, by tokens x width: GPT-2 style 0.26 M (2 layers)
         431 / 365, 0.77 M (6 layers) 1417 / 1127, 1.6 M 2107 / 1892, 3.1 M 2919 / 2700, 6.3 M 4607 / 4569; Llama style 1.0 M (4 layers) 1596 / 1516, 4.2 M
-        2565 / 2545 and 5603 / 5544.  Behind 4 M there is nothing to gain, and what is held until the end of the pass (nine widths a token and layer) adds up.
-        A sharded store hands its buckets on as they are complete, so its gradients stay in line."""
+        2565 / 2545 and 5603 / 5544.  Behind 4 M there is nothing to gain.  A sharded store hands its buckets on as they are complete, so its
+        gradients stay in line."""
         if self.device.type != "cuda" or type(self.params) is not FlatParams or tokens * self.cfg.d_model > 4 << 20:
             return None
         if self._side is None:

@@ -218,3 +218,37 @@ def test_resume_with_optimizer_state_continues_bit_for_bit():
         resumed.load_optimizer_state(opt_tensors, dict(opt_meta, world=2))
     with pytest.raises(SerializationError):
         resumed.load_optimizer_state({"adam.m": opt_tensors["adam.m"]}, opt_meta)
+
+
+def test_gradients_held_for_the_other_stream_are_bounded(monkeypatch):
+    """However many layers hand their gradients over, no more than the limit is held (one larger gradient alone excepted), and none is let go before the
+    main stream has waited for the work that reads it."""
+    import contextlib
+    import weakref
+    from rustral_b200.runtime import fused_gpt
+
+    class Stream:
+        device, waits = None, 0
+
+        def wait_stream(self, other):
+            self.waits += 1
+
+    main, side = Stream(), Stream()
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: main)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    limit = 8 * 4096
+    monkeypatch.setattr(fused_gpt._Beside, "MOST_HELD", limit)
+    beside, x = fused_gpt._Beside(side), torch.zeros(4)
+    handed = []                                       # (gradient, its bytes, waits of the main stream when it was handed over)
+    for i in range(60):
+        dy = torch.zeros(64, (16, 48, 8, 200)[i % 4], dtype=torch.bfloat16)
+        if i == 30:
+            dy = torch.zeros(2 * limit, dtype=torch.uint8)
+        beside.run(lambda: None, dy, x)
+        handed.append((weakref.ref(dy), dy.numel() * dy.element_size(), main.waits))
+        del dy
+        alive = [h for h in handed if h[0]() is not None]
+        assert sum(n for _, n, _ in alive) <= (2 * limit if i == 30 else limit)
+        assert all(main.waits > w for ref, _, w in handed if ref() is None)
+    beside.join()
+    assert all(ref() is None and main.waits > w for ref, _, w in handed) and side.waits == 60

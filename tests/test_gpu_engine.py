@@ -68,3 +68,32 @@ def test_weight_gradients_beside_the_chain_are_those_in_line(name, cuda_status):
         torch.cuda.synchronize()
         grads.append(torch.stack(out))
     assert torch.equal(grads[0], grads[1])
+
+
+def test_split_weight_gradients_and_joins_beside_the_chain(monkeypatch, cuda_status):
+    """Enough tokens for split contractions, whose slabs and column sums then lie on the other stream, and limits on what is held that make the main stream
+    wait after every gradient, after a few and not before the end: equal bits."""
+    from rustral_b200 import _native as N
+    from rustral_b200.models.config import GPTConfig
+    from rustral_b200.ops import matmul
+    from rustral_b200.runtime import fused_gpt
+    cfg = GPTConfig(vocab_size=1000, seq_len=512, n_layer=3, n_head=6, n_kv_head=6, d_model=384, ffn_dim=1536, arch="gpt2")
+    T = 4 * cfg.seq_len
+    a = N.RbGemmArgs()
+    a.M, a.N, a.K, a.a_mn_major, a.b_mn_major, a.out_f32, a.alpha, a.col_sum = 384, 384, T, 1, 1, 1, 1.0, 256
+    assert N.kernels().rb_gemm_workspace(a, matmul.WORKSPACE_BYTES) > 0
+    g = torch.Generator().manual_seed(4)
+    batches = [[torch.randint(0, cfg.vocab_size, (4, cfg.seq_len), generator=g).cuda() for _ in range(2)] for _ in range(5)]
+    grads = []
+    for limit in (None, 1, 8 << 20, 1 << 40):
+        e = FusedGPTEngine(cfg, "cuda", micro_batch=4, seed=5, max_grad_norm=1.0)
+        if limit is None:
+            e._beside = lambda tokens: None
+        else:
+            monkeypatch.setattr(fused_gpt._Beside, "MOST_HELD", limit)
+        out = []
+        for ids, tg in batches:
+            e.train_step(ids, tg, do_step=False)
+            out.append(e.params.grad.clone())
+        grads.append(torch.stack(out))
+    assert all(torch.equal(grads[0], x) for x in grads[1:])
