@@ -28,6 +28,11 @@ from . import decoder_body
 from .kv_cache import PagedCache
 
 
+# Keys and values gathered for later portions of prompts live until their launch, which several portions share: at most this many bytes of them (or one
+# portion's) at a time, however many portions a step has.
+MOST_GATHERED = 256 << 20
+
+
 class StepBatch:
     """The rows of one model pass: prompt portions first (`spans`), then one row per decoded sequence (from row `rd`).
     `segments`: the same sequences for layers with recurrent state (None: the model has none).  `arrived`: given for a step of decoded
@@ -201,7 +206,7 @@ class ModelRunner:
             bt, seq = sb.row_tables()
             return paged_ops.paged_attention_rows(q, kc, vc, bt, seq, sb.pos, scale, rule, gate, out, head_gate)
         a = out if out is not None else torch.empty((T, H * dv), dtype=q.dtype, device=self.device)
-        parts = []
+        parts, gathered = [], 0                       # portions of the next launch; bytes of their gathered keys and values
         for i, (r0, r1, start) in enumerate(sb.spans):
             L = r1 - r0
             kept, first = rule.key_ranges(start) if rule is not None else (0, 0)
@@ -209,6 +214,11 @@ class ModelRunner:
                 kk, vv = k2[r0:r1].view(1, L, G, dk), v2[r0:r1].view(1, L, G, dv)
             else:
                 cs = sb.key_slots(i, first, kept)
+                size = cs.numel() * G * (dk + dv) * kc.element_size()
+                if parts and gathered + size > MOST_GATHERED:
+                    attn_ops.prompt_attention_many(parts, scale)
+                    parts, gathered = [], 0
+                gathered += size
                 kk = ops.gather_rows(kc.view(nb * bs, G * dk), cs).view(1, -1, G, dk)
                 vv = ops.gather_rows(vc.view(nb * bs, G * dv), cs).view(1, -1, G, dv)
             qq, oo = q[r0:r1].view(1, L, H, dk), a[r0:r1].view(1, L, H, dv)

@@ -414,3 +414,38 @@ def test_aborting_during_chunked_prefill_drops_the_prefill_progress():
     a = eng2.submit(list(range(1, 30)), 3)
     eng2.step()
     assert eng2.abort_all() == [a] and not eng2._prefill_pos and not eng2.scheduler.has_work()
+
+
+def test_gathered_keys_of_later_portions_are_bounded(monkeypatch):
+    """A step with many later portions of prompts holds the gathered keys and values of as many of them as the limit has room for, of one at least,
+    and its logits do not hang on that."""
+    from rustral_b200.models.config import preset
+    from rustral_b200.ops import attention as attn_ops
+    from rustral_b200.serve import model_runner
+    cfg = preset("llama-test")
+    r = model_runner.ModelRunner(cfg, device="cpu", num_blocks=64, seed=3)
+    starts = [8, 17, 40, 3, 24, 9]
+    prompts = [[(7 * i + t) % cfg.vocab_size for t in range(s + 6)] for i, s in enumerate(starts)]
+    for i, p in enumerate(prompts):
+        assert r.cache.allocate(i, len(p))
+    r.step_mixed([(i, p[:s], 0, False) for i, (p, s) in enumerate(zip(prompts, starts))], [], [], [])
+    launches = []
+    real = attn_ops.prompt_attention_many
+
+    def spy(parts, scale):
+        launches.append(sum(k.numel() * k.element_size() + v.numel() * v.element_size() for _, k, v, _ in parts))
+        return real(parts, scale)
+
+    monkeypatch.setattr(attn_ops, "prompt_attention_many", spy)
+    later = [(i, p[s:], s, True) for i, (p, s) in enumerate(zip(prompts, starts))]
+    want = torch.stack(r.step_mixed(later, [], [], [])[0])
+    assert len(launches) == cfg.n_layer                       # the usual limit holds all of them
+    row = 2 * r.n_kv_head * cfg.head_dim * r.cache.k[0].element_size()
+    sizes = [row * len(p) for p in prompts]
+    assert launches[0] == sum(sizes)
+    for limit in (1, max(sizes), 2 * max(sizes)):
+        launches.clear()
+        monkeypatch.setattr(model_runner, "MOST_GATHERED", limit)
+        got = torch.stack(r.step_mixed(later, [], [], [])[0])
+        assert max(launches) <= max(limit, max(sizes)) and sum(launches) == cfg.n_layer * sum(sizes)
+        assert torch.equal(got, want)
