@@ -21,6 +21,7 @@
 #define RB_INLINE_WAITS
 #include "gemm_rows.h"
 
+#include "norm_row.cuh"
 #include "pdl.cuh"
 #include "rb_common.cuh"
 
@@ -69,29 +70,23 @@ __device__ __forceinline__ float rows_act(int act, float v) {
   return v;
 }
 
-// Sum over the 128 threads of warps 2 to 5; `red`: 4 floats per use.
-__device__ __forceinline__ float rows_sum128(float v, float* red) {
-  v = warp_sum(v);
-  const int w = (threadIdx.x >> 5) - 2;
-  if ((threadIdx.x & 31) == 0) red[w] = v;
-  asm volatile("bar.sync 1, 128;" ::: "memory");
-  return red[0] + red[1] + red[2] + red[3];
-}
-
-// What warps 2 to 5 do first (NORM, the 16-byte pieces of a row that a thread holds): statistics of the rows, then the normed columns of k-blocks
-// kb0 .. kb1 into the first stages and, for stages that are filled again, into `later`.
+// What warps 2 to 5 do first (NORM: the warps that a row belongs to): statistics of the rows, then the normed columns of k-blocks kb0 .. kb1 into the
+// first stages and, for stages that are filled again, into `later`.  Lanes, order and roundings are those of the norm's own kernel, so that a row's bits
+// do not hang on how many rows there are.
 template <int NORM>
 __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int kb0, int kb1, int stages, int stage_bytes, uint32_t base,
                                           uint8_t* later, float* red, bool w_constant) {
-  const int t = threadIdx.x - 64;
+  constexpr int kRows = 4 / NORM;                // at a time
+  const int warp = (threadIdx.x >> 5) - 2, lane = threadIdx.x & 31, wr = warp % NORM;
   const float inv_n = 1.f / static_cast<float>(K);
+  auto col = [&](int i) { return norm_col<4, NORM>(wr, i, lane); };
   // the norm's weights are the model's like W: asked for before the kernel in front has ended
-  uint4 gamma[NORM], beta[NORM];
+  uint4 gamma[4], beta[4];
   auto weights = [&]() {
 #pragma unroll
-    for (int i = 0; i < NORM; ++i) {
-      const int c = (i * 128 + t) * 8, kb = c >> 6;
-      const bool mine = c < K && kb >= kb0 && kb < kb1;
+    for (int i = 0; i < 4; ++i) {
+      const int c = col(i), kb = c >> 6;
+      const bool mine = c < K && kb >= kb0 && kb < kb1 && warp / NORM < M;
       gamma[i] = mine ? *reinterpret_cast<const uint4*>(nm.gamma + c) : make_uint4(0u, 0u, 0u, 0u);
       beta[i] = mine && nm.beta ? *reinterpret_cast<const uint4*>(nm.beta + c) : make_uint4(0u, 0u, 0u, 0u);
     }
@@ -100,62 +95,77 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
   pdl_wait();
   pdl_launch();
   if (!w_constant) weights();
-  uint4 next[NORM];
+  uint4 next[4];
   auto fetch = [&](int m) {
 #pragma unroll
-    for (int i = 0; i < NORM; ++i) {
-      const int c = (i * 128 + t) * 8;
-      next[i] = c < K ? *reinterpret_cast<const uint4*>(nm.x + m * nm.ldx + c) : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < 4; ++i) {
+      const int c = col(i);
+      next[i] = m < M && c < K ? *reinterpret_cast<const uint4*>(nm.x + m * nm.ldx + c) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
   auto unpack = [](const uint4& a, float (&v)[8]) {
     const float2 f0 = unpack_bf16x2(a.x), f1 = unpack_bf16x2(a.y), f2 = unpack_bf16x2(a.z), f3 = unpack_bf16x2(a.w);
     v[0] = f0.x; v[1] = f0.y; v[2] = f1.x; v[3] = f1.y; v[4] = f2.x; v[5] = f2.y; v[6] = f3.x; v[7] = f3.y;
   };
-  fetch(0);
-#pragma unroll 1
-  for (int m = 0; m < M; ++m) {
-    uint4 u[NORM];
+  // `at`: 4 floats per row and use
+  auto row_sum = [&](float v, float* at) {
+    v = warp_sum(v);
+    if (NORM == 1) return v;
+    if (lane == 0) at[wr] = v;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < NORM; ++i) u[i] = next[i];
-    if (m + 1 < M) fetch(m + 1);
+    for (int i = 0; i < NORM; ++i) s += at[i];
+    return s;
+  };
+  fetch(warp / NORM);
+#pragma unroll 1
+  for (int m0 = 0; m0 < M; m0 += kRows) {
+    const int m = m0 + warp / NORM;              // M or more: nothing is read or written, the barriers are kept
+    uint4 u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = next[i];
+    fetch(m + kRows);
     float mean = 0.f;
     if (!nm.rms) {
       float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < NORM; ++i) {
+      for (int i = 0; i < 4; ++i) {
         float v[8];
         unpack(u[i], v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += v[j];
       }
-      mean = rows_sum128(s, red + m * 8) * inv_n;
+      mean = norm_mean(row_sum(s, red + m * 8), inv_n);
     }
     float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < NORM; ++i) {
-      if ((i * 128 + t) * 8 < K) {
+    for (int i = 0; i < 4; ++i) {
+      if (col(i) < K) {
         float v[8];
         unpack(u[i], v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { const float d = v[j] - mean; sq += d * d; }
+        for (int j = 0; j < 8; ++j) sq = norm_square(v[j], mean, sq);
       }
     }
-    const float rstd = rsqrtf(rows_sum128(sq, red + m * 8 + 4) * inv_n + nm.eps);
+    const float rstd = norm_rstd(row_sum(sq, red + m * 8 + 4), inv_n, nm.eps);
+    if (m >= M) continue;
 #pragma unroll
-    for (int i = 0; i < NORM; ++i) {
-      const int c = (i * 128 + t) * 8, kb = c >> 6;
+    for (int i = 0; i < 4; ++i) {
+      const int c = col(i), kb = c >> 6;
       if (kb >= kb0 && kb < kb1) {               // the last block's columns behind the row are zero
         float v[8] = {}, g[8];
         if (c < K) {
           unpack(u[i], v);
           unpack(gamma[i], g);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = (v[j] - mean) * rstd * g[j];
           if (nm.beta) {
-            unpack(beta[i], g);
+            float b[8];
+            unpack(beta[i], b);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] += g[j];
+            for (int j = 0; j < 8; ++j) v[j] = norm_value(v[j], mean, rstd, g[j], b[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = norm_value(v[j], mean, rstd, g[j]);
           }
         }
         const uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
@@ -173,7 +183,7 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-// NORM: 0, or the 16-byte pieces of a row per thread of the norm (1, 2, 4: K up to 1024, 2048, 4096)
+// NORM: 0, or the warps that share a row of the norm (1, 2, 4: K up to 1024, 2048, 4096)
 template <int NORM>
 __global__ void __launch_bounds__(kRowsThreads)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, int M, int N, int K, int mpad,

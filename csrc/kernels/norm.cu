@@ -9,6 +9,7 @@
 // root (crates/nn/src/normalization.rs:87-158; backward crates/autodiff/src/lib.rs:1167-1214).
 #include "norm.h"
 
+#include "norm_row.cuh"
 #include "pdl.cuh"
 #include "rb_common.cuh"
 
@@ -45,14 +46,11 @@ __device__ __forceinline__ float row_sum(float v, float* red, int warp) {
 }
 
 template <int CHUNKS, int WPR>
-__device__ __forceinline__ int col_of(int wr, int c, int lane) { return ((wr * CHUNKS + c) * 32 + lane) * 8; }
-
-template <int CHUNKS, int WPR>
 __device__ __forceinline__ void load_row(const __nv_bfloat16* p, int n, int wr, int lane, bool valid,
                                          float (&x)[CHUNKS][8]) {
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
-    const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+    const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
     if (valid && col < n) {
       load8(p + col, x[c]);
     } else {
@@ -89,21 +87,17 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_b
       for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += v[c][j];
-      mean = row_sum<WPR>(s, red, warp) * inv_n;
+      mean = norm_mean(row_sum<WPR>(s, red, warp), inv_n);
     }
     float sq = 0.f;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      if (col_of<CHUNKS, WPR>(wr, c, lane) < n) {
+      if (norm_col<CHUNKS, WPR>(wr, c, lane) < n) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float d = v[c][j] - mean;
-          sq += d * d;
-        }
+        for (int j = 0; j < 8; ++j) sq = norm_square(v[c][j], mean, sq);
       }
     }
-    const float var = row_sum<WPR>(sq, red, warp) * inv_n;
-    const float rstd = rsqrtf(var + eps);
+    const float rstd = norm_rstd(row_sum<WPR>(sq, red, warp), inv_n, eps);
     if (!valid) continue;
     if (lane == 0 && wr == 0) {
       if (mean_out) mean_out[row] = mean;
@@ -111,16 +105,13 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_b
     }
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+      const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
       if (col < n) {
         float g[8], b[8], o[8];
         load8(gamma + col, g);
         if (beta) load8(beta + col, b);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          o[j] = (v[c][j] - mean) * rstd * g[j];
-          if (beta) o[j] += b[j];
-        }
+        for (int j = 0; j < 8; ++j) o[j] = beta ? norm_value(v[c][j], mean, rstd, g[j], b[j]) : norm_value(v[c][j], mean, rstd, g[j]);
         store8(y + row * ldy + col, o);
       }
     }
@@ -164,7 +155,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
   uint4 gpk[CHUNKS];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
-    const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+    const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
     gpk[c] = col < n ? *reinterpret_cast<const uint4*>(gamma + col) : make_uint4(0u, 0u, 0u, 0u);
   }
   // The three input rows (x, dy, residual-branch gradient) of the NEXT row this warp will process are requested
@@ -175,7 +166,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
     const bool valid = row < rows;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+      const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
       const bool in = valid && col < n;
       nx[c] = in ? *reinterpret_cast<const uint4*>(x + row * ldx + col) : make_uint4(0u, 0u, 0u, 0u);
       ny[c] = in ? *reinterpret_cast<const uint4*>(dy + row * lddy + col) : make_uint4(0u, 0u, 0u, 0u);
@@ -206,7 +197,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+      const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
       if (valid && col < n) {
         float g[8];
         unpack8(gpk[c], g);
@@ -229,7 +220,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
     if (!valid) continue;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+      const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
       if (col < n) {
         float o[8];
 #pragma unroll
@@ -247,7 +238,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv
 
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
-    const int col = col_of<CHUNKS, WPR>(wr, c, lane);
+    const int col = norm_col<CHUNKS, WPR>(wr, c, lane);
 #pragma unroll
     for (int j = 0; j < 8; ++j) { sg[col + j] = ag[c][j]; sb[col + j] = ab[c][j]; }
   }

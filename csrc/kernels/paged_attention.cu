@@ -89,6 +89,8 @@ __device__ __forceinline__ float pa_sigmoid(float x) { return __fdividef(1.f, 1.
 // k-steps of mma.sync, the softmax runs on the accumulator fragments, and O += P V reuses those fragments as the A
 // operand against ldmatrix.trans-fed V.  One query token per sequence gives M <= 16, far below the 64-row minimum
 // of a tcgen05 tile, which is why this kernel is on the warp-level tensor path; it is bound by the K / V reads.
+// Products and sums are contracted explicitly, here, in the merge and in the one-launch form (paged_step.cu), so that a sequence gets the same
+// bits whichever of them its batch takes.
 //
 // DK / DV are the key / value head sizes rounded up to a compiled size; columns beyond the real sizes are zero-filled in
 // shared memory and never leave it.  RULE adds a score cap, a linear and a logarithmic distance bias, chunked or windowed visibility, a
@@ -356,7 +358,7 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const bool ok = n * 8 + 2 * tq + j < n_tok;
-          float v0 = s[n][j] * scale, v1 = s[n][2 + j] * scale;
+          float v0 = __fmul_rn(s[n][j], scale), v1 = __fmul_rn(s[n][2 + j], scale);
           if (RULE) {
             if (rule.softcap > 0.f) {
               v0 = pa_softcap(v0, rule.softcap, two_over_cap);
@@ -399,8 +401,8 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
       sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
       sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
       sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
-      l0 = l0 * al0 + sum0;
-      l1 = l1 * al1 + sum1;
+      l0 = __fmaf_rn(l0, al0, sum0);
+      l1 = __fmaf_rn(l1, al1, sum1);
       m0 = mn0;
       m1 = mn1;
 #pragma unroll
@@ -447,8 +449,8 @@ paged_decode_split_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, c
 #pragma unroll
       for (int w = 0; w < kPaWarps; ++w) {
         const float sc = (m_sh[w][g] == -INFINITY) ? 0.f : __expf(m_sh[w][g] - mx);
-        num += merge[w * kMergeStride + g * VROW + d] * sc;
-        den += l_sh[w][g] * sc;
+        num = __fmaf_rn(merge[w * kMergeStride + g * VROW + d], sc, num);
+        den = __fmaf_rn(l_sh[w][g], sc, den);
       }
       if (direct_out) {                        // a single slice: this is the result
         const long long col = static_cast<long long>(h_base + g) * dv + d;
@@ -491,8 +493,8 @@ paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restri
     for (int s = 0; s < n; ++s) {
       const float ms = base[s * (dv + 2)];
       const float sc = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-      num += base[s * (dv + 2) + 2 + d] * sc;
-      den += base[s * (dv + 2) + 1] * sc;
+      num = __fmaf_rn(base[s * (dv + 2) + 2 + d], sc, num);
+      den = __fmaf_rn(base[s * (dv + 2) + 1], sc, den);
     }
   } else {
     // Long contexts: a slice's factor is formed once, by one thread, and the sums run over independent loads (in the same order).  Attention of
@@ -516,8 +518,8 @@ paged_decode_merge_kernel(const float* __restrict__ partial, const int* __restri
       if (d < dv) {
 #pragma unroll 8
         for (int s = 0; s < m; ++s) {
-          num += base[(from + s) * (dv + 2) + 2 + d] * scale_sh[s];
-          den += sum_sh[s] * scale_sh[s];
+          num = __fmaf_rn(base[(from + s) * (dv + 2) + 2 + d], scale_sh[s], num);
+          den = __fmaf_rn(sum_sh[s], scale_sh[s], den);
         }
       }
     }

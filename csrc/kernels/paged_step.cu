@@ -6,8 +6,8 @@
 // cached tokens of a sequence for one KV head, four warps take 32 tokens each and then 32 more, and all their K and V rows are asked for, with
 // slots looked up and angles formed, while the projection still runs.  Behind it come the queries and the new token's row, which goes from the
 // projection into the tiles and into the cache.  A CTA leaves (max, sum, accumulator) of its slice; the last one of a sequence and KV head to count
-// itself in adds up the slices in their order.  Slices, the order inside them and the arithmetic are those of `paged_decode_split_kernel`
-// (paged_attention.cu), so a sequence gets the same bits alone as beside many others.
+// itself in adds up the slices in their order.  Slices, the order inside them and the arithmetic, contractions included, are those of
+// `paged_decode_split_kernel` (paged_attention.cu), so a sequence gets the same bits alone as beside many others.
 //
 // One B200, a layer of a step in a captured chain, us, rotation and append, slices and merge in launches of their own / this kernel: 1 sequence of 2047,
 // 4 KV heads of 128 14.4 / 7.2; of 300, 12 heads of 64 9.2 / 5.1.  As a form of `paged_decode_split_kernel` the one launch took 12.8 and 8.5: half of
@@ -85,9 +85,9 @@ __device__ __forceinline__ void step_merge(const float* partial, int n, int nspl
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
         const float f = __shfl_sync(0xffffffffu, factor, (s0 + s) & 31), l = __shfl_sync(0xffffffffu, ml.y, (s0 + s) & 31);
-        den += l * f;
+        den = __fmaf_rn(l, f, den);
 #pragma unroll
-        for (int j = 0; j < P; ++j) { num[j].x += v[s][j].x * f; num[j].y += v[s][j].y * f; }
+        for (int j = 0; j < P; ++j) num[j] = make_float2(__fmaf_rn(v[s][j].x, f, num[j].x), __fmaf_rn(v[s][j].y, f, num[j].y));
       }
     }
 #pragma unroll
@@ -246,8 +246,8 @@ paged_step_kernel(const StepParams p RB_BOUNDS_PARAM) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const bool ok = n * 8 + 2 * tq + j < n_tok;
-        s[n][j] = ok ? s[n][j] * p.scale : -INFINITY;
-        s[n][2 + j] = ok ? s[n][2 + j] * p.scale : -INFINITY;
+        s[n][j] = ok ? __fmul_rn(s[n][j], p.scale) : -INFINITY;
+        s[n][2 + j] = ok ? __fmul_rn(s[n][2 + j], p.scale) : -INFINITY;
         mx0 = fmaxf(mx0, s[n][j]);
         mx1 = fmaxf(mx1, s[n][2 + j]);
       }
@@ -274,8 +274,8 @@ paged_step_kernel(const StepParams p RB_BOUNDS_PARAM) {
     sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
     sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
     sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
-    l0 = l0 * al0 + sum0;
-    l1 = l1 * al1 + sum1;
+    l0 = __fmaf_rn(l0, al0, sum0);
+    l1 = __fmaf_rn(l1, al1, sum1);
     m0 = mn0;
     m1 = mn1;
 #pragma unroll
@@ -319,8 +319,8 @@ paged_step_kernel(const StepParams p RB_BOUNDS_PARAM) {
 #pragma unroll
     for (int w = 0; w < kStepWarps; ++w) {
       const float m = factor_sh[w * kStepGroup + g], sc = (m == -INFINITY) ? 0.f : __expf(m - mx);
-      num += all[w * kWarpPitch + g * L::kRow + d] * sc;
-      den += sum_sh[w * kStepGroup + g] * sc;
+      num = __fmaf_rn(all[w * kWarpPitch + g * L::kRow + d], sc, num);
+      den = __fmaf_rn(sum_sh[w * kStepGroup + g], sc, den);
     }
     if (direct) {
       p.out[b * p.ld_o + static_cast<long long>(hk * group + g) * D + d] = __float2bfloat16(num / den);

@@ -192,3 +192,75 @@ def test_norm_inside_a_product_with_few_rows(rows, n, k, rms, cuda_status):
         want = rotary.swiglu_product(h, weight) if act == "swiglu" else matmul.gemm(h, weight, bias=b, act=act)
         e = (got.float() - want.float()).abs()
         assert (e <= 2.0 ** -7 * want.float().abs() + 2.0 ** -8 * want.float().pow(2).mean().sqrt()).all(), e.max()
+
+
+@pytest.mark.parametrize("rows,n,k", [(1, 768, 768), (4, 640, 4096), (8, 528, 2048), (7, 272, 1024), (3, 272, 200), (5, 264, 1032), (2, 28672, 4096), (3, 520, 3000)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_inside_a_product_has_the_bits_of_norm_and_product(rows, n, k, rms, cuda_status):
+    """One, two and four warps to a row, rows that leave warps without one, blocks that end inside 64 columns; a row has the same bits beside others."""
+    from rustral_b200.ops import matmul, norm as norm_ops
+    g = torch.Generator(device="cuda").manual_seed(rows * n)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    x, w, gamma = rand(rows, k + 8)[:, :k] * 3 + 1, rand(n, k) * 0.05, rand(k)
+    beta, bias = (None, None) if rms else (rand(k), rand(n))
+    for act in ("none", "gelu", "swiglu") if n % 16 == 0 else ("none", "gelu"):        # swiglu: halves of whole 16-byte pieces
+        b = None if act == "swiglu" else bias
+        before = N.launch_count
+        got = matmul.norm_gemm(x, gamma, beta, 1e-5, rms, w, bias=b, act=act, b_constant=True)
+        assert N.launch_count - before == 1
+        h = norm_ops.norm_forward(x, gamma, beta, 1e-5, rms)[0]
+        assert torch.equal(got, rotary.swiglu_product(h, w) if act == "swiglu" else matmul.gemm(h, w, bias=b, act=act))
+        assert torch.equal(got[-1:], matmul.norm_gemm(x[-1:], gamma, beta, 1e-5, rms, w, bias=b, act=act))
+
+
+@pytest.mark.parametrize("batch,heads,kv,dim,longest,width,theta", [
+    (1, 8, 2, 128, 2500, 400, 10000.0), (36, 8, 4, 128, 1300, 96, 500000.0), (10, 32, 16, 64, 700, 64, 10000.0), (3, 4, 4, 64, 257, 1024, 0.0),
+    (2, 16, 1, 128, 20000, 1250, 10000.0), (3, 12, 1, 64, 9000, 600, 0.0)])
+def test_attention_step_has_the_bits_of_the_three_launches(batch, heads, kv, dim, longest, width, theta, cuda_status):
+    """One slice, some and more than 32; both forms of the merge; lengths at the edges of tiles and slices."""
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    need = (longest + 15) // 16
+    kc, vc = (torch.randn(batch * need, 16, kv, dim, device="cuda", generator=g).bfloat16() for _ in range(2))
+    table = torch.zeros(batch, width, dtype=torch.int32, device="cuda")
+    table[:, :need] = torch.randperm(batch * need, device="cuda", generator=g).view(batch, need).int()
+    edges = [n for n in (1, 32, 33, 128, 129, 256, 257, 512, 513, 2048, 2049, longest) if n <= longest]
+    lens = torch.tensor([longest] + [edges[i % len(edges)] for i in range(batch - 1)], dtype=torch.int32, device="cuda")
+    qkv = torch.randn(batch, (heads + 2 * kv) * dim, device="cuda", generator=g).bfloat16()
+    pos = (lens - 1).long()
+    slots = table.gather(1, (pos // 16)[:, None]).view(-1).long() * 16 + pos % 16
+    other, k2, v2 = qkv.clone(), kc.clone(), vc.clone()
+    if theta:
+        rotary.rope_append_(other, heads, kv, dim, pos, theta, k2, v2, slots)
+    else:
+        paged.kv_append(other[:, heads * dim:(heads + kv) * dim], other[:, (heads + kv) * dim:], k2, v2, slots)
+    arrived = torch.zeros(batch * kv, dtype=torch.int32, device="cuda")
+    for scale in (dim ** -0.5, 0.37):
+        want = paged.paged_attention_decode(other[:, :heads * dim], k2, v2, table, lens, scale)
+        got = paged.attention_step(qkv, heads, kv, dim, theta, kc, vc, table, lens, arrived, scale)
+        assert torch.equal(got, want) and torch.equal(kc, k2) and torch.equal(vc, v2)
+
+
+@pytest.mark.parametrize("arch,d,heads,kv,blocks", [("gpt2", 768, 12, 12, 1024), ("llama", 2048, 16, 4, 1024), ("llama", 4096, 32, 8, 700)])
+def test_a_decoded_sequence_has_the_same_bits_beside_others(arch, d, heads, kv, blocks, cuda_status):
+    """Logits, keys and values of one sequence alone and in batches on both sides of every limit: norms inside the products (8 rows, 16384 numbers),
+    attention in one launch (slices that the tables have room for), replayed and eager."""
+    from rustral_b200.models.config import GPTConfig
+    from rustral_b200.serve.model_runner import ModelRunner
+    from rustral_b200.serve.weights import InferenceWeights
+    cfg = GPTConfig(vocab_size=1000, seq_len=1024 if arch == "gpt2" else 8192, n_layer=2, n_head=heads, n_kv_head=kv, d_model=d, ffn_dim=2 * d, arch=arch)
+    weights = InferenceWeights.random_llama(cfg, "cuda", seed=3) if arch == "llama" else None
+    r = ModelRunner(cfg, params=weights, device="cuda", num_blocks=blocks, block_size=16, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(d)
+    lens = [700] + [(97 * i) % 300 + 1 for i in range(33)]
+    for i, n in enumerate(lens):
+        assert r.cache.allocate(i, n)
+    for l in range(2):
+        r.cache.k[l].normal_(0.0, 0.9, generator=g)
+        r.cache.v[l].normal_(0.0, 0.9, generator=g)
+    for graphs in (True, False):
+        r.use_graphs = graphs
+        alone = r.decode([0], [17], lens[:1]).clone()
+        for batch in (2, 3, 4, 5, 8, 9, 16, 34):
+            ids = list(range(1, batch)) + [0]
+            got = r.decode(ids, [5] * (batch - 1) + [17], [lens[i] for i in ids])
+            assert torch.equal(got[-1:], alone), batch
