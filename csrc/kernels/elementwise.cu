@@ -474,6 +474,12 @@ RB_API int rb_sum_dim0_staged(const void* a, long long lda, float* out, float* p
   return static_cast<int>(cudaGetLastError());
 }
 
+// The second stage alone, for partial sums that another kernel has left (one row for each of rb_sum_dim0_staged's slabs).
+RB_API int rb_sum_dim0_fold(const float* partial, int slabs, float* out, int cols, int accumulate, void* stream_v) {
+  if (slabs <= 0 || cols <= 0 || !partial || !out) return -1;
+  return static_cast<int>(rbhost::launch_pdl(rb::sum_dim0_stage2, dim3((cols + 31) / 32), dim3(1024), 0, RB_STREAM, 1, partial, slabs, out, cols, accumulate));
+}
+
 RB_API int rb_sum_all(const void* a, long long n, int dtype, float* scratch, float* out, void* stream_v) {
   if (n <= 0 || !scratch || !out) return -1;
   long long want = (n + 4095) / 4096;

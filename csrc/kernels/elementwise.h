@@ -24,6 +24,7 @@ int rb_sum_dim0(const void* a, long long lda, float* out, long long rows, int co
 int rb_sum_dim0_slabs(void);
 int rb_sum_dim0_staged(const void* a, long long lda, float* out, float* partial, long long rows, int cols, int dtype,
                        int accumulate, void* stream);
+int rb_sum_dim0_fold(const float* partial, int slabs, float* out, int cols, int accumulate, void* stream);
 // out[0] = sum(a); scratch >= 1024 floats
 int rb_sum_all(const void* a, long long n, int dtype, float* scratch, float* out, void* stream);
 // 2-D transpose out[c, r] = a[r, c]

@@ -18,6 +18,7 @@
 // op sequences (crates/candle-backend/src/lib.rs:220-312).
 #include "gemm_tcgen05.h"
 
+#include "elementwise.h"
 #include "gemm_rows.h"
 
 #include <stdlib.h>
@@ -56,8 +57,10 @@ struct EpiParams {
   int side;     // staged == 2: what TMA loads into the tiles before the accumulator is complete: 0 nothing, 1 residual, 2 aux_in
   const float* row_scale;   // fp32 [M] or nullptr: multiplies row i of the accumulator (8-bit operands: per-token scale)
   const float* col_scale;   // fp32 [N] or nullptr: multiplies column j (per-output-channel weight scale)
-  float* col_sum;           // fp32 [M] (or [splits][M], slabs), column sums of A; kernels of the EXTRA form with MN-major A only
-  int col_accumulate;
+  float* col_sum;           // fp32 [slabs][M], column sums of A over every col_rows rows; kernels of the EXTRA form with MN-major A only
+  int col_rows;
+  const __nv_bfloat16* col_src;   // A once more, [K, M] with pitch col_ld: rows of a slab that another part of the contraction loads
+  long long col_ld;
   int fp8_b_format;         // 8-bit operands: format of B in the instruction descriptor (0 = e4m3, 1 = e5m2); A is e4m3
 };
 
@@ -604,8 +607,11 @@ __device__ __forceinline__ void epilogue_swiglu(const CUtensorMap* tmD, uint32_t
 // k-block of 64, when the issuer has seen them land (it arrives at bar_read; for a pair of CTAs a commit does, behind the products: an arrival at the
 // peer's barrier took the issuer so long that the product took three times as long) and before they are loaded over (bar_summed, for which the
 // producer waits).  Warp w sums 32 columns: lane r + 8 c the rows r, r + 8, .. of 8 columns, a swizzle chunk, so that eight lanes read a row of banks.
-// The eight rows of a lane are added up first and then to its running sum; lanes are added by shuffles, splits by the kernel that folds the slabs: the
-// order is fixed.  As a kernel of its own the sum read dy once more and took two launches: 32768 x 3072 46 + 3 us of a step's backward pass.
+// The sums are those of `rb_sum_dim0_staged`, bit for bit: its slabs of `col_rows` rows (whole k-blocks), its lanes (every eighth row, one after the other), its order of lanes;
+// a slab leaves a row of partial sums, which `rb_sum_dim0_fold` adds up.  A slab belongs to the part of the contraction in which it begins; rows
+// of it that the next part loads are read from memory.  (A running sum over a whole part, folded with the parts, needed no second launch, but was
+// further from 64 bits from 6000 rows on: of the norm, 32768 rows around zero, 2.2e-7 against 1.3e-7.)  As kernels of its own the sum reads dy once more: 46
+// us for 32768 x 3072.
 constexpr int kSumWarps = 4;
 template <int STAGES>
 struct SumProducer {                               // what the TMA producer keeps
@@ -619,39 +625,85 @@ struct SumProducer {                               // what the TMA producer keep
     return true;
   }
 };
-// One k-block.
-__device__ __forceinline__ void sum_block(uint32_t a_tile, int w, int lane, float (&acc)[8]) {
-  const int chunk = 4 * w + (lane >> 3), r = lane & 7;
-  const uint32_t at = a_tile + (chunk >> 3) * (kBlockK * 128) + r * 128 + (((chunk & 7) ^ r) << 4);
-  Pair v[4];
+__device__ __forceinline__ void sum_add(const uint32_t (&u)[4], Pair (&acc)[4]) {
 #pragma unroll
-  for (int i = 0; i < kBlockK / 8; ++i) {
-    uint32_t u[4];
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + i * 1024));
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = i == 0 ? pair_of(u[j]) : add2(v[j], pair_of(u[j]));
-  }
+  for (int j = 0; j < 4; ++j) acc[j] = add2(acc[j], pair_of(u[j]));
+}
+// Row `slab` of the partial sums; begins the next one.
+__device__ __forceinline__ void sum_store(const EpiParams& ep, int slab, int row0, int M, int w, int lane, Pair (&acc)[4]) {
+  float v[8];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float2 f = floats(v[j]);
-    acc[2 * j] += f.x;
-    acc[2 * j + 1] += f.y;
+    const float2 f = floats(acc[j]);
+    v[2 * j] = f.x;
+    v[2 * j + 1] = f.y;
+    acc[j] = pair_of(0.f, 0.f);
   }
+  // eight lanes x eight columns, transposed: lane r then has column r of all of them, lane by lane
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i & o) continue;
+      const float got = __shfl_xor_sync(0xffffffffu, lane & o ? v[i] : v[i | o], o);
+      if (lane & o) v[i] = got;
+      else v[i | o] = got;
+    }
+  }
+  float t = 0.f;
+#pragma unroll
+  for (int y = 0; y < 8; ++y) t += v[y];
+  const int m = row0 + 32 * w + lane;
+  if (m < M) ep.col_sum[static_cast<long long>(slab) * M + m] = t;
 }
-__device__ __forceinline__ void sum_store(const EpiParams& ep, int split, int num_splits, int row0, int M, int w, int lane, float (&acc)[8]) {
+
+// What a warp keeps of the slab that it is in.
+struct SumSlab {
+  int slab, lo;                                  // lo: its first row
+  Pair acc[4];
+  __device__ __forceinline__ SumSlab(int kb0, int rows) {
+    slab = (kb0 * kBlockK + rows - 1) / rows;    // the first that begins in this part
+    lo = slab * rows;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+    for (int j = 0; j < 4; ++j) acc[j] = pair_of(0.f, 0.f);
   }
-  const int m0 = row0 + (4 * w + (lane >> 3)) * 8;
-  if ((lane & 7) == 0) {
-    float* dst = ep.col_sum + (num_splits > 1 ? static_cast<long long>(split) * M : 0);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (m0 + j < M) dst[m0 + j] = ep.col_accumulate && num_splits == 1 ? dst[m0 + j] + acc[j] : acc[j];
+  __device__ __forceinline__ void done(const EpiParams& ep, int row0, int M, int w, int lane) {
+    sum_store(ep, slab, row0, M, w, lane, acc);
+    ++slab;
+    lo += ep.col_rows;
   }
-}
+  // One k-block in shared memory; rows behind K are zero there (and a sum is never -0).
+  __device__ __forceinline__ void block(const EpiParams& ep, uint32_t a_tile, int kb, int K, int row0, int M, int w, int lane) {
+    if (lo > kb * kBlockK) return;               // a slab of the part in front
+    const int chunk = 4 * w + (lane >> 3), r = lane & 7;
+    const uint32_t at = a_tile + (chunk >> 3) * (kBlockK * 128) + r * 128 + (((chunk & 7) ^ r) << 4);
+#pragma unroll
+    for (int i = 0; i < kBlockK / 8; ++i) {
+      uint32_t u[4];
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + i * 1024));
+      sum_add(u, acc);
+    }
+    if ((kb + 1) * kBlockK >= min(lo + ep.col_rows, K)) done(ep, row0, M, w, lane);
+  }
+  // Behind the last block of a part: the rest of a slab that has begun in it.
+  __device__ __forceinline__ void rest(const EpiParams& ep, int kb1, int K, int row0, int M, int w, int lane) {
+    const int from = kb1 * kBlockK, hi = min(lo + ep.col_rows, K), m = row0 + (4 * w + (lane >> 3)) * 8;
+    if (lo >= from || hi <= from) return;
+    for (int at = from; at < hi; at += 64) {
+      const int row = at + (lane & 7);
+      uint4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        v[i] = row + 8 * i < hi && m < M ? __ldg(reinterpret_cast<const uint4*>(ep.col_src + (row + 8 * i) * ep.col_ld + m)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        sum_add(u, acc);
+      }
+    }
+    done(ep, row0, M, w, lane);
+  }
+};
 
 // FP8 = 1: both operands hold e4m3 bytes (K-major only).  A 128-byte swizzle row then carries 128 elements, so K, lda
 // and ldb arrive halved (in units of two bytes) and only the TMA coordinates, which count elements, are doubled back.
@@ -899,16 +951,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int m_blk, n_blk, kb0, kb1, outer;
       decode_tile(tile, m_blk, n_blk, kb0, kb1, outer);
       if (n_blk != 0) { it += kb1 - kb0; continue; }
-      float acc[8] = {};
+      const int row0 = m_blk * kBlockM;
+      SumSlab sum(kb0, ep.col_rows);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const uint32_t s = it % STAGES;
         if (!mbar_wait(bar_read + 8 * s, phase >> s & 1, abort_flag, status, 9)) { ok = false; break; }
         phase ^= 1u << s;
-        sum_block(smem_base + s * L::kStageBytes, w, lane, acc);
+        sum.block(ep, smem_base + s * L::kStageBytes, kb, K, row0, M, w, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_summed + 8 * s);
       }
-      if (ok) sum_store(ep, outer, num_splits, m_blk * kBlockM, M, w, lane, acc);
+      if (ok) sum.rest(ep, kb1, K, row0, M, w, lane);
     }
   } else {
     // -------------------------------------------------------------------- epilogue warps
@@ -1299,16 +1352,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int m_blk, n_blk, kb0, kb1, split;
       decode_tile(tile, m_blk, n_blk, kb0, kb1, split);
       if (n_blk != 0) { it += kb1 - kb0; continue; }
-      float acc[8] = {};
+      const int row0 = m_blk * kPairM + static_cast<int>(cta_rank) * kBlockM;
+      SumSlab sum(kb0, ep.col_rows);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const uint32_t s = it % STAGES;
         if (!mbar_wait(bar_read + 8 * s, phase >> s & 1, abort_flag, status, 9)) { ok = false; break; }
         phase ^= 1u << s;
-        sum_block(smem_base + s * L::kStageBytes, w, lane, acc);
+        sum.block(ep, smem_base + s * L::kStageBytes, kb, K, row0, M, w, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_summed + 8 * s);
       }
-      if (ok) sum_store(ep, split, num_splits, m_blk * kPairM + static_cast<int>(cta_rank) * kBlockM, M, w, lane, acc);
+      if (ok) sum.rest(ep, kb1, K, row0, M, w, lane);
     }
   } else {
     // -------------------------------------------------------------------- epilogue warps (both CTAs)
@@ -1384,16 +1438,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slab, void* d, long long ldd, int M, int N,
                      int out_f32, int accumulate, const __nv_bfloat16* __restrict__ bias,
-                     const __nv_bfloat16* __restrict__ residual, long long ldr, const float* __restrict__ sum_ws, float* col_sum) {
+                     const __nv_bfloat16* __restrict__ residual, long long ldr) {
   pdl_wait();
   pdl_launch();
-  if (sum_ws != nullptr) {                          // column sums: slabs of M numbers
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-      float acc = sum_ws[i];
-      for (int s = 1; s < splits; ++s) acc += sum_ws[static_cast<long long>(s) * M + i];
-      col_sum[i] = accumulate ? col_sum[i] + acc : acc;
-    }
-  }
   const long long n4 = static_cast<long long>(M) * N / 4;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -1480,9 +1527,9 @@ int plan_epilogue(const RbGemmArgs& g, int splits, rb::EpiParams& ep, const CUte
   ep.col_scale = reinterpret_cast<const float*>(g.b_scale);
   ep.fp8_b_format = g.ab_fp8 == 2 ? 1 : 0;
   ep.staged = 0; ep.side = 0;
-  ep.col_sum = g.col_sum; ep.col_accumulate = g.accumulate;
+  ep.col_sum = g.col_sum; ep.col_rows = g.col_rows;
+  ep.col_src = reinterpret_cast<const __nv_bfloat16*>(g.a); ep.col_ld = g.lda;
   if (splits > 1) {
-    if (g.col_sum) ep.col_sum = reinterpret_cast<float*>(g.workspace) + static_cast<long long>(splits) * g.M * g.N;
     ep.d = g.workspace; ep.ldd = g.N; ep.out_f32 = 1; ep.accumulate = 0;
     ep.bias = nullptr; ep.residual = nullptr;          // applied once, by the kernel that folds the slabs
   }
@@ -1579,8 +1626,7 @@ int launch(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* tb, in
   rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
-                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr,
-                                                      g.col_sum ? ep.col_sum : nullptr, g.col_sum);
+                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1659,8 +1705,7 @@ int launch_pair(const RbGemmArgs& g, const CUtensorMap* ta, const CUtensorMap* t
   rbhost::launch_pdl(rb::splitk_reduce_kernel, dim3(rgrid), dim3(256), 0, stream, 1, reinterpret_cast<const float*>(g.workspace), splits, slab, g.d,
                                                       g.ldd, g.M, g.N, g.out_f32, g.accumulate,
                                                       reinterpret_cast<const __nv_bfloat16*>(g.bias),
-                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr,
-                                                      g.col_sum ? ep.col_sum : nullptr, g.col_sum);
+                                                      reinterpret_cast<const __nv_bfloat16*>(g.residual), g.ldr);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1680,11 +1725,6 @@ double plan_cost(int M, int N, int K, int bn, int splits, int experts, int sms, 
   double us = waves * width * (wc / 100.0) * (static_cast<double>(K) / (splits * experts)) * 0.0065 + 1.5 * width;
   if (splits > 1) us += 2.0 + (2.0 * splits + 1.0) * M * static_cast<double>(N) * 4.0 / 5.0e6;
   return us;
-}
-
-// Workspace of a split contraction: a slab of results for each part, and behind them one of column sums where the call wants those.
-long long split_bytes(const RbGemmArgs& g, int splits) {
-  return static_cast<long long>(splits) * g.M * (g.N + (g.col_sum ? 1 : 0)) * 4;
 }
 
 void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
@@ -1707,7 +1747,7 @@ void pick_plan(const RbGemmArgs& g, int sms, int& bn_out, int& splits_out) {
       if (sp > 1) {
         if (!can_split) continue;
         if (g.splits <= 0 && g.K / sp < 768) continue;
-        if (split_bytes(g, sp) > g.workspace_bytes) continue;
+        if (static_cast<long long>(sp) * g.M * g.N * 4 > g.workspace_bytes) continue;
       }
       const double cost = plan_cost(g.M, g.N, g.K, bn, sp, experts, sms, pair_ok);
       if (best < 0.0 || cost < best) { best = cost; bn_out = bn; splits_out = sp; }
@@ -1772,16 +1812,12 @@ RB_API long long rb_gemm_workspace(const RbGemmArgs* args, long long most) {
   g.workspace = &g;                           // any address: nothing is launched
   g.workspace_bytes = most;
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.act == RB_ACT_SWIGLU || rbhost::gemm_rows_takes(g)) return 0;
-  // `most` bounds the slabs alone: the plan of a weight gradient, chosen here or named by a table, is the same with column sums as without
-  g.col_sum = nullptr;
   int bn = 128, splits = 1;
   pick_plan(g, rbhost::device_sm_count(), bn, splits);
-  return splits > 1 ? split_bytes(*args, splits) : 0;
+  return splits > 1 ? static_cast<long long>(splits) * g.M * g.N * 4 : 0;
 }
 
-RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
-  const RbGemmArgs& g = *args;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+static int gemm_bf16(const RbGemmArgs& g, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return -1;
   // TMA needs 16-byte aligned bases and pitches
   if ((reinterpret_cast<uintptr_t>(g.a) & 15) || (reinterpret_cast<uintptr_t>(g.b) & 15)) return -2;
@@ -1818,7 +1854,7 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
     if (g.block_n == 0) {
       forced = g;
       forced.block_n = want;
-      return rb_gemm_bf16(&forced, stream_v);
+      return gemm_bf16(forced, stream);
     }
   }
   if (g.peer_mode != 0) {
@@ -1833,7 +1869,7 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
     if (g.peer_mode == 1 && (!g.ready_flags || g.lda != g.K)) return -11;       // a_full is dense [M, K]
   }
   if (g.col_sum && (!g.a_mn_major || !g.b_mn_major || g.group_mode || g.peer_mode || g.ab_fp8 || g.act != RB_ACT_NONE ||
-                    (reinterpret_cast<uintptr_t>(g.col_sum) & 3)))
+                    (reinterpret_cast<uintptr_t>(g.col_sum) & 3) || !g.col_out || g.col_rows <= 0 || g.col_rows % rb::kBlockK || (g.M & 7)))
     return -9;
   if (g.act == RB_ACT_SWIGLU) return gemm_swiglu(g, stream);
   const int sms = rbhost::device_sm_count();
@@ -1879,4 +1915,10 @@ RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
     case 128: return dispatch_major<128, 5>(g, ta, tb, grid, splits, stream);
     default: return dispatch_major<64, 8>(g, ta, tb, grid, splits, stream);
   }
+}
+
+RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
+  const RbGemmArgs& g = *args;
+  const int rc = gemm_bf16(g, reinterpret_cast<cudaStream_t>(stream_v));
+  return rc != 0 || !g.col_sum ? rc : rb_sum_dim0_fold(g.col_sum, (g.K + g.col_rows - 1) / g.col_rows, g.col_out, g.M, g.accumulate, stream_v);
 }

@@ -76,15 +76,17 @@ typedef struct RbGemmArgs {
   const void* norm_beta;       // or NULL
   float norm_eps;
   int norm_rms;
-  // sums over the contraction of A's columns, fp32 [M]: col_sum[i] = sum_k A[k, i] (added to it with `accumulate`), or NULL.  MN-major A and B, plain
-  // problems only.  In a weight gradient dW = dy^T x it is the bias gradient, formed while dy is in shared memory anyway.
+  // col_out: column sums of A, fp32 [M] (added to it with `accumulate`), or NULL: in a weight gradient dW = dy^T x the bias gradient, formed while dy is in
+  // shared memory anyway.  MN-major A and B, plain problems with M a multiple of 8.  col_sum: scratch of the sums over every `col_rows` rows (a multiple of
+  // 64), fp32 [ceil(K / col_rows)][M], that `rb_sum_dim0_fold` makes the result of: with the slabs of `rb_sum_dim0_staged` it has that one's bits.
   float* col_sum;
+  float* col_out;
+  int col_rows;
 } RbGemmArgs;
 
 // Returns 0 on success, a negative code for rejected arguments, a positive cudaError otherwise.
 int rb_gemm_bf16(const RbGemmArgs* args, void* stream);
-// Bytes of workspace that rb_gemm_bf16 makes use of for this call when its slabs may take up to `most` (col_sum: a slab of sums each comes on top);
-// 0: none.
+// Bytes of workspace that rb_gemm_bf16 makes use of for this call when it may have up to `most`; 0: none.
 long long rb_gemm_workspace(const RbGemmArgs* args, long long most);
 
 #ifdef __cplusplus

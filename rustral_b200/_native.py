@@ -38,7 +38,7 @@ class RbGemmArgs(C.Structure):
         ("peer_epoch", C.c_uint), ("ready_flags", c_void_p), ("peer_ptrs", c_void_p * 8),
         ("tile_arrived", c_void_p), ("tile_expected", c_void_p),
         ("ab_fp8", c_int), ("a_scale", c_void_p), ("b_scale", c_void_p), ("b_constant", c_int),
-        ("norm_gamma", c_void_p), ("norm_beta", c_void_p), ("norm_eps", c_float), ("norm_rms", c_int), ("col_sum", c_void_p),
+        ("norm_gamma", c_void_p), ("norm_beta", c_void_p), ("norm_eps", c_float), ("norm_rms", c_int), ("col_sum", c_void_p), ("col_out", c_void_p), ("col_rows", c_int),
     ]
 
 

@@ -168,12 +168,10 @@ N.optional_sig("rb_gemm_workspace", [N.C.POINTER(N.RbGemmArgs), N.c_ll], N.c_ll)
 
 def _give_workspace(g, device, need: int):
     """Names the split-K scratch in `g`; what is returned has to live until the launch.  `need`: what the plan takes (`rb_gemm_workspace`); with
-    none the plan is the same without scratch.  A captured graph gets its own: graphs that name one buffer could not be replayed side by side.  So does
-    a call whose column sums come on top of slabs that fill the kept buffer."""
+    none the plan is the same without scratch.  A captured graph gets its own: graphs that name one buffer could not be replayed side by side."""
     if not need:
         return None
-    own = need > WORKSPACE_BYTES or torch.cuda.is_current_stream_capturing()
-    ws = torch.empty(need, dtype=torch.uint8, device=device) if own else _workspace(device)
+    ws = torch.empty(need, dtype=torch.uint8, device=device) if torch.cuda.is_current_stream_capturing() else _workspace(device)
     g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
     return ws
 
@@ -218,13 +216,32 @@ def _gemm_f32(a, b, out, alpha, tile_expert=None, num_tiles=None, expert_stride=
     return out
 
 
+_sum_scratch: dict = {}
+
+
+def _sum_columns(a, out, accumulate: bool) -> None:
+    from .elementwise import sum_dim0
+    sum_dim0(a, out=out, accumulate=accumulate)
+
+
+def _sum_rows(M: int, K: int) -> int:
+    """Rows of a slab in which `sum_dim0` adds up the columns of [K, M], where a product forms the slabs' sums beside itself: slabs of whole k-blocks (up to
+    8192 rows in whole blocks a slab for each, 16384 or 32768 rows two or four).  0: elsewhere.  (Slabs that begin and end inside blocks were read
+    from shared memory row by row; with two folds a block the sums held up the product: 6 layers of 384 with 1998 tokens 1333 us a step, 1135 with
+    launches of their own.)"""
+    if M & 7:
+        return 0
+    rows = -(-K // min(N.kernels().rb_sum_dim0_slabs(), (K + 63) // 64))
+    return 0 if rows & 63 else rows
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, aux_out=None, out=None, out_dtype=None, accumulate: bool = False,
          alpha: float = 1.0, block_n: int = 0, group_m: int = 0, max_ctas: int = 0, splits: int = 0,
          peer: dict | None = None, row_scale=None, col_scale=None, b_constant: bool = False, col_sum=None) -> torch.Tensor:
     """`b_constant`: the kernel in front of this call in its stream does not write `b` (a served model's weights), so reading `b` may
     begin while that kernel still runs.  `col_sum` (fp32 [M], weight gradients: both operands transposed): receives the sums of a's columns, the bias
-    gradient, added to what it holds with `accumulate`.  `row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
+    gradient, added to what it holds with `accumulate`; the bits are those of `sum_dim0`.  `row_scale` (fp32 [M]) / `col_scale` (fp32 [N]) multiply the accumulator's rows / columns before the bias (weight
     scales of quantised layers).  `peer` selects the tensor-parallel modes of the kernel (see parallel/fused_tp.py): a dict with `mode`
     (1: remote row blocks of A are pulled from the peers' shards inside the kernel; 2: output row blocks are
     stored into their owner's receive slot), `world`, `rank`, `rows_per_rank`, `epoch`, `ready_flags` (pointer,
@@ -244,11 +261,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if not (a_mn and b_mn) or act != "none" or peer is not None or col_sum.dtype != torch.float32 or col_sum.shape != (M,) or \
                 not col_sum.is_contiguous() or col_sum.device != a.device:
             raise ValueError("gemm: column sums go with a plain product of two transposed operands, into a contiguous fp32 vector")
-        if not a.is_cuda or a.dtype != torch.bfloat16 or not K or not M or not Nn or \
+        plain = bias is None and residual is None and aux_in is None and aux_out is None and row_scale is None and col_scale is None
+        if not a.is_cuda or not a.dtype is b.dtype is torch.bfloat16 or not K or not M or not Nn or not plain or \
                 _needs_padding(a, b, bias, residual, aux_in, aux_out, out, out_dtype, Nn):
-            from .elementwise import sum_dim0
             if M:
-                sum_dim0(a, out=col_sum, accumulate=accumulate and out is not None)
+                _sum_columns(a, col_sum, accumulate and out is not None)
             col_sum = None
     if not a.is_cuda:
         if row_scale is not None or col_scale is not None:
@@ -319,13 +336,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             g.alpha = alpha
             g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
             g.b_constant = int(b_constant)
-            g.col_sum = N.ptr(col_sum)
             need = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES) if splits != 1 and K >= 2048 and act == "none" else 0
+            g.col_rows = 0 if col_sum is None else _sum_rows(M, K)
             cache[key] = g, need
         else:
             g, need = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
-        g.col_sum = N.ptr(col_sum)
+        if g.col_rows:
+            partial = N.scratch(_sum_scratch, a.device, -(-K // g.col_rows) * M, torch.float32, 4096)
+            g.col_sum, g.col_out = partial.data_ptr(), col_sum.data_ptr()
+            N.launch_count += 1
+        elif col_sum is not None:
+            _sum_columns(a, col_sum, accumulate)
         ws = _give_workspace(g, a.device, need)  # noqa: F841
         N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
         return out
@@ -350,7 +372,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     g.alpha = alpha
     g.block_n, g.group_m, g.max_ctas, g.splits = block_n, group_m, max_ctas, splits
     g.b_constant = int(b_constant)
-    g.col_sum = N.ptr(col_sum)
     for t, n_, nm in ((row_scale, M, "row_scale"), (col_scale, Nn, "col_scale")):
         if t is not None and (t.dtype != torch.float32 or t.numel() != n_ or not t.is_contiguous() or t.device != a.device):
             raise TypeError(f"gemm: {nm} must be a contiguous fp32 vector of {n_} elements on the operands' device")
@@ -366,7 +387,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         g.splits = 1
     elif splits != 1 and K >= 2048 and act == "none":
         cache = _plain_args()
-        key = (M, Nn, K, a_mn, b_mn, accumulate, block_n, group_m, max_ctas, splits, aux_in is None, aux_out is None, col_sum is None)
+        key = (M, Nn, K, a_mn, b_mn, accumulate, block_n, group_m, max_ctas, splits, aux_in is None, aux_out is None)
         need = cache.get(key)
         if need is None:
             need = cache[key] = N.kernels().rb_gemm_workspace(g, WORKSPACE_BYTES)
@@ -378,7 +399,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta, eps: float, rms: bool, w: torch.Tensor, *, bias=None, act: str = "none",
               b_constant: bool = False) -> torch.Tensor:
     """act(norm(x) @ w^T + bias) for inference (`act` "swiglu": w = [gate; up], see rotary.swiglu_product).  For a few rows one launch, in which
-    every block forms the norm itself; else the norm's kernel and the product's, with the same result up to the order of the norm's sums."""
+    every block forms the norm itself; else the norm's kernel and the product's, with the same bits."""
     from . import norm as norm_ops
     from .rotary import swiglu_product
     M, K = x.shape

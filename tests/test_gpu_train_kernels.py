@@ -276,3 +276,28 @@ def test_a_split_that_fills_the_scratch_takes_column_sums_too(hook, captured, cu
     assert torch.equal(w, plain)
     want = dy.double().sum(0)
     assert ((b.double() - want).abs() <= 2.0 ** -24 * (tokens / 64 + 16) * dy.double().abs().sum(0) + 2.0 ** -23 * want.abs()).all()
+
+
+@pytest.mark.parametrize("tokens,out,inp,splits,inside", [
+    (1, 64, 64, 0, False), (64, 64, 64, 0, True), (70, 8, 24, 0, False), (127, 136, 64, 0, True), (1024, 256, 256, 0, True), (1998, 1152, 384, 0, False),
+    (4096, 2304, 768, 0, True), (6144, 776, 768, 3, True), (6144, 780, 256, 0, False), (8192, 3072, 768, 2, True), (8200, 264, 256, 12, False),
+    (8256, 256, 256, 0, False), (16384, 768, 768, 0, True), (32768, 2304, 768, 0, True), (32768, 256, 520, 3, True), (32767, 200, 768, 6, True)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_bias_gradient_has_the_bits_of_a_column_sum(tokens, out, inp, splits, inside, accumulate, cuda_status):
+    """Inside the weight gradient's product where the slabs of `sum_dim0` are whole k-blocks: one and several blocks to a slab, slabs that reach into the next
+    part of the contraction, a last one that is cut short, ragged columns; in launches of its own elsewhere."""
+    from rustral_b200 import _native as N
+    from rustral_b200.ops import matmul, sum_dim0
+    g = torch.Generator(device="cuda").manual_seed(tokens + out)
+    dy = (torch.randn(tokens, out + 8 - out % 8, device="cuda", generator=g) * 3 + 0.1).bfloat16()[:, :out]
+    x = torch.randn(tokens, inp, device="cuda", generator=g).bfloat16()
+    b0 = torch.randn(out, device="cuda", generator=g)
+    w, b, plain, want = torch.zeros(out, inp, device="cuda"), b0.clone(), torch.zeros(out, inp, device="cuda"), b0.clone()
+    call = lambda d, **kw: matmul.gemm(dy, x, a_mn=True, b_mn=True, out=d, accumulate=accumulate, splits=splits, **kw)  # noqa: E731
+    before = N.launch_count
+    call(plain)
+    product = N.launch_count - before
+    call(w, col_sum=b)
+    assert (N.launch_count - before - 2 * product == 1) == inside
+    sum_dim0(dy, out=want, accumulate=accumulate)
+    assert torch.equal(b, want) and torch.equal(w, plain)
