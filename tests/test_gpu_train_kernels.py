@@ -301,3 +301,18 @@ def test_bias_gradient_has_the_bits_of_a_column_sum(tokens, out, inp, splits, in
     assert (N.launch_count - before - 2 * product == 1) == inside
     sum_dim0(dy, out=want, accumulate=accumulate)
     assert torch.equal(b, want) and torch.equal(w, plain)
+
+
+@pytest.mark.parametrize("vocab,tokens", [(31, 100), (16385, 4000), (50257, 9000)])
+def test_embedding_gradient_leaves_out_ids_out_of_range(vocab, tokens, cuda_status):
+    """Negative ids and ids behind the table add to no row."""
+    from rustral_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    ids = torch.randint(0, vocab, (tokens,), device="cuda", generator=g)
+    ids[::5], ids[1::5], ids[2], ids[3] = -1, vocab, vocab + 12345, -(1 << 40)
+    dy = torch.randn(tokens, 64, device="cuda", generator=g).bfloat16()
+    got = torch.zeros(vocab, 64, device="cuda")
+    ops.embedding_backward(ids, dy, got, None, tokens)
+    real = (ids >= 0) & (ids < vocab)
+    want, often = (torch.zeros(vocab, 64, dtype=torch.float64, device="cuda").index_add(0, ids[real], v[real]) for v in (dy.double(), dy.double().abs()))
+    assert ((got.double() - want).abs() <= 2.0 ** -24 * (torch.bincount(ids[real], minlength=vocab)[:, None] + 1) * often).all()
