@@ -65,7 +65,7 @@ class GPTBody:
 
     def embed(self, sb):
         P, cfg = self.r.params, self.cfg
-        if cfg.arch == "gpt2" and sb.arrived is not None:
+        if cfg.arch == "gpt2" and not sb.spans and sb.ids.is_cuda:
             return ops.embedding_forward(sb.ids, P.w("tok_embed.embed"), P.w("pos_embed.embed"), lengths=sb.ctx)
         x = ops.embedding_forward(sb.ids, P.w("tok_embed.embed"))
         if cfg.arch == "gpt2":

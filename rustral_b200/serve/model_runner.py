@@ -373,10 +373,13 @@ class ModelRunner:
     def _decode_segments(self, seq_ids, context_lens) -> list:
         return [(i, 1, self.cache.state_slot(s), n - 1) for i, (s, n) in enumerate(zip(seq_ids, context_lens))]
 
-    def _step_counters(self, batch: int):
-        """Zeros that the steps of one stream share (see ops.paged.attention_step); None: the model's layers do not use them."""
-        if self.device.type != "cuda" or not isinstance(self.body, decoder_body.GPTBody):
-            return None
+    def _attends_in_one_launch(self, context_lens, width: int) -> bool:
+        """Whether a decoding step's layers attend in one launch (see ops.paged.step_pays)."""
+        return self.device.type == "cuda" and isinstance(self.body, decoder_body.GPTBody) and \
+            paged_ops.step_pays(context_lens, self.n_kv_head, self.cfg.head_dim, width, self.block_size, self.device)
+
+    def _step_counters(self, batch: int) -> torch.Tensor:
+        """Zeros that the steps of one stream share (see ops.paged.attention_step)."""
         return torch.zeros(batch * self.n_kv_head, dtype=torch.int32, device=self.device)
 
     def _decode_body(self, ids, ctx, bt, segments=None, arrived=None):
@@ -397,7 +400,8 @@ class ModelRunner:
         self.cache.fill_tables(seq_ids, bt)
         bt = bt.to(dev)
         seg = Segments.of(self._decode_segments(seq_ids, context_lens), dev) if self.recurrent else None
-        return self._decode_body(ids, ctx, bt, seg, self._step_counters(len(seq_ids)))
+        one = self._attends_in_one_launch(context_lens, max_blocks)
+        return self._decode_body(ids, ctx, bt, seg, self._step_counters(len(seq_ids)) if one else None)
 
     def _table_width(self, context_lens) -> int:
         """Block-table columns of a graphed decode step: the model's whole context when that is at most 1024 blocks, else
@@ -414,20 +418,22 @@ class ModelRunner:
                 "bt": buf[12 * B:].view(torch.int32).view(B, width)}
 
     def _decode_graphed(self, seq_ids, last_tokens, context_lens) -> torch.Tensor:
-        """Replays one captured CUDA graph per batch size: the 10 to 20 launches per layer of a decode step are
+        """Replays one captured CUDA graph per batch size, table width and form of the attention: the 10 to 20 launches per layer of a decode step are
         launch-bound from Python, the graph submits them in one call.  Inputs live in a static device buffer that
         one copy refreshes before each replay."""
         B = len(seq_ids)
         dev = self.device
         width = self._table_width(context_lens)
-        g = self._graphs.get((B, width))
+        one = self._attends_in_one_launch(context_lens, width)
+        g = self._graphs.get((B, width, one))
         if g is None:
             # ids (int64), context lengths and block tables (int32) behind one another: one copy refreshes all three
             buf = torch.zeros(12 * B + 4 * B * width, dtype=torch.uint8, device=dev)
-            g = {"buf": buf, "seg": None, "graph": None, "out": None, "arrived": self._step_counters(B), **self._step_views(buf, B, width)}
+            g = {"buf": buf, "seg": None, "graph": None, "out": None, "arrived": self._step_counters(B) if one else None,
+                 **self._step_views(buf, B, width)}
             if self.recurrent:
                 g["seg"] = Segments(torch.zeros((B, 4), dtype=torch.int32, device=dev), None)
-            self._graphs[(B, width)] = g
+            self._graphs[(B, width, one)] = g
         memory, copied = self._memory.take(g["buf"].numel())
         host = memory[:g["buf"].numel()]
         view = self._step_views(host, B, width)

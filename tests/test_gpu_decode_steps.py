@@ -264,3 +264,34 @@ def test_a_decoded_sequence_has_the_same_bits_beside_others(arch, d, heads, kv, 
             ids = list(range(1, batch)) + [0]
             got = r.decode(ids, [5] * (batch - 1) + [17], [lens[i] for i in ids])
             assert torch.equal(got[-1:], alone), batch
+
+
+@pytest.mark.parametrize("dim,many", [(128, False), (64, True)])
+def test_attention_goes_by_the_slices_that_are_there(dim, many, monkeypatch, cuda_status):
+    """In tables of one width: twelve short sequences attend in one launch, twelve long ones with heads of 128 in three, eager and captured, in turn; a short
+    one has the same bits beside both."""
+    from rustral_b200.models.config import GPTConfig
+    from rustral_b200.ops import paged as paged_ops
+    from rustral_b200.serve.model_runner import ModelRunner
+    from rustral_b200.serve.weights import InferenceWeights
+    cfg = GPTConfig(vocab_size=512, seq_len=4096, n_layer=2, n_head=8, n_kv_head=4, d_model=8 * dim, ffn_dim=512, arch="llama")
+    r = ModelRunner(cfg, params=InferenceWeights.random_llama(cfg, "cuda", seed=3), device="cuda", num_blocks=12 * 256, block_size=16, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    for i in range(12):
+        assert r.cache.allocate(i, 4096)
+    for l in range(2):
+        r.cache.k[l].normal_(0.0, 0.9, generator=g)
+        r.cache.v[l].normal_(0.0, 0.9, generator=g)
+    short, long = [300 + i for i in range(12)], [300] + [4090 - i for i in range(11)]
+    calls = []
+    real = paged_ops.attention_step
+    monkeypatch.setattr(paged_ops, "attention_step", lambda *a: calls.append(1) or real(*a))
+    first = []
+    for graphs in (False, True):
+        r.use_graphs = graphs
+        for lens in (short, long, short, long):
+            before = len(calls)
+            first.append(r.decode(list(range(12)), list(range(12)), lens)[0].clone())
+            fresh = not graphs or len(first) <= (5 if many else 6)    # a replay calls nothing; with heads of 64 all share a graph
+            assert (len(calls) > before) == (fresh and (lens is short or many)), (graphs, lens)
+    assert all(torch.equal(first[0], x) for x in first)
