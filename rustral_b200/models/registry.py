@@ -53,7 +53,7 @@ def _layered_weights(cfg, device, dtype, tensors, seed):
 
 
 _GPT_KERNELS = ("gemm_tcgen05", "gemm_rows", "embedding", "elementwise", "norm", "rope", "attention", "attention_tc", "attention_fwd2",
-                "paged_attention", "optim")
+                "paged_attention", "paged_step", "optim")
 _LAYERED_KERNELS = ("gemm_tcgen05", "gemm_rows", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe",
                     "attention_fwd2", "paged_attention")
 _HYBRID_KERNELS = ("gemm_tcgen05", "gemm_rows", "gemm_f32", "embedding", "elementwise", "residual_norm", "head_prep", "moe", "attention_fwd2",
