@@ -73,32 +73,29 @@ __device__ __forceinline__ float rows_act(int act, float v) {
 // What warps 2 to 5 do first (NORM: the warps that a row belongs to): statistics of the rows, then the normed columns of k-blocks kb0 .. kb1 into the
 // first stages and, for stages that are filled again, into `later`.  Lanes, order and roundings are those of the norm's own kernel, so that a row's bits
 // do not hang on how many rows there are.
-template <int NORM>
+template <int NORM, int CHUNKS>
 __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int kb0, int kb1, int stages, int stage_bytes, uint32_t base,
                                           uint8_t* later, float* red, bool w_constant) {
   constexpr int kRows = 4 / NORM;                // at a time
   const int warp = (threadIdx.x >> 5) - 2, lane = threadIdx.x & 31, wr = warp % NORM;
   const float inv_n = 1.f / static_cast<float>(K);
-  auto col = [&](int i) { return norm_col<4, NORM>(wr, i, lane); };
+  auto col = [&](int i) { return norm_col<CHUNKS, NORM>(wr, i, lane); };
   // the norm's weights are the model's like W: asked for before the kernel in front has ended
-  uint4 gamma[4], beta[4];
-  auto weights = [&]() {
+  uint4 gamma[CHUNKS], beta[CHUNKS];
+  if (!w_constant) pdl_wait();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = col(i), kb = c >> 6;
-      const bool mine = c < K && kb >= kb0 && kb < kb1 && warp / NORM < M;
-      gamma[i] = mine ? *reinterpret_cast<const uint4*>(nm.gamma + c) : make_uint4(0u, 0u, 0u, 0u);
-      beta[i] = mine && nm.beta ? *reinterpret_cast<const uint4*>(nm.beta + c) : make_uint4(0u, 0u, 0u, 0u);
-    }
-  };
-  if (w_constant) weights();
+  for (int i = 0; i < CHUNKS; ++i) {
+    const int c = col(i), kb = c >> 6;
+    const bool mine = c < K && kb >= kb0 && kb < kb1 && warp / NORM < M;
+    gamma[i] = mine ? *reinterpret_cast<const uint4*>(nm.gamma + c) : make_uint4(0u, 0u, 0u, 0u);
+    beta[i] = mine && nm.beta ? *reinterpret_cast<const uint4*>(nm.beta + c) : make_uint4(0u, 0u, 0u, 0u);
+  }
   pdl_wait();
   pdl_launch();
-  if (!w_constant) weights();
-  uint4 next[4];
+  uint4 next[CHUNKS];
   auto fetch = [&](int m) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
       const int c = col(i);
       next[i] = m < M && c < K ? *reinterpret_cast<const uint4*>(nm.x + m * nm.ldx + c) : make_uint4(0u, 0u, 0u, 0u);
     }
@@ -122,15 +119,16 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
 #pragma unroll 1
   for (int m0 = 0; m0 < M; m0 += kRows) {
     const int m = m0 + warp / NORM;              // M or more: nothing is read or written, the barriers are kept
-    uint4 u[4];
+    if (NORM == 1 && m >= M) break;              // (there are none)
+    uint4 u[CHUNKS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) u[i] = next[i];
+    for (int i = 0; i < CHUNKS; ++i) u[i] = next[i];
     fetch(m + kRows);
     float mean = 0.f;
     if (!nm.rms) {
       float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < CHUNKS; ++i) {
         float v[8];
         unpack(u[i], v);
 #pragma unroll
@@ -140,7 +138,7 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
     }
     float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
       if (col(i) < K) {
         float v[8];
         unpack(u[i], v);
@@ -151,22 +149,16 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
     const float rstd = norm_rstd(row_sum(sq, red + m * 8 + 4), inv_n, nm.eps);
     if (m >= M) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
       const int c = col(i), kb = c >> 6;
       if (kb >= kb0 && kb < kb1) {               // the last block's columns behind the row are zero
-        float v[8] = {}, g[8];
+        float v[8] = {}, g[8], b[8];
         if (c < K) {
           unpack(u[i], v);
           unpack(gamma[i], g);
-          if (nm.beta) {
-            float b[8];
-            unpack(beta[i], b);
+          unpack(beta[i], b);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = norm_value(v[j], mean, rstd, g[j], b[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = norm_value(v[j], mean, rstd, g[j]);
-          }
+          for (int j = 0; j < 8; ++j) v[j] = norm_value(v[j], mean, rstd, g[j], b[j]);     // without beta + 0: the same number
         }
         const uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
         const int it = kb - kb0, chunk = (c & 63) >> 3;
@@ -183,8 +175,8 @@ __device__ __forceinline__ void rows_norm(const RowsNorm& nm, int M, int K, int 
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-// NORM: 0, or the warps that share a row of the norm (1, 2, 4: K up to 1024, 2048, 4096)
-template <int NORM>
+// NORM: 0, or the warps that share a row of the norm (1, 2, 4: K up to 1024, 2048, 4096), CHUNKS: the norm's 16-byte pieces per lane
+template <int NORM, int CHUNKS = 4>
 __global__ void __launch_bounds__(kRowsThreads)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, int M, int N, int K, int mpad,
                  int parts, int stages, int w_constant, const RowsEpi ep, const RowsNorm nm, unsigned int* status) {
@@ -270,7 +262,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       pdl_wait();
       pdl_launch();
     } else {
-      rows_norm<NORM>(nm, M, K, kb0, kb1, stages, stage_bytes, base, later, red, w_constant);
+      rows_norm<NORM, CHUNKS>(nm, M, K, kb0, kb1, stages, stage_bytes, base, later, red, w_constant);
       if (warp == 2) {
         if (lane < min(stages, kb1 - kb0)) mbar_arrive(bar_full + 8 * lane);
         for (int it = stages; it < kb1 - kb0; ++it) {
@@ -423,12 +415,14 @@ int gemm_rows(const RbGemmArgs& g, cudaStream_t stream) {
   const CUtensorMap* tx = norm ? tw : get_tmap_2d(g.a, 2, (uint64_t)g.K, (uint64_t)g.M, (uint64_t)g.lda, 64, (uint32_t)mpad, 1, &err);
   if (!tx) return err ? err : -5;
   const int smem = stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024 + later;
-  const int form = !norm ? 0 : g.K <= 1024 ? 1 : g.K <= 2048 ? 2 : 3;
+  // the norm's own kernel takes rows of up to 768 in three pieces a lane
+  const int form = !norm ? 0 : g.K <= 768 ? 1 : g.K <= 1024 ? 2 : g.K <= 2048 ? 3 : 4;
   auto kern = form == 0   ? rb::gemm_rows_kernel<0>
-              : form == 1 ? rb::gemm_rows_kernel<1>
-              : form == 2 ? rb::gemm_rows_kernel<2>
+              : form == 1 ? rb::gemm_rows_kernel<1, 3>
+              : form == 2 ? rb::gemm_rows_kernel<1>
+              : form == 3 ? rb::gemm_rows_kernel<2>
                           : rb::gemm_rows_kernel<4>;
-  static bool configured_dev[4][64] = {{false}};
+  static bool configured_dev[5][64] = {{false}};
   bool& configured = configured_dev[form][device_slot()];
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 114 * 1024);
