@@ -109,9 +109,10 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_b
       if (col < n) {
         float g[8], b[8], o[8];
         load8(gamma + col, g);
-        if (beta) load8(beta + col, b);
+        const bool shifted = !RMS && beta != nullptr;
+        if (shifted) load8(beta + col, b);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = beta ? norm_value(v[c][j], mean, rstd, g[j], b[j]) : norm_value(v[c][j], mean, rstd, g[j]);
+        for (int j = 0; j < 8; ++j) o[j] = shifted ? norm_value(v[c][j], mean, rstd, g[j], b[j]) : norm_value(v[c][j], mean, rstd, g[j]);
         store8(y + row * ldy + col, o);
       }
     }
