@@ -1919,6 +1919,13 @@ static int gemm_bf16(const RbGemmArgs& g, cudaStream_t stream) {
 
 RB_API int rb_gemm_bf16(const RbGemmArgs* args, void* stream_v) {
   const RbGemmArgs& g = *args;
+  if (g.col_out && g.col_rows == 0) {              // slabs that a product cannot form beside itself
+    if (!g.a_mn_major || !g.b_mn_major || g.group_mode || g.peer_mode || g.ab_fp8 || !g.col_sum || g.M <= 0 || g.K <= 0) return -9;
+    RbGemmArgs plain = g;
+    plain.col_sum = plain.col_out = nullptr;
+    const int rc = rb_sum_dim0_staged(g.a, g.lda, g.col_out, g.col_sum, g.K, g.M, 1, g.accumulate, stream_v);
+    return rc != 0 ? rc : gemm_bf16(plain, reinterpret_cast<cudaStream_t>(stream_v));
+  }
   const int rc = gemm_bf16(g, reinterpret_cast<cudaStream_t>(stream_v));
   return rc != 0 || !g.col_sum ? rc : rb_sum_dim0_fold(g.col_sum, (g.K + g.col_rows - 1) / g.col_rows, g.col_out, g.M, g.accumulate, stream_v);
 }

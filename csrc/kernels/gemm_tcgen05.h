@@ -79,6 +79,7 @@ typedef struct RbGemmArgs {
   // col_out: column sums of A, fp32 [M] (added to it with `accumulate`), or NULL: in a weight gradient dW = dy^T x the bias gradient, formed while dy is in
   // shared memory anyway.  MN-major A and B, plain problems with M a multiple of 8.  col_sum: scratch of the sums over every `col_rows` rows (a multiple of
   // 64), fp32 [ceil(K / col_rows)][M], that `rb_sum_dim0_fold` makes the result of: with the slabs of `rb_sum_dim0_staged` it has that one's bits.
+  // col_rows 0: that function itself, in front of the product (col_sum: its scratch; any M).
   float* col_sum;
   float* col_out;
   int col_rows;

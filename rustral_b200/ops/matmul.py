@@ -219,11 +219,6 @@ def _gemm_f32(a, b, out, alpha, tile_expert=None, num_tiles=None, expert_stride=
 _sum_scratch: dict = {}
 
 
-def _sum_columns(a, out, accumulate: bool) -> None:
-    from .elementwise import sum_dim0
-    sum_dim0(a, out=out, accumulate=accumulate)
-
-
 def _sum_rows(M: int, K: int) -> int:
     """Rows of a slab in which `sum_dim0` adds up the columns of [K, M], where a product forms the slabs' sums beside itself: slabs of whole k-blocks (up to
     8192 rows in whole blocks a slab for each, 16384 or 32768 rows two or four).  0: elsewhere.  (Slabs that begin and end inside blocks were read
@@ -264,8 +259,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         plain = bias is None and residual is None and aux_in is None and aux_out is None and row_scale is None and col_scale is None
         if not a.is_cuda or not a.dtype is b.dtype is torch.bfloat16 or not K or not M or not Nn or not plain or \
                 _needs_padding(a, b, bias, residual, aux_in, aux_out, out, out_dtype, Nn):
+            from .elementwise import sum_dim0
             if M:
-                _sum_columns(a, col_sum, accumulate and out is not None)
+                sum_dim0(a, out=col_sum, accumulate=accumulate and out is not None)
             col_sum = None
     if not a.is_cuda:
         if row_scale is not None or col_scale is not None:
@@ -342,12 +338,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         else:
             g, need = g
         g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), out.data_ptr()
-        if g.col_rows:
-            partial = N.scratch(_sum_scratch, a.device, -(-K // g.col_rows) * M, torch.float32, 4096)
+        if col_sum is not None:
+            slabs = -(-K // g.col_rows) if g.col_rows else N.kernels().rb_sum_dim0_slabs()
+            partial = N.scratch(_sum_scratch, a.device, slabs * M, torch.float32, 4096)
             g.col_sum, g.col_out = partial.data_ptr(), col_sum.data_ptr()
-            N.launch_count += 1
-        elif col_sum is not None:
-            _sum_columns(a, col_sum, accumulate)
+            N.launch_count += 1 if g.col_rows else 2
         ws = _give_workspace(g, a.device, need)  # noqa: F841
         N.check(N.kernels().rb_gemm_bf16(g, N.stream_ptr()), "rb_gemm_bf16")
         return out
