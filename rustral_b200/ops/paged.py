@@ -111,22 +111,22 @@ N.optional_sig("rb_paged_attention_step_takes", [N.c_int, N.c_int, N.c_int, N.c_
 
 
 def step_supported(qkv, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables) -> bool:
-    """Whether `attention_step` takes these operands: tables with room for six slices per SM (see `step_pays` for when it is the faster way)."""
+    """Whether `attention_step` takes these operands: tables with room for six slices per SM (see `step_most_slices` for when it is the faster way)."""
     return qkv.is_cuda and qkv.dtype is torch.bfloat16 and head_dim in (64, 128) and heads <= 16 * kv_heads and qkv.stride(1) == 1 and \
         not qkv.stride(0) & 7 and not qkv.data_ptr() & 15 and k_cache.is_contiguous() and v_cache.is_contiguous() and \
         k_cache.dtype is torch.bfloat16 and k_cache.shape == v_cache.shape and k_cache.shape[2:] == (kv_heads, head_dim) and \
         bool(N.kernels().rb_paged_attention_step_takes(block_tables.shape[0], kv_heads, block_tables.shape[1], k_cache.shape[1]))
 
 
-def step_pays(context_lens, kv_heads: int, head_dim: int, width: int, block_size: int, device) -> bool:
-    """Whether `attention_step` is the faster way for sequences of these lengths (a list), counted in the slices of 256 tokens that are there.
+def step_most_slices(batch: int, kv_heads: int, head_dim: int, width: int, block_size: int) -> float:
+    """Up to how many slices (256 tokens of a sequence for a KV head) `attention_step` is the faster way on the current device, in tables of this width.
     With heads of 128 an SM holds one of its blocks where the split kernel has three, so it loses behind two slices per SM.  One B200, a layer of a captured
     chain with its projection, us, one launch / three, by slices per SM: 0.6 13.9 / 20.5, 1.2 18.5 / 22.7, 1.7 20.8 / 23.8, 1.9 22.3 / 25.9, 2.2 24.6 / 26.3 and (2 KV
     heads) 30.6 / 27.9, 2.6 30.2 / 28.0, 3.5 38.3 / 36.2, 4.3 43.5 / 38.6, 5.8 57.0 / 42.8; three sequences in tables of 64 slices, 5.2 per SM if they were full, 0.14 of
     them there 11.5 / 19.7.  Heads of 64: 2.6 17.8 / 19.0, 4.3 24.9 / 27.8, 5.8 27.8 / 29.5."""
-    if not N.kernels().rb_paged_attention_step_takes(len(context_lens), kv_heads, width, block_size):
-        return False
-    return head_dim <= 64 or kv_heads * sum((n + 255) // 256 for n in context_lens) <= 2 * torch.cuda.get_device_properties(device).multi_processor_count
+    if not N.kernels().rb_paged_attention_step_takes(batch, kv_heads, width, block_size):
+        return 0
+    return math.inf if head_dim <= 64 else 2 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
 
 
 def attention_step(qkv, heads: int, kv_heads: int, head_dim: int, theta: float, k_cache, v_cache, block_tables, context_lens, arrived, scale: float):

@@ -11,6 +11,7 @@ and the cached decode its TransformerDecoder::generate_token does not have (full
 from __future__ import annotations
 
 import gc
+import math
 from collections import deque
 
 import torch
@@ -187,6 +188,7 @@ class ModelRunner:
         self._memory = _StepMemory(self.device)
         self.use_graphs = True          # CUDA-graph replay of decode steps
         self._graphs: dict = {}
+        self._most_slices: dict = {}    # (batch, table width) -> ops.paged.step_most_slices
 
     # ---- attention over the rows of a step -------------------------------------------------------------------------
     def attend(self, l: int, q, k2, v2, sb: StepBatch, scale: float, rule=None, gate=None, head_gate=None, out=None) -> torch.Tensor:
@@ -374,9 +376,16 @@ class ModelRunner:
         return [(i, 1, self.cache.state_slot(s), n - 1) for i, (s, n) in enumerate(zip(seq_ids, context_lens))]
 
     def _attends_in_one_launch(self, context_lens, width: int) -> bool:
-        """Whether a decoding step's layers attend in one launch (see ops.paged.step_pays)."""
-        return self.device.type == "cuda" and isinstance(self.body, decoder_body.GPTBody) and \
-            paged_ops.step_pays(context_lens, self.n_kv_head, self.cfg.head_dim, width, self.block_size, self.device)
+        """Whether a decoding step's layers attend in one launch: by the slices that its lengths have."""
+        if self.device.type != "cuda" or not isinstance(self.body, decoder_body.GPTBody):
+            return False
+        key = (len(context_lens), width)
+        most = self._most_slices.get(key)
+        if most is None:
+            if len(self._most_slices) > 4096:
+                self._most_slices.clear()
+            most = self._most_slices[key] = paged_ops.step_most_slices(len(context_lens), self.n_kv_head, self.cfg.head_dim, width, self.block_size)
+        return 0 < most and (most == math.inf or self.n_kv_head * sum((n + 255) // 256 for n in context_lens) <= most)
 
     def _step_counters(self, batch: int) -> torch.Tensor:
         """Zeros that the steps of one stream share (see ops.paged.attention_step)."""

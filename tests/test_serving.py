@@ -461,7 +461,7 @@ def test_a_checkout_without_built_files_compiles_what_serving_calls(arch):
     from rustral_b200.ops import attention, embed, matmul, norm, paged, rotary
     files = Path(__file__).resolve().parent.parent / "csrc" / "kernels"
     where = {name: f.stem for f in files.glob("*.cu") for name in re.findall(r"RB_API\s[^;(]*?\b(rb_\w+)\s*\(", f.read_text())}
-    called = (paged.attention_step, paged.step_pays, paged.step_supported, paged.paged_attention_decode, paged.kv_append, matmul.gemm, matmul.norm_gemm,
+    called = (paged.attention_step, paged.step_most_slices, paged.step_supported, paged.paged_attention_decode, paged.kv_append, matmul.gemm, matmul.norm_gemm,
               norm.norm_forward, attention.prompt_attention_many, rotary.rope_append_, rotary.swiglu_product, embed.embedding_forward)
     names = {n for f in called for n in re.findall(r"kernels\(\)\.(rb_\w+)|lib\.(rb_\w+)", inspect.getsource(f)) for n in n if n}
     assert {"rb_paged_attention_step", "rb_gemm_bf16", "rb_norm_fwd", "rb_kv_append"} <= names
