@@ -295,3 +295,50 @@ def test_attention_goes_by_the_slices_that_are_there(dim, many, monkeypatch, cud
             fresh = not graphs or len(first) <= (5 if many else 6)    # a replay calls nothing; with heads of 64 all share a graph
             assert (len(calls) > before) == (fresh and (lens is short or many)), (graphs, lens)
     assert all(torch.equal(first[0], x) for x in first)
+
+
+def test_attention_in_one_launch_on_a_tensor_parallel_shard(monkeypatch, cuda_status):
+    """A rank's shard (half of the heads, exchanges that return the rank's own part): the decoding step with attention in one launch has the bits of the
+    three launches, eager and replayed."""
+    from rustral_b200.models.config import GPTConfig
+    from rustral_b200.ops import paged as paged_ops
+    from rustral_b200.serve.model_runner import ModelRunner
+
+    class Shard:
+        world, rank = 2, 1
+
+        def __init__(self):
+            self.memory = {}
+
+        def staging(self, rows, cols):
+            return self.memory.setdefault((rows, cols), torch.zeros(rows, cols, device="cuda", dtype=torch.bfloat16))
+
+        def all_reduce(self, rows, cols, residual=None):
+            return self.staging(rows, cols) + residual
+
+        def all_gather_cols(self, rows, cols):
+            return self.staging(rows, cols).clone()
+
+        def end_step(self):
+            pass
+
+    cfg = GPTConfig(vocab_size=1024, seq_len=2048, n_layer=2, n_head=16, n_kv_head=8, d_model=1024, ffn_dim=2048, arch="llama")
+    lens = [1, 300, 1000]
+    got = []
+    for one in (True, False):
+        if not one:
+            monkeypatch.setattr(paged_ops, "step_most_slices", lambda *a: 0)
+        r = ModelRunner(cfg, device="cuda", num_blocks=128, block_size=16, seed=3, tp=Shard())
+        g = torch.Generator(device="cuda").manual_seed(1)
+        for i, n in enumerate(lens):
+            assert r.cache.allocate(i, n)
+        for l in range(2):
+            r.cache.k[l].normal_(0.0, 0.9, generator=g)
+            r.cache.v[l].normal_(0.0, 0.9, generator=g)
+        assert r.n_kv_head == 4 and r._attends_in_one_launch(lens, 128) == one
+        for graphs in (False, True, True):
+            r.use_graphs = graphs
+            got.append((r.decode([0, 1, 2], [5, 6, 7], lens).clone(), *(c.clone() for c in (*r.cache.k, *r.cache.v))))
+    assert torch.isfinite(got[0][0]).all()
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
