@@ -5,8 +5,8 @@
 // that; 128 rows of W form a tile, and a cluster of up to 8 CTAs shares a tile: each CTA contracts over its part of K with its own ring
 // of TMA stages, leaves its partial sums in shared memory, and takes its share of the tile's results, adding the partial sums of all
 // CTAs in rank order through distributed shared memory (bit-reproducible, no workspace, no second kernel).  Measured on one B200, one
-// row, in a captured chain: 28672 x 4096 41 us = 5.7 TB/s (the tile kernel: 54), 65536 x 4096 6.5 TB/s, 2048 x 2048 5.4 us (12.0), of which
-// launch, first load, exchange and last store are about 4.
+// row, in a captured chain of one product on weights of their own: 28672 x 4096 41 us = 5.7 TB/s (the tile kernel: 54), 65536 x 4096 6.5
+// TB/s, 2048 x 2048 5.4 us (12.0), of which launch, first load, exchange and last store are about 4.
 //
 // Roles: warp 0 TMA, warp 1 MMA issue and TMEM, warps 2 to 5 accumulator -> shared memory; then all warps the epilogue.
 //
@@ -14,10 +14,13 @@
 // decoding step; here every CTA reads the whole rows (at most 32 KB, from L2), forms their statistics and puts its part of the normed rows, rounded
 // to bf16 as the norm's own kernel does, into the operand tiles itself, while the first stages of W are on their way.  Warps 2 to 5 do that.
 // A decoded token of GPT-2 small, 25 norms, with the attention step in one launch 479 -> 392 us on one B200; of 8 Llama style layers of 2048 518 -> 497.
+// Lanes and order are those of the norm's kernel; sums over all 128 threads in an order of their own saved 2 % of that (328 / 320 us a token today), but gave a
+// sequence other bits beside eight others than beside seven.
 //
 // A kernel's last barrier across the cluster only keeps shared memory alive: as a release it waited 2000 to 3000 cycles for the results' stores.  Without
-// that, with the partial sums of all CTAs asked for at once and the norm's weights under the kernel in front, us per product in a chain, before /
-// now: 1 row 768 x 3072 6.45 / 5.63, 2048 x 2048 8.1 / 7.1, 2048 x 8192 13.4 / 12.3; 64 rows 2048 x 8192 15.8 / 14.1.
+// that, with the partial sums of all CTAs asked for at once and the norm's weights under the kernel in front, us per product, before / now, both in one
+// chain that is not the one above (their difference counts): 1 row 768 x 3072 6.45 / 5.63, 2048 x 2048 8.1 / 7.1, 2048 x 8192 13.4 / 12.3; 64 rows
+// 2048 x 8192 15.8 / 14.1.  In the one above 4.3, 5.4, 10.5 and 12.8; again and again on the same weights 4.4, 4.7, 7.8 and 10.4.
 #define RB_INLINE_WAITS
 #include "gemm_rows.h"
 

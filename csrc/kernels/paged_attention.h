@@ -22,8 +22,8 @@ int rb_paged_attention_decode(const void* q, long long ld_q, void* out, long lon
 // Decode attention of one layer of a decoding step, from the packed projection: rotation of queries and keys (theta 0: none), append and attention
 // in one launch.  qkv [batch, (heads + 2 kv_heads) * head_dim], pitch ld_qkv, is not changed; context_lens count the new token, whose cache slot
 // follows from the tables.  Neither tables, lengths nor the cached tokens may be written by the kernel in front in the stream.  At most 16 query
-// heads per KV head; head_dim 64 or 128.  -9 where the tables have room for more slices than fit the GPU twice (the other entries are faster
-// there; rb_paged_attention_step_takes).  arrived: [batch * kv_heads], zero before the first call; a call leaves it zero.  scratch as above.
+// heads per KV head; head_dim 64 or 128.  -9 where the tables have room for more than six slices per SM (rb_paged_attention_step_takes; with head_dim
+// 128 the other entries are faster from two slices per SM that are there).  arrived: [batch * kv_heads], zero before the first call; a call leaves it zero.  scratch as above.
 typedef struct RbPagedStepArgs {
   const void* qkv;
   long long ld_qkv;

@@ -365,7 +365,10 @@ int step_launch(const rb::StepParams& p, int batch, cudaStream_t stream) {
 }
 }  // namespace
 
-// Up to six times as many slices as SMs in the tables: the batches and table widths that `paged_decode_split_kernel` works on as a grid of slices.
+// Up to six times as many slices as SMs in the tables: the batches and table widths that `paged_decode_split_kernel` works on as a grid of slices.  With
+// heads of 64 (75 KB of shared memory) this kernel is faster up to there: 5.8 slices per SM 27.8 us a layer with its projection, three launches
+// 29.5.  With heads of 128 (141 KB, one CTA on an SM) it is so up to about two slices per SM that are there: 1.9 22.3 / 25.9, 2.6 30.3 / 28.5, 5.8 57.0 / 42.8; callers
+// that know the lengths decide by them, since tables are mostly wider than their sequences.
 // Behind it, where slices are dealt as a list to CTAs that stay, counting and summing at a CTA's end cost more than the launches (a list form of this
 // kernel, us per layer: 64 sequences of 100 to 4000 tokens 69.2 in three launches, 90.6 in one; 24 of 128 to 2560 42.6, 46.7).
 RB_API int rb_paged_attention_step_takes(int batch, int kv_heads, int max_blocks, int block_size) {

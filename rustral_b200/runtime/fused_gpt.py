@@ -239,7 +239,8 @@ class _Beside:
     gradients they read were allocated on the main stream, so they are held until that stream has waited for them; it does so whenever more than
     `MOST_HELD` bytes are held, whatever the depth and the widths of the model are."""
 
-    # Six layers of 2048 tokens x 384 hold 105 MB, twelve of 4096 x 768 700 MB (without a limit).
+    # A step of 4096 tokens on one B200, without a limit / 256 / 64 MiB: GPT-2 style, 12 layers of 768, 4.51 / 4.12 / 3.94 GB at the peak and 5940 / 5975 /
+    # 6070 us; Llama style, 24 layers of 1024, 13.6 / 11.7 / 11.6 GB and 18360 / 18500 / 18720 us.
     MOST_HELD = 256 << 20
 
     def __init__(self, stream):
